@@ -230,6 +230,8 @@ gkc_status gkc_ctx_create(int device_id, uint64_t hbm_budget_bytes, gkc_ctx **ou
   // thread's setting and launch.
   if (set_dyn_smem_limit((const void *)k_partition, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bin_place, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_sort<uint64_t>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_sort<u128>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_count<uint64_t>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_count<u128>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_scatter<uint64_t>, c->max_smem_optin) != cudaSuccess ||
@@ -609,7 +611,10 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   const uint32_t nbins = (uint32_t)prm->nbins;
   uint32_t max_bits = kCoarseMaxBits;
   while (max_bits > 0 && ((uint64_t)nbins << max_bits) > (1ull << 20)) max_bits--;
-  const uint64_t max_buckets = (uint64_t)nbins << max_bits;
+  const uint32_t bucket_keys = bucket_target<K>(c->tune.coarse_target ? c->tune.coarse_target : kCoarseTarget);
+  // a bin has a bucket per bucket_keys keys, or one per digit where the digits hold more than half of that
+  const uint64_t max_buckets =
+      std::min<uint64_t>((uint64_t)nbins << max_bits, keys_cap / (bucket_keys / 2) + nbins + 1);
   const uint64_t cap_skm = std::max<uint64_t>(c->part_cap_skm, 1);
   WS(err, uint32_t, "err", 4);
   const unsigned long long *n_skm_dev = (const unsigned long long *)c->bufs["cursors"].p;
@@ -635,7 +640,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   pl.nbins = nbins;
   pl.bin_start = bin_start;
   pl.bin_kstart = bin_kstart;
-  pl.coarse_target = c->tune.coarse_target ? c->tune.coarse_target : kCoarseTarget;
+  pl.bucket_keys = bucket_keys;
   pl.max_bits = max_bits;
   const uint64_t chunk_kmers = c->tune.chunk_kmers ? c->tune.chunk_kmers : kChunkKmers;
   pl.chunk_kmers = chunk_kmers;
@@ -645,13 +650,15 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   pl.bucket_base = bucket_base;
   pl.chunk_base = chunk_base;
   pl.hist_base = hist_base;
-  k_count_plan<<<1, 32, 0, c->st>>>(pl);
+  k_count_plan<<<1, kCountPlanThreads, 0, c->st>>>(pl);
   LAUNCHED(c);
 
   // chunks: at most keys_cap / kChunkKmers + nbins; histogram cells: chunks << max_bits
   const uint64_t max_chunks = keys_cap / chunk_kmers + nbins + 1;
   WS(chunk_s0, uint64_t, "chunk_s0", max_chunks);
   WS(hist, uint32_t, "bucket_hist", max_chunks << max_bits);
+  WS(lut, uint16_t, "bucket_lut", (uint64_t)nbins << max_bits);
+  WS(digit_total, uint32_t, "digit_total", (uint64_t)nbins << max_bits);
   WS(keys, K, "keys", keys_cap);
   // the result's key array holds the k-mer-order keys until the count stage is done with them
   WS(out_keys, K, slot_name(c, "out_keys").c_str(), keys_cap);
@@ -673,23 +680,30 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   ea.k = prm->k;
   ea.chunk_s0 = chunk_s0;
   ea.hist = hist;
+  ea.lut = lut;
+  ea.digit_total = digit_total;
+  ea.max_bits = max_bits;
+  ea.bucket_keys = bucket_keys;
   ea.keys = keys;
   ea.flat = out_keys;
   ea.keys_cap = keys_cap;
   ea.err = err;
-  k_chunk_first<<<(unsigned)std::min<uint64_t>((max_chunks + 255) / 256, 65535), 256, 0, c->st>>>(ea);
+  const uint64_t first_n = std::max(max_chunks, ((uint64_t)nbins << max_bits) / 8);
+  k_chunk_first<<<(unsigned)std::min<uint64_t>((first_n + 255) / 256, 65535), 256, 0, c->st>>>(ea);
   LAUNCHED(c);
   k_bucket_hist<K><<<c->n_sms * 8, kBucketHistThreads, 0, c->st>>>(ea);
   LAUNCHED(c);
-  WS(bbin, uint32_t, "bucket_bin", max_buckets + 1);
   WS(big_list, uint32_t, "big_list", max_buckets + 1);
   // [0] bucket ticket, [1] unused, [2] large buckets listed, [3] their ticket
   WS(ticket, unsigned long long, "count_ticket", 4);
   CK(cudaMemsetAsync(ticket, 0, 32, c->st));
   ea.big_list = big_list;
   ea.big_count = ticket + 2;
-  ea.big_min = bucket_count_cap<K>();
-  k_bucket_scan<<<std::min<uint32_t>(nbins, 65535), kBucketScanThreads, 0, c->st>>>(ea, bstart, bsize, bbin);
+  ea.big_min = bucket_count_cap<K>() + 1;
+  k_bucket_scan<<<std::min<uint32_t>(nbins, 65535), kBucketScanThreads, 0, c->st>>>(ea, bstart, bsize);
+  LAUNCHED(c);
+  k_bucket_offsets<<<(unsigned)std::min<uint64_t>((max_buckets + kBucketOffsetThreads - 1) / kBucketOffsetThreads, 65535),
+                     kBucketOffsetThreads, 0, c->st>>>(ea, bstart);
   LAUNCHED(c);
   stage_mark(c, 4);
   const size_t sct_smem = bucket_scatter_smem_bytes<K>();
@@ -708,12 +722,9 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   SortCountArgs sa;
   memset(&sa, 0, sizeof(sa));
   sa.nbins = nbins;
-  sa.k = prm->k;
   sa.bucket_base = bucket_base;
-  sa.bin_bits = bin_bits;
   sa.bucket_start = bstart;
   sa.bucket_size = bsize;
-  sa.bucket_bin = bbin;
   sa.keys = keys;
   sa.scratch = out_keys;
   sa.stage_keys = keys;
@@ -731,10 +742,14 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   int occ = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bucket_count<K>, kBucketCountThreads, smem));
   stage_mark(c, 5);
-  // persistent, buckets taken by ticket
+  const size_t sort_smem = bucket_sort_smem_bytes<K>();
+  if ((int)sort_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "sort areas exceed shared memory");
+  int sort_occ = 0;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sort_occ, k_bucket_sort<K>, kBucketSortThreads, sort_smem));
+  k_bucket_sort<K><<<c->n_sms * std::max(sort_occ, 1), kBucketSortThreads, sort_smem, c->st>>>(sa);
+  LAUNCHED(c);
+  // the large and rejected buckets, persistent, taken by ticket
   const int ctas = std::max(1, std::min(occ, c->tune.count_ctas ? (int)c->tune.count_ctas : 2));
-  WS(sstarts, uint32_t, "slice_starts", (uint64_t)c->n_sms * ctas * 4097);
-  sa.slice_starts = sstarts;
   k_bucket_count<K><<<c->n_sms * ctas, kBucketCountThreads, smem, c->st>>>(sa);
   LAUNCHED(c);
   stage_mark(c, 6);

@@ -133,6 +133,34 @@ GKC_DEV uint32_t block_exclusive_scan(uint32_t v, uint32_t *tmp, uint32_t *total
   return res;
 }
 
+// The same for one uint64 per thread; `tmp` holds >= 32 words.
+template <int NT>
+GKC_DEV uint64_t block_exclusive_scan_u64(uint64_t v, uint64_t *tmp, uint64_t *total) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint64_t x = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint64_t y = __shfl_up_sync(0xffffffffu, x, d);
+    if (lane >= d) x += y;
+  }
+  if (lane == 31) tmp[warp] = x;
+  __syncthreads();
+  if (warp == 0) {
+    uint64_t w = (lane < NT / 32) ? tmp[lane] : 0ull;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint64_t y = __shfl_up_sync(0xffffffffu, w, d);
+      if (lane >= d) w += y;
+    }
+    tmp[lane] = w;
+  }
+  __syncthreads();
+  const uint64_t res = (warp ? tmp[warp - 1] : 0ull) + x - v;
+  *total = tmp[NT / 32 - 1];
+  __syncthreads();
+  return res;
+}
+
 template <int NT>
 GKC_DEV uint64_t block_sum_u64(uint64_t v, uint64_t *tmp) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;

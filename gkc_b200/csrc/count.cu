@@ -4,36 +4,35 @@
 // every superkmer of a bin, canonicalised as min(x, revcomp(x)), sorted
 // ascending, run-length counted (count clamped to 2^32-1), per bin.
 //
-// The keys of a bin are split into 2^cb coarse buckets by the top bits of an
-// order-preserving map of the key (eq_map), so a bin's sorted list is the
-// concatenation of its buckets' sorted lists.  Device stages:
-//   1. k_bucket_hist    - per chunk of a bin's k-mers, a histogram of coarse
-//                         digits.  Warps take 32 consecutive k-mers at a time,
+// The keys of a bin are split into buckets of about 3 K (1.5 K 16-byte) keys:
+// runs of digits, the digit being the top bits of an order-preserving map of
+// the key (eq_map), so a bin's sorted list is the concatenation of its
+// buckets' sorted lists.  Device stages:
+//   1. k_bucket_hist    - expands every k-mer once, in k-mer order, and per
+//                         chunk of a bin's k-mers counts the digits.  Warps take 32 consecutive k-mers at a time,
 //                         one per lane: each lane finds its superkmer by a
 //                         search over the next 32 superkmers' k-mer ends and
 //                         extracts its k-mer from aligned 8-byte words;
-//   2. k_bucket_scan    - one CTA per bin turns the (chunk, digit) counts
-//                         into each chunk's write offset per digit and each
-//                         bucket's start, size and bin;
-//   3. k_bucket_scatter - expands every k-mer once the same way and writes
-//                         it at its chunk's offset for its digit plus its
-//                         rank there (a shared-memory atomic);
-//   4. k_bucket_count   - persistent, buckets taken by ticket, each counted
-//                         on its own: its keys aggregated in a shared-memory
-//                         hash table and the distinct (key, count) pairs
-//                         sorted by a bitonic network; a bucket with too many
-//                         distinct keys is counting-sorted by sub-bucket
-//                         instead (the digit that follows the common prefix
-//                         of its smallest and largest key), each sub-bucket
-//                         reduced by its thread or a warp.  The runs are staged at the bucket's own key
-//                         range and its distinct count recorded;
-//                         k_compact_runs then moves them to the scan of the
-//                         counts.  A bucket larger than shared memory is
-//                         placed by sub-bucket in a scratch area and counted
-//                         in slices; a single sub-bucket too large for a slice
-//                         is aggregated in a shared-memory hash table over key
-//                         ranges that are halved until a range's distinct keys
-//                         fit.
+//   2. k_bucket_scan    - one CTA per bin packs the digits into buckets;
+//                         k_bucket_offsets turns the (chunk, digit) counts
+//                         into each chunk's write offset per bucket;
+//   3. k_bucket_scatter - moves every key to its chunk's offset for its
+//                         bucket plus its rank there;
+//   4. k_bucket_sort    - persistent, buckets taken by ticket, each counted
+//                         on its own: split into groups of about 100 keys by
+//                         splitters taken from its keys, the groups sorted
+//                         by warps in registers and run-length encoded.  The
+//                         runs are staged at the bucket's own key range and
+//                         its distinct count recorded; k_compact_runs then
+//                         moves them to the scan of the counts;
+//      k_bucket_count   - the buckets too large for that, and those in which
+//                         copies of one key fill a group: the keys aggregated
+//                         in a shared-memory hash table and the distinct ones
+//                         sorted by a sample sort.  A bucket with too many
+//                         distinct keys is sorted by the digit that follows
+//                         the common prefix of its smallest and largest key
+//                         and counted in slices; a digit larger than a slice
+//                         is opened the same way, one prefix further on.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -95,26 +94,57 @@ GKC_DEV void prefetch_l2(const void *p) { asm volatile("prefetch.global.L2 [%0];
 
 // ------------------------------------------------------------------ planning
 
-__global__ void k_count_plan(CountPlan pl) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Digit bits of a bin of nk keys: none where one bucket holds them, else
+// digits of about an eighth of a bucket (so that the buckets packed from them
+// come out even although the digits do not), at most max_bits.
+GKC_DEV uint32_t plan_bits(uint64_t nk, uint32_t bucket_keys, uint32_t max_bits, uint32_t key_bits) {
+  uint32_t bits = 0;
+  if (nk > bucket_keys)
+    while (bits < max_bits && bits < key_bits && (nk >> bits) > bucket_keys / 8) bits++;
+  return bits;
+}
+// Whether each digit is a bucket of its own: digits too large to be packed.
+GKC_DEV bool plan_whole(uint64_t nk, uint32_t bucket_keys, uint32_t bits) {
+  return bits == 0 || (nk >> bits) > bucket_keys / 2;
+}
+// Buckets of the bin: a bucket takes the digits that start within its span of
+// bucket_keys keys.
+GKC_DEV uint64_t plan_buckets(uint64_t nk, uint32_t bucket_keys, uint32_t bits) {
+  return plan_whole(nk, bucket_keys, bits) ? 1ull << bits : (nk + bucket_keys - 1) / bucket_keys;
+}
+
+// One CTA: the digits, buckets and chunks of every bin and their prefixes
+// (one bin per thread; one thread for all bins took 71-134 us at 256 bins).
+__global__ void __launch_bounds__(kCountPlanThreads) k_count_plan(CountPlan pl) {
+  constexpr int NT = kCountPlanThreads;
+  __shared__ uint64_t tmp[32];
   const bool dead = (*pl.err & (ERR_CAPACITY | ERR_BAD_READ)) != 0;
   uint64_t bb = 0, cb = 0, hb = 0;
-  for (uint32_t b = 0; b < pl.nbins; b++) {
-    const uint64_t nk = dead ? 0 : pl.bin_kstart[b + 1] - pl.bin_kstart[b];
-    uint32_t bits = 0;
-    while (bits < pl.max_bits && (int)bits < 2 * pl.k && (nk >> bits) > pl.coarse_target) bits++;
+  for (uint32_t b0 = 0; b0 < pl.nbins; b0 += NT) {
+    const uint32_t b = b0 + threadIdx.x;
+    const bool in = b < pl.nbins;
+    const uint64_t nk = dead || !in ? 0 : pl.bin_kstart[b + 1] - pl.bin_kstart[b];
+    const uint32_t bits = plan_bits(nk, pl.bucket_keys, pl.max_bits, 2 * pl.k);
     const uint64_t nch = (nk + pl.chunk_kmers - 1) / pl.chunk_kmers;
-    pl.bin_bits[b] = bits;
-    pl.bucket_base[b] = bb;
-    pl.chunk_base[b] = cb;
-    pl.hist_base[b] = hb;
-    bb += 1ull << bits;
-    cb += nch;
-    hb += nch << bits;
+    uint64_t nb, nc, nh;
+    const uint64_t ob = block_exclusive_scan_u64<NT>(in ? plan_buckets(nk, pl.bucket_keys, bits) : 0ull, tmp, &nb);
+    const uint64_t oc = block_exclusive_scan_u64<NT>(nch, tmp, &nc);
+    const uint64_t oh = block_exclusive_scan_u64<NT>(nch << bits, tmp, &nh);
+    if (in) {
+      pl.bin_bits[b] = bits;
+      pl.bucket_base[b] = bb + ob;
+      pl.chunk_base[b] = cb + oc;
+      pl.hist_base[b] = hb + oh;
+    }
+    bb += nb;
+    cb += nc;
+    hb += nh;
   }
-  pl.bucket_base[pl.nbins] = bb;
-  pl.chunk_base[pl.nbins] = cb;
-  pl.hist_base[pl.nbins] = hb;
+  if (threadIdx.x == 0) {
+    pl.bucket_base[pl.nbins] = bb;
+    pl.chunk_base[pl.nbins] = cb;
+    pl.hist_base[pl.nbins] = hb;
+  }
 }
 
 GKC_DEV uint32_t find_bin(const uint64_t *base, uint32_t nbins, uint64_t c) {
@@ -138,9 +168,12 @@ __global__ void k_skm_nk(const uint64_t *desc, const unsigned long long *n_skm_d
 }
 
 // First superkmer of every chunk: the last superkmer of the bin whose k-mer
-// prefix is at most the chunk's first k-mer.
+// prefix is at most the chunk's first k-mer.  Clears the digit totals, too.
 __global__ void k_chunk_first(ExpandArgs a) {
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
+  const uint64_t n_tot = (uint64_t)a.nbins << a.max_bits;
+  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_tot; i += (uint64_t)gridDim.x * blockDim.x)
+    a.digit_total[i] = 0;
   const uint64_t n_chunks = a.chunk_base[a.nbins];
   for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n_chunks;
        c += (uint64_t)gridDim.x * blockDim.x) {
@@ -310,73 +343,109 @@ __global__ void __launch_bounds__(HS_NT) k_bucket_hist(ExpandArgs a) {
     }
     __syncthreads();
     uint32_t *row = a.hist + a.hist_base[b] + j * nd;  // the chunk's row, digits contiguous
-    for (uint32_t d = threadIdx.x; d < nd; d += HS_NT) row[d] = hist[d];
+    uint32_t *tot = a.digit_total + ((uint64_t)b << a.max_bits);
+    for (uint32_t d = threadIdx.x; d < nd; d += HS_NT) {
+      const uint32_t v = hist[d];
+      row[d] = v;
+      if (v) atomicAdd(&tot[d], v);
+    }
     __syncthreads();
   }
 }
 
 // ----------------------------------------------------------------- 2. scan
 
-// One CTA per bin: column sums of the bin's (chunk, digit) counts, an
-// exclusive scan over digits (the bucket starts), then every chunk's write
-// offset per digit, written over its count; offsets are relative to the
-// bin's first key.
+// One CTA per bin: the exclusive scan of the bin's digit totals; the digits
+// packed into buckets (a bucket takes those that start within its span of
+// keys, so buckets are even where digits are not: the keys of a minimizer bin
+// crowd at the minimizers' own values); the buckets' starts and sizes.
 constexpr int BS_NT = 1024;
 __global__ void __launch_bounds__(BS_NT) k_bucket_scan(ExpandArgs a, uint64_t *bucket_start,
-                                                       uint64_t *bucket_size, uint32_t *bucket_bin) {
+                                                       uint64_t *bucket_size) {
   __shared__ uint32_t tmp[64];
+  __shared__ uint32_t first[1 << kCoarseMaxBits];  // start of every bucket, relative to the bin
   constexpr int DPT = (1 << kCoarseMaxBits) / BS_NT;
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   for (uint32_t b = blockIdx.x; b < a.nbins; b += gridDim.x) {
-    const uint32_t nd = 1u << a.bin_bits[b];
-    const uint64_t nch = a.chunk_base[b + 1] - a.chunk_base[b];
-    if (a.bin_kstart[b + 1] - a.bin_kstart[b] >= (1ull << 32)) {  // offsets in a bin are 32-bit
+    const uint32_t bits = a.bin_bits[b], nd = 1u << bits;
+    const uint64_t nk = a.bin_kstart[b + 1] - a.bin_kstart[b];
+    const uint64_t g0 = a.bucket_base[b];
+    const uint32_t nu = (uint32_t)(a.bucket_base[b + 1] - g0);  // at most nd
+    if (nk >= (1ull << 32)) {  // offsets in a bin are 32-bit
       if (threadIdx.x == 0) atomicOr(a.err, ERR_BIN_TOO_LARGE);
       continue;
     }
-    uint32_t *M = a.hist + a.hist_base[b];
+    const bool whole = plan_whole(nk, a.bucket_keys, bits);
     // thread t holds the contiguous digits [t * DPT, t * DPT + DPT)
-    uint32_t col[DPT];
-#pragma unroll
-    for (int u = 0; u < DPT; u++) col[u] = 0;
-    for (uint64_t jj = 0; jj < nch; jj++) {
-#pragma unroll
-      for (int u = 0; u < DPT; u++) {
-        const uint32_t d = threadIdx.x * DPT + u;
-        if (d < nd) col[u] += M[jj * nd + d];
-      }
-    }
-    uint32_t s = 0;
-#pragma unroll
-    for (int u = 0; u < DPT; u++) s += col[u];
-    uint32_t tot;
-    uint32_t run = block_exclusive_scan<BS_NT>(s, tmp, &tot);
-    const uint64_t g0 = a.bucket_base[b];
-    uint32_t start[DPT];
+    const uint32_t d0 = threadIdx.x * DPT;
+    const uint32_t *total = a.digit_total + ((uint64_t)b << a.max_bits);
+    uint32_t col[DPT], s = 0;
 #pragma unroll
     for (int u = 0; u < DPT; u++) {
-      const uint32_t d = threadIdx.x * DPT + u;
-      start[u] = run;
-      if (d < nd) {
-        bucket_start[g0 + d] = a.bin_kstart[b] + run;
-        bucket_size[g0 + d] = col[u];
-        bucket_bin[g0 + d] = b;
-        if (col[u] >= a.big_min) a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)(g0 + d);
-      }
-      run += col[u];
+      col[u] = d0 + u < nd ? total[d0 + u] : 0u;
+      s += col[u];
     }
-    for (uint64_t jj = 0; jj < nch; jj++) {
+    for (uint32_t u = threadIdx.x; u < nu; u += BS_NT) first[u] = ~0u;
+    uint32_t tot;
+    uint32_t at = block_exclusive_scan<BS_NT>(s, tmp, &tot);  // ends with a barrier
 #pragma unroll
-      for (int u = 0; u < DPT; u++) {
-        const uint32_t d = threadIdx.x * DPT + u;
-        if (d < nd) {
-          const uint32_t v = M[jj * nd + d];
-          M[jj * nd + d] = start[u];
-          start[u] += v;
-        }
+    for (int u = 0; u < DPT; u++) {
+      const uint32_t d = d0 + u;
+      if (d < nd) {
+        const uint32_t unit = whole ? d : min(at / a.bucket_keys, nu - 1);
+        a.lut[((uint64_t)b << a.max_bits) + d] = (uint16_t)unit;
+        atomicMin(&first[unit], at);
+        at += col[u];
       }
     }
     __syncthreads();
+    for (uint32_t u = threadIdx.x; u < nu; u += BS_NT) {
+      const uint32_t st = first[u];
+      uint32_t next = u + 1;  // buckets in which no digit starts are empty
+      while (next < nu && first[next] == ~0u) next++;
+      const uint32_t end = next < nu ? first[next] : (uint32_t)nk;
+      const uint64_t size = st == ~0u ? 0 : end - st;
+      bucket_start[g0 + u] = a.bin_kstart[b] + (st == ~0u ? end : st);
+      bucket_size[g0 + u] = size;
+      if (size >= a.big_min) a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)(g0 + u);
+    }
+    __syncthreads();
+  }
+}
+
+// Every chunk's write offset per bucket, relative to the bin's first key: one
+// thread per bucket adds up its digits chunk after chunk and leaves each
+// offset at the count of the bucket's first digit.
+__global__ void __launch_bounds__(kBucketOffsetThreads) k_bucket_offsets(ExpandArgs a, const uint64_t *bucket_start) {
+  if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
+  const uint64_t n_buckets = a.bucket_base[a.nbins];
+  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n_buckets;
+       g += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t b = find_bin(a.bucket_base, a.nbins, g);
+    const uint32_t u = (uint32_t)(g - a.bucket_base[b]), nd = 1u << a.bin_bits[b];
+    // the bucket's digits [lo, hi): a run in the ascending table
+    const uint16_t *lut = a.lut + ((uint64_t)b << a.max_bits);
+    uint32_t lo = 0, hi = nd;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (lut[mid] < u) lo = mid + 1; else hi = mid;
+    }
+    hi = lo;
+    for (uint32_t h = nd; hi < h;) {
+      const uint32_t mid = (hi + h) >> 1;
+      if (lut[mid] <= u) hi = mid + 1; else h = mid;
+    }
+    if (lo == hi) continue;  // no digit starts in it
+    const uint64_t nch = a.chunk_base[b + 1] - a.chunk_base[b];
+    uint32_t *M = a.hist + a.hist_base[b];
+    uint32_t run = (uint32_t)(bucket_start[g] - a.bin_kstart[b]);
+#pragma unroll 4
+    for (uint64_t jj = 0; jj < nch; jj++) {
+      uint32_t v = 0;
+      for (uint32_t d = lo; d < hi; d++) v += M[jj * nd + d];
+      M[jj * nd + lo] = run;
+      run += v;
+    }
   }
 }
 
@@ -388,21 +457,22 @@ constexpr int SC_THREADS = 1024;
 template <typename K> constexpr int sc_tile() { return sizeof(K) == 8 ? 16384 : 8192; }
 
 // Moves every key of `flat` to its bucket.  Each CTA takes whole chunks, a
-// tile of SC_TILE keys at a time: the tile is counting-sorted by digit in
-// shared memory (a key's rank within its digit from a shared-memory atomic),
-// then written out in that order, so the keys of one digit leave as a
-// contiguous run at the chunk's write offset for the digit (from the scan)
-// plus the digit's keys of the chunk's earlier tiles.
+// tile of SC_TILE keys at a time: the tile is counting-sorted by bucket in
+// shared memory (a key's rank within its bucket from a shared-memory atomic),
+// then written out in that order, so the keys of one bucket leave as a
+// contiguous run at the chunk's write offset for the bucket (from the scan)
+// plus the bucket's keys of the chunk's earlier tiles.
 template <typename K>
 __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) {
   constexpr int SC_TILE = sc_tile<K>(), KPT = SC_TILE / SC_THREADS;
   constexpr int ND = 1 << kCoarseMaxBits;
   extern __shared__ __align__(16) uint8_t sc_smem[];
   K *S = reinterpret_cast<K *>(sc_smem);                      // the tile, by digit
-  uint16_t *Sd = reinterpret_cast<uint16_t *>(S + SC_TILE);   // digits of S
+  uint16_t *Sd = reinterpret_cast<uint16_t *>(S + SC_TILE);   // buckets of S
   uint32_t *gbase = reinterpret_cast<uint32_t *>(Sd + SC_TILE);  // chunk's write offsets
-  uint32_t *done = gbase + ND;                                // digit's keys of the chunk's earlier tiles
+  uint32_t *done = gbase + ND;                                // bucket's keys of the chunk's earlier tiles
   uint32_t *toff = done + ND;                                 // tile counts, then tile offsets (ND + 1)
+  uint16_t *lut = reinterpret_cast<uint16_t *>(toff + ND + 1 + 64);  // bucket of every digit
   uint32_t *tmp = toff + ND + 1;                              // block scan
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   K *keys = reinterpret_cast<K *>(a.keys);
@@ -414,14 +484,17 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
     const uint32_t b = find_bin(a.chunk_base, a.nbins, c);
     const uint64_t j = c - a.chunk_base[b];
     const int cb = (int)a.bin_bits[b];
-    const uint32_t nd = 1u << cb;
+    const uint32_t nd = (uint32_t)(a.bucket_base[b + 1] - a.bucket_base[b]);  // buckets
     const uint64_t kbase = a.bin_kstart[b];
     const uint64_t q0 = kbase + j * a.chunk_kmers;
     const uint64_t q1 = min(q0 + a.chunk_kmers, a.bin_kstart[b + 1]);
-    const uint32_t *row = a.hist + a.hist_base[b] + j * nd;
-    for (uint32_t d = tid; d < nd; d += SC_THREADS) {
-      gbase[d] = row[d];
-      done[d] = 0;
+    const uint32_t *row = a.hist + a.hist_base[b] + (j << cb);
+    for (uint32_t d = tid; d < nd; d += SC_THREADS) done[d] = 0;
+    const uint16_t *glut = a.lut + ((uint64_t)b << a.max_bits);
+    for (uint32_t d = tid; d < (1u << cb); d += SC_THREADS) {
+      const uint16_t u = glut[d];
+      lut[d] = u;
+      if (d == 0 || glut[d - 1] != u) gbase[u] = row[d];  // the bucket's first digit holds its offset
     }
     for (uint64_t t0 = q0; t0 < q1; t0 += SC_TILE) {
       const uint32_t tn = (uint32_t)min((uint64_t)SC_TILE, q1 - t0);
@@ -433,15 +506,14 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
       for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
       __syncthreads();
       K xs[KPT];
-      uint32_t rk[KPT / 2];  // ranks within the digit, two 16-bit halves (< SC_TILE)
-#pragma unroll
-      for (int u = 0; u < KPT / 2; u++) rk[u] = 0;
+      uint32_t rk[KPT];  // bucket << 16 | rank within it (< SC_TILE)
 #pragma unroll
       for (int u = 0; u < KPT; u++) {
         const uint32_t i = u * SC_THREADS + tid;
         if (i < tn) {
           xs[u] = flat[t0 + i];
-          rk[u / 2] |= atomicAdd(&toff[coarse_digit<K>(xs[u], key_bits, cb)], 1u) << (16 * (u & 1));
+          const uint32_t d = lut[coarse_digit<K>(xs[u], key_bits, cb)];
+          rk[u] = (d << 16) | atomicAdd(&toff[d], 1u);
         }
       }
       __syncthreads();
@@ -462,8 +534,8 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
       for (int u = 0; u < KPT; u++) {
         const uint32_t i = u * SC_THREADS + tid;
         if (i < tn) {
-          const uint32_t d = coarse_digit<K>(xs[u], key_bits, cb);
-          const uint32_t at = toff[d] + ((rk[u / 2] >> (16 * (u & 1))) & 0xFFFFu);
+          const uint32_t d = rk[u] >> 16;
+          const uint32_t at = toff[d] + (rk[u] & 0xFFFFu);
           S[at] = xs[u];
           Sd[at] = (uint16_t)d;
         }
@@ -485,63 +557,107 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
 template <typename K> size_t bucket_scatter_smem_bytes() {
   constexpr int ND = 1 << kCoarseMaxBits;
   static_assert(sc_tile<K>() <= 65536 && sc_tile<K>() % SC_THREADS == 0, "16-bit ranks, whole rounds");
-  return (size_t)sc_tile<K>() * (sizeof(K) + 2) + 4 * (3 * ND + 1 + 64);
+  return (size_t)sc_tile<K>() * (sizeof(K) + 2) + 4 * (3 * ND + 1 + 64) + 2 * ND;
 }
 template size_t bucket_scatter_smem_bytes<uint64_t>();
 template size_t bucket_scatter_smem_bytes<u128>();
 
 // ---------------------------------------------------------------- 4. count
 
+// CAP: the most distinct keys a bucket (or a slice of one) is counted with in
+// shared memory; SLOTS: its hash table, at most two thirds full.
 template <typename K> struct CountShape;
-template <> struct CountShape<uint64_t> { static constexpr int NT = 512, CAP = 8192; };
-template <> struct CountShape<u128> { static constexpr int NT = 512, CAP = 4096; };
-constexpr int CC_SB_MAX = 12;        // sub-bucket bits
+template <> struct CountShape<uint64_t> { static constexpr int NT = 512, CAP = 4096, SLOTS = 6144; };
+template <> struct CountShape<u128> { static constexpr int NT = 512, CAP = 3072, SLOTS = 4608; };
+constexpr int CC_SB_MAX = 12;        // sub-bucket bits of an oversized bucket
 constexpr int CC_NSUB_MAX = 1 << CC_SB_MAX;
-constexpr uint32_t CC_THREAD_MAX = 8;  // larger sub-buckets are reduced by warps
-constexpr int CC_BIG_LIST = 1024;      // > CAP / (CC_THREAD_MAX + 1): every larger sub-bucket fits
+// k_bucket_sort: threads per CTA; a bucket is split into groups of at most
+// GROUP keys on average, sorted by one warp with at most RMAX keys a lane.
+template <typename K> struct SortShape;
+template <> struct SortShape<uint64_t> { static constexpr int NT = 256, GROUP = 128, RMAX = 16, CTAS = 5; };
+template <> struct SortShape<u128> { static constexpr int NT = 256, GROUP = 64, RMAX = 8, CTAS = 4; };
+constexpr int CS_GROUPS = 64;       // most groups of a bucket
+constexpr uint32_t CC_SPLIT_MAX = 512;  // groups of the sample sort (one per thread)
 constexpr uint32_t CC_TICKETS = 4;     // buckets taken per ticket
-constexpr int CC_STACK = 2 * 129 + 2;  // key-range halving: at most 128 levels, two entries each
+constexpr int CC_LEVELS = 130;      // open levels of an oversized bucket: each one fixes at least a bit
 
-// Heavy-slice hash table: keys, counts and a slot state (0 free, 1 being
-// written, 2 holds a key), inside the key area of the shared memory.
-template <typename K> struct HeavyTab {
-  static constexpr int SLOTS = (CountShape<K>::CAP * sizeof(K)) / (sizeof(K) + 8);
-  static constexpr int N = SLOTS >= 4096 ? 4096 : (SLOTS >= 2048 ? 2048 : 1024);
-  K key[N];
-  uint32_t cnt[N];
-  uint32_t state[N];
+// The hash table of a bucket and the areas of the sample sort of its distinct
+// keys.  8-byte keys: the table holds the keys (claimed by compare-and-swap)
+// and 16-bit counts beside them; an element's handle is its slot.
+template <typename K> struct HashArea {
+  static constexpr int CAP = CountShape<K>::CAP, SLOTS = CountShape<K>::SLOTS;
+  typedef uint64_t Member;     // groups hold the keys themselves
+  K T[SLOTS];                  // keys; at the end the sorted keys
+  uint32_t TC[SLOTS / 2];      // counts, two 16-bit halves a word; at the end the sorted counts
+  union {
+    Member G[CAP];             // the distinct keys, group after group
+    K spl[2 * CC_SPLIT_MAX];   // samples (runs of 32), then the sorted splitters
+  } g;
+  uint16_t L[CAP];             // handles of the distinct keys, then the group of every G entry
+  uint16_t GC[CAP];            // counts in G order
+};
+// 16-byte keys (no 128-bit compare-and-swap in shared memory): the bucket's
+// keys stay in shared memory and a slot holds (index of the key's first
+// claimant + 1) and the count in one word; an element's handle is that index.
+template <> struct HashArea<u128> {
+  static constexpr int CAP = CountShape<u128>::CAP, SLOTS = CountShape<u128>::SLOTS;
+  typedef uint16_t Member;     // groups hold handles
+  u128 A[CAP];                 // the bucket's keys
+  uint32_t T[SLOTS];           // 0: free, else (index + 1) | count << 13
+  union {
+    struct {
+      uint16_t G[CAP];         // handles of the distinct keys, group after group
+      uint16_t GC[CAP];        // counts in G order
+      uint16_t P[CAP];         // sorted order: G index of every output
+    } m;
+    u128 spl[2 * CC_SPLIT_MAX];
+  } g;
+  uint16_t L[CAP];             // slots of the distinct keys, then the group of every G entry
+};
+static_assert(CountShape<u128>::CAP < (1 << 13) - 1, "index + 1 fits 13 bits");
+
+// A bucket split into groups by splitters taken from its keys.
+template <typename K, int NT, int CAP_> struct SortArea {
+  static constexpr int CAP = CAP_;
+  K A[CAP];                             // keys, group after group; then each group's runs
+  uint16_t C[CAP];                      // group of each key; then first position of each run in its sorted group
+  K spl[CS_GROUPS];                     // splitters, in the order of a breadth-first search tree
+  uint32_t gcnt[CS_GROUPS];             // keys per group
+  uint32_t cur[CS_GROUPS];              // placement cursors
+  uint16_t goff[NT / 32][CS_GROUPS + 2];  // group starts, a copy for every warp
+  uint16_t gd[CS_GROUPS];               // runs per group
+  uint32_t next, same;                  // next group to sort; one key fills too much of the bucket
+};
+
+// Hash table of k_bucket_sort, for buckets of few distinct 8-byte keys: small
+// enough that five CTAs stay on an SM with the sort's areas for CAP keys.
+struct DedupArea {
+  static constexpr int SLOTS = 2560, CAP = 1280;
+  uint64_t T[SLOTS];
+  uint32_t TC[SLOTS / 2];               // counts, two 16-bit halves a word
+  uint16_t L[CAP];                      // slots of the distinct keys
 };
 
 template <typename K>
 struct CountSmem {
   static constexpr int CAP = CountShape<K>::CAP, NT = CountShape<K>::NT;
   union {
-    K A[CAP];  // keys of a bucket or a slice
-    HeavyTab<K> h;
+    HashArea<K> h;
+    SortArea<K, CountShape<K>::NT, CountShape<K>::CAP> s;
+    uint32_t sub[CC_NSUB_MAX];        // sub-bucket counts of an oversized bucket, then placement cursors
   } u;
-  // run counts; cursors of the oversized path (as 32-bit words)
-  uint16_t C[CAP > 2 * CC_NSUB_MAX ? CAP : 2 * CC_NSUB_MAX];
-  uint32_t cnt[CC_NSUB_MAX + 1];  // sub-bucket counts, then starts
-  uint32_t seg_pos[NT];           // output position of each thread's runs (exclusive scan)
-  uint32_t seg_src[NT];           // first run of each thread's segment in A
-  uint16_t big[CC_BIG_LIST];      // sub-buckets reduced by warps
+  uint32_t goff[CC_SPLIT_MAX + 1];    // group counts, then starts
   uint32_t tmp[64];
-  uint32_t nbig, hfill, nsub;
-  int flag, sp;
-  uint64_t g, start, n, out_base, run, tbase;
-  uint64_t pf_start, pf_n;        // the next bucket's keys, prefetched into L2
-  K red[64];                      // block min / max
-  uint32_t b;
-  union {
-    struct {
-      K lo[CC_STACK], hi[CC_STACK];
-    } stk;                       // key-range stack of the heavy path
-    uint16_t dc[CC_NSUB_MAX];    // distinct keys of each sub-bucket of a slice
-  } w;
+  uint32_t hfill;
+  int flag;
+  uint64_t g, start, n;
+  K red[64];                          // block min / max
+  // open levels of an oversized bucket: keys up to `end` are in buffer `buf`,
+  // in the order of the sb bits after the first cp
+  uint64_t lend[CC_LEVELS];
+  uint8_t lcp[CC_LEVELS], lsb[CC_LEVELS], lbuf[CC_LEVELS];
 };
-
-static_assert(CountShape<uint64_t>::CAP / (CC_THREAD_MAX + 1) < CC_BIG_LIST, "big list holds every large sub-bucket");
-static_assert(CountShape<u128>::CAP / (CC_THREAD_MAX + 1) < CC_BIG_LIST, "big list holds every large sub-bucket");
+static_assert(sizeof(CountSmem<uint64_t>) <= 115712 && sizeof(CountSmem<u128>) <= 115712, "two CTAs per SM");
 
 template <typename K> size_t bucket_count_smem_bytes() { return sizeof(CountSmem<K>); }
 template <typename K> uint64_t bucket_count_cap() { return CountShape<K>::CAP; }
@@ -550,141 +666,50 @@ template uint64_t bucket_count_cap<u128>();
 template size_t bucket_count_smem_bytes<uint64_t>();
 template size_t bucket_count_smem_bytes<u128>();
 
-// In-place ascending sort of A[0, m) by one warp (bitonic network whose
-// comparators put the smaller key first, so indices >= m act as +infinity).
-template <typename K>
-GKC_DEV void warp_sort(K *A, uint32_t m) {
-  uint32_t P = 1;
-  while (P < m) P <<= 1;
-  const uint32_t lane = threadIdx.x & 31u;
-  for (uint32_t size = 2; size <= P; size <<= 1) {
-    const uint32_t half = size >> 1;
-    for (uint32_t i = lane; i < P / 2; i += 32) {
-      const uint32_t blk = i / half, off = i % half;
-      const uint32_t lo = blk * size + off, hi = blk * size + size - 1 - off;
-      if (hi < m) {
-        const K x = A[lo], y = A[hi];
-        if (y < x) {
-          A[lo] = y;
-          A[hi] = x;
-        }
-      }
-    }
-    __syncwarp();
-    for (uint32_t stride = size >> 2; stride >= 1; stride >>= 1) {
-      for (uint32_t i = lane; i < P / 2; i += 32) {
-        const uint32_t blk = i / stride, off = i % stride;
-        const uint32_t lo = blk * 2 * stride + off, hi = lo + stride;
-        if (hi < m) {
-          const K x = A[lo], y = A[hi];
-          if (y < x) {
-            A[lo] = y;
-            A[hi] = x;
-          }
-        }
-      }
-      __syncwarp();
-    }
-  }
-}
+template <typename K> struct SortSmem {
+  static constexpr int NT = SortShape<K>::NT;
+  union {
+    SortArea<K, NT, CountShape<K>::CAP> s;
+    struct {
+      DedupArea t;
+      SortArea<K, NT, DedupArea::CAP> s;
+    } d;                              // 8-byte keys only
+  } u;
+  uint32_t tmp[64];
+  uint32_t hfill;
+  int flag;
+  uint64_t g, start;
+  uint32_t n;
+  uint64_t bg[CC_TICKETS], bstart[CC_TICKETS];  // the batch of buckets in hand
+  uint32_t bn[CC_TICKETS];
+  uint64_t pf_start;                  // the next bucket's keys, prefetched into L2
+  uint32_t pf_n;
+};
+static_assert(sizeof(SortSmem<uint64_t>) <= 45568, "five CTAs per SM");
+template <typename K> size_t bucket_sort_smem_bytes() { return sizeof(SortSmem<K>); }
+template size_t bucket_sort_smem_bytes<uint64_t>();
+template size_t bucket_sort_smem_bytes<u128>();
 
-// The same network over (key, count) pairs, by the whole block.
-template <typename K, int NT>
-GKC_DEV void block_sort_pairs(K *A, uint32_t *cv, uint32_t m) {
-  uint32_t P = 1;
-  while (P < m) P <<= 1;
-  for (uint32_t size = 2; size <= P; size <<= 1) {
-    const uint32_t half = size >> 1;
-    for (uint32_t i = threadIdx.x; i < P / 2; i += NT) {
-      const uint32_t blk = i / half, off = i % half;
-      const uint32_t lo = blk * size + off, hi = blk * size + size - 1 - off;
-      if (hi < m && A[hi] < A[lo]) {
-        const K x = A[lo];
-        A[lo] = A[hi];
-        A[hi] = x;
-        const uint32_t c = cv[lo];
-        cv[lo] = cv[hi];
-        cv[hi] = c;
-      }
-    }
-    __syncthreads();
-    for (uint32_t stride = size >> 2; stride >= 1; stride >>= 1) {
-      for (uint32_t i = threadIdx.x; i < P / 2; i += NT) {
-        const uint32_t blk = i / stride, off = i % stride;
-        const uint32_t lo = blk * 2 * stride + off, hi = lo + stride;
-        if (hi < m && A[hi] < A[lo]) {
-          const K x = A[lo];
-          A[lo] = A[hi];
-          A[hi] = x;
-          const uint32_t c = cv[lo];
-          cv[lo] = cv[hi];
-          cv[hi] = c;
-        }
-      }
-      __syncthreads();
-    }
-  }
-}
-
-// Exclusive scan of S.cnt[0, nsub) in place (thread-contiguous groups).
-template <typename K, int NT>
-GKC_DEV void scan_sub(CountSmem<K> &S, uint32_t nsub) {
+// Exclusive scan of cnt[0, nsub) in place (thread-contiguous groups).
+template <int NT>
+GKC_DEV void scan_sub(uint32_t *cnt, uint32_t *tmp, uint32_t nsub) {
   const uint32_t per = (nsub + NT - 1) / NT, c0 = threadIdx.x * per;
   uint32_t s = 0;
-  for (uint32_t jj = c0; jj < c0 + per && jj < nsub; jj++) s += S.cnt[jj];
+  for (uint32_t jj = c0; jj < c0 + per && jj < nsub; jj++) s += cnt[jj];
   uint32_t tot;
-  uint32_t run = block_exclusive_scan<NT>(s, S.tmp, &tot);
+  uint32_t run = block_exclusive_scan<NT>(s, tmp, &tot);
   for (uint32_t jj = c0; jj < c0 + per && jj < nsub; jj++) {
-    const uint32_t v = S.cnt[jj];
-    S.cnt[jj] = run;
+    const uint32_t v = cnt[jj];
+    cnt[jj] = run;
     run += v;
   }
   __syncthreads();
-}
-
-template <typename K>
-GKC_DEV void insertion_sort(K *A, uint32_t b0, uint32_t b1) {
-  for (uint32_t p = b0 + 1; p < b1; p++) {
-    const K x = A[p];
-    uint32_t q = p;
-    while (q > b0 && x < A[q - 1]) {
-      A[q] = A[q - 1];
-      q--;
-    }
-    A[q] = x;
-  }
-}
-
-// Run-length encodes the sorted A[b0, b1) in place (keys in A, counts in C
-// from b0); returns the number of runs.
-template <typename K>
-GKC_DEV uint32_t rle_in_place(K *A, uint16_t *C, uint32_t b0, uint32_t b1) {
-  uint32_t u = 0;
-  for (uint32_t i = b0; i < b1;) {
-    const K x = A[i];
-    uint32_t c = 1;
-    i++;
-    while (i < b1 && A[i] == x) {
-      c++;
-      i++;
-    }
-    A[b0 + u] = x;
-    C[b0 + u] = (uint16_t)c;  // c <= m <= CAP < 2^16
-    u++;
-  }
-  return u;
 }
 
 template <typename K> GKC_DEV K shfl_xor_k(K v, int m) { return __shfl_xor_sync(0xffffffffu, v, m); }
 template <> GKC_DEV u128 shfl_xor_k<u128>(u128 v, int m) {
   const uint64_t lo = __shfl_xor_sync(0xffffffffu, (uint64_t)v, m);
   const uint64_t hi = __shfl_xor_sync(0xffffffffu, (uint64_t)(v >> 64), m);
-  return ((u128)hi << 64) | lo;
-}
-template <typename K> GKC_DEV K shfl_up_k(K v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
-template <> GKC_DEV u128 shfl_up_k<u128>(u128 v, int d) {
-  const uint64_t lo = __shfl_up_sync(0xffffffffu, (uint64_t)v, d);
-  const uint64_t hi = __shfl_up_sync(0xffffffffu, (uint64_t)(v >> 64), d);
   return ((u128)hi << 64) | lo;
 }
 
@@ -712,6 +737,310 @@ GKC_DEV void block_minmax(CountSmem<K> &S, K &lo, K &hi) {
   __syncthreads();
 }
 
+// ---- a bucket (or a slice of one) in shared memory: its keys aggregated in
+// a hash table, so that only its distinct keys are sorted, then a sample sort
+// of those.  Keys of a minimizer bin are far from uniform in their leading
+// bases (those holding the minimizer near their start share them), so the
+// sort takes its splitters from the keys: the table's slots are in hash
+// order, which makes any fixed choice of them a random sample.
+
+constexpr uint64_t HT_MAX_KEYS = 65535;  // counts are 16-bit (8-byte keys)
+constexpr uint64_t HT_EMPTY = ~0ull;     // never a canonical key: the reverse complement of all-T is all-A
+
+GKC_DEV uint32_t ht_slot(uint64_t x, uint32_t slots) {
+  return __umulhi((uint32_t)((x * 0x9E3779B97F4A7C15ull) >> 32), slots);
+}
+GKC_DEV uint32_t ht_slot(u128 x, uint32_t slots) {
+  const uint64_t y = (uint64_t)x * 0x9E3779B97F4A7C15ull + (uint64_t)(x >> 64) * 0xC2B2AE3D27D4EB4Full;
+  return __umulhi((uint32_t)(y >> 32), slots);
+}
+
+// Slots for n keys: twice as many, whole rounds of the block.
+template <typename K>
+GKC_DEV uint32_t ht_slots(uint64_t n) {
+  constexpr uint32_t NT = CountShape<K>::NT, SLOTS = CountShape<K>::SLOTS;
+  return 2 * n >= SLOTS ? SLOTS : max(NT, ((uint32_t)(2 * n) + NT - 1) / NT * NT);
+}
+
+// Inserts the n keys into the table tab (S holds the fill counter and the
+// flag); false when they hold more than CAP distinct ones (only possible for
+// n > CAP).  At most CAP + NT slots are ever taken, so every probe chain ends
+// at a free slot.
+template <int NT, uint32_t CAP, uint32_t SLOTS, typename SM>
+GKC_DEV bool table_insert64(SM &S, uint64_t *tab, uint32_t *counts, const uint64_t *src, uint64_t n, uint32_t slots) {
+  constexpr int U = 8;  // keys in flight per thread
+  static_assert(CAP + NT < SLOTS, "a free slot is always left");
+  const int tid = threadIdx.x;
+  const bool limited = n > CAP;
+  for (uint32_t i = tid; i < slots; i += NT) tab[i] = HT_EMPTY;
+  for (uint32_t i = tid; i < slots / 2; i += NT) counts[i] = 0;
+  if (tid == 0) {
+    S.hfill = 0;
+    S.flag = 0;
+  }
+  __syncthreads();
+  volatile uint64_t *T = tab;
+  for (uint64_t i0 = tid; i0 < n; i0 += (uint64_t)U * NT) {
+    uint64_t xs[U];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint64_t i = i0 + (uint64_t)u * NT;
+      xs[u] = i < n ? __ldcg(reinterpret_cast<const unsigned long long *>(src) + i) : HT_EMPTY;
+    }
+    if (limited && *(volatile int *)&S.flag) break;
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const uint64_t x = xs[u];
+      if (x == HT_EMPTY || (limited && *(volatile int *)&S.flag)) break;  // past the end, or given up
+      uint32_t h = ht_slot(x, slots);
+      while (true) {
+        uint64_t cur = T[h];
+        if (cur == HT_EMPTY) {
+          cur = atomicCAS(reinterpret_cast<unsigned long long *>(tab + h), (unsigned long long)HT_EMPTY,
+                          (unsigned long long)x);
+          if (cur == HT_EMPTY) {
+            if (limited && atomicAdd(&S.hfill, 1u) + 1 > CAP) S.flag = 1;
+            cur = x;
+          }
+        }
+        if (cur == x) break;
+        h = h + 1 == slots ? 0 : h + 1;
+      }
+      atomicAdd(&counts[h >> 1], 1u << (16 * (h & 1u)));
+    }
+  }
+  __syncthreads();
+  return !(limited && S.flag);
+}
+template <int NT>
+GKC_DEV bool table_insert(CountSmem<uint64_t> &S, const uint64_t *src, uint64_t n, uint32_t slots) {
+  return table_insert64<NT, CountShape<uint64_t>::CAP, CountShape<uint64_t>::SLOTS>(S, S.u.h.T, S.u.h.TC, src, n, slots);
+}
+GKC_DEV bool slot_taken(const CountSmem<uint64_t> &S, uint32_t slot) { return S.u.h.T[slot] != HT_EMPTY; }
+GKC_DEV uint64_t slot_key(const CountSmem<uint64_t> &S, uint32_t slot) { return S.u.h.T[slot]; }
+GKC_DEV void put_member(CountSmem<uint64_t> &S, uint32_t at, uint32_t slot) {
+  HashArea<uint64_t> &H = S.u.h;
+  H.g.G[at] = H.T[slot];
+  H.GC[at] = (uint16_t)(H.TC[slot >> 1] >> (16 * (slot & 1u)));
+}
+GKC_DEV uint64_t member_key(const CountSmem<uint64_t> &S, uint32_t i) { return S.u.h.g.G[i]; }
+GKC_DEV void put_sorted(CountSmem<uint64_t> &S, uint32_t at, uint32_t i, uint64_t x) {
+  HashArea<uint64_t> &H = S.u.h;  // the table is no longer read
+  H.T[at] = x;
+  reinterpret_cast<uint16_t *>(H.TC)[at] = H.GC[i];
+}
+GKC_DEV void get_sorted(const CountSmem<uint64_t> &S, uint32_t at, uint64_t &x, uint32_t &c) {
+  x = S.u.h.T[at];
+  c = reinterpret_cast<const uint16_t *>(S.u.h.TC)[at];
+}
+
+// 16-byte keys: n <= CAP, so they never hold too many distinct ones.
+template <int NT>
+GKC_DEV bool table_insert(CountSmem<u128> &S, const u128 *src, uint64_t n, uint32_t slots) {
+  HashArea<u128> &H = S.u.h;
+  const int tid = threadIdx.x;
+  if (n > (uint64_t)CountShape<u128>::CAP) return false;
+  for (uint32_t i = tid; i < (uint32_t)n; i += NT) {
+    const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(src) + i);
+    H.A[i] = ((u128)v.y << 64) | v.x;
+  }
+  for (uint32_t i = tid; i < slots; i += NT) H.T[i] = 0;
+  __syncthreads();
+  volatile uint32_t *T = H.T;
+  for (uint32_t i = tid; i < (uint32_t)n; i += NT) {
+    const u128 x = H.A[i];
+    uint32_t h = ht_slot(x, slots);
+    while (true) {
+      uint32_t cur = T[h];
+      if (cur == 0) {
+        cur = atomicCAS(&H.T[h], 0u, (i + 1) | (1u << 13));
+        if (cur == 0) break;
+      }
+      if (H.A[(cur & 8191u) - 1] == x) {
+        atomicAdd(&H.T[h], 1u << 13);
+        break;
+      }
+      h = h + 1 == slots ? 0 : h + 1;
+    }
+  }
+  __syncthreads();
+  return true;
+}
+GKC_DEV bool slot_taken(const CountSmem<u128> &S, uint32_t slot) { return S.u.h.T[slot] != 0; }
+GKC_DEV u128 slot_key(const CountSmem<u128> &S, uint32_t slot) { return S.u.h.A[(S.u.h.T[slot] & 8191u) - 1]; }
+GKC_DEV void put_member(CountSmem<u128> &S, uint32_t at, uint32_t slot) {
+  HashArea<u128> &H = S.u.h;
+  const uint32_t t = H.T[slot];
+  H.g.m.G[at] = (uint16_t)((t & 8191u) - 1);
+  H.g.m.GC[at] = (uint16_t)(t >> 13);
+}
+GKC_DEV u128 member_key(const CountSmem<u128> &S, uint32_t i) { return S.u.h.A[S.u.h.g.m.G[i]]; }
+GKC_DEV void put_sorted(CountSmem<u128> &S, uint32_t at, uint32_t i, u128) { S.u.h.g.m.P[at] = (uint16_t)i; }
+GKC_DEV void get_sorted(const CountSmem<u128> &S, uint32_t at, u128 &x, uint32_t &c) {
+  const uint32_t i = S.u.h.g.m.P[at];
+  x = member_key(S, i);
+  c = S.u.h.g.m.GC[i];
+}
+
+// Counts the n keys src[0, n) through the table and writes their sorted runs
+// to the staging arrays at `out_at`; their number is left in S.hfill.
+// Returns false, with nothing written, when there are more than CAP distinct
+// keys (the caller then splits them).  Not inlined: it is called for whole
+// buckets and for the slices of large ones.
+template <typename K, int NT>
+__device__ __noinline__ bool hash_count(CountSmem<K> &S, const SortCountArgs &a, const K *src, uint64_t n,
+                                        uint64_t out_at) {
+  constexpr int CAP = CountShape<K>::CAP;
+  constexpr int EPT = CAP / NT;                     // elements per thread
+  constexpr int SPT = CountShape<K>::SLOTS / NT;    // slots per thread
+  static_assert(CAP % NT == 0 && CountShape<K>::SLOTS % NT == 0 && CC_SPLIT_MAX == NT, "whole rounds");
+  static_assert(CountShape<K>::SLOTS <= 8192 && SPT <= 32, "13-bit slots, one mask per thread");
+  const int tid = threadIdx.x, lane = tid & 31;
+  HashArea<K> &H = S.u.h;
+  const uint32_t slots = ht_slots<K>(n);
+  if (!table_insert<NT>(S, src, n, slots)) {
+    __syncthreads();
+    return false;
+  }
+  // the taken slots, listed
+  uint32_t mask = 0;
+#pragma unroll
+  for (int q = 0; q < SPT; q++) {
+    const uint32_t slot = q * NT + tid;
+    if (slot < slots && slot_taken(S, slot)) mask |= 1u << q;
+  }
+  uint32_t D;
+  {
+    uint32_t pos = block_exclusive_scan<NT>(__popc(mask), S.tmp, &D);
+    while (mask) {
+      const int q = __ffs(mask) - 1;
+      mask &= mask - 1;
+      H.L[pos++] = (uint16_t)(q * NT + tid);
+    }
+  }
+  S.goff[tid] = 0;
+  __syncthreads();
+  // ns - 1 splitters, so groups of about D / ns in (4, 8] keys: ns samples,
+  // runs of 32 sorted by warps, then ranked against every other run
+  uint32_t ns = 1;
+  while (8 * ns < D && ns < CC_SPLIT_MAX) ns <<= 1;
+  if (ns > 1) {
+    K x = ~(K)0;
+    const uint32_t nw = max(ns, 32u);
+    if ((uint32_t)tid < nw) {
+      if ((uint32_t)tid < ns) x = slot_key(S, H.L[(uint32_t)tid * D / ns]);
+#pragma unroll
+      for (int size = 2; size <= 32; size <<= 1) {
+#pragma unroll
+        for (int stride = size >> 1; stride > 0; stride >>= 1) {
+          const K y = shfl_xor_k<K>(x, stride);
+          const bool keep_min = ((lane & stride) == 0) == ((lane & size) == 0);
+          x = keep_min ? (y < x ? y : x) : (x < y ? y : x);
+        }
+      }
+      H.g.spl[tid] = x;
+    }
+    __syncthreads();
+    if ((uint32_t)tid < ns) {
+      uint32_t rank = lane;
+      for (uint32_t r = 0; r < ns; r += 32) {
+        if (r == (uint32_t)(tid & ~31)) continue;
+        const K *R = H.g.spl + r;
+        uint32_t p = 0;
+#pragma unroll
+        for (uint32_t st = 16; st > 0; st >>= 1)
+          if (R[p + st - 1] < x) p += st;
+        rank += p + (R[p] < x ? 1u : 0u);
+      }
+      H.g.spl[CC_SPLIT_MAX + rank] = x;
+    }
+    __syncthreads();
+  }
+  // each key's group (the splitters below it) and place in the group
+  uint32_t es[EPT], er[EPT];  // slot | group << 13; place
+  const K *spl = H.g.spl + CC_SPLIT_MAX;
+#pragma unroll
+  for (int u = 0; u < EPT; u++) {
+    const uint32_t i = u * NT + tid;
+    if (i < D) {
+      const uint32_t slot = H.L[i];
+      const K x = slot_key(S, slot);
+      uint32_t p = 0;
+      for (uint32_t st = ns >> 1; st > 0; st >>= 1)
+        if (spl[p + st - 1] < x) p += st;
+      es[u] = slot | (p << 13);
+      er[u] = atomicAdd(&S.goff[p], 1u);
+    }
+  }
+  __syncthreads();
+  {
+    const uint32_t c = S.goff[tid];
+    uint32_t tot;
+    const uint32_t o = block_exclusive_scan<NT>(c, S.tmp, &tot);
+    S.goff[tid] = o;
+    if (tid == 0) S.goff[NT] = tot;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int u = 0; u < EPT; u++) {
+    const uint32_t i = u * NT + tid;
+    if (i < D) {
+      const uint32_t p = es[u] >> 13, at = S.goff[p] + er[u];
+      put_member(S, at, es[u] & 8191u);
+      H.L[at] = (uint16_t)p;  // the list of slots is no longer read
+    }
+  }
+  __syncthreads();
+  // rank within the group
+  for (uint32_t i = tid; i < D; i += NT) {
+    const uint32_t p = H.L[i], b0 = S.goff[p], b1 = S.goff[p + 1];
+    const K x = member_key(S, i);
+    uint32_t at = b0;
+    for (uint32_t j = b0; j < b1; j++) at += member_key(S, j) < x ? 1u : 0u;
+    put_sorted(S, at, i, x);
+  }
+  __syncthreads();
+  K *out = reinterpret_cast<K *>(a.stage_keys);
+  for (uint32_t i = tid; i < D; i += NT) {
+    if (out_at + i < a.stage_cap) {
+      K x;
+      uint32_t c;
+      get_sorted(S, i, x, c);
+      out[out_at + i] = x;
+      a.stage_counts[out_at + i] = c;
+    } else {
+      atomicOr(a.err, ERR_CAPACITY);
+    }
+  }
+  if (tid == 0) S.hfill = D;
+  __syncthreads();
+  return true;
+}
+
+
+// ---- a bucket (or a slice of one) sorted without a table: split into groups
+// of about 100 keys by splitters taken from its keys, each group sorted by a
+// warp in registers.
+
+template <typename K> GKC_DEV K shfl_up_k(K v, int d) { return __shfl_up_sync(0xffffffffu, v, d); }
+template <typename K> GKC_DEV K shfl_k(K v, int l) { return __shfl_sync(0xffffffffu, v, l); }
+template <> GKC_DEV u128 shfl_k<u128>(u128 v, int l) {
+  const uint64_t lo = __shfl_sync(0xffffffffu, (uint64_t)v, l);
+  const uint64_t hi = __shfl_sync(0xffffffffu, (uint64_t)(v >> 64), l);
+  return ((u128)hi << 64) | lo;
+}
+// A key read once (L2 only: the staged runs overwrite it).
+GKC_DEV uint64_t load_key(const uint64_t *p) { return __ldcg(reinterpret_cast<const unsigned long long *>(p)); }
+GKC_DEV u128 load_key(const u128 *p) {
+  const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(p));
+  return ((u128)v.y << 64) | v.x;
+}
+template <> GKC_DEV u128 shfl_up_k<u128>(u128 v, int d) {
+  const uint64_t lo = __shfl_up_sync(0xffffffffu, (uint64_t)v, d);
+  const uint64_t hi = __shfl_up_sync(0xffffffffu, (uint64_t)(v >> 64), d);
+  return ((u128)hi << 64) | lo;
+}
+
 GKC_DEV uint32_t warp_exclusive_scan(uint32_t c, uint32_t *total) {
   const uint32_t lane = threadIdx.x & 31u;
   uint32_t inc = c;
@@ -724,51 +1053,75 @@ GKC_DEV uint32_t warp_exclusive_scan(uint32_t c, uint32_t *total) {
   return inc - c;
 }
 
-// Sorts A[b0, b0 + n), n <= 32 R, with the calling warp: lane l holds
-// positions l R .. l R + R - 1 in registers (positions past n hold the
-// largest key, so the first n sorted positions are A's keys), a bitonic
-// network over 32 R positions; then run-length encodes the sorted keys in
-// place (keys in A, counts in C from b0).  Returns the number of runs.
+// Bitonic merge of each lane's R keys (ascending if asc).
 template <typename K, int R>
-GKC_DEV uint32_t warp_sort_rle(K *A, uint16_t *C, uint32_t b0, uint32_t n) {
-  constexpr uint32_t N = 32 * R;
+GKC_DEV void lane_merge(K (&v)[R], bool asc) {
+#pragma unroll
+  for (int stride = R / 2; stride > 0; stride >>= 1) {
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if ((r & stride) == 0) {
+        const K x = v[r], y = v[r + stride];
+        const bool sw = (y < x) == asc;
+        v[r] = sw ? y : x;
+        v[r + stride] = sw ? x : y;
+      }
+  }
+}
+
+// Sorts the warp's 32 R keys ascending, sorted position e in lane e / R,
+// register e % R: a bitonic network whose strides below R stay in a lane, so
+// that only 15 of its steps exchange keys between lanes, whatever R.  The
+// steps between lanes are a loop, not unrolled: straight-line networks of
+// several sizes are more code than the instruction cache holds, and their
+// fetches cost more than the network (count stage of 135 M keys: 7.1 ms
+// unrolled, 3.4 ms with one size left).
+template <typename K, int R>
+GKC_DEV void warp_bitonic(K (&v)[R]) {
+  const uint32_t lane = threadIdx.x & 31u;
+#pragma unroll
+  for (int size = 2; size <= R; size <<= 1) {
+#pragma unroll
+    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+#pragma unroll
+      for (int r = 0; r < R; r++)
+        if ((r & stride) == 0) {
+          const bool asc = size < R ? (r & size) == 0 : (lane & 1u) == 0;
+          const K x = v[r], y = v[r + stride];
+          const bool sw = (y < x) == asc;
+          v[r] = sw ? y : x;
+          v[r + stride] = sw ? x : y;
+        }
+    }
+  }
+#pragma unroll 1
+  for (uint32_t lsize = 2; lsize <= 32; lsize <<= 1) {
+    const bool asc = (lane & lsize) == 0;
+#pragma unroll 1
+    for (uint32_t lm = lsize >> 1; lm > 0; lm >>= 1) {
+      const bool keep_min = ((lane & lm) == 0) == asc;
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const K y = shfl_xor_k<K>(v[r], (int)lm);
+        v[r] = (y < v[r]) == keep_min ? y : v[r];
+      }
+    }
+    lane_merge<K, R>(v, asc);
+  }
+}
+
+// Sorts A[b0, b0 + n), n <= 32 R, with the calling warp and leaves its runs
+// there: the distinct keys in A, the first position of each in C.  Returns
+// their number.
+template <typename K, int R>
+GKC_DEV uint32_t warp_sort_runs(K *A, uint16_t *C, uint32_t b0, uint32_t n) {
   const uint32_t lane = threadIdx.x & 31u;
   K v[R];
 #pragma unroll
-  for (int r = 0; r < R; r++) {
-    const uint32_t e = lane * R + r;
-    v[r] = e < n ? A[b0 + e] : ~(K)0;
-  }
-#pragma unroll
-  for (uint32_t size = 2; size <= N; size <<= 1) {
-#pragma unroll
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride < (uint32_t)R) {
-#pragma unroll
-        for (int r = 0; r < R; r++)
-          if ((r & stride) == 0) {
-            const bool asc = ((lane * R + r) & size) == 0;
-            const K x = v[r], y = v[r + stride];
-            const bool sw = asc ? (y < x) : (x < y);
-            v[r] = sw ? y : x;
-            v[r + stride] = sw ? x : y;
-          }
-      } else {
-        const int lm = (int)(stride / R);
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const K y = shfl_xor_k<K>(v[r], lm);
-          const bool asc = ((lane * R + r) & size) == 0;
-          const bool low = (lane & (uint32_t)lm) == 0;  // the lower position of the pair
-          const bool keep_min = low == asc;
-          v[r] = keep_min ? (y < v[r] ? y : v[r]) : (v[r] < y ? y : v[r]);
-        }
-      }
-    }
-  }
-  // run heads among the first n positions
+  for (int r = 0; r < R; r++) v[r] = r * 32 + lane < n ? A[b0 + r * 32 + lane] : ~(K)0;
+  warp_bitonic<K, R>(v);
   const K before = shfl_up_k<K>(v[R - 1], 1);
-  uint32_t hb = 0;
+  uint32_t hb = 0;  // run heads among the first n positions
 #pragma unroll
   for (int r = 0; r < R; r++) {
     const uint32_t e = lane * R + r;
@@ -776,765 +1129,458 @@ GKC_DEV uint32_t warp_sort_rle(K *A, uint16_t *C, uint32_t b0, uint32_t n) {
     if (e < n && (e == 0 || p != v[r])) hb |= 1u << r;
   }
   uint32_t D;
-  const uint32_t rank0 = warp_exclusive_scan(__popc(hb), &D);
-  __syncwarp();
-  uint32_t rank = rank0;
+  uint32_t rank = b0 + warp_exclusive_scan(__popc(hb), &D);
 #pragma unroll
   for (int r = 0; r < R; r++)
     if ((hb >> r) & 1u) {
-      A[b0 + rank] = v[r];
-      C[b0 + rank] = (uint16_t)(lane * R + r);  // the run's first position, < 32 R
-      rank++;
-    }
-  __syncwarp();
-  uint32_t nxt[R];
-  rank = rank0;
-#pragma unroll
-  for (int r = 0; r < R; r++)
-    if ((hb >> r) & 1u) {
-      nxt[r] = rank + 1 < D ? C[b0 + rank + 1] : n;
-      rank++;
-    }
-  __syncwarp();
-  rank = rank0;
-#pragma unroll
-  for (int r = 0; r < R; r++)
-    if ((hb >> r) & 1u) {
-      C[b0 + rank] = (uint16_t)(nxt[r] - (lane * R + r));
+      A[rank] = v[r];
+      C[rank] = (uint16_t)(lane * R + r);
       rank++;
     }
   __syncwarp();
   return D;
 }
 
-template <typename K> GKC_DEV K warp_min_k(K v) {
+constexpr uint32_t SORT_REJECTED = ~0u;
+
+// Counts the n <= CAP keys src[0, n) and writes their sorted runs to the
+// staging arrays at `out_at`; returns their number, or SORT_REJECTED with
+// nothing written when a group is too large for a warp (copies of one key
+// cannot be split): the caller takes the hash table then.
+//
+// What bounds it is instruction issue and the shared-memory port, so it keeps
+// the keys in registers where it can: 128 samples are sorted by one warp and
+// every second to fourth (fewer groups: more) becomes a splitter, which keeps
+// groups even whatever the keys' distribution; a key's group is found in a
+// breadth-first tree (the nodes of a level are neighbours, so the lanes'
+// loads meet in few banks); the groups' network needs 15 exchanges between
+// lanes at any size.
+// Keys in global memory: a run's count is its length.
+template <typename K> struct GlobalKeys {
+  const K *p;
+  GKC_DEV K key(uint32_t i) const { return load_key(p + i); }
+  GKC_DEV uint32_t count(K, uint32_t run) const { return run; }
+};
+// The distinct keys of the table: a key's count is found in its slot.
+struct TableKeys {
+  const DedupArea &t;
+  GKC_DEV uint64_t key(uint32_t i) const { return t.T[t.L[i]]; }
+  GKC_DEV uint32_t count(uint64_t x, uint32_t) const {
+    uint32_t h = ht_slot(x, DedupArea::SLOTS);
+    while (t.T[h] != x) h = h + 1 == DedupArea::SLOTS ? 0 : h + 1;  // x is in the table
+    return (t.TC[h >> 1] >> (16 * (h & 1u))) & 0xFFFFu;
+  }
+};
+
+template <typename K, int NT, typename Src, typename Area>
+GKC_DEV uint32_t sort_count(Area &S, const SortCountArgs &a, const Src &src, uint32_t n, uint64_t out_at) {
+  constexpr int CAP = Area::CAP, W = NT / 32, RMAX = SortShape<K>::RMAX;
+  static_assert(CAP <= 65535 && (CS_GROUPS * SortShape<K>::GROUP) >= CAP, "16-bit positions");
+  const uint32_t tid = threadIdx.x, lane = tid & 31u, w = tid >> 5;
+  int lg = 0;
+  while (((uint32_t)SortShape<K>::GROUP << lg) < n || (lg < 3 && (32u << lg) < n)) lg++;  // few keys: a group for every warp
+  const uint32_t G = 1u << lg;  // <= CS_GROUPS
+  if (tid < CS_GROUPS) S.gcnt[tid] = lg == 0 && tid == 0 ? n : 0u;
+  if (tid == NT - 1) {
+    S.next = 0;
+    if (lg == 0) S.same = 0;
+  }
+  if (lg > 0 && w == 0) {
+    // splitter j (1 .. G - 1) is sample j * (samples / G); as a node of the
+    // tree it is number j >> (t + 1) of its level, t its trailing zero bits
+    K v[4];
+    uint32_t any = 0;
+    if (G <= 8) {  // n > 32 here: 32 samples, one a lane
+      K u[1] = {src.key(lane * n / 32)};
+      warp_bitonic<K, 1>(u);
+      const uint32_t j = lane * G / 32;
+      if (j > 0 && j * 32 == lane * G) {
+        const int t = __ffs((int)j) - 1;
+        S.spl[(1u << (lg - 1 - t)) + (j >> (t + 1))] = u[0];
+      }
+    } else {
 #pragma unroll
-  for (int m = 16; m > 0; m >>= 1) {
-    const K y = shfl_xor_k<K>(v, m);
-    v = y < v ? y : v;
-  }
-  return v;
-}
-
-// Run-length encodes A[b0, b0 + n) with the calling warp when it holds at
-// most 32 distinct keys: each round takes the smallest key above the last
-// one and counts its copies.  Returns the number of runs, or 0 (A untouched)
-// when there are more.
-template <typename K>
-GKC_DEV uint32_t warp_select_rle(K *A, uint16_t *C, uint32_t b0, uint32_t n) {
-  const uint32_t lane = threadIdx.x & 31u;
-  K mine = 0;
-  uint32_t mine_c = 0, d = 0, seen = 0;
-  K last = 0;
-  while (seen < n) {
-    if (d == 32) return 0;
-    K lo = ~(K)0;
-    bool any = false;
-    for (uint32_t i = lane; i < n; i += 32) {
-      const K x = A[b0 + i];
-      if ((d == 0 || last < x) && (!any || x < lo)) {
-        lo = x;
-        any = true;
-      }
-    }
-    // lanes with nothing above `last` offer the largest key, which is only
-    // taken when no lane has a smaller one; the copies counted below decide
-    const K key = warp_min_k<K>(lo);
-    uint32_t c = 0;
-    for (uint32_t i = lane; i < n; i += 32) c += A[b0 + i] == key ? 1u : 0u;
+      for (int r = 0; r < 4; r++) v[r] = src.key((uint32_t)(r * 32 + lane) * n / 128);
+      warp_bitonic<K, 4>(v);
+      const uint32_t j = lane * 4 * G / 128;  // G <= 32: every (128 / G)th sample is a lane's first
 #pragma unroll
-    for (int m = 16; m > 0; m >>= 1) c += __shfl_xor_sync(0xffffffffu, c, m);
-    if (lane == d) {
-      mine = key;
-      mine_c = c;
-    }
-    last = key;
-    seen += c;
-    d++;
-  }
-  __syncwarp();
-  if (lane < d) {
-    A[b0 + lane] = mine;
-    C[b0 + lane] = (uint16_t)mine_c;
-  }
-  __syncwarp();
-  return d;
-}
-
-// The m keys in S.u.A are grouped by sub-bucket: sub-bucket jb + jj starts at
-// S.cnt[jb + jj] - s0 for jj in [0, nsl) (the last one ends at m).  Each
-// sub-bucket is reduced to its runs in place: by the thread that owns it
-// (insertion sort) when it holds at most CC_THREAD_MAX keys, else by a warp
-// (a register bitonic sort up to 128 keys; above that, rounds that take the
-// next smallest key while there are at most 32 distinct ones; else a bitonic
-// sort in shared memory).  A k-mer seen many times fills a sub-bucket with
-// copies of itself and of its sequencing-error variants, which share its
-// leading bases.  Each thread then packs the runs of the sub-buckets it owns
-// together from their first key on (keys in A, counts in C).  Sets
-// S.seg_src / S.seg_pos (exclusive scan of the run counts) and returns the
-// slice's distinct keys.
-template <typename K, int NT>
-GKC_DEV uint32_t slice_runs(CountSmem<K> &S, uint32_t m, uint32_t jb, uint32_t nsl, uint32_t s0) {
-  const int tid = threadIdx.x;
-  K *A = S.u.A;
-  uint16_t *dc = S.w.dc;
-  auto start_of = [&](uint32_t jj) -> uint32_t { return jj < nsl ? S.cnt[jb + jj] - s0 : m; };
-  const uint32_t j0 = (uint32_t)(((uint64_t)tid * nsl) / NT), j1 = (uint32_t)(((uint64_t)(tid + 1) * nsl) / NT);
-  if (tid == 0) S.nbig = 0;
-  __syncthreads();
-  for (uint32_t jj = j0; jj < j1; jj++) {
-    const uint32_t b0 = start_of(jj), b1 = start_of(jj + 1);
-    if (b1 - b0 <= CC_THREAD_MAX) {
-      insertion_sort<K>(A, b0, b1);
-      dc[jj] = (uint16_t)rle_in_place<K>(A, S.C, b0, b1);
-    } else {
-      S.big[atomicAdd(&S.nbig, 1u)] = (uint16_t)jj;  // fewer than CC_BIG_LIST (static_assert)
-    }
-  }
-  __syncthreads();
-  const uint32_t nbig = S.nbig, lane = threadIdx.x & 31u;
-  for (uint32_t t = threadIdx.x >> 5; t < nbig; t += NT / 32) {
-    const uint32_t jj = S.big[t];
-    const uint32_t b0 = start_of(jj), n = start_of(jj + 1) - b0;
-    uint32_t d;
-    if (n <= 32) {
-      d = warp_sort_rle<K, 1>(A, S.C, b0, n);
-    } else if (n <= 64) {
-      d = warp_sort_rle<K, 2>(A, S.C, b0, n);
-    } else if (n <= 128) {
-      d = warp_sort_rle<K, 4>(A, S.C, b0, n);
-    } else {
-      d = warp_select_rle<K>(A, S.C, b0, n);
-      if (d == 0) {
-        warp_sort<K>(A + b0, n);
-        if (lane == 0) d = rle_in_place<K>(A, S.C, b0, b0 + n);
-        d = __shfl_sync(0xffffffffu, d, 0);
+      for (int r = 0; r < 4; r += 2) {        // G = 64: every second one
+        const uint32_t e = lane * 4 + r, jj = r ? e * G / 128 : j;
+        if (jj > 0 && jj * 128 == e * G) {
+          const int t = __ffs((int)jj) - 1;
+          S.spl[(1u << (lg - 1 - t)) + (jj >> (t + 1))] = v[r];
+        }
       }
+      // 32 equal samples: one key fills about a quarter of the bucket
+      const K far = shfl_k<K>(v[0], min(lane + 8, 31u));
+      any = __any_sync(0xffffffffu, lane < 24 && v[0] == far && n > 4u * 32 * RMAX);
     }
-    if (lane == 0) dc[jj] = (uint16_t)d;
-    __syncwarp();
+    if (lane == 0) S.same = any;
   }
   __syncthreads();
-  const uint32_t s = start_of(j0);
-  uint32_t u = 0;
-  for (uint32_t jj = j0; jj < j1; jj++) {
-    const uint32_t b0 = start_of(jj), d = dc[jj];
-    if (b0 != s + u)
-      for (uint32_t i = 0; i < d; i++) {
-        A[s + u + i] = A[b0 + i];
-        S.C[s + u + i] = S.C[b0 + i];
-      }
-    u += d;
+  if (S.same) {
+    __syncthreads();
+    return SORT_REJECTED;
   }
-  uint32_t D;
-  const uint32_t pos = block_exclusive_scan<NT>(u, S.tmp, &D);
-  S.seg_pos[tid] = pos;
-  S.seg_src[tid] = s;
+  // groups counted, each key's group kept in C
+  if (lg > 0) {
+#pragma unroll 4
+    for (uint32_t i = tid; i < n; i += NT) {
+      const K x = src.key(i);
+      uint32_t node = 1;
+      for (int l = 0; l < lg; l++) node = 2 * node + (x < S.spl[node] ? 0u : 1u);
+      S.C[i] = (uint16_t)(node - G);
+      atomicAdd(&S.gcnt[node - G], 1u);
+    }
+  }
   __syncthreads();
-  return D;
-}
-
-// Writes the D runs of the slice (S.seg_* from slice_runs) to the staging
-// arrays at [ob, ob+D), coalesced: output i comes from the thread whose runs
-// cover it.
-template <typename K, int NT>
-GKC_DEV void write_runs(CountSmem<K> &S, const SortCountArgs &a, uint32_t D, uint64_t ob) {
-  K *out_keys = reinterpret_cast<K *>(a.stage_keys);
-  for (uint32_t i = threadIdx.x; i < D; i += NT) {
-    uint32_t lo = 0, hi = NT - 1;
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi + 1) >> 1;
-      if (S.seg_pos[mid] <= i) lo = mid; else hi = mid - 1;
+  uint16_t *goff = S.goff[w];
+  {
+    const uint32_t c0 = S.gcnt[2 * lane], c1 = S.gcnt[2 * lane + 1];
+    uint32_t tot;
+    const uint32_t o = warp_exclusive_scan(c0 + c1, &tot);
+    goff[2 * lane] = (uint16_t)o;
+    goff[2 * lane + 1] = (uint16_t)(o + c0);
+    if (lane == 31) goff[CS_GROUPS] = (uint16_t)tot;
+    if (w == 0) {
+      S.cur[2 * lane] = o;
+      S.cur[2 * lane + 1] = o + c0;
     }
-    const uint32_t src = S.seg_src[lo] + (i - S.seg_pos[lo]);
-    if (ob + i < a.stage_cap) {
-      out_keys[ob + i] = S.u.A[src];
-      a.stage_counts[ob + i] = S.C[src];
-    } else {
-      atomicOr(a.err, ERR_CAPACITY);
-    }
+    const bool large = __reduce_max_sync(0xffffffffu, max(c0, c1)) > 32u * RMAX;  // the same in every warp
+    __syncthreads();
+    if (large) return SORT_REJECTED;
   }
-}
-
-// One sub-bucket of n keys at tmp[0, n), too many for shared memory: key
-// ranges are aggregated in the hash table; a range whose distinct keys fill
-// more than 3/4 of it is halved and both halves retried (lower first).  Runs
-// are appended to the staging arrays at S.out_base + S.run.
-template <typename K, int NT>
-GKC_DEV void heavy_slice(CountSmem<K> &S, const SortCountArgs &a, const K *src, uint64_t n) {
-  constexpr int HN = HeavyTab<K>::N;
-  HeavyTab<K> &T = S.u.h;
-  K *out_keys = reinterpret_cast<K *>(a.stage_keys);
-  const int tid = threadIdx.x;
-  if (tid == 0) {
-    S.sp = 1;
-    S.w.stk.lo[0] = (K)0;
-    S.w.stk.hi[0] = ~(K)0;
+  if (lg > 0) {
+#pragma unroll 4
+    for (uint32_t i = tid; i < n; i += NT) S.A[atomicAdd(&S.cur[S.C[i]], 1u)] = src.key(i);
+  } else {
+    for (uint32_t i = tid; i < n; i += NT) S.A[i] = src.key(i);
   }
   __syncthreads();
   while (true) {
-    if (S.sp == 0) break;
-    const K lo = S.w.stk.lo[S.sp - 1], hi = S.w.stk.hi[S.sp - 1];
-    for (int s = tid; s < HN; s += NT) {
-      T.cnt[s] = 0;
-      T.state[s] = 0;
-    }
-    __syncthreads();
-    if (tid == 0) {
-      S.sp--;
-      S.flag = 0;
-      S.hfill = 0;
-    }
-    __syncthreads();
-    for (uint64_t i = tid; i < n; i += NT) {
-      const K x = src[i];
-      if (x < lo || x > hi) continue;
-      uint64_t hh = (uint64_t)x ^ (uint64_t)(x >> (4 * sizeof(K))) ^ (uint64_t)(x >> (8 * sizeof(K) - 8));
-      hh = (hh ^ (hh >> 29)) * 0xBF58476D1CE4E5B9ull;
-      uint32_t slot = (uint32_t)(hh >> 40) & (HN - 1);
-      for (uint32_t probes = 0;; probes++) {
-        if (probes >= (uint32_t)HN || *(volatile int *)&S.flag) {
-          S.flag = 1;
-          break;
-        }
-        uint32_t st = *(volatile uint32_t *)&T.state[slot];
-        if (st == 0) {
-          if (atomicCAS(&T.state[slot], 0u, 1u) == 0u) {
-            T.key[slot] = x;
-            __threadfence_block();
-            atomicExch(&T.state[slot], 2u);
-            atomicAdd(&T.cnt[slot], 1u);
-            if (atomicAdd(&S.hfill, 1u) + 1 > (uint32_t)(HN * 3 / 4)) S.flag = 1;
-            break;
-          }
-          st = 1;
-        }
-        if (st == 1) {  // another thread is writing this slot's key
-          uint32_t w = 0;
-          while ((st = *(volatile uint32_t *)&T.state[slot]) != 2u && ++w < (1u << 22)) {
-          }
-          if (st != 2u) {
-            atomicOr(a.err, ERR_SPIN_TIMEOUT);
-            S.flag = 1;
-            break;
-          }
-        }
-        if (*(volatile K *)&T.key[slot] == x) {
-          atomicAdd(&T.cnt[slot], 1u);
-          break;
-        }
-        slot = (slot + 1) & (HN - 1);
-      }
-    }
-    __syncthreads();
-    if (S.flag && lo < hi) {
-      if (tid == 0) {
-        const K mid = lo + ((hi - lo) >> 1);
-        if (S.sp + 2 <= CC_STACK) {
-          S.w.stk.lo[S.sp] = mid + 1;  // upper half below the lower half
-          S.w.stk.hi[S.sp] = hi;
-          S.w.stk.lo[S.sp + 1] = lo;
-          S.w.stk.hi[S.sp + 1] = mid;
-          S.sp += 2;
-        } else {
-          atomicOr(a.err, ERR_BOUNDS);
-        }
-      }
-      __syncthreads();
-      continue;
-    }
-    // the occupied slots to the front (through registers), sorted, written
-    constexpr int PT = HN / NT;
-    K mk[PT];
-    uint32_t mc[PT], mine = 0;
-#pragma unroll
-    for (int u = 0; u < PT; u++) {
-      const int s = u * NT + tid;
-      if (T.state[s] == 2u) {
-        mk[mine] = T.key[s];
-        mc[mine] = T.cnt[s];
-        mine++;
-      }
-    }
-    __syncthreads();
-    if (tid == 0) S.hfill = 0;
-    __syncthreads();
-    const uint32_t first = atomicAdd(&S.hfill, mine);
-#pragma unroll
-    for (int u = 0; u < PT; u++)
-      if ((uint32_t)u < mine) {
-        T.key[first + u] = mk[u];
-        T.cnt[first + u] = mc[u];
-      }
-    __syncthreads();
-    const uint32_t nd = S.hfill;
-    block_sort_pairs<K, NT>(T.key, T.cnt, nd);
-    const uint64_t ob = S.out_base + S.run;
-    for (uint32_t i = tid; i < nd; i += NT) {
-      if (ob + i < a.stage_cap) {
-        out_keys[ob + i] = T.key[i];
-        a.stage_counts[ob + i] = T.cnt[i];
-      } else {
-        atomicOr(a.err, ERR_CAPACITY);
-      }
-    }
-    __syncthreads();
-    if (tid == 0) S.run += nd;
-    __syncthreads();
-  }
-}
-
-// Sorts the 32 R keys (with counts) at Kb / Cb by the calling warp in
-// registers: lane l holds positions r 32 + l, a bitonic network (strides
-// below 32 across lanes by shuffles, larger ones across a lane's registers).
-template <int R, typename CT>
-GKC_DEV void warp_sort_run(uint64_t *Kb, CT *Cb) {
-  const uint32_t lane = threadIdx.x & 31u;
-  uint64_t v[R];
-  uint32_t c[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    v[r] = Kb[r * 32 + lane];
-    c[r] = Cb[r * 32 + lane];
-  }
-#pragma unroll
-  for (uint32_t size = 2; size <= 32u * R; size <<= 1) {
-#pragma unroll
-    for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-      if (stride >= 32) {
-        const int rs = (int)(stride / 32);
-#pragma unroll
-        for (int r = 0; r < R; r++)
-          if ((r & rs) == 0) {
-            const bool asc = ((r * 32 + lane) & size) == 0;
-            const uint64_t x = v[r], y = v[r + rs];
-            if (asc ? (y < x) : (x < y)) {
-              v[r] = y;
-              v[r + rs] = x;
-              const uint32_t t = c[r];
-              c[r] = c[r + rs];
-              c[r + rs] = t;
-            }
-          }
-      } else {
-#pragma unroll
-        for (int r = 0; r < R; r++) {
-          const bool asc = ((r * 32 + lane) & size) == 0;
-          const uint64_t y = __shfl_xor_sync(0xffffffffu, v[r], stride);
-          const uint32_t cy = __shfl_xor_sync(0xffffffffu, c[r], stride);
-          const bool keep_min = ((lane & stride) == 0) == asc;
-          if (keep_min ? (y < v[r]) : (v[r] < y)) {
-            v[r] = y;
-            c[r] = cy;
-          }
-        }
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < R; r++) {
-    Kb[r * 32 + lane] = v[r];
-    Cb[r * 32 + lane] = (CT)c[r];
-  }
-}
-
-// Merges the sorted runs of length L of (sk, sc) pairwise into (dk, dc): each
-// thread writes P / NT consecutive outputs (at least one), starting from a
-// merge-path search of its first one.
-template <int NT, typename CT>
-GKC_DEV void merge_round(const uint64_t *sk, const CT *sc, uint64_t *dk, CT *dc, uint32_t P, uint32_t L) {
-  const uint32_t per = P >= (uint32_t)NT ? P / NT : 1u;
-  const uint32_t o0 = threadIdx.x * per;
-  if (o0 < P) {
-    const uint32_t a0 = o0 & ~(2 * L - 1);
-    const uint64_t *A = sk + a0, *Bk = sk + a0 + L;
-    const uint32_t o = o0 - a0;
-    uint32_t lo = o > L ? o - L : 0u, hi = o < L ? o : L;
-    while (lo < hi) {  // i = outputs before o taken from A (ties from A first)
-      const uint32_t mid = (lo + hi) >> 1;
-      if (A[mid] <= Bk[o - mid - 1]) lo = mid + 1; else hi = mid;
-    }
-    uint32_t i = lo, j = o - lo;
-    for (uint32_t t = 0; t < per; t++) {
-      if (j >= L || (i < L && A[i] <= Bk[j])) {
-        dk[o0 + t] = A[i];
-        dc[o0 + t] = sc[a0 + i];
-        i++;
-      } else {
-        dk[o0 + t] = Bk[j];
-        dc[o0 + t] = sc[a0 + L + j];
-        j++;
-      }
-    }
+    uint32_t t = 0;
+    if (lane == 0) t = atomicAdd(&S.next, 1u);
+    t = __shfl_sync(0xffffffffu, t, 0);
+    if (t >= G) break;
+    const uint32_t b0 = goff[t], m = goff[t + 1] - b0;
+    uint32_t d;
+    if (m <= 64) d = warp_sort_runs<K, 2>(S.A, S.C, b0, m);
+    else if (m <= 128) d = warp_sort_runs<K, 4>(S.A, S.C, b0, m);
+    else if (RMAX <= 8 || m <= 256) d = warp_sort_runs<K, 8>(S.A, S.C, b0, m);
+    else d = warp_sort_runs<K, RMAX>(S.A, S.C, b0, m);
+    if (lane == 0) S.gd[t] = (uint16_t)d;
   }
   __syncthreads();
-}
-
-// Sorts P keys with counts (P a power of two in [32, 4096]) held in buffer 0
-// (k0, c0), using buffer 1 (k1, c1) as well: runs of P / W keys sorted by W
-// warps in registers, then merged pairwise.  Returns the buffer that holds
-// the result.
-template <int NT, typename CT>
-GKC_DEV int block_merge_sort(uint64_t *k0, CT *c0, uint64_t *k1, CT *c1, uint32_t P) {
-  const uint32_t W = min((uint32_t)NT / 32, P / 32), C = P / W, w = threadIdx.x >> 5;
-  if (w < W) {
-    switch (C / 32) {
-      case 1: warp_sort_run<1, CT>(k0 + w * C, c0 + w * C); break;
-      case 2: warp_sort_run<2, CT>(k0 + w * C, c0 + w * C); break;
-      case 4: warp_sort_run<4, CT>(k0 + w * C, c0 + w * C); break;
-      default: warp_sort_run<8, CT>(k0 + w * C, c0 + w * C); break;
+  const uint32_t d0 = 2 * lane < G ? S.gd[2 * lane] : 0u, d1 = 2 * lane + 1 < G ? S.gd[2 * lane + 1] : 0u;
+  uint32_t D;
+  const uint32_t o = warp_exclusive_scan(d0 + d1, &D);
+  K *out = reinterpret_cast<K *>(a.stage_keys);
+  const bool fits = out_at + n <= a.stage_cap;
+  if (!fits && tid == 0) atomicOr(a.err, ERR_CAPACITY);
+  for (uint32_t t = w; t < G; t += W) {
+    const uint32_t at = __shfl_sync(0xffffffffu, o, t >> 1) + (t & 1u ? __shfl_sync(0xffffffffu, d0, t >> 1) : 0u);
+    const uint32_t d = __shfl_sync(0xffffffffu, t & 1u ? d1 : d0, t >> 1);
+    const uint32_t b0 = goff[t], m = goff[t + 1] - b0;
+    for (uint32_t i = lane; i < d && fits; i += 32) {
+      const uint32_t e = i + 1 < d ? S.C[b0 + i + 1] : m;
+      const K x = S.A[b0 + i];
+      out[out_at + at + i] = x;
+      a.stage_counts[out_at + at + i] = src.count(x, e - S.C[b0 + i]);
     }
   }
-  __syncthreads();
-  int src = 0;
-  for (uint32_t L = C; L < P; L <<= 1) {
-    if (src == 0) merge_round<NT, CT>(k0, c0, k1, c1, P, L);
-    else merge_round<NT, CT>(k1, c1, k0, c0, P, L);
-    src ^= 1;
-  }
-  return src;
-}
-
-// ---- hash path (8-byte keys): a bucket's keys aggregated in a shared-memory
-// table first, so that only its distinct keys are sorted, by comparisons
-// (keys of a minimizer bin are far from uniform in their leading bases:
-// those holding the minimizer near their start share them, so digit splits
-// of a bucket can be very uneven).  The keys are read from global memory, so
-// a bucket of any size with few enough distinct keys takes this path.  The
-// table lives in the upper half of the key area (keys) and in the run-count
-// area (counts); the distinct keys go to the lower half of the key area,
-// their counts to the per-sub-bucket array, and are merge-sorted with the
-// table's two areas as the second buffer.  The slices of a bucket too large
-// for the table are counted the same way.
-constexpr uint32_t HT_SLOTS = 4096;
-constexpr uint32_t HT_MAX_DISTINCT = 3072;  // 3/4 full: beyond it the bucket takes the sub-bucket path
-constexpr uint64_t HT_MAX_KEYS = 65535;     // counts of the sorted pairs are 16-bit
-constexpr uint32_t HT_MAX_PROBE = 64;       // a longer probe chain also abandons the table
-constexpr uint64_t HT_EMPTY = ~0ull;        // never a canonical key: the reverse complement of all-T is all-A
-
-GKC_DEV uint32_t ht_slot(uint64_t x) { return (uint32_t)((x * 0x9E3779B97F4A7C15ull) >> 52); }
-
-template <int NT, typename K>
-GKC_DEV bool hash_count(CountSmem<K> &, const SortCountArgs &, const K *, uint64_t, uint64_t) {
-  return false;  // 16-byte keys: no 128-bit compare-and-swap in shared memory here
-}
-
-// Counts the n keys src[0, n) (read from global memory; n < 2^16, so counts
-// fit 16 bits) through the table and writes their sorted runs to the staging
-// arrays at `out_at`; their number is left in S.hfill.  Returns false, with
-// nothing written, when there are more than HT_MAX_DISTINCT distinct keys
-// (the caller then takes another path).  Uses the key area, the run-count
-// area and the per-sub-bucket array only (S.cnt is left as it is).  Not
-// inlined: its registers are then not added to the count kernel's.
-template <int NT>
-__device__ __noinline__ bool hash_count(CountSmem<uint64_t> &S, const SortCountArgs &a, const uint64_t *src,
-                                        uint64_t n, uint64_t out_at) {
-  static_assert(2 * HT_SLOTS <= (uint32_t)CountShape<uint64_t>::CAP, "table and sorted keys share the key area");
-  static_assert(sizeof(S.C) >= HT_SLOTS * 4, "table counts fit the run-count area");
-  static_assert(sizeof(S.w.dc) >= HT_SLOTS * 2, "sorted counts fit the per-sub-bucket array");
-  constexpr uint32_t SPT = HT_SLOTS / NT;
-  constexpr int U = 8;  // keys in flight per thread
-  if (n > HT_MAX_KEYS) return false;
-  volatile uint64_t *T = S.u.A + HT_SLOTS;
-  uint32_t *TC = reinterpret_cast<uint32_t *>(S.C);
-  uint64_t *B = S.u.A;
-  uint16_t *BC = S.w.dc;
-  const int tid = threadIdx.x;
-  for (uint32_t i = tid; i < HT_SLOTS; i += NT) {
-    T[i] = HT_EMPTY;
-    TC[i] = 0;
-  }
-  if (tid == 0) {
-    S.hfill = 0;
-    S.flag = 0;
-  }
-  __syncthreads();
-  for (uint64_t i0 = tid; i0 < n; i0 += (uint64_t)U * NT) {
-    if (*(volatile int *)&S.flag) break;
-    uint64_t xs[U];
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const uint64_t i = i0 + (uint64_t)u * NT;
-      xs[u] = i < n ? __ldg(reinterpret_cast<const unsigned long long *>(src) + i) : HT_EMPTY;
-    }
-#pragma unroll
-    for (int u = 0; u < U; u++) {
-      const uint64_t x = xs[u];
-      if (i0 + (uint64_t)u * NT >= n || *(volatile int *)&S.flag) break;
-      uint32_t h = ht_slot(x);
-      for (uint32_t probe = 0;; probe++) {
-        if (probe == HT_MAX_PROBE) {  // a long chain: the table is too full, give up
-          S.flag = 1;
-          break;
-        }
-        uint64_t cur = T[h];
-        if (cur == HT_EMPTY) {
-          cur = atomicCAS((unsigned long long *)(S.u.A + HT_SLOTS + h), (unsigned long long)HT_EMPTY,
-                          (unsigned long long)x);
-          if (cur == HT_EMPTY) {
-            atomicAdd(&TC[h], 1u);
-            if (atomicAdd(&S.hfill, 1u) + 1 > HT_MAX_DISTINCT) S.flag = 1;
-            break;
-          }
-        }
-        if (cur == x) {
-          atomicAdd(&TC[h], 1u);
-          break;
-        }
-        h = (h + 1) & (HT_SLOTS - 1);
-      }
-    }
-  }
-  __syncthreads();
-  if (S.flag) return false;
-  const uint32_t D = S.hfill;
-  // the distinct keys, in slot order, to B[0, D), their counts to BC; the
-  // rest of the power of two above D holds the largest key
-  uint32_t own = 0;
-#pragma unroll
-  for (int q = 0; q < (int)SPT; q++) own += T[q * NT + tid] != HT_EMPTY ? 1u : 0u;
-  uint32_t tot;
-  uint32_t pos = block_exclusive_scan<NT>(own, S.tmp, &tot);
-#pragma unroll
-  for (int q = 0; q < (int)SPT; q++) {
-    const uint32_t slot = q * NT + tid;
-    const uint64_t x = T[slot];
-    if (x != HT_EMPTY) {
-      B[pos] = x;
-      BC[pos] = (uint16_t)TC[slot];  // <= n < 2^16
-      pos++;
-    }
-  }
-  uint32_t P = 32;
-  while (P < D) P <<= 1;
-  for (uint32_t i = D + tid; i < P; i += NT) {
-    B[i] = HT_EMPTY;
-    BC[i] = 0;
-  }
-  __syncthreads();
-  // the table is free now: its two areas are the sort's second buffer
-  uint64_t *B1 = S.u.A + HT_SLOTS;
-  uint16_t *BC1 = S.C;
-  const int res = block_merge_sort<NT, uint16_t>(B, BC, B1, BC1, P);
-  const uint64_t *RK = res ? B1 : B;
-  const uint16_t *RC = res ? BC1 : BC;
-  uint64_t *out = reinterpret_cast<uint64_t *>(a.stage_keys);
-  for (uint32_t i = tid; i < D; i += NT) {
-    if (out_at + i < a.stage_cap) {
-      out[out_at + i] = RK[i];
-      a.stage_counts[out_at + i] = RC[i];
-    } else {
-      atomicOr(a.err, ERR_CAPACITY);
-    }
-  }
-  __syncthreads();
-  return true;
-}
-
-// Counts the m <= CAP keys src[0, m) in shared memory and stages their runs
-// at out_at; returns their number.  The keys are counting-sorted by the
-// sub-bucket digit that follows the common prefix of their smallest and
-// largest key, then each sub-bucket is reduced to runs (slice_runs).  Not
-// inlined: it is called for whole buckets and for the slices of large ones.
-template <typename K, int NT, int KPT>
-__device__ __noinline__ uint32_t smem_count(CountSmem<K> &S, const SortCountArgs &a, const K *src, uint32_t m,
-                                            uint64_t out_at) {
-  const int tid = threadIdx.x;
-  K xs[KPT];
-  K lo = ~(K)0, hi = 0;
-#pragma unroll
-  for (int u = 0; u < KPT; u++) {
-    const uint32_t i = u * NT + tid;
-    if (i < m) {
-      xs[u] = src[i];
-      lo = xs[u] < lo ? xs[u] : lo;
-      hi = xs[u] > hi ? xs[u] : hi;
-    }
-  }
-  block_minmax<K, NT>(S, lo, hi);
-  int cp, sb;
-  prefix_split<K>(lo, hi, m, CC_SB_MAX, &cp, &sb);
-  const uint32_t nsub = 1u << sb;
-  for (uint32_t jj = tid; jj < nsub; jj += NT) S.cnt[jj] = 0;
-  __syncthreads();
-  uint32_t rk[(KPT + 1) / 2];
-#pragma unroll
-  for (int u = 0; u < (KPT + 1) / 2; u++) rk[u] = 0;
-#pragma unroll
-  for (int u = 0; u < KPT; u++) {
-    const uint32_t i = u * NT + tid;
-    if (i < m) rk[u / 2] |= atomicAdd(&S.cnt[prefix_digit<K>(xs[u], cp, sb)], 1u) << (16 * (u & 1));
-  }
-  __syncthreads();
-  scan_sub<K, NT>(S, nsub);
-#pragma unroll
-  for (int u = 0; u < KPT; u++) {
-    const uint32_t i = u * NT + tid;
-    if (i < m) S.u.A[S.cnt[prefix_digit<K>(xs[u], cp, sb)] + ((rk[u / 2] >> (16 * (u & 1))) & 0xFFFFu)] = xs[u];
-  }
-  __syncthreads();
-  const uint32_t D = slice_runs<K, NT>(S, m, 0, nsub, 0);
-  write_runs<K, NT>(S, a, D, out_at);
   __syncthreads();
   return D;
 }
 
+// A bucket of n <= 65535 8-byte keys, its distinct keys (their number is
+// returned; SORT_REJECTED when there are more than the table takes or sorted
+// groups are too large) aggregated in the table first and then sorted.
+template <int NT>
+__device__ __noinline__ uint32_t dedup_count(SortSmem<uint64_t> &S, const SortCountArgs &a, const uint64_t *src,
+                                             uint32_t n, uint64_t out_at) {
+  DedupArea &H = S.u.d.t;
+  constexpr int SPT = DedupArea::SLOTS / NT;
+  static_assert(DedupArea::SLOTS % NT == 0 && SPT <= 32, "one mask per thread");
+  if (!table_insert64<NT, DedupArea::CAP, DedupArea::SLOTS>(S, H.T, H.TC, src, n, DedupArea::SLOTS)) {
+    __syncthreads();
+    return SORT_REJECTED;
+  }
+  uint32_t mask = 0;
+#pragma unroll
+  for (int q = 0; q < SPT; q++)
+    if (H.T[q * NT + threadIdx.x] != HT_EMPTY) mask |= 1u << q;
+  uint32_t D;
+  uint32_t pos = block_exclusive_scan<NT>(__popc(mask), S.tmp, &D);
+  while (mask) {
+    const int q = __ffs(mask) - 1;
+    mask &= mask - 1;
+    H.L[pos++] = (uint16_t)(q * NT + threadIdx.x);
+  }
+  __syncthreads();
+  return sort_count<uint64_t, NT>(S.u.d.s, a, TableKeys{H}, D, out_at);
+}
+template <int NT>
+GKC_DEV uint32_t dedup_count(SortSmem<u128> &, const SortCountArgs &, const u128 *, uint32_t, uint64_t) {
+  return SORT_REJECTED;
+}
+
+template <typename K, int NT>
+__device__ __noinline__ uint32_t slice_count(SortArea<K, NT, CountShape<K>::CAP> &S, const SortCountArgs &a,
+                                             const K *src, uint32_t n, uint64_t out_at) {
+  return sort_count<K, NT>(S, a, GlobalKeys<K>{src}, n, out_at);
+}
+
+// Buckets of at most CAP keys, persistent, taken by ticket.  Those that
+// sort_count rejects join the list of large ones (k_bucket_count).  256
+// threads and 45 KB, so that five CTAs (four for 16-byte keys) on an SM hide
+// each other's barriers.  Count stage (this kernel and k_bucket_count) on a
+// B200, against counting each bucket in a 4096-slot hash table with a merge
+// sort, or by insertion and warp sorts of 4096 fixed digits: 720 M 31-mers at
+// 30x 9.7 ms (14.7), 134.7 M mostly distinct 21-mers 3.4 ms (10.6), 150.9 M
+// 25-mers of compressed long reads 4.5 ms (14.8), 112.8 M 63-mers 3.5 ms (9.9).
 template <typename K>
-__global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_count(SortCountArgs a) {
-  constexpr int NT = CountShape<K>::NT, CAP = CountShape<K>::CAP, KPT = CAP / NT;
+__global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket_sort(SortCountArgs a) {
+  constexpr int NT = SortShape<K>::NT;
   extern __shared__ __align__(16) uint8_t smem_raw[];
-  CountSmem<K> &S = *reinterpret_cast<CountSmem<K> *>(smem_raw);
+  SortSmem<K> &S = *reinterpret_cast<SortSmem<K> *>(smem_raw);
   const K *keys = reinterpret_cast<const K *>(a.keys);
-  K *tmp = reinterpret_cast<K *>(a.scratch);
   const int tid = threadIdx.x;
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   const uint64_t n_buckets = a.bucket_base[a.nbins];
-  int hash_skip = 0;                // the same in every thread of the block
-  int slice_skip = 0;               // the same, for the slices of large buckets
-  uint64_t t_next = 0, t_end = 0;   // thread 0: the rest of its batch of tickets
-  bool big_phase = true;            // thread 0: the large buckets first, so none is left for the end
+  // several buckets per ticket only where every CTA gets many: with few, a
+  // batch would leave CTAs without any
+  const uint32_t batch = n_buckets >= 16ull * CC_TICKETS * gridDim.x ? CC_TICKETS : 1;
+  uint32_t bi = 0, bm = 0;          // thread 0: next and end of its batch of buckets
+  uint32_t repeats = 0;             // the same in every thread of the block
   while (true) {
     if (tid == 0) {
-      uint64_t gg = n_buckets;
-      if (big_phase) {
-        const unsigned long long bi = atomicAdd(a.big_ticket, 1ull);
-        if (bi < *a.big_count) gg = a.big_list[bi];
-        else big_phase = false;
-      }
-      if (!big_phase) {
-        while (true) {
-          if (t_next == t_end) {
-            t_next = atomicAdd(a.ticket, (unsigned long long)CC_TICKETS);
-            t_end = t_next + CC_TICKETS;
+      while (bi == bm) {  // a new batch, without the large ones
+        const uint64_t t0 = atomicAdd(a.ticket, (unsigned long long)batch);
+        bi = bm = 0;
+        if (t0 >= n_buckets) {
+          S.bg[0] = n_buckets;
+          S.bn[0] = 0;
+          S.bstart[0] = 0;
+          bm = 1;
+          break;
+        }
+        uint64_t sz[CC_TICKETS], st[CC_TICKETS];
+#pragma unroll
+        for (uint32_t j = 0; j < CC_TICKETS; j++) {
+          const bool in = j < batch && t0 + j < n_buckets;
+          sz[j] = in ? a.bucket_size[t0 + j] : ~0ull;
+          st[j] = in ? a.bucket_start[t0 + j] : 0;
+        }
+#pragma unroll
+        for (uint32_t j = 0; j < CC_TICKETS; j++)
+          if (sz[j] < a.big_min) {
+            S.bg[bm] = t0 + j;
+            S.bstart[bm] = st[j];
+            S.bn[bm] = (uint32_t)sz[j];
+            bm++;
           }
-          gg = t_next++;
-          if (gg >= n_buckets || a.bucket_size[gg] < a.big_min) break;  // a large one: taken from the list
-        }
       }
-      S.g = gg;
-      if (gg < n_buckets) {
-        S.b = a.bucket_bin[gg];
-        S.start = a.bucket_start[gg];
-        S.n = a.bucket_size[gg];
-      }
-      // the next bucket of the batch, if it is a regular one
-      S.pf_n = 0;
-      if (!big_phase && t_next < t_end && t_next < n_buckets) {
-        const uint64_t nn = a.bucket_size[t_next];
-        if (nn < a.big_min) {
-          S.pf_start = a.bucket_start[t_next];
-          S.pf_n = nn;
-        }
-      }
+      S.g = S.bg[bi];
+      S.start = S.bstart[bi];
+      S.n = S.bn[bi];
+      bi++;
+      S.pf_n = bi < bm ? S.bn[bi] : 0;
+      S.pf_start = bi < bm ? S.bstart[bi] : 0;
     }
     __syncthreads();
-    const uint64_t g = S.g;
+    const uint64_t g = S.g, start = S.start;
+    const uint32_t n = S.n;
     if (g >= n_buckets) break;
-    const uint64_t start = S.start, n = S.n;
     {
       constexpr int KPL = 128 / (int)sizeof(K);
       const uint64_t ps = S.pf_start, pe = ps + S.pf_n;
       for (uint64_t i = ps + (uint64_t)tid * KPL; i < pe; i += (uint64_t)NT * KPL) prefetch_l2(keys + i);
     }
-    // distinct keys through the table first, unless the last bucket that
-    // tried it had too many (then skip it for a few buckets)
-    if (n <= HT_MAX_KEYS) {
+    // Which way is faster depends on how often keys repeat, which changes
+    // little from bucket to bucket: the last bucket's share decides.  8-byte
+    // keys: the table first where two keys in three or more are repeats.
+    // 16-byte keys have no table here: the next 15 such buckets go to the
+    // list, then one is sorted again.
+    uint32_t D = SORT_REJECTED;
+    if (sizeof(K) == 8 && repeats) D = dedup_count<NT>(S, a, keys + start, n, start);
+    if (D == SORT_REJECTED && (sizeof(K) == 8 || repeats == 0))
+      D = sort_count<K, NT>(S.u.s, a, GlobalKeys<K>{keys + start}, n, start);
+    if (D != SORT_REJECTED) repeats = 3 * D <= n ? 15 : 0;
+    else if (sizeof(K) == 8) repeats = 0;
+    else if (repeats) repeats--;
+    if (tid == 0) {  // the counting's last barrier protects S.g too
+      if (D != SORT_REJECTED) a.bucket_d[g] = D;
+      else a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)g;
+    }
+    if (sizeof(K) == 16) __syncthreads();  // S.g is read before the next bucket, also where nothing was sorted
+  }
+}
+
+// Opens the keys [b, e) of an oversized bucket (`from`: its keys, `to`: the
+// same range of the other buffer): sorted into `to` by the up to 12 bits after
+// their common prefix, so that at least the first differing bit is among
+// them.  Returns false when all keys are equal (*key), nothing moved then.
+template <typename K, int NT>
+__device__ __noinline__ bool open_level(CountSmem<K> &S, const K *from, K *to, uint64_t b, uint64_t e, int *cp, int *sb,
+                                        K *key) {
+  constexpr int U = sizeof(K) == 8 ? 8 : 4;  // keys in flight per thread
+  const int tid = threadIdx.x;
+  uint32_t *sub = S.u.sub;
+  K lo = ~(K)0, hi = 0;
+#pragma unroll U
+  for (uint64_t i = b + tid; i < e; i += NT) {
+    const K x = load_key(from + i);
+    lo = x < lo ? x : lo;
+    hi = x > hi ? x : hi;
+  }
+  block_minmax<K, NT>(S, lo, hi);
+  *key = lo;
+  if (lo == hi) return false;
+  prefix_split<K>(lo, hi, e - b, CC_SB_MAX, cp, sb);
+  const uint32_t nsub = 1u << *sb;
+  for (uint32_t jj = tid; jj < nsub; jj += NT) sub[jj] = 0;
+  __syncthreads();
+#pragma unroll U
+  for (uint64_t i = b + tid; i < e; i += NT) atomicAdd(&sub[prefix_digit<K>(load_key(from + i), *cp, *sb)], 1u);
+  __syncthreads();
+  scan_sub<NT>(sub, S.tmp, nsub);
+#pragma unroll U
+  for (uint64_t i = b + tid; i < e; i += NT) {
+    const K x = load_key(from + i);
+    to[b + atomicAdd(&sub[prefix_digit<K>(x, *cp, *sb)], 1u)] = x;
+  }
+  __syncthreads();
+  return true;
+}
+
+// The listed buckets: larger than CAP, or rejected by k_bucket_sort.
+template <typename K>
+__global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_count(SortCountArgs a) {
+  constexpr int NT = CountShape<K>::NT, CAP = CountShape<K>::CAP;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  CountSmem<K> &S = *reinterpret_cast<CountSmem<K> *>(smem_raw);
+  K *keys = reinterpret_cast<K *>(a.keys);
+  const int tid = threadIdx.x;
+  if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
+  const uint64_t n_big = *a.big_count;
+  int hash_skip = 0;                // the same in every thread of the block
+  while (true) {
+    if (tid == 0) {
+      const uint64_t t = atomicAdd(a.big_ticket, 1ull);
+      S.g = t < n_big ? a.big_list[t] : ~0ull;
+      if (t < n_big) {
+        S.start = a.bucket_start[S.g];
+        S.n = a.bucket_size[S.g];
+      }
+    }
+    __syncthreads();
+    const uint64_t g = S.g;
+    if (g == ~0ull) break;
+    const uint64_t start = S.start, n = S.n;
+    // the whole bucket through the table: always possible up to CAP keys,
+    // else tried unless the last larger one had too many distinct keys
+    bool done = false;
+    if (n <= (uint64_t)CAP) {
+      done = hash_count<K, NT>(S, a, keys + start, n, start);
+    } else if (sizeof(K) == 8 && n <= HT_MAX_KEYS) {
       if (hash_skip == 0) {
-        if (hash_count<NT>(S, a, keys + start, n, start)) {
-          if (tid == 0) a.bucket_d[g] = S.hfill;
-          __syncthreads();
-          continue;
-        }
-        hash_skip = 8;
+        done = hash_count<K, NT>(S, a, keys + start, n, start);
+        if (!done) hash_skip = 8;
       } else {
         hash_skip--;
       }
     }
-    if (n <= (uint64_t)CAP) {
-      // ---- the whole bucket in shared memory; the runs go to the staging
-      // arrays at the bucket's own key range (its keys are all on chip by
-      // then), and a later pass moves them to their final place
-      const uint32_t D = smem_count<K, NT, KPT>(S, a, keys + start, (uint32_t)n, start);
-      if (tid == 0) a.bucket_d[g] = D;
+    if (done) {
+      if (tid == 0) a.bucket_d[g] = S.hfill;
+      __syncthreads();
       continue;
     }
 
-    // ---- oversized bucket: placed by sub-bucket in the scratch area, then
-    // counted in slices of at most CAP keys in key order
-    K lo = ~(K)0, hi = 0;
-    for (uint64_t i = tid; i < n; i += NT) {
-      const K x = keys[start + i];
-      lo = x < lo ? x : lo;
-      hi = x > hi ? x : hi;
-    }
-    block_minmax<K, NT>(S, lo, hi);
-    int cp, sb;
-    prefix_split<K>(lo, hi, n, CC_SB_MAX, &cp, &sb);
-    const uint32_t nsub = 1u << sb;
-    for (uint32_t jj = tid; jj < nsub; jj += NT) S.cnt[jj] = 0;
-    __syncthreads();
-    // the bucket's own key range of the scratch array (the result's key
-    // array, written only after this kernel)
-    K *place = tmp + start;
-    for (uint64_t i = tid; i < n; i += NT) atomicAdd(&S.cnt[prefix_digit<K>(keys[start + i], cp, sb)], 1u);
-    __syncthreads();
-    scan_sub<K, NT>(S, nsub);
-    static_assert(sizeof(S.C) / 4 >= CC_NSUB_MAX, "cursors fit in C");
-    uint32_t *cur = reinterpret_cast<uint32_t *>(S.C);
-    for (uint32_t jj = tid; jj < nsub; jj += NT) cur[jj] = S.cnt[jj];
-    __syncthreads();
-    for (uint64_t i = tid; i < n; i += NT) {
-      const K x = keys[start + i];
-      place[atomicAdd(&cur[prefix_digit<K>(x, cp, sb)], 1u)] = x;
-    }
-    // the sub-bucket starts go to this CTA's global area: the slices are
-    // counted with the shared-memory counters
-    uint32_t *gst = a.slice_starts + (uint64_t)blockIdx.x * (CC_NSUB_MAX + 1);
-    for (uint32_t jj = tid; jj < nsub; jj += NT) gst[jj] = S.cnt[jj];
-    __threadfence_block();
-    __syncthreads();
-    if (tid == 0) {
-      S.out_base = start;  // staged at the bucket's own key range (all its keys are in the scratch area)
-      S.run = 0;
-    }
-    __syncthreads();
-    uint32_t jlo = 0;
-    while (jlo < nsub) {
-      // next slice: sub-buckets [jlo, jhi), at most CAP keys, or one heavy sub-bucket
-      const uint32_t s0 = gst[jlo];
-      uint32_t lo = jlo + 1, hi = nsub;
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        const uint64_t e = mid < nsub ? gst[mid] : n;
-        if (e - s0 <= (uint64_t)CAP) lo = mid; else hi = mid - 1;
-      }
-      const uint32_t jhi = lo;
-      const uint64_t se = jhi < nsub ? gst[jhi] : n;
-      const uint64_t ns = se - s0;
-      if (ns <= (uint64_t)CAP) {
-        uint32_t D;
-        bool hashed = false;
-        if (slice_skip == 0) {
-          hashed = hash_count<NT>(S, a, place + s0, ns, S.out_base + S.run);
-          if (!hashed) slice_skip = 8;
-        } else {
-          slice_skip--;
+    // ---- oversized bucket: sorted by digit into the other buffer, then
+    // counted in slices of at most CAP keys in key order; a digit of more
+    // keys is opened in turn, back into the first buffer.  Buffer 0 is the
+    // bucket's own key range, buffer 1 the same range of the scratch array
+    // (the result's key array, written only after this kernel).  The runs are
+    // staged from the start of the key range on and never pass the keys
+    // already counted.
+    K *const buf[2] = {keys + start, reinterpret_cast<K *>(a.scratch) + start};
+    uint64_t pos = 0, end = n, run = 0;  // [pos, end): what is opened next; the same in every thread
+    int from = 0, level = 0;
+    while (true) {
+      int cp, sb;
+      K key;
+      if (open_level<K, NT>(S, buf[from], buf[from ^ 1], pos, end, &cp, &sb, &key)) {
+        if (level == CC_LEVELS) {  // not possible: every level fixes a bit of the key
+          if (tid == 0) atomicOr(a.err, ERR_BOUNDS);
+          break;
         }
-        if (hashed) D = S.hfill;
-        else D = smem_count<K, NT, KPT>(S, a, place + s0, (uint32_t)ns, S.out_base + S.run);
-        __syncthreads();
-        if (tid == 0) S.run += D;
-        __syncthreads();
-      } else if (hash_count<NT>(S, a, place + s0, ns, S.out_base + S.run)) {
-        // one sub-bucket larger than a slice with few distinct keys
-        if (tid == 0) S.run += S.hfill;
-        __syncthreads();
-      } else {
-        heavy_slice<K, NT>(S, a, place + s0, ns);
+        if (tid == 0) {
+          S.lend[level] = end;
+          S.lcp[level] = (uint8_t)cp;
+          S.lsb[level] = (uint8_t)sb;
+          S.lbuf[level] = (uint8_t)(from ^ 1);
+        }
+        level++;
+      } else {  // one key
+        if (tid == 0) {
+          if (start + run < a.stage_cap) {
+            reinterpret_cast<K *>(a.stage_keys)[start + run] = key;
+            a.stage_counts[start + run] = (uint32_t)(end - pos);
+          } else {
+            atomicOr(a.err, ERR_CAPACITY);
+          }
+        }
+        run++;
+        pos = end;
       }
-      jlo = jhi;
+      __syncthreads();
+      // slices of the innermost open level, until one has to be opened
+      bool open = false;
+      while (level > 0 && !open) {
+        const uint64_t lend = S.lend[level - 1];
+        if (pos == lend) {
+          level--;
+          continue;
+        }
+        const int lcp = S.lcp[level - 1], lsb = S.lsb[level - 1];
+        from = S.lbuf[level - 1];
+        const K *src = buf[from];
+        end = lend;
+        if (lend - pos > (uint64_t)CAP) {
+          // the digit of the first key that does not fit ends the slice
+          const uint32_t d = prefix_digit<K>(load_key(src + pos + CAP), lcp, lsb);
+          uint64_t l = pos, h = pos + CAP;  // first key of digit d
+          while (l < h) {
+            const uint64_t mid = (l + h) >> 1;
+            if (prefix_digit<K>(load_key(src + mid), lcp, lsb) < d) l = mid + 1; else h = mid;
+          }
+          end = l;
+          if (l == pos) {  // digit d alone is larger than a slice
+            l = pos + CAP + 1;
+            h = lend;
+            while (l < h) {
+              const uint64_t mid = (l + h) >> 1;
+              if (prefix_digit<K>(load_key(src + mid), lcp, lsb) <= d) l = mid + 1; else h = mid;
+            }
+            end = l;
+            open = true;
+            break;
+          }
+        }
+        const uint32_t ns = (uint32_t)(end - pos);
+        uint32_t D = slice_count<K, NT>(S.u.s, a, src + pos, ns, start + run);
+        if (D == SORT_REJECTED) {
+          hash_count<K, NT>(S, a, src + pos, ns, start + run);  // at most CAP keys: never too many
+          D = S.hfill;
+          __syncthreads();
+        }
+        run += D;
+        pos = end;
+      }
+      if (!open) break;
+      __syncthreads();  // the level's parameters are read before a new one is written
     }
-    if (tid == 0) a.bucket_d[g] = S.run;
+    if (tid == 0) a.bucket_d[g] = run;
     __syncthreads();
   }
 }
@@ -1572,6 +1618,8 @@ template __global__ void k_bucket_hist<uint64_t>(ExpandArgs);
 template __global__ void k_bucket_hist<u128>(ExpandArgs);
 template __global__ void k_bucket_scatter<uint64_t>(ExpandArgs);
 template __global__ void k_bucket_scatter<u128>(ExpandArgs);
+template __global__ void k_bucket_sort<uint64_t>(SortCountArgs);
+template __global__ void k_bucket_sort<u128>(SortCountArgs);
 template __global__ void k_bucket_count<uint64_t>(SortCountArgs);
 template __global__ void k_bucket_count<u128>(SortCountArgs);
 

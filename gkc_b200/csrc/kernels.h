@@ -54,18 +54,19 @@ struct CountPlan {
   uint32_t nbins;
   const uint64_t *bin_start;   // superkmers per bin (exclusive prefix, nbins+1)
   const uint64_t *bin_kstart;  // k-mers per bin (exclusive prefix, nbins+1)
-  uint32_t coarse_target;      // desired largest mean keys per coarse bucket
-  uint32_t max_bits;           // coarse bucket bits cap (<= kCoarseMaxBits)
+  uint32_t bucket_keys;        // keys of a bucket
+  uint32_t max_bits;           // digit bits cap (<= kCoarseMaxBits)
   uint64_t chunk_kmers;        // k-mers per expansion chunk
   int k;
   const uint32_t *err;         // nothing is planned after an upstream overflow
   // outputs
-  uint32_t *bin_bits;          // coarse bucket bits per bin
-  uint64_t *bucket_base;       // first coarse bucket of each bin (nbins+1)
+  uint32_t *bin_bits;          // digit bits per bin
+  uint64_t *bucket_base;       // first bucket of each bin (nbins+1)
   uint64_t *chunk_base;        // first chunk of each bin (nbins+1)
   uint64_t *hist_base;         // first (digit, chunk) entry of each bin (nbins+1)
 };
 __global__ void k_count_plan(CountPlan pl);
+constexpr int kCountPlanThreads = 1024;
 
 struct ExpandArgs {
   const uint64_t *desc;        // bin-ordered superkmer descriptors
@@ -81,7 +82,11 @@ struct ExpandArgs {
   uint64_t chunk_kmers;
   int k;
   uint64_t *chunk_s0;          // first superkmer of each chunk
-  uint32_t *hist;              // (bin, chunk, digit) counts, then write offsets in the bin
+  uint32_t *hist;              // (bin, chunk, digit) counts, then write offsets in the bin per bucket
+  uint32_t *digit_total;       // per (bin, digit), 1 << max_bits entries per bin
+  uint16_t *lut;               // bucket (of its bin) of every digit, 1 << max_bits entries per bin
+  uint32_t max_bits;
+  uint32_t bucket_keys;
   void *keys;                  // scatter output (uint64 or u128)
   void *flat;                  // the keys in k-mer order (written by the histogram, read by the scatter)
   uint64_t keys_cap;          // of keys and flat
@@ -92,7 +97,9 @@ struct ExpandArgs {
 };
 __global__ void k_chunk_first(ExpandArgs a);
 template <typename K> __global__ void k_bucket_hist(ExpandArgs a);
-__global__ void k_bucket_scan(ExpandArgs a, uint64_t *bucket_start, uint64_t *bucket_size, uint32_t *bucket_bin);
+__global__ void k_bucket_scan(ExpandArgs a, uint64_t *bucket_start, uint64_t *bucket_size);
+__global__ void k_bucket_offsets(ExpandArgs a, const uint64_t *bucket_start);
+constexpr int kBucketOffsetThreads = 128;
 template <typename K> __global__ void k_bucket_scatter(ExpandArgs a);
 constexpr int kBucketScanThreads = 1024;
 constexpr int kBucketHistThreads = 256;
@@ -103,29 +110,28 @@ __global__ void k_skm_nk(const uint64_t *desc, const unsigned long long *n_skm_d
 
 struct SortCountArgs {
   uint32_t nbins;
-  int k;
   const uint64_t *bucket_base;    // buckets per bin (prefix, nbins + 1)
-  const uint32_t *bin_bits;
   const uint64_t *bucket_start;   // first key of each bucket
   const uint64_t *bucket_size;
-  const uint32_t *bucket_bin;     // bin of each bucket
-  const void *keys;               // bucketed keys
-  void *scratch;                  // oversized buckets, placed by sub-bucket at their own key range
-  uint32_t *slice_starts;         // per CTA: sub-bucket starts of its current large bucket (4097 each)
+  void *keys;                     // bucketed keys
+  void *scratch;                  // second buffer of oversized buckets, at their own key range
   void *stage_keys;               // runs of bucket g at [bucket_start[g], + its distinct count)
   uint32_t *stage_counts;
   uint64_t stage_cap;
   unsigned long long *bucket_d;   // distinct keys of each bucket
   unsigned long long *ticket;     // zeroed
-  const uint32_t *big_list;       // buckets of at least big_min keys, taken before the others
-  const unsigned long long *big_count;
+  uint32_t *big_list;             // buckets of at least big_min keys (from the scan), then rejected ones
+  unsigned long long *big_count;
   unsigned long long *big_ticket;  // zeroed
   uint64_t big_min;
   uint32_t *err;
 };
+template <typename K> __global__ void k_bucket_sort(SortCountArgs a);
+template <typename K> size_t bucket_sort_smem_bytes();
+constexpr int kBucketSortThreads = 256;
 template <typename K> __global__ void k_bucket_count(SortCountArgs a);
 template <typename K> size_t bucket_count_smem_bytes();
-template <typename K> uint64_t bucket_count_cap();  // keys of the largest bucket counted in shared memory
+template <typename K> uint64_t bucket_count_cap();  // largest bucket of k_bucket_sort
 template <typename K>
 __global__ void k_compact_runs(const K *stage_keys, const uint32_t *stage_counts, const uint64_t *bucket_start,
                                const unsigned long long *bucket_d, const uint64_t *bucket_out,
@@ -133,6 +139,12 @@ __global__ void k_compact_runs(const K *stage_keys, const uint32_t *stage_counts
                                uint64_t *bin_out, const uint32_t *err);
 constexpr int kBucketCountThreads = 512;
 constexpr uint32_t kCoarseTarget = 8192;
+// Keys of a bucket for a tuned target (an upper bound of the mean): at the
+// default target 2816 8-byte or 1536 16-byte keys, so that with the digit
+// that passes the span a bucket still fits the 4096 (3072) of k_bucket_sort.
+template <typename K> constexpr uint32_t bucket_target(uint32_t target) {
+  return sizeof(K) == 8 ? target / 16 * 11 / 2 : target / 16 * 3;
+}
 constexpr uint32_t kCoarseMaxBits = 12;
 constexpr uint64_t kChunkKmers = 65536;
 
