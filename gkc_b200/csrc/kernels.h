@@ -25,8 +25,8 @@ struct PartArgs {
   uint32_t *err;
 };
 
-constexpr int kPartThreads = 512;
-constexpr int kPartTile = 4096;
+constexpr int kPartThreads = 256;
+constexpr int kPartTile = 3584;
 size_t partition_smem_bytes(int nbins_smem);
 __global__ void k_partition(PartArgs a);
 constexpr int kBinChunk = 8192;          // superkmers per placement chunk

@@ -12,437 +12,242 @@
 // Reads shorter than k produce nothing.
 //
 // The fused kernel is persistent and tiled over the concatenated read bytes:
-// each tile of PT_T window positions (+ halo) is loaded with 16-byte vector
-// loads into shared memory, minimizers are computed with a sliding-window
-// minimum over per-position filtered p-mer values, superkmer breaks are
-// compacted with a block scan, and the packed bytes are written as coalesced
-// 32-bit words.
+// the minimizers of a tile's windows stay in registers (tile.cuh), breaks are
+// bitmaps of 32 windows a word, superkmers are compacted from them, and the
+// packed bytes are written as coalesced 16-byte words.
 #include "common.cuh"
 #include "kernels.h"
 #include "minimizer.cuh"
+#include "tile.cuh"
 
 namespace gkc {
 
-constexpr int PT_NT = 512;
-constexpr int PT_T = 4096;                       // core windows per tile
-constexpr int PT_H = 512;                        // halo windows to find superkmer ends
-constexpr int PT_PRE = 64;                       // local index of the first core window
-constexpr int PT_NLOC = PT_PRE + PT_T + PT_H + 64;  // bytes held per tile (k <= 64)
-constexpr int PT_NW = PT_T + PT_H;               // windows with break flags
-constexpr int PT_WORDS = PT_NLOC / 32;
-constexpr int PT_PER_THREAD = PT_NW / PT_NT;     // 9 contiguous windows per thread
-constexpr int PT_PT = 9;                         // positions per rolling p-mer task
+constexpr int PT_NT = TL_NT;
+constexpr int PT_PRE = 32;                       // local index of the first core window
+constexpr int PT_T = kPartTile;                  // core windows per tile; the rest find superkmer ends
 constexpr int PT_STG = 6144;                     // packed bytes of a tile staged in shared memory
-static_assert(PT_NW % PT_NT == 0, "windows per thread");
-static_assert(PT_NLOC % 64 == 0, "tile alignment");
+static_assert(PT_T % 32 == 0 && PT_PRE + PT_T < TL_NW && kPartThreads == TL_NT, "whole words, a halo after the core");
 
 struct PartSmem {
-  uint8_t cd[PT_NLOC];             // 2-bit code, or 255
-  uint32_t badw[PT_WORDS];         // bit i: byte i is not ACGTU
-  uint32_t rsw[PT_WORDS];          // bit i: a read starts at byte i
-  uint32_t validw[PT_WORDS];       // bit l: window l lies inside one read
-  uint32_t touchw[PT_WORDS];       // bit l: window l covers a byte that is not ACGTU
-  union {
-    uint32_t g[PT_NLOC];           // filtered p-mer minimum per position, then suffix minima
-    uint32_t boff[PT_NLOC];        // per superkmer: byte offset in the tile
-  } a;
-  union {
-    uint32_t pre[PT_NLOC];         // prefix minima
-    uint32_t smm[PT_T + 1];        // minimizer of each core superkmer (after the window pass)
-  } b;
-  uint32_t pk[PT_NLOC / 16 + 1];   // the tile's bases, 2 bits each, first base in the top bits
+  TileBases t;
+  uint32_t brkw[TL_WORDS];         // bit i: window i starts a superkmer or lies in none
+  uint32_t smm[PT_T];              // minimizer of each core superkmer
+  uint32_t boff[PT_T];             // its byte offset in the tile
+  uint16_t spos[PT_T];             // its first window
+  uint16_t send[PT_T];             // its end window (PT_EXT: ext_end)
   alignas(16) uint8_t stg[PT_STG]; // the tile's packed superkmers before they are written out (read as uint4)
-  uint8_t code_tab[256];           // byte -> 2-bit code or 255
-  uint16_t brk[PT_NW + 1];         // local positions of breaks, ascending
-  uint16_t skm[PT_T + 1];          // break index of each core superkmer start
   uint32_t scan_tmp[64];
-  uint64_t red_tmp[32];
+  uint32_t lastmm[TL_WARPS], wcnt[TL_WARPS];
   int ext_end;                     // local end window of an extended last superkmer
-  int use_stg;                     // the tile's superkmers are packed through stg
-  uint32_t n_brk, n_skm, n_bytes;
   unsigned long long base_skm, base_byte;
 };
+constexpr uint32_t PT_EXT = 0xFFFFu;
 
-// Filtered p-mer minimum of every tile position (forward and reverse
-// complement), rolling over tasks of PT_PT consecutive positions; an odd
-// stride between threads keeps their shared-memory accesses in different
-// banks.  The filter is fixed per instantiation so the inner loop holds no
-// branch on it.
-template <int FILT>
-GKC_DEV void pmer_minima(PartSmem &S, int p, uint32_t M, int tid) {
-  const int npos = PT_NLOC - p + 1;
-  const int ntask = (npos + PT_PT - 1) / PT_PT;
-  for (int task = tid; task < ntask; task += PT_NT) {
-    int a0 = task * PT_PT;
-    uint32_t f = 0, r = 0;
-    for (int j = 0; j < p - 1; j++) {
-      uint32_t c = S.cd[a0 + j] & 3u;
-      f = (f << 2) | c;
-      r = (r >> 2) | ((3u - c) << (2 * p - 2));
-    }
-    int e = min(a0 + PT_PT, npos);
-    for (int i = a0; i < e; i++) {
-      uint32_t c = S.cd[i + p - 1] & 3u;
-      f = ((f << 2) | c) & M;
-      r = (r >> 2) | ((3u - c) << (2 * p - 2));
-      uint32_t vf = mm_filter(f, p, FILT) ? f : M;
-      uint32_t vr = mm_filter(r, p, FILT) ? r : M;
-      S.a.g[i] = vf < vr ? vf : vr;
-    }
-  }
-}
-
-GKC_DEV bool bit_at(const uint32_t *w, int i) { return (w[i >> 5] >> (i & 31)) & 1u; }
-
-// Any bit set in [a, b] (inclusive), b - a < 96.
-GKC_DEV bool any_bits(const uint32_t *w, int a, int b) {
-  if (a > b) return false;
-  int wa = a >> 5, wb = b >> 5;
-  if (wa == wb) {
-    uint32_t m = (0xFFFFFFFFu >> (31 - (b & 31))) & (0xFFFFFFFFu << (a & 31));
-    return (w[wa] & m) != 0u;
-  }
-  if (w[wa] & (0xFFFFFFFFu << (a & 31))) return true;
-  for (int x = wa + 1; x < wb; x++)
-    if (w[x]) return true;
-  return (w[wb] & (0xFFFFFFFFu >> (31 - (b & 31)))) != 0u;
-}
-
-// Bit i (0..31) of the result = OR of bits i .. i+n-1 of the 96-bit value
-// (x2:x1:x0), for 1 <= n <= 64: a sliding OR built by doubling shifts.
-GKC_DEV uint32_t span_or(uint32_t x0, uint32_t x1, uint32_t x2, int n) {
-  uint64_t lo = (uint64_t)x0 | ((uint64_t)x1 << 32);
-  uint64_t hi = x2;
-  int m = 1;
-  while (2 * m <= n) {  // lo:hi now holds the OR over m consecutive bits
-    lo |= (lo >> m) | (hi << (64 - m));
-    hi |= hi >> m;
-    m *= 2;
-  }
-  const int r = n - m;  // 0 <= r < m: cover the remaining bits with an overlapping shift
-  if (r > 0) lo |= (lo >> r) | (hi << (64 - r));
-  return (uint32_t)lo;
-}
-
-__global__ void __launch_bounds__(PT_NT, 3) k_partition(PartArgs a) {
+// Bound by instruction issue and the barriers between its phases: 256 threads
+// and 64 registers, so that four CTAs on an SM overlap, the next tile's bytes
+// loaded while this one is worked on.  900 M bases of 150 b reads (k 31, p 11)
+// on a B200: see k_partition's figures at its launch.
+__global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PartSmem &S = *reinterpret_cast<PartSmem *>(smem_raw);
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int k = a.k, p = a.p, omega = a.k - a.p + 1;
-  const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * p);
   if (a.nbytes_dev) a.nbytes = *a.nbytes_dev;
   const uint64_t n_tiles = (a.nbytes + PT_T - 1) / PT_T;
 
-  // per-CTA bin histograms (small bin counts only)
-  unsigned long long *h_km = reinterpret_cast<unsigned long long *>(smem_raw + sizeof(PartSmem));
-  uint32_t *h_skm = reinterpret_cast<uint32_t *>(h_km + a.nbins_smem);
-  for (int i = tid; i < a.nbins_smem; i += PT_NT) {
-    h_skm[i] = 0;
-    h_km[i] = 0;
-  }
-  for (int i = tid; i < 256; i += PT_NT) S.code_tab[i] = (uint8_t)code_of_byte((uint32_t)i);
-  __syncthreads();
+  // per-CTA bin histograms (small bin counts only): superkmers, k-mers
+  uint32_t *h_skm = reinterpret_cast<uint32_t *>(smem_raw + sizeof(PartSmem));
+  uint32_t *h_km = h_skm + a.nbins_smem;
+  for (int i = tid; i < 2 * a.nbins_smem; i += PT_NT) h_skm[i] = 0;
 
+  uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
+  if (blockIdx.x < n_tiles && tid < TL_GROUPS)
+    bytes = tile_fetch(a.reads, a.nbytes, a.aligned16, (int64_t)blockIdx.x * PT_T - PT_PRE, tid);
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int64_t ts = (int64_t)tile * PT_T;
-    const int64_t G0 = ts - PT_PRE;  // global position of local 0 (64-aligned)
-
-    // ---- load bytes -> codes (16 per thread, one 16-byte store), bad-code
-    //      bitmap (lane pairs combine their 16-bit halves), read-start bitmap ----
-    static_assert(PT_NLOC % 16 == 0 && PT_NLOC / 16 <= PT_NT, "one 16-byte group per thread");
-    if ((tid & ~31) * 16 < PT_NLOC) {  // warps with at least one group
-      const int q = tid * 16;
-      const bool act = q < PT_NLOC;
-      uint32_t cw[4] = {0u, 0u, 0u, 0u};
-      uint32_t bad16 = 0, pkw = 0;
-      if (act) {
-        const int64_t g = G0 + q;
-        const bool fast = g >= 0 && (uint64_t)(g + 16) <= a.nbytes && a.aligned16;
-        if (fast) {
-          const uint4 v = __ldg(reinterpret_cast<const uint4 *>(a.reads + g));
-          const uint32_t vw[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-          for (int t = 0; t < 16; t++) {
-            const uint32_t c = S.code_tab[(vw[t >> 2] >> (8 * (t & 3))) & 0xFFu];
-            cw[t >> 2] |= c << (8 * (t & 3));
-            bad16 |= (c >> 7) << t;
-            pkw |= (c & 3u) << (30 - 2 * t);
-          }
-        } else {
-#pragma unroll
-          for (int t = 0; t < 16; t++) {
-            const uint32_t c = global_code(a.reads, a.nbytes, g + t);
-            cw[t >> 2] |= c << (8 * (t & 3));
-            bad16 |= (c >> 7) << t;
-            pkw |= (c & 3u) << (30 - 2 * t);
-          }
-        }
-        *reinterpret_cast<uint4 *>(S.cd + q) = make_uint4(cw[0], cw[1], cw[2], cw[3]);
-        S.pk[q >> 4] = pkw;
-      }
-      const uint32_t other = __shfl_xor_sync(0xffffffffu, bad16, 1);
-      if (act && (tid & 1) == 0) S.badw[q >> 5] = bad16 | (other << 16);
-    }
-    for (int w = tid; w < PT_WORDS; w += PT_NT) {
-      int64_t gw = (G0 >> 5) + w;  // G0 is a multiple of 64
-      S.rsw[w] = (gw >= 0 && (uint64_t)gw < a.rs_words) ? a.rs_bits[gw] : 0u;
-      S.validw[w] = 0u;
-    }
-    if (tid == 0) S.pk[PT_NLOC / 16] = 0u;
+    const int64_t G0 = (int64_t)(tile * PT_T) - PT_PRE;  // global position of local 0 (32-aligned)
+    tile_store(S.t, bytes, a.rs_bits, a.rs_words, G0);
+    if (tid == 0) S.ext_end = -1;
     __syncthreads();
-    // Windows are valid when no read starts inside them (after their first
-    // byte) and they lie inside the data; they touch a bad byte when one of
-    // their k bytes is not ACGTU.  32 windows per word, by sliding ORs.
-    for (int w = tid; w < PT_WORDS; w += PT_NT) {
-      const uint32_t r0 = S.rsw[w], r1 = w + 1 < PT_WORDS ? S.rsw[w + 1] : 0u,
-                     r2 = w + 2 < PT_WORDS ? S.rsw[w + 2] : 0u;
-      // read starts at window bytes 1 .. k-1: shift the span right by one
-      const uint32_t hit = k > 1 ? span_or((r0 >> 1) | (r1 << 31), (r1 >> 1) | (r2 << 31), r2 >> 1, k - 1) : 0u;
-      const uint32_t b0 = S.badw[w], b1 = w + 1 < PT_WORDS ? S.badw[w + 1] : 0u,
-                     b2 = w + 2 < PT_WORDS ? S.badw[w + 2] : 0u;
-      S.touchw[w] = span_or(b0, b1, b2, k);
-      // windows inside the data: G0 + l >= 0 and G0 + l + k <= nbytes
-      const int64_t s0 = G0 + 32 * (int64_t)w;
-      const int64_t ilo = s0 < 0 ? -s0 : 0;
-      const int64_t ihi = (int64_t)a.nbytes - k - s0;
-      uint32_t range = 0u;
-      if (ihi >= 0 && ilo <= 31) {
-        const int lo_i = (int)ilo, hi_i = (int)(ihi > 31 ? 31 : ihi);
-        if (hi_i >= lo_i) range = (0xFFFFFFFFu >> (31 - hi_i)) & (0xFFFFFFFFu << lo_i);
-      }
-      S.validw[w] = ~hit & range;
-    }
+    if (tile + gridDim.x < n_tiles && tid < TL_GROUPS)
+      bytes = tile_fetch(a.reads, a.nbytes, a.aligned16, (int64_t)((tile + gridDim.x) * PT_T) - PT_PRE, tid);
 
-    // ---- filtered p-mer minimum per position ----
+    // ---- minimizers: lane l, register r hold window 32 (w0 + r) + l ----
+    const int w0 = warp * TL_TW;
+    uint32_t vw = 0, tw = 0;  // lane r + 1: word w0 + r; lane 0: the word before
+    if (lane <= TL_TW && w0 + lane >= 1)
+      tile_valid(S.t, w0 + lane - 1, G0, 0, (int64_t)a.nbytes, k, &vw, &tw);
+    uint32_t m[TL_TW + 2], none[1];
     switch (a.filter) {
-      case FILTER_ALL: pmer_minima<FILTER_ALL>(S, p, M, tid); break;
-      case FILTER_NEW: pmer_minima<FILTER_NEW>(S, p, M, tid); break;
-      case FILTER_SIGNATURE: pmer_minima<FILTER_SIGNATURE>(S, p, M, tid); break;
-      default: pmer_minima<FILTER_NEW2>(S, p, M, tid); break;
+      case FILTER_ALL: tile_minima<FILTER_ALL, false>(S.t, w0, p, omega, m, none); break;
+      case FILTER_NEW: tile_minima<FILTER_NEW, false>(S.t, w0, p, omega, m, none); break;
+      case FILTER_SIGNATURE: tile_minima<FILTER_SIGNATURE, false>(S.t, w0, p, omega, m, none); break;
+      default: tile_minima<FILTER_NEW2, false>(S.t, w0, p, omega, m, none); break;
     }
-    __syncthreads();
-
-    // ---- van Herk / Gil-Werman: prefix and suffix minima in blocks of omega ----
-    {
-      const int npos = PT_NLOC - p + 1;
-      const int nblk = (npos + omega - 1) / omega;
-      for (int blk = tid; blk < nblk; blk += PT_NT) {
-        int b0 = blk * omega, b1 = min(b0 + omega, npos);
-        uint32_t m = 0xFFFFFFFFu;
-        for (int i = b0; i < b1; i++) {
-          m = min(m, S.a.g[i]);
-          S.b.pre[i] = m;
-        }
-        m = 0xFFFFFFFFu;
-        for (int i = b1 - 1; i >= b0; i--) {
-          m = min(m, S.a.g[i]);
-          S.a.g[i] = m;  // suffix minima in place
-        }
-      }
-    }
-    __syncthreads();
-
-    // ---- window minimizers and breaks, thread-contiguous: windows
-    //      [lw0 - 1, lw0 + 9), the first only for the comparison ----
-    uint32_t nb_local = 0, ns_local = 0;
-    uint32_t brkbits = 0, startbits = 0;
-    const int lw0 = PT_PRE + tid * PT_PER_THREAD;
-    uint32_t mmv[PT_PER_THREAD + 1];
-    uint32_t vbits, tbits, rbits;  // bit j: window lw0 - 1 + j
-    {
-      const int l0 = lw0 - 1, w0 = l0 >> 5, sh = l0 & 31;
-      auto bits10 = [&](const uint32_t *arr) -> uint32_t {
-        const uint64_t v = (uint64_t)arr[w0] | ((uint64_t)(w0 + 1 < PT_WORDS ? arr[w0 + 1] : 0u) << 32);
-        return (uint32_t)(v >> sh) & 0x3FFu;
-      };
-      vbits = bits10(S.validw);
-      tbits = bits10(S.touchw);
-      rbits = bits10(S.rsw);
+    if (__any_sync(0xffffffffu, (tw & vw) != 0u)) {
 #pragma unroll
-      for (int j = 0; j <= PT_PER_THREAD; j++) {
-        const int l = l0 + j;
-        mmv[j] = 0xFFFFFFFFu;
-        if ((vbits >> j) & 1u) {
-          if (!((tbits >> j) & 1u)) {
-            mmv[j] = min(S.a.g[l], S.b.pre[l + omega - 1]);
-          } else {
-            const uint8_t *cw = S.cd + l;
-            mmv[j] = exact_window_minimizer([&](int i) { return (uint32_t)cw[i]; }, k, p, a.filter);
-          }
+      for (int r = 0; r < TL_TW; r++) {
+        const uint32_t t = __shfl_sync(0xffffffffu, tw & vw, r + 1);
+        if ((t >> lane) & 1u) {
+          const int l = 32 * (w0 + r) + lane;
+          m[r] = exact_window_minimizer([&](int i) { return tile_code(S.t, l + i); }, k, p, a.filter);
         }
       }
+    }
+    if (lane == 31) S.lastmm[warp] = m[TL_TW - 1];
+    __syncthreads();
+
+    // ---- breaks and superkmer starts, 32 windows a word ----
+    uint32_t st[TL_TW], cnt = 0;
+    {
+      uint32_t carry = warp ? S.lastmm[warp - 1] : 0u;  // minimizer of the window before
+      uint32_t pv = __shfl_sync(0xffffffffu, vw, 0);
+#pragma unroll
+      for (int r = 0; r < TL_TW; r++) {
+        const uint32_t before = __shfl_sync(0xffffffffu, m[r], (lane + 31) & 31);
+        const uint32_t diff = __ballot_sync(0xffffffffu, m[r] != (lane ? before : carry));
+        carry = before;  // lane 0: this word's last window
+        const uint32_t v = __shfl_sync(0xffffffffu, vw, r + 1);
+        const uint32_t start = v & (S.t.rsw[w0 + r] | diff | ~((v << 1) | (pv >> 31)));
+        pv = v;
+        if (lane == 0) S.brkw[w0 + r] = start | ~v;
+        const bool core = w0 + r >= PT_PRE / 32 && w0 + r < (PT_PRE + PT_T) / 32;
+        st[r] = core ? start : 0u;
+        cnt += __popc(st[r]);
+      }
+    }
+    if (lane == 0) S.wcnt[warp] = cnt;
+    __syncthreads();
+    uint32_t n_skm = 0, at = 0;
+#pragma unroll
+    for (int x = 0; x < TL_WARPS; x++) {
+      const uint32_t c = S.wcnt[x];
+      if (x < warp) at += c;
+      n_skm += c;
     }
 #pragma unroll
-    for (int j = 0; j < PT_PER_THREAD; j++) {
-      const int l = lw0 + j;
-      const bool valid = (vbits >> (j + 1)) & 1u;
-      const bool start = valid && (((rbits >> (j + 1)) & 1u) || mmv[j + 1] != mmv[j] || !((vbits >> j) & 1u));
-      const bool brk = !valid || start;
-      brkbits |= (brk ? 1u : 0u) << j;
-      const bool core_start = start && l < PT_PRE + PT_T;
-      startbits |= (core_start ? 1u : 0u) << j;
-      nb_local += brk;
-      ns_local += core_start;
-    }
-    uint32_t tot;
-    uint32_t excl = block_exclusive_scan<PT_NT>(nb_local | (ns_local << 16), S.scan_tmp, &tot);
-    {
-      uint32_t bi = excl & 0xFFFFu, si = excl >> 16;
-#pragma unroll
-      for (int j = 0; j < PT_PER_THREAD; j++) {
-        if ((brkbits >> j) & 1u) {
-          if ((startbits >> j) & 1u) {
-            S.b.smm[si] = mmv[j + 1];  // pre[] is no longer read: the scan above ended with a barrier
-            S.skm[si++] = (uint16_t)bi;
-          }
-          S.brk[bi++] = (uint16_t)(lw0 + j);
-        }
+    for (int r = 0; r < TL_TW; r++) {
+      if ((st[r] >> lane) & 1u) {
+        const uint32_t i = at + __popc(st[r] & ((1u << lane) - 1u));
+        S.spos[i] = (uint16_t)(32 * (w0 + r) + lane);
+        S.smm[i] = m[r];
       }
-    }
-    if (tid == 0) {
-      S.n_brk = tot & 0xFFFFu;
-      S.n_skm = tot >> 16;
-      S.ext_end = -1;
-    }
-    __syncthreads();
-    const uint32_t n_brk = S.n_brk, n_skm = S.n_skm;
-
-    // ---- the last core superkmer may run past the halo: extend it ----
-    if (n_skm > 0 && tid == 0) {
-      uint32_t jlast = S.skm[n_skm - 1];
-      if (jlast + 1 >= n_brk) {
-        uint32_t mv = S.b.smm[n_skm - 1];
-        uint64_t w = (uint64_t)(G0 + PT_PRE + PT_NW);
-        // walk windows beyond the halo with the exact rule until a break
-        while (w < a.nbytes) {
-          if (global_rs(a.rs_bits, w) || !global_window_valid(a.rs_bits, a.nbytes, w, k)) break;
-          uint32_t v = exact_window_minimizer(
-              [&](int i) { return global_code(a.reads, a.nbytes, (int64_t)w + i); }, k, p, a.filter);
-          if (v != mv) break;
-          w++;
-        }
-        S.ext_end = (int)((int64_t)w - G0);
-      }
+      at += __popc(st[r]);
     }
     __syncthreads();
 
-    // ---- superkmer sizes -> byte offsets (contiguous chunks of 8 per thread) ----
+    // ---- ends, byte offsets: consecutive superkmers per thread ----
+    const uint32_t per = (n_skm + PT_NT - 1) / PT_NT, i0 = min(tid * per, n_skm), i1 = min(i0 + per, n_skm);
     uint32_t my_bytes = 0;
-    const int sk0 = tid * 8;
-    for (int i = sk0; i < sk0 + 8 && i < (int)n_skm; i++) {
-      uint32_t j = S.skm[i];
-      int l = S.brk[j];
-      int e = (j + 1 < n_brk) ? S.brk[j + 1] : S.ext_end;
-      uint32_t len = (uint32_t)(e - l) + k - 1;
-      my_bytes += (len + 3) / 4;
+    for (uint32_t i = i0; i < i1; i++) {
+      const uint32_t l = S.spos[i];
+      int w = (int)(l >> 5);
+      uint32_t bits = S.brkw[w] & (0xFFFFFFFEu << (l & 31));
+      while (!bits && ++w < TL_WORDS) bits = S.brkw[w];
+      uint32_t e = bits ? 32 * (uint32_t)w + __ffs((int)bits) - 1 : PT_EXT, end = e;
+      if (!bits) {
+        // the last superkmer runs past the tile: walk on with the exact rule until a break
+        const uint32_t mv = S.smm[i];
+        uint64_t x = (uint64_t)(G0 + TL_NW);
+        while (x < a.nbytes) {
+          if (global_rs(a.rs_bits, x) || !global_window_valid(a.rs_bits, a.nbytes, x, k)) break;
+          const uint32_t v = exact_window_minimizer(
+              [&](int u) { return global_code(a.reads, a.nbytes, (int64_t)x + u); }, k, p, a.filter);
+          if (v != mv) break;
+          x++;
+        }
+        end = (uint32_t)((int64_t)x - G0);
+        S.ext_end = (int)end;
+      }
+      S.send[i] = (uint16_t)e;
+      const uint32_t nb = (end - l + k - 1 + 3) / 4;
+      S.boff[i] = my_bytes;  // relative to the thread's first
+      my_bytes += nb;
     }
     uint32_t tile_bytes;
-    uint32_t boff = block_exclusive_scan<PT_NT>(my_bytes, S.scan_tmp, &tile_bytes);
-    // S.a.g is no longer needed: reuse it for per-superkmer byte offsets
-    for (int i = sk0; i < sk0 + 8 && i < (int)n_skm; i++) {
-      uint32_t j = S.skm[i];
-      int l = S.brk[j];
-      int e = (j + 1 < n_brk) ? S.brk[j + 1] : S.ext_end;
-      uint32_t len = (uint32_t)(e - l) + k - 1;
-      S.a.boff[i] = boff;
-      boff += (len + 3) / 4;
-    }
+    const uint32_t off0 = block_exclusive_scan<PT_NT>(my_bytes, S.scan_tmp, &tile_bytes);
+    for (uint32_t i = i0; i < i1; i++) S.boff[i] += off0;
+    const uint32_t rounded = (tile_bytes + 15u) & ~15u;
     if (tid == 0) {
-      S.n_bytes = tile_bytes;
-      uint32_t rounded = (tile_bytes + 15u) & ~15u;
-      // the staged packing needs every superkmer's bases in the tile's data
-      S.use_stg = rounded <= (uint32_t)PT_STG && (S.ext_end < 0 || S.ext_end + k - 1 <= PT_NLOC);
-      S.base_skm = n_skm ? atomicAdd(a.cursors + 0, (unsigned long long)n_skm) : 0ull;
-      S.base_byte = rounded ? atomicAdd(a.cursors + 1, (unsigned long long)rounded) : 0ull;
-      if (S.base_skm + n_skm > a.cap_skm || S.base_byte + rounded > a.cap_bytes)
-        atomicOr(a.err, ERR_CAPACITY);
+      const unsigned long long bs = n_skm ? atomicAdd(a.cursors + 0, (unsigned long long)n_skm) : 0ull;
+      const unsigned long long bb = rounded ? atomicAdd(a.cursors + 1, (unsigned long long)rounded) : 0ull;
+      S.base_skm = bs;
+      S.base_byte = bb;
+      if (bs + n_skm > a.cap_skm || bb + rounded > a.cap_bytes) atomicOr(a.err, ERR_CAPACITY);
     }
     __syncthreads();
+    const int ext_end = S.ext_end;
+    // the staged packing needs every superkmer's bases in the tile's data
+    const bool use_stg = rounded <= (uint32_t)PT_STG && (ext_end < 0 || ext_end + k - 1 <= 32 * TL_BWORDS);
     const unsigned long long base_skm = S.base_skm, base_byte = S.base_byte;
-    const bool fits = base_skm + n_skm <= a.cap_skm && base_byte + ((tile_bytes + 15u) & ~15u) <= a.cap_bytes;
+    const bool fits = base_skm + n_skm <= a.cap_skm && base_byte + rounded <= a.cap_bytes;
 
-    // ---- descriptors, bin histograms ----
-    for (int i = tid; i < (int)n_skm; i += PT_NT) {
-      uint32_t j = S.skm[i];
-      int l = S.brk[j];
-      int e = (j + 1 < n_brk) ? S.brk[j + 1] : S.ext_end;
-      uint32_t nk = (uint32_t)(e - l);
-      uint32_t len = nk + k - 1;
-      uint32_t mv = S.b.smm[i];
-      uint32_t bin = mv % (uint32_t)a.nbins;
+    // ---- descriptors, bin histograms; each superkmer's bases cut from the
+    //      tile's 2-bit words into the staging area ----
+    for (uint32_t i = tid; i < n_skm; i += PT_NT) {
+      const uint32_t l = S.spos[i];
+      const uint32_t e = S.send[i] == PT_EXT ? (uint32_t)ext_end : S.send[i];
+      const uint32_t nk = e - l, len = nk + k - 1, mv = S.smm[i], bin = mv % (uint32_t)a.nbins;
       if (len > 0xFFFFFFu) atomicOr(a.err, ERR_BAD_READ);
       if (fits && len <= 0xFFFFFFu) {
-        uint64_t off = base_byte + S.a.boff[i];
-        a.skm_desc[base_skm + i] = (off << 24) | (uint64_t)len;
+        a.skm_desc[base_skm + i] = ((base_byte + S.boff[i]) << 24) | (uint64_t)len;
         a.skm_mm[base_skm + i] = mv;
         if (a.skm_gpos) a.skm_gpos[base_skm + i] = (uint64_t)(G0 + l);
       }
       if (bin < (uint32_t)a.nbins_smem) {
         atomicAdd(&h_skm[bin], 1u);
-        atomicAdd(&h_km[bin], (unsigned long long)nk);
+        atomicAdd(&h_km[bin], nk);
       } else {
         atomicAdd(&a.bin_nskm[bin], 1ull);
         atomicAdd(&a.bin_nkmers[bin], (unsigned long long)nk);
       }
-    }
-
-    // ---- packed bytes: each superkmer's bases cut from the tile's 2-bit
-    //      stream into the staging area, then written out in 16-byte pieces ----
-    if (fits && S.use_stg) {
-      for (int i = tid; i < (int)n_skm; i += PT_NT) {
-        const uint32_t j = S.skm[i];
-        const int l = S.brk[j];
-        const int e = (j + 1 < n_brk) ? S.brk[j + 1] : S.ext_end;
-        const uint32_t len = (uint32_t)(e - l) + k - 1, nb = (len + 3) / 4;
-        uint8_t *dst = S.stg + S.a.boff[i];
-        for (uint32_t m = 0; 16 * m < len; m++) {
-          const uint32_t B = (uint32_t)l + 16 * m, w = B >> 4, sh = 2 * (B & 15u);
-          uint32_t v = sh ? (S.pk[w] << sh) | (S.pk[w + 1] >> (32 - sh)) : S.pk[w];
-          const uint32_t rem = len - 16 * m;
+      if (fits && use_stg) {
+        const uint32_t nb = (len + 3) / 4;
+        uint8_t *dst = S.stg + S.boff[i];
+        for (uint32_t x = 0; 16 * x < len; x++) {
+          const uint32_t B = l + 16 * x, w = B >> 4;
+          uint32_t v = __funnelshift_l(S.t.pk[w + 1].x, S.t.pk[w].x, 2 * (B & 15u));
+          const uint32_t rem = len - 16 * x;
           if (rem < 16) v &= 0xFFFFFFFFu << (32 - 2 * rem);  // zero padding after the last base
 #pragma unroll
           for (int u = 0; u < 4; u++)
-            if (4 * m + u < nb) dst[4 * m + u] = (uint8_t)(v >> (24 - 8 * u));
+            if (4 * x + u < nb) dst[4 * x + u] = (uint8_t)(v >> (24 - 8 * u));
         }
       }
-      if (tid < 16 && tile_bytes + tid < ((tile_bytes + 15u) & ~15u)) S.stg[tile_bytes + tid] = 0;
+    }
+    if (fits && use_stg) {
+      if (tid < 16 && tile_bytes + tid < rounded) S.stg[tile_bytes + tid] = 0;
       __syncthreads();
-      const uint32_t n16 = (tile_bytes + 15u) / 16u;
       uint4 *dst16 = reinterpret_cast<uint4 *>(a.packed + base_byte);
       const uint4 *src16 = reinterpret_cast<const uint4 *>(S.stg);
-      for (uint32_t v = tid; v < n16; v += PT_NT) dst16[v] = src16[v];
+      for (uint32_t v = tid; v < rounded / 16; v += PT_NT) dst16[v] = src16[v];
     } else if (fits) {
       const uint32_t nwords = (tile_bytes + 3) / 4;
       uint32_t *dst = reinterpret_cast<uint32_t *>(a.packed + base_byte);
       for (uint32_t w = tid; w < nwords; w += PT_NT) {
         uint32_t word = 0;
         // superkmer holding the word's first byte: last i with boff[i] <= 4w
-        int lo = 0;
-        {
-          int hi = (int)n_skm - 1;
-          while (lo < hi) {
-            int mid = (lo + hi + 1) >> 1;
-            if (S.a.boff[mid] <= w * 4) lo = mid; else hi = mid - 1;
-          }
+        int lo = 0, hi = (int)n_skm - 1;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (S.boff[mid] <= w * 4) lo = mid; else hi = mid - 1;
         }
 #pragma unroll
         for (int u = 0; u < 4; u++) {
-          uint32_t q = w * 4 + u;
+          const uint32_t q = w * 4 + u;
           if (q >= tile_bytes) break;
-          while (lo + 1 < (int)n_skm && S.a.boff[lo + 1] <= q) lo++;
-          uint32_t j = S.skm[lo];
-          int l = S.brk[j];
-          int e = (j + 1 < n_brk) ? S.brk[j + 1] : S.ext_end;
-          uint32_t len = (uint32_t)(e - l) + k - 1;
-          uint32_t bb = q - S.a.boff[lo];
+          while (lo + 1 < (int)n_skm && S.boff[lo + 1] <= q) lo++;
+          const uint32_t l = S.spos[lo];
+          const uint32_t e = S.send[lo] == PT_EXT ? (uint32_t)ext_end : S.send[lo];
+          const uint32_t len = e - l + k - 1, bb = q - S.boff[lo];
           uint32_t byte = 0;
 #pragma unroll
           for (int t = 0; t < 4; t++) {
-            uint32_t bi = bb * 4 + t;
+            const uint32_t bi = bb * 4 + t;
             uint32_t c = 0;
             if (bi < len) {
-              int lp = l + (int)bi;
-              c = (lp < PT_NLOC) ? (S.cd[lp] & 3u) : (global_code(a.reads, a.nbytes, G0 + lp) & 3u);
+              const uint32_t lp = l + bi;
+              c = lp < 32u * TL_BWORDS ? tile_code(S.t, (int)lp) & 3u
+                                       : global_code(a.reads, a.nbytes, G0 + (int64_t)lp) & 3u;
             }
             byte = (byte << 2) | c;
           }
@@ -455,14 +260,15 @@ __global__ void __launch_bounds__(PT_NT, 3) k_partition(PartArgs a) {
   }
 
   // flush bin histograms
+  __syncthreads();
   for (int i = tid; i < a.nbins_smem; i += PT_NT) {
     if (h_skm[i]) atomicAdd(&a.bin_nskm[i], (unsigned long long)h_skm[i]);
-    if (h_km[i]) atomicAdd(&a.bin_nkmers[i], h_km[i]);
+    if (h_km[i]) atomicAdd(&a.bin_nkmers[i], (unsigned long long)h_km[i]);
   }
 }
 
 size_t partition_smem_bytes(int nbins_smem) {
-  return sizeof(PartSmem) + (size_t)nbins_smem * (sizeof(uint32_t) + sizeof(unsigned long long)) + 16;
+  return sizeof(PartSmem) + (size_t)nbins_smem * 2 * sizeof(uint32_t) + 16;
 }
 
 // Read-start bitmap: bit offs[r]-offs[0] for every read, plus bit nbytes as

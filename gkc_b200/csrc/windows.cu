@@ -21,6 +21,7 @@
 #include "kernels.h"
 #include "minimizer.cuh"
 #include "onesweep.h"
+#include "tile.cuh"
 
 namespace gkc {
 
@@ -37,21 +38,6 @@ __global__ void k_window_starts(const uint64_t *offs, uint64_t n_reads, uint64_t
     }
     atomicOr(&bits[pos >> 5], 1u << (pos & 31));
   }
-}
-
-// Window [i, i + k) inside one read: lo <= i, i + k <= hi, and no read start
-// at positions i+1 .. i+k-1.
-GKC_DEV bool window_inside(const uint32_t *bits, uint64_t i, int k, uint64_t lo, uint64_t hi) {
-  if (i < lo || i + k > hi) return false;
-  for (uint64_t q = i + 1; q < i + k;) {
-    const uint32_t w = bits[q >> 5] >> (q & 31);
-    const uint64_t left = i + k - q, room = 32 - (q & 31);
-    const uint32_t span = (uint32_t)(left < room ? left : room);
-    const uint32_t m = span == 32 ? 0xFFFFFFFFu : ((1u << span) - 1u);
-    if (w & m) return false;
-    q += span;
-  }
-  return true;
 }
 
 struct WinMin {
@@ -87,50 +73,123 @@ GKC_DEV WinMin window_min_pos(const uint8_t *reads, uint64_t i, int k, int p, in
   return w;
 }
 
-__global__ void k_window_minimizers(const uint8_t *reads, uint64_t n_bytes, const uint64_t *offs,
-                                    uint64_t n_reads, const uint32_t *bits, int k, int p, int filter,
-                                    uint32_t *mm, uint8_t *pos, int8_t *strand) {
-  const uint64_t lo = offs[0], hi = offs[n_reads];
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_bytes;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    WinMin w{0xFFFFFFFFu, 255, 0};
-    if (hi <= n_bytes && window_inside(bits, i, k, lo, hi)) w = window_min_pos(reads, i, k, p, filter);
-    mm[i] = w.mm;
-    if (pos) pos[i] = w.pos;
-    if (strand) strand[i] = w.strand;
+struct WinArgs {
+  const uint8_t *reads;
+  uint64_t n_bytes;
+  int aligned16;
+  const uint64_t *offs;
+  uint64_t n_reads;
+  const uint32_t *bits;  // read starts
+  uint64_t bit_words;
+  int k, p, filter;
+};
+
+// The warp's windows of a tile (tile.cuh): m[r] and, with POS, q[r] for word
+// w0 + r; valid and touched words in lane r of *vw and *tw.
+template <bool POS>
+GKC_DEV void tile_windows(const TileBases &S, const WinArgs &a, int64_t G0, int64_t lo, int64_t hi, int w0,
+                          uint32_t (&m)[TL_TW + 2], uint32_t (&q)[POS ? TL_TW + 2 : 1], uint32_t *vw, uint32_t *tw) {
+  const int lane = threadIdx.x & 31, omega = a.k - a.p + 1;
+  *vw = *tw = 0;
+  if (lane < TL_TW) tile_valid(S, w0 + lane, G0, lo, hi, a.k, vw, tw);
+  switch (a.filter) {
+    case FILTER_ALL: tile_minima<FILTER_ALL, POS>(S, w0, a.p, omega, m, q); break;
+    case FILTER_NEW: tile_minima<FILTER_NEW, POS>(S, w0, a.p, omega, m, q); break;
+    case FILTER_SIGNATURE: tile_minima<FILTER_SIGNATURE, POS>(S, w0, a.p, omega, m, q); break;
+    default: tile_minima<FILTER_NEW2, POS>(S, w0, a.p, omega, m, q); break;
+  }
+}
+
+// Minimizer, position and strand of every window, one tile per CTA turn.
+// Windows with a byte that is no base follow the exact per-window rule, and so
+// do those whose minimizer is the largest p-mer value (it may stand for "none
+// passed", which has no position).
+__global__ void __launch_bounds__(TL_NT, 3) k_window_minimizers(WinArgs a, uint32_t *mm, uint8_t *pos,
+                                                                int8_t *strand) {
+  __shared__ TileBases S;
+  const uint64_t hi = a.offs[a.n_reads];
+  const int64_t lo = (int64_t)a.offs[0], end = hi <= a.n_bytes ? (int64_t)hi : 0;
+  const uint64_t n_tiles = (a.n_bytes + TL_NW - 1) / TL_NW;
+  const int lane = threadIdx.x & 31, w0 = (threadIdx.x >> 5) * TL_TW;
+  const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * a.p);
+  uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
+  if (blockIdx.x < n_tiles && threadIdx.x < TL_GROUPS)
+    bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, (int64_t)blockIdx.x * TL_NW, threadIdx.x);
+  for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const int64_t G0 = (int64_t)(tile * TL_NW);
+    tile_store(S, bytes, a.bits, a.bit_words, G0);
+    __syncthreads();
+    if (tile + gridDim.x < n_tiles && threadIdx.x < TL_GROUPS)
+      bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, (int64_t)((tile + gridDim.x) * TL_NW), threadIdx.x);
+    uint32_t m[TL_TW + 2], q[TL_TW + 2], vw, tw;
+    tile_windows<true>(S, a, G0, lo, end, w0, m, q, &vw, &tw);
+#pragma unroll
+    for (int r = 0; r < TL_TW; r++) {
+      const uint32_t v = __shfl_sync(0xffffffffu, vw, r), t = __shfl_sync(0xffffffffu, tw, r);
+      const uint32_t l = 32 * (uint32_t)(w0 + r) + lane;
+      const uint64_t i = (uint64_t)G0 + l;
+      if (i < a.n_bytes) {
+        WinMin w{0xFFFFFFFFu, 255, 0};
+        if ((v >> lane) & 1u) {
+          if (((t >> lane) & 1u) || m[r] == M) {
+            w = window_min_pos(a.reads, i, a.k, a.p, a.filter);
+          } else {
+            const uint32_t code = q[r] & 3u;
+            w.mm = m[r];
+            w.pos = (uint8_t)((q[r] >> 2) - l);
+            w.strand = (int8_t)(code == 2u ? -1 : (int)code);
+          }
+        }
+        mm[i] = w.mm;
+        if (pos) pos[i] = w.pos;
+        if (strand) strand[i] = w.strand;
+      }
+    }
+    __syncthreads();  // before the next tile's bases
   }
 }
 
 // ---- subsampling: windows whose minimizer % mod == 0, in window order ----
 
-constexpr int SUB_NT = 256;
-constexpr int SUB_ITEMS = 16;
-constexpr int SUB_TILE = SUB_NT * SUB_ITEMS;  // windows per tile = 128 bitmap words
+constexpr int SUB_NT = TL_NT;
+constexpr int SUB_WORDS = TL_WORDS;  // selection words per tile
+constexpr int SUB_TILE = TL_NW;      // windows per tile
+static_assert(SUB_WORDS * 2 <= SUB_NT, "two threads per selection word");
 
 // Tile t covers windows [t*SUB_TILE, (t+1)*SUB_TILE): selection bitmap and count.
-__global__ void k_sub_flags(const uint8_t *reads, uint64_t n_bytes, const uint64_t *offs,
-                            uint64_t n_reads, const uint32_t *bits, int k, int p, int filter,
-                            uint32_t mod, uint32_t *sel, unsigned long long *tile_cnt) {
-  __shared__ uint64_t tmp[32];
-  const uint64_t lo = offs[0], hi = offs[n_reads];
-  const uint64_t t = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  uint64_t cnt = 0;
-  // warp w handles bitmap words t*128 + w*16 + r: 32 consecutive windows each
-  for (int r = 0; r < SUB_ITEMS; r++) {
-    const uint64_t word = t * (SUB_TILE / 32) + (uint64_t)warp * SUB_ITEMS + r;
-    const uint64_t i = word * 32 + lane;
-    bool f = false;
-    if (i < n_bytes && hi <= n_bytes && window_inside(bits, i, k, lo, hi)) {
-      const uint32_t m = exact_window_minimizer([&](int j) { return code_of_byte(reads[i + j]); }, k, p, filter);
-      f = (m % mod) == 0u;
+__global__ void __launch_bounds__(SUB_NT, 4) k_sub_flags(WinArgs a, uint32_t mod, uint32_t *sel,
+                                                         unsigned long long *tile_cnt, uint64_t n_tiles) {
+  __shared__ TileBases S;
+  __shared__ uint32_t cnt[TL_WARPS];
+  const uint64_t hi = a.offs[a.n_reads];
+  const int64_t lo = (int64_t)a.offs[0], end = hi <= a.n_bytes ? (int64_t)hi : 0;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * TL_TW;
+  for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const int64_t G0 = (int64_t)(tile * TL_NW);
+    uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < TL_GROUPS) bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, G0, threadIdx.x);
+    tile_store(S, bytes, a.bits, a.bit_words, G0);
+    __syncthreads();
+    uint32_t m[TL_TW + 2], none[1], vw, tw, c = 0;
+    tile_windows<false>(S, a, G0, lo, end, w0, m, none, &vw, &tw);
+#pragma unroll
+    for (int r = 0; r < TL_TW; r++) {
+      const uint32_t v = __shfl_sync(0xffffffffu, vw, r), t = __shfl_sync(0xffffffffu, tw & vw, r);
+      const int l = 32 * (w0 + r) + lane;
+      if ((t >> lane) & 1u)
+        m[r] = exact_window_minimizer([&](int j) { return tile_code(S, l + j); }, a.k, a.p, a.filter);
+      const uint32_t f = __ballot_sync(0xffffffffu, ((v >> lane) & 1u) && m[r] % mod == 0u);
+      if (lane == 0) sel[tile * SUB_WORDS + w0 + r] = f;
+      c += __popc(f);
     }
-    const uint32_t b = __ballot_sync(0xffffffffu, f);
-    if (lane == 0 && word * 32 < n_bytes) sel[word] = b;
-    cnt += __popc(b) * (lane == 0);
+    if (lane == 0) cnt[warp] = c;
+    __syncthreads();  // also before the next tile's bases
+    if (threadIdx.x == 0) {
+      uint32_t s = 0;
+      for (int x = 0; x < TL_WARPS; x++) s += cnt[x];
+      tile_cnt[tile] = s;
+    }
   }
-  cnt = block_sum_u64<SUB_NT>(cnt, tmp);
-  if (threadIdx.x == 0) tile_cnt[t] = cnt;
 }
 
 template <typename K>
@@ -143,20 +202,17 @@ GKC_DEV K window_canonical(const uint8_t *reads, uint64_t i, int k) {
 
 // Writes (canonical key, window start) of the selected windows in window order.
 template <typename K>
-__global__ void k_sub_write(const uint8_t *reads, uint64_t n_bytes, const uint32_t *sel,
-                            const uint64_t *tile_off, int k, K *keys, uint32_t *posv) {
+__global__ void __launch_bounds__(SUB_NT) k_sub_write(const uint8_t *reads, uint64_t n_bytes, const uint32_t *sel,
+                                                      const uint64_t *tile_off, int k, K *keys, uint32_t *posv) {
   __shared__ uint32_t tmp[64];
   const uint64_t t = blockIdx.x;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // thread (warp, lane) owns bitmap word t*128 + warp*16 + lane/2, half lane&1
-  const uint64_t word = t * (SUB_TILE / 32) + (uint64_t)warp * SUB_ITEMS + (lane >> 1);
-  const bool in = word * 32 < n_bytes;
-  uint32_t b = in ? sel[word] : 0u;
-  b = (lane & 1) ? (b >> 16) : (b & 0xFFFFu);
-  const uint32_t c = __popc(b);
+  // thread x owns half x & 1 of the tile's selection word x / 2
+  const uint32_t x = threadIdx.x;
+  uint32_t b = x < 2 * SUB_WORDS ? sel[t * SUB_WORDS + (x >> 1)] : 0u;
+  b = (x & 1) ? (b >> 16) : (b & 0xFFFFu);
   uint32_t total;
-  uint64_t o = tile_off[t] + block_exclusive_scan<SUB_NT>(c, tmp, &total);
-  const uint64_t i0 = word * 32 + (lane & 1) * 16;
+  uint64_t o = tile_off[t] + block_exclusive_scan<SUB_NT>(__popc(b), tmp, &total);
+  const uint64_t i0 = t * SUB_TILE + 16 * (uint64_t)x;
   while (b) {
     const int q = __ffs(b) - 1;
     b &= b - 1;
@@ -210,6 +266,12 @@ static gkc_status mark_starts(gkc_ctx *c, const uint64_t *d_offs, uint64_t n_rea
   return GKC_OK;
 }
 
+static WinArgs win_args(const gkc_ctx *c, const gkc_params *prm, const uint8_t *reads, uint64_t n_bytes,
+                        const uint64_t *offs, uint64_t n_reads, const uint32_t *bits) {
+  return WinArgs{reads,  n_bytes, ((uintptr_t)reads % 16) == 0, offs,   n_reads, bits, (n_bytes + 1) / 32 + 3,
+                 prm->k, prm->p,  c->filter};
+}
+
 static gkc_status read_err(gkc_ctx *c, const uint32_t *err) {
   uint32_t e = 0;
   CK(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, c->st));
@@ -230,9 +292,10 @@ gkc_status gkc_minimizers_device(gkc_ctx *c, const gkc_params *prm, const char *
   uint32_t *bits, *err;
   s = mark_starts(c, d_offs, n_reads, n_bytes, &bits, &err);
   if (s != GKC_OK) return s;
-  k_window_minimizers<<<c->n_sms * 16, 256, 0, c->st>>>(reinterpret_cast<const uint8_t *>(d_reads), n_bytes,
-                                                         d_offs, n_reads, bits, prm->k, prm->p, c->filter, d_minimizer,
-                                                         d_pos, d_strand);
+  const uint64_t tiles = (n_bytes + TL_NW - 1) / TL_NW;
+  k_window_minimizers<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 3), TL_NT, 0, c->st>>>(
+      win_args(c, prm, reinterpret_cast<const uint8_t *>(d_reads), n_bytes, d_offs, n_reads, bits), d_minimizer, d_pos,
+      d_strand);
   CK(cudaPeekAtLastError());
   return read_err(c, err);
 }
@@ -245,12 +308,12 @@ static gkc_status subsample_t(gkc_ctx *c, const gkc_params *prm, uint32_t mod, c
   gkc_status s = mark_starts(c, d_offs, n_reads, n_bytes, &bits, &err);
   if (s != GKC_OK) return s;
   const uint64_t tiles = (n_bytes + SUB_TILE - 1) / SUB_TILE;
-  WS(sel, uint32_t, "win_sel", tiles * (SUB_TILE / 32) + 1);
+  WS(sel, uint32_t, "win_sel", tiles * SUB_WORDS + 1);
   WS(tcnt, unsigned long long, "win_tile_cnt", tiles + 1);
   WS(toff, uint64_t, "win_tile_off", tiles + 2);
   WS(stmp, uint64_t, "win_scan_tmp", scan_u64_tmp_words(tiles + 1) + 8);
-  k_sub_flags<<<(unsigned)tiles, SUB_NT, 0, c->st>>>(reads, n_bytes, d_offs, n_reads, bits, prm->k, prm->p,
-                                                     c->filter, mod, sel, tcnt);
+  k_sub_flags<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 4), SUB_NT, 0, c->st>>>(
+      win_args(c, prm, reads, n_bytes, d_offs, n_reads, bits), mod, sel, tcnt, tiles);
   scan_u64(tcnt, toff, tiles, stmp, c->st);
   CK(cudaPeekAtLastError());
   uint64_t n = 0;
