@@ -338,6 +338,7 @@ static gkc_status check_params(gkc_ctx *c, const gkc_params *prm) {
 
 // --------------------------------------------------------------- totals
 
+// The totals go straight to the slot's page-locked record (no copy follows).
 __global__ void k_finalize(DevTotals *t, const unsigned long long *cursors, const uint32_t *err,
                            const uint64_t *bin_kstart, uint32_t nbins, const uint64_t *n_bytes_dev,
                            const uint64_t *bin_out) {
@@ -347,6 +348,7 @@ __global__ void k_finalize(DevTotals *t, const unsigned long long *cursors, cons
   t->n_kmers = bin_kstart ? bin_kstart[nbins] : 0;
   t->n_bytes = n_bytes_dev ? *n_bytes_dev : 0;
   t->n_distinct = bin_out ? bin_out[nbins] : 0;
+  __threadfence_system();
 }
 
 // ------------------------------------------------------------- partition
@@ -404,8 +406,6 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
   WS(tot, unsigned long long, "cursors", 4);
   WS(err, uint32_t, "err", 4);
   stage_mark(c, 0);
-  CK(cudaMemsetAsync(tot, 0, 4 * sizeof(unsigned long long), c->st));
-  CK(cudaMemsetAsync(err, 0, 4 * sizeof(uint32_t), c->st));
   c->part_hpc_reads = nullptr;
   c->part_hpc_offs = nullptr;
   c->part_hpc_orig = nullptr;
@@ -417,8 +417,7 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
     WS(stmp, uint64_t, "scan_tmp", scan_u64_tmp_words(n_reads + 1) + 8);
     k_hpc_count<<<c->n_sms * 8, 256, 0, c->st>>>(src, offs, n_reads, runlen);
     LAUNCHED(c);
-    scan_u64(runlen, hoffs, n_reads, stmp, c->st);
-    c->launches += 4;
+    c->launches += scan_u64(runlen, hoffs, n_reads, stmp, c->st);
     k_hpc_write<<<c->n_sms * 8, 256, 0, c->st>>>(src, offs, n_reads, hoffs, hreads, horig);
     LAUNCHED(c);
     src = hreads;
@@ -430,7 +429,11 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
   }
   const uint64_t rs_words = (n_bytes + 1 + 31) / 32 + 2;
   WS(rs, uint32_t, "rs_bits", rs_words);
-  CK(cudaMemsetAsync(rs, 0, rs_words * 4, c->st));
+  WS(bin_nskm, unsigned long long, "bin_nskm", nbins + 1);
+  WS(bin_nkm, unsigned long long, "bin_nkmers", nbins + 1);
+  const ClearArgs ca{tot, err, bin_nskm, bin_nkm, nbins, rs, rs_words};
+  k_partition_clear<<<(unsigned)std::min<uint64_t>(rs_words / 1024 + 1, (uint64_t)c->n_sms * 8), 256, 0, c->st>>>(ca);
+  LAUNCHED(c);
   k_read_start_bits<<<(unsigned)std::min<uint64_t>((n_reads + 256) / 256, 65535), 256, 0, c->st>>>(
       offs, n_reads, rs);
   LAUNCHED(c);
@@ -438,10 +441,6 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
   WS(desc, uint64_t, "skm_desc_tile", cap_skm);
   WS(mm, uint32_t, "skm_mm_tile", cap_skm);
   WS(packed, uint8_t, "packed", cap_bytes);
-  WS(bin_nskm, unsigned long long, "bin_nskm", nbins + 1);
-  WS(bin_nkm, unsigned long long, "bin_nkmers", nbins + 1);
-  CK(cudaMemsetAsync(bin_nskm, 0, (nbins + 1) * 8, c->st));
-  CK(cudaMemsetAsync(bin_nkm, 0, (nbins + 1) * 8, c->st));
 
   PartArgs a;
   memset(&a, 0, sizeof(a));
@@ -479,24 +478,25 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
 
   WS(bin_start, uint64_t, "bin_start", nbins + 1);
   WS(bin_kstart, uint64_t, "bin_kstart", nbins + 1);
-  k_bin_prefix<<<1, 32, 0, c->st>>>(bin_nskm, bin_nkm, nbins, bin_start, bin_kstart);
+  k_bin_prefix<<<1, kBinPrefixThreads, 0, c->st>>>(bin_nskm, bin_nkm, nbins, bin_start, bin_kstart);
   LAUNCHED(c);
   WS(bdesc, uint64_t, "skm_desc_bin", cap_skm);
   WS(bmm, uint32_t, "skm_mm_bin", cap_skm);
   if (nbins <= (uint32_t)kBinPlaceMaxBins) {
     // (bin, chunk) counts, one scan, then placement: no global atomics
-    const uint64_t nch_cap = (cap_skm + kBinChunk - 1) / kBinChunk;
+    // few superkmers: chunks of one round, so that more CTAs share them
+    const uint32_t chunk = cap_skm < (uint64_t)kBinChunk * c->n_sms * 2 ? kBinRound : kBinChunk;
+    const uint64_t nch_cap = (cap_skm + chunk - 1) / chunk;
     const uint64_t cells = nch_cap * nbins;
     WS(bmat, unsigned long long, "bin_chunk_cnt", cells + 1);
     WS(boff, uint64_t, "bin_chunk_off", cells + 2);
     WS(btmp, uint64_t, "bin_chunk_scan", scan_u64_tmp_words(cells + 1) + 8);
     const unsigned g = (unsigned)std::min<uint64_t>(nch_cap, (uint64_t)c->n_sms * 8);
-    k_bin_count<<<g, 256, nbins * 4, c->st>>>(tot, mm, nbins, nch_cap, bmat, err);
+    k_bin_count<<<g, 256, nbins * 4, c->st>>>(tot, mm, nbins, chunk, nch_cap, bmat, err);
     LAUNCHED(c);
-    scan_u64(bmat, boff, cells, btmp, c->st);
-    c->launches += 4;
+    c->launches += scan_u64(bmat, boff, cells, btmp, c->st);
     k_bin_place<<<(unsigned)std::min<uint64_t>(nch_cap, (uint64_t)c->n_sms * 2), kBinPlaceThreads,
-                  bin_place_smem_bytes(nbins), c->st>>>(tot, desc, mm, nbins, nch_cap, boff, bdesc, bmm, err);
+                  bin_place_smem_bytes(nbins), c->st>>>(tot, desc, mm, nbins, chunk, nch_cap, boff, bdesc, bmm, err);
     LAUNCHED(c);
   } else {
     WS(bfill, unsigned long long, "bin_fill", nbins + 1);
@@ -539,11 +539,9 @@ static gkc_status fill_partition_view(gkc_ctx *c, const gkc_params *prm, uint64_
 static gkc_status read_totals(gkc_ctx *c, bool with_count, uint32_t nbins) {
   const uint64_t *bk = (const uint64_t *)c->bufs["bin_kstart"].p;
   const uint64_t *bo = with_count ? (const uint64_t *)c->bufs[slot_name(c, "bin_out")].p : nullptr;
-  WS(dt, DevTotals, "totals", 1);
-  k_finalize<<<1, 1, 0, c->st>>>(dt, (const unsigned long long *)c->bufs["cursors"].p,
+  k_finalize<<<1, 1, 0, c->st>>>(c->h_tot, (const unsigned long long *)c->bufs["cursors"].p,
                                  (const uint32_t *)c->bufs["err"].p, bk, nbins, c->part_nbytes_dev, bo);
   LAUNCHED(c);
-  CK(cudaMemcpyAsync(c->h_tot, dt, sizeof(DevTotals), cudaMemcpyDeviceToHost, c->st));
   stage_mark(c, 7);
   return GKC_OK;
 }
@@ -624,13 +622,9 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
 
   // k-mer offset of every bin-ordered superkmer
   stage_mark(c, 3);
-  WS(nk, unsigned long long, "skm_nk", cap_skm + 1);
   WS(koff, uint64_t, "skm_koff", cap_skm + 2);
   WS(stmp, uint64_t, "scan_tmp2", scan_u64_tmp_words(cap_skm + 1) + 8);
-  k_skm_nk<<<c->n_sms * 8, 256, 0, c->st>>>(desc, n_skm_dev, prm->k, nk);
-  LAUNCHED(c);
-  scan_u64_dev(nk, koff, cap_skm, (const uint64_t *)n_skm_dev, stmp, c->st);
-  c->launches += 4;
+  c->launches += scan_kmers_dev(desc, prm->k, koff, cap_skm, (const uint64_t *)n_skm_dev, stmp, c->st);
 
   WS(bin_bits, uint32_t, "bin_bits", nbins + 1);
   WS(bucket_base, uint64_t, "bucket_base", nbins + 1);
@@ -650,6 +644,9 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   pl.bucket_base = bucket_base;
   pl.chunk_base = chunk_base;
   pl.hist_base = hist_base;
+  // [0] bucket ticket, [1] unused, [2] large buckets listed, [3] their ticket
+  WS(ticket, unsigned long long, "count_ticket", 4);
+  pl.tickets = ticket;
   k_count_plan<<<1, kCountPlanThreads, 0, c->st>>>(pl);
   LAUNCHED(c);
 
@@ -688,15 +685,12 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   ea.flat = out_keys;
   ea.keys_cap = keys_cap;
   ea.err = err;
-  const uint64_t first_n = std::max(max_chunks, ((uint64_t)nbins << max_bits) / 8);
+  const uint64_t first_n = std::max(32 * max_chunks, ((uint64_t)nbins << max_bits) / 8);
   k_chunk_first<<<(unsigned)std::min<uint64_t>((first_n + 255) / 256, 65535), 256, 0, c->st>>>(ea);
   LAUNCHED(c);
   k_bucket_hist<K><<<c->n_sms * 8, kBucketHistThreads, 0, c->st>>>(ea);
   LAUNCHED(c);
   WS(big_list, uint32_t, "big_list", max_buckets + 1);
-  // [0] bucket ticket, [1] unused, [2] large buckets listed, [3] their ticket
-  WS(ticket, unsigned long long, "count_ticket", 4);
-  CK(cudaMemsetAsync(ticket, 0, 32, c->st));
   ea.big_list = big_list;
   ea.big_count = ticket + 2;
   ea.big_min = bucket_count_cap<K>() + 1;
@@ -754,8 +748,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   LAUNCHED(c);
   stage_mark(c, 6);
   // final offsets: the exclusive scan of the distinct counts (the bucket count is read on the device)
-  scan_u64_dev(bucket_d, bucket_out, max_buckets, bucket_base + nbins, dtmp, c->st);
-  c->launches += 4;
+  c->launches += scan_u64_dev(bucket_d, bucket_out, max_buckets, bucket_base + nbins, dtmp, c->st);
   WS(out_counts, uint32_t, slot_name(c, "counts").c_str(), keys_cap);
   WS(bin_out, uint64_t, slot_name(c, "bin_out").c_str(), nbins + 1);
   k_compact_runs<K><<<c->n_sms * 8, 256, 0, c->st>>>(keys, stage_counts, bstart, bucket_d, bucket_out, bucket_base,

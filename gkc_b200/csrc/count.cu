@@ -140,11 +140,26 @@ __global__ void __launch_bounds__(kCountPlanThreads) k_count_plan(CountPlan pl) 
     cb += nc;
     hb += nh;
   }
+  if (threadIdx.x < 4) pl.tickets[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     pl.bucket_base[pl.nbins] = bb;
     pl.chunk_base[pl.nbins] = cb;
     pl.hist_base[pl.nbins] = hb;
   }
+}
+
+// The last index i in [lo, hi] with a[i] <= x (a ascending, a[lo] <= x), by
+// the whole warp: 32 probes a step, so that few dependent loads follow on
+// another.
+GKC_DEV uint64_t warp_last_le(const uint64_t *a, uint64_t lo, uint64_t hi, uint64_t x) {
+  const uint32_t lane = threadIdx.x & 31u;
+  while (lo < hi) {
+    const uint64_t step = (hi - lo) / 32 + 1, at = lo + lane * step;
+    const uint32_t le = __ballot_sync(0xffffffffu, at <= hi && __ldg(a + at) <= x);
+    lo += (uint64_t)(__popc(le) - 1) * step;
+    hi = min(hi, lo + step - 1);
+  }
+  return lo;
 }
 
 GKC_DEV uint32_t find_bin(const uint64_t *base, uint32_t nbins, uint64_t c) {
@@ -156,35 +171,19 @@ GKC_DEV uint32_t find_bin(const uint64_t *base, uint32_t nbins, uint64_t c) {
   return lo;
 }
 
-// Number of k-mers of each bin-ordered superkmer (for the k-mer prefix).
-__global__ void k_skm_nk(const uint64_t *desc, const unsigned long long *n_skm_dev, int k,
-                         unsigned long long *nk) {
-  const uint64_t n = *n_skm_dev;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n;
-       i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t len = (uint32_t)(desc[i] & 0xFFFFFFu);
-    nk[i] = len >= (uint32_t)k ? len - k + 1 : 0;
-  }
-}
-
 // First superkmer of every chunk: the last superkmer of the bin whose k-mer
 // prefix is at most the chunk's first k-mer.  Clears the digit totals, too.
 __global__ void k_chunk_first(ExpandArgs a) {
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
+  const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t n_tot = (uint64_t)a.nbins << a.max_bits;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_tot; i += (uint64_t)gridDim.x * blockDim.x)
-    a.digit_total[i] = 0;
+  for (uint64_t i = t; i < n_tot; i += nt) a.digit_total[i] = 0;
   const uint64_t n_chunks = a.chunk_base[a.nbins];
-  for (uint64_t c = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; c < n_chunks;
-       c += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t b = find_bin(a.chunk_base, a.nbins, c);
+  for (uint64_t c = t >> 5; c < n_chunks; c += nt >> 5) {  // a warp per chunk
+    const uint32_t b = (uint32_t)warp_last_le(a.chunk_base, 0, a.nbins - 1, c);
     const uint64_t q0 = a.bin_kstart[b] + (c - a.chunk_base[b]) * a.chunk_kmers;
-    uint64_t lo = a.bin_start[b], hi = a.bin_start[b + 1] - 1;
-    while (lo < hi) {
-      const uint64_t mid = (lo + hi + 1) >> 1;
-      if (a.koff[mid] <= q0) lo = mid; else hi = mid - 1;
-    }
-    a.chunk_s0[c] = lo;
+    const uint64_t s = warp_last_le(a.koff, a.bin_start[b], a.bin_start[b + 1] - 1, q0);
+    if ((threadIdx.x & 31u) == 0) a.chunk_s0[c] = s;
   }
 }
 
@@ -300,7 +299,7 @@ GKC_DEV uint64_t warp_run(const ExpandArgs &a, uint64_t c, uint32_t b, uint64_t 
   *qb = min(*qa + per, q1);
   const uint64_t lo = a.chunk_s0[c];
   const uint64_t hi = (c + 1 < a.chunk_base[b + 1]) ? a.chunk_s0[c + 1] : a.bin_start[b + 1] - 1;
-  return skm_of_kmer(a.koff, lo, hi, *qa);
+  return warp_last_le(a.koff, lo, hi, *qa);
 }
 
 // ----------------------------------------------------------- 1. histogram
@@ -321,7 +320,7 @@ __global__ void __launch_bounds__(HS_NT) k_bucket_hist(ExpandArgs a) {
   const int key_bits = 2 * a.k;
   const int w = threadIdx.x >> 5;
   for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-    const uint32_t b = find_bin(a.chunk_base, a.nbins, c);
+    const uint32_t b = (uint32_t)warp_last_le(a.chunk_base, 0, a.nbins - 1, c);
     const uint64_t j = c - a.chunk_base[b];
     const int cb = (int)a.bin_bits[b];
     const uint32_t nd = 1u << cb;
@@ -481,7 +480,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
   const int key_bits = 2 * a.k;
   const int tid = threadIdx.x;
   for (uint64_t c = blockIdx.x; c < n_chunks; c += gridDim.x) {
-    const uint32_t b = find_bin(a.chunk_base, a.nbins, c);
+    const uint32_t b = (uint32_t)warp_last_le(a.chunk_base, 0, a.nbins - 1, c);
     const uint64_t j = c - a.chunk_base[b];
     const int cb = (int)a.bin_bits[b];
     const uint32_t nd = (uint32_t)(a.bucket_base[b + 1] - a.bucket_base[b]);  // buckets
@@ -1586,24 +1585,41 @@ __global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_count(SortCount
 }
 
 // Moves each bucket's staged runs to its final offset (the exclusive scan of
-// the buckets' distinct counts), one warp per bucket; bin_out[b] is the
-// offset of the bin's first bucket.
+// the buckets' distinct counts); bin_out[b] is the offset of the bin's first
+// bucket.  A warp per bucket where there are buckets for every warp, else
+// several warps share one; four entries a lane in flight.
 template <typename K>
 __global__ void k_compact_runs(const K *stage_keys, const uint32_t *stage_counts, const uint64_t *bucket_start,
                                const unsigned long long *bucket_d, const uint64_t *bucket_out,
                                const uint64_t *bucket_base, uint32_t nbins, K *out_keys, uint32_t *out_counts,
                                uint64_t *bin_out, const uint32_t *err) {
   if (*err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
+  constexpr int U = 4;
   const uint64_t nb = bucket_base[nbins];
   const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x;
   const uint64_t nt = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t b = t; b <= nbins; b += nt) bin_out[b] = bucket_out[bucket_base[b]];
   const uint32_t lane = threadIdx.x & 31u;
-  for (uint64_t g = t >> 5; g < nb; g += nt >> 5) {
+  const uint64_t warps = nt >> 5;
+  const uint32_t parts = nb == 0 || nb >= warps ? 1 : (uint32_t)min(warps / nb, (uint64_t)32);
+  for (uint64_t x = t >> 5; x < nb * parts; x += warps) {
+    const uint64_t g = x / parts;
     const uint64_t s = bucket_start[g], d = bucket_d[g], o = bucket_out[g];
-    for (uint64_t i = lane; i < d; i += 32) {
-      out_keys[o + i] = stage_keys[s + i];
-      out_counts[o + i] = stage_counts[s + i];
+    for (uint64_t i0 = (x - g * parts) * 32 * U + lane; i0 < d; i0 += (uint64_t)parts * 32 * U) {
+      K kv[U];
+      uint32_t cv[U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (i0 + 32 * u < d) {
+          kv[u] = stage_keys[s + i0 + 32 * u];
+          cv[u] = stage_counts[s + i0 + 32 * u];
+        }
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (i0 + 32 * u < d) {
+          out_keys[o + i0 + 32 * u] = kv[u];
+          out_counts[o + i0 + 32 * u] = cv[u];
+        }
     }
   }
 }

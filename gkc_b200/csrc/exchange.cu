@@ -125,9 +125,8 @@ gkc_status gkc_exchange_pack(gkc_ctx *c, uint32_t n_dest, const uint32_t *bin_lo
   std::vector<uint64_t> hoff(n_dest + 1, 0);
   if (n) {
     k_xchg_nbytes<<<grid_for(c, n), 256, 0, c->st>>>(v.skm_desc, n, nbytes);
-    scan_u64(nbytes, off, n, stmp, c->st);
+    c->launches += 1 + scan_u64(nbytes, off, n, stmp, c->st);  // with the byte-length kernel
     CK(cudaPeekAtLastError());
-    c->launches += 5;  // the byte-length kernel and the scan's four
     // byte offset of every destination's first superkmer (and the total)
     for (uint32_t r = 0; r <= n_dest; r++)
       CK(cudaMemcpyAsync(&hoff[r], off + seg[r], 8, cudaMemcpyDeviceToHost, c->st));

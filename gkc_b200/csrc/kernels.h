@@ -29,21 +29,32 @@ constexpr int kPartThreads = 256;
 constexpr int kPartTile = 3584;
 size_t partition_smem_bytes(int nbins_smem);
 __global__ void k_partition(PartArgs a);
-constexpr int kBinChunk = 8192;          // superkmers per placement chunk
+constexpr int kBinChunk = 8192;          // superkmers per placement chunk (kBinRound where there are few)
 constexpr int kBinRound = 2048;          // superkmers grouped by bin at a time
 constexpr int kBinPlaceThreads = 512;
 size_t bin_place_smem_bytes(uint32_t nbins);
 constexpr int kBinPlaceMaxBins = 2048;   // larger bin counts use k_bin_scatter
-__global__ void k_bin_count(const unsigned long long *n_skm_ptr, const uint32_t *mm, uint32_t nbins,
+__global__ void k_bin_count(const unsigned long long *n_skm_ptr, const uint32_t *mm, uint32_t nbins, uint32_t chunk,
                             uint64_t nch_cap, unsigned long long *mat, const uint32_t *err);
 __global__ void k_bin_place(const unsigned long long *n_skm_ptr, const uint64_t *desc, const uint32_t *mm,
-                            uint32_t nbins, uint64_t nch_cap, const uint64_t *off, uint64_t *out_desc,
+                            uint32_t nbins, uint32_t chunk, uint64_t nch_cap, const uint64_t *off, uint64_t *out_desc,
                             uint32_t *out_mm, const uint32_t *err);
+// Zeroes the partition's counters and the read-start bitmap.
+struct ClearArgs {
+  unsigned long long *cursors;  // 4
+  uint32_t *err;                // 4
+  unsigned long long *bin_nskm, *bin_nkmers;  // nbins + 1
+  uint32_t nbins;
+  uint32_t *rs_bits;
+  uint64_t rs_words;
+};
+__global__ void k_partition_clear(ClearArgs a);
 __global__ void k_read_start_bits(const uint64_t *offs, uint64_t n_reads, uint32_t *bits);
 __global__ void k_bin_scatter(const unsigned long long *n_skm_ptr, const uint64_t *desc,
                               const uint32_t *mm, uint32_t nbins, const uint64_t *bin_start,
                               unsigned long long *bin_fill, uint64_t *out_desc, uint32_t *out_mm,
                               const uint64_t *gpos, uint64_t *out_gpos, const uint32_t *err);
+constexpr int kBinPrefixThreads = 1024;
 __global__ void k_bin_prefix(const unsigned long long *bin_nskm,
                              const unsigned long long *bin_nkmers, uint32_t nbins,
                              uint64_t *bin_start, uint64_t *bin_kstart);
@@ -64,6 +75,7 @@ struct CountPlan {
   uint64_t *bucket_base;       // first bucket of each bin (nbins+1)
   uint64_t *chunk_base;        // first chunk of each bin (nbins+1)
   uint64_t *hist_base;         // first (digit, chunk) entry of each bin (nbins+1)
+  unsigned long long *tickets; // 4, zeroed
 };
 __global__ void k_count_plan(CountPlan pl);
 constexpr int kCountPlanThreads = 1024;
@@ -105,8 +117,6 @@ constexpr int kBucketScanThreads = 1024;
 constexpr int kBucketHistThreads = 256;
 constexpr int kBucketScatterThreads = 1024;
 template <typename K> size_t bucket_scatter_smem_bytes();
-__global__ void k_skm_nk(const uint64_t *desc, const unsigned long long *n_skm_dev, int k,
-                         unsigned long long *nk);
 
 struct SortCountArgs {
   uint32_t nbins;
@@ -148,13 +158,16 @@ template <typename K> constexpr uint32_t bucket_target(uint32_t target) {
 constexpr uint32_t kCoarseMaxBits = 12;
 constexpr uint64_t kChunkKmers = 65536;
 
-// device-wide exclusive scan of uint64 counters (n <= 2^31)
-void scan_u64(const unsigned long long *in, uint64_t *out, uint64_t n, uint64_t *block_tmp,
-              cudaStream_t st);
+// device-wide exclusive scan of uint64 counters (n <= 2^31); out[n] = total.
+// Returns the kernels launched.
+uint32_t scan_u64(const unsigned long long *in, uint64_t *out, uint64_t n, uint64_t *block_tmp, cudaStream_t st);
 size_t scan_u64_tmp_words(uint64_t n);
-// the same over a device-side length min(*n_dev, n_cap); out[n] = total
-void scan_u64_dev(const unsigned long long *in, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
-                  uint64_t *block_tmp, cudaStream_t st);
+// the same over a device-side length min(*n_dev, n_cap)
+uint32_t scan_u64_dev(const unsigned long long *in, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
+                      uint64_t *block_tmp, cudaStream_t st);
+// the same over the k-mers of each superkmer
+uint32_t scan_kmers_dev(const uint64_t *desc, int k, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
+                        uint64_t *block_tmp, cudaStream_t st);
 
 }  // namespace gkc
 

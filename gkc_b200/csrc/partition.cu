@@ -271,6 +271,16 @@ size_t partition_smem_bytes(int nbins_smem) {
   return sizeof(PartSmem) + (size_t)nbins_smem * 2 * sizeof(uint32_t) + 16;
 }
 
+__global__ void k_partition_clear(ClearArgs a) {
+  const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
+  if (t < 4) {
+    a.cursors[t] = 0;
+    a.err[t] = 0;
+  }
+  for (uint64_t i = t; i <= a.nbins; i += nt) a.bin_nskm[i] = a.bin_nkmers[i] = 0;
+  for (uint64_t i = t; i < a.rs_words; i += nt) a.rs_bits[i] = 0;
+}
+
 // Read-start bitmap: bit offs[r]-offs[0] for every read, plus bit nbytes as
 // the end-of-data sentinel.
 __global__ void k_read_start_bits(const uint64_t *offs, uint64_t n_reads, uint32_t *bits) {
@@ -312,11 +322,11 @@ __global__ void k_bin_scatter(const unsigned long long *n_skm_ptr, const uint64_
 }
 
 // Bin placement without global atomics, for nbins <= kBinPlaceMaxBins.
-// k_bin_count: superkmers per (bin, chunk of kBinChunk superkmers), stored
+// k_bin_count: superkmers per (bin, chunk of superkmers), stored
 // bin-major (mat[b * nch_cap + c]) so that one exclusive scan gives every
 // (bin, chunk) its first slot in bin order; k_bin_place then moves each
 // chunk's superkmers with shared-memory cursors per bin.
-__global__ void k_bin_count(const unsigned long long *n_skm_ptr, const uint32_t *mm, uint32_t nbins,
+__global__ void k_bin_count(const unsigned long long *n_skm_ptr, const uint32_t *mm, uint32_t nbins, uint32_t chunk,
                             uint64_t nch_cap, unsigned long long *mat, const uint32_t *err) {
   extern __shared__ uint32_t hcnt[];
   if (*err & (ERR_CAPACITY | ERR_BAD_READ)) return;
@@ -324,8 +334,8 @@ __global__ void k_bin_count(const unsigned long long *n_skm_ptr, const uint32_t 
   for (uint64_t c = blockIdx.x; c < nch_cap; c += gridDim.x) {
     for (uint32_t b = threadIdx.x; b < nbins; b += blockDim.x) hcnt[b] = 0;
     __syncthreads();
-    const uint64_t i1 = min(n, (c + 1) * (uint64_t)kBinChunk);
-    for (uint64_t i = c * (uint64_t)kBinChunk + threadIdx.x; i < i1; i += blockDim.x)
+    const uint64_t i1 = min(n, (c + 1) * (uint64_t)chunk);
+    for (uint64_t i = c * (uint64_t)chunk + threadIdx.x; i < i1; i += blockDim.x)
       atomicAdd(&hcnt[mm[i] % nbins], 1u);
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < nbins; b += blockDim.x) mat[(uint64_t)b * nch_cap + c] = hcnt[b];
@@ -338,7 +348,7 @@ __global__ void k_bin_count(const unsigned long long *n_skm_ptr, const uint32_t 
 // bin's superkmers leave as a run of consecutive slots.
 __global__ void __launch_bounds__(kBinPlaceThreads, 2) k_bin_place(const unsigned long long *n_skm_ptr,
                                                                 const uint64_t *desc, const uint32_t *mm,
-                                                                uint32_t nbins, uint64_t nch_cap,
+                                                                uint32_t nbins, uint32_t chunk, uint64_t nch_cap,
                                                                 const uint64_t *off, uint64_t *out_desc,
                                                                 uint32_t *out_mm, const uint32_t *err) {
   extern __shared__ __align__(16) uint8_t bp_raw[];
@@ -350,12 +360,12 @@ __global__ void __launch_bounds__(kBinPlaceThreads, 2) k_bin_place(const unsigne
   __shared__ uint32_t tmp[64];
   if (*err & (ERR_CAPACITY | ERR_BAD_READ)) return;
   const uint64_t n = *n_skm_ptr;
-  const uint64_t nch = min(nch_cap, (n + kBinChunk - 1) / kBinChunk);
+  const uint64_t nch = min(nch_cap, (n + chunk - 1) / chunk);
   const int tid = threadIdx.x;
   for (uint64_t c = blockIdx.x; c < nch; c += gridDim.x) {
     for (uint32_t b = tid; b < nbins; b += kBinPlaceThreads) cur[b] = off[(uint64_t)b * nch_cap + c];
-    const uint64_t c1 = min(n, (c + 1) * (uint64_t)kBinChunk);
-    for (uint64_t r0 = c * (uint64_t)kBinChunk; r0 < c1; r0 += kBinRound) {
+    const uint64_t c1 = min(n, (c + 1) * (uint64_t)chunk);
+    for (uint64_t r0 = c * (uint64_t)chunk; r0 < c1; r0 += kBinRound) {
       const uint32_t m = (uint32_t)min((uint64_t)kBinRound, c1 - r0);
       for (uint32_t b = tid; b < nbins; b += kBinPlaceThreads) cnt[b] = 0;
       __syncthreads();
@@ -412,19 +422,30 @@ size_t bin_place_smem_bytes(uint32_t nbins) {
   return (size_t)kBinRound * 12 + (size_t)nbins * 16;
 }
 
-// Exclusive scans of the per-bin counters (one thread; nbins is small).
-__global__ void k_bin_prefix(const unsigned long long *bin_nskm, const unsigned long long *bin_nkmers,
-                             uint32_t nbins, uint64_t *bin_start, uint64_t *bin_kstart) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
+// Exclusive scans of the per-bin counters, one CTA (one thread alone took 22-25
+// us at 256 bins).
+__global__ void __launch_bounds__(kBinPrefixThreads) k_bin_prefix(const unsigned long long *bin_nskm,
+                                                                  const unsigned long long *bin_nkmers, uint32_t nbins,
+                                                                  uint64_t *bin_start, uint64_t *bin_kstart) {
+  constexpr int NT = kBinPrefixThreads;
+  __shared__ uint64_t tmp[32];
   uint64_t cs = 0, ck = 0;
-  for (uint32_t b = 0; b < nbins; b++) {
-    bin_start[b] = cs;
-    bin_kstart[b] = ck;
-    cs += bin_nskm[b];
-    ck += bin_nkmers[b];
+  for (uint32_t b0 = 0; b0 < nbins; b0 += NT) {
+    const uint32_t b = b0 + threadIdx.x;
+    uint64_t ts, tk;
+    const uint64_t s = block_exclusive_scan_u64<NT>(b < nbins ? bin_nskm[b] : 0ull, tmp, &ts);
+    const uint64_t kk = block_exclusive_scan_u64<NT>(b < nbins ? bin_nkmers[b] : 0ull, tmp, &tk);
+    if (b < nbins) {
+      bin_start[b] = cs + s;
+      bin_kstart[b] = ck + kk;
+    }
+    cs += ts;
+    ck += tk;
   }
-  bin_start[nbins] = cs;
-  bin_kstart[nbins] = ck;
+  if (threadIdx.x == 0) {
+    bin_start[nbins] = cs;
+    bin_kstart[nbins] = ck;
+  }
 }
 
 }  // namespace gkc
