@@ -154,7 +154,6 @@ __global__ void __launch_bounds__(TL_NT, 3) k_window_minimizers(WinArgs a, uint3
 constexpr int SUB_NT = TL_NT;
 constexpr int SUB_WORDS = TL_WORDS;  // selection words per tile
 constexpr int SUB_TILE = TL_NW;      // windows per tile
-static_assert(SUB_WORDS * 2 <= SUB_NT, "two threads per selection word");
 
 // Tile t covers windows [t*SUB_TILE, (t+1)*SUB_TILE): selection bitmap and count.
 __global__ void __launch_bounds__(SUB_NT, 4) k_sub_flags(WinArgs a, uint32_t mod, uint32_t *sel,
@@ -192,34 +191,53 @@ __global__ void __launch_bounds__(SUB_NT, 4) k_sub_flags(WinArgs a, uint32_t mod
   }
 }
 
+// The 2k bits of the k bases from tile base l on (a byte that is no base
+// counts as T, as in the packed superkmers).
 template <typename K>
-GKC_DEV K window_canonical(const uint8_t *reads, uint64_t i, int k) {
+GKC_DEV K tile_kmer(const TileBases &S, int l, int k) {
+  const int j = l >> 4;
+  const uint32_t sh = 2 * (uint32_t)(l & 15);
+  uint32_t w[sizeof(K) / 4 + 1];
+#pragma unroll
+  for (int t = 0; t <= (int)sizeof(K) / 4; t++) w[t] = S.pk[j + t].x;
   K x = 0;
-  for (int j = 0; j < k; j++) x = (x << 2) | (K)(code_of_byte(reads[i + j]) & 3u);  // N -> T
-  const K r = revcomp_k<K>(x, k);
-  return x < r ? x : r;
+#pragma unroll
+  for (int t = 0; t < (int)sizeof(K) / 4; t++) x = (x << 32) | (K)__funnelshift_l(w[t + 1], w[t], sh);
+  return x >> (8 * (int)sizeof(K) - 2 * k);
 }
 
-// Writes (canonical key, window start) of the selected windows in window order.
+// Writes (canonical key, window start) of the selected windows in window
+// order: a warp takes its words of the tile, each lane the k-mer of its own
+// window from the tile's packed bases.
 template <typename K>
-__global__ void __launch_bounds__(SUB_NT) k_sub_write(const uint8_t *reads, uint64_t n_bytes, const uint32_t *sel,
-                                                      const uint64_t *tile_off, int k, K *keys, uint32_t *posv) {
-  __shared__ uint32_t tmp[64];
-  const uint64_t t = blockIdx.x;
-  // thread x owns half x & 1 of the tile's selection word x / 2
-  const uint32_t x = threadIdx.x;
-  uint32_t b = x < 2 * SUB_WORDS ? sel[t * SUB_WORDS + (x >> 1)] : 0u;
-  b = (x & 1) ? (b >> 16) : (b & 0xFFFFu);
-  uint32_t total;
-  uint64_t o = tile_off[t] + block_exclusive_scan<SUB_NT>(__popc(b), tmp, &total);
-  const uint64_t i0 = t * SUB_TILE + 16 * (uint64_t)x;
-  while (b) {
-    const int q = __ffs(b) - 1;
-    b &= b - 1;
-    const uint64_t i = i0 + q;
-    keys[o] = window_canonical<K>(reads, i, k);
-    posv[o] = (uint32_t)i;
-    o++;
+__global__ void __launch_bounds__(SUB_NT) k_sub_write(WinArgs a, const uint32_t *sel, const uint64_t *tile_off,
+                                                      K *keys, uint32_t *posv, uint64_t n_tiles) {
+  __shared__ TileBases S;
+  __shared__ uint32_t cnt[TL_WARPS];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * TL_TW;
+  for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
+    const int64_t G0 = (int64_t)(tile * TL_NW);
+    uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
+    if (threadIdx.x < TL_GROUPS) bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, G0, threadIdx.x);
+    const uint32_t mine = lane < TL_TW ? sel[tile * SUB_WORDS + w0 + lane] : 0u;
+    tile_store(S, bytes, a.bits, a.bit_words, G0);
+    const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(mine));
+    if (lane == 0) cnt[warp] = c;
+    __syncthreads();
+    uint64_t o = tile_off[tile];
+    for (int x = 0; x < warp; x++) o += cnt[x];
+    for (int r = 0; r < TL_TW; r++) {
+      const uint32_t f = __shfl_sync(0xffffffffu, mine, r);
+      if ((f >> lane) & 1u) {
+        const int l = 32 * (w0 + r) + lane;
+        const K x = tile_kmer<K>(S, l, a.k), rc = revcomp_k<K>(x, a.k);
+        const uint64_t at = o + __popc(f & ((1u << lane) - 1u));
+        keys[at] = x < rc ? x : rc;
+        posv[at] = (uint32_t)(G0 + l);
+      }
+      o += __popc(f);
+    }
+    __syncthreads();  // before the next tile's bases
   }
 }
 
@@ -327,7 +345,8 @@ static gkc_status subsample_t(gkc_ctx *c, const gkc_params *prm, uint32_t mod, c
   WS(out_keys, K, "win_out_keys", n + 16);
   WS(pos_off, uint64_t, "win_pos_off", n + 2);
   if (n) {
-    k_sub_write<K><<<(unsigned)tiles, SUB_NT, 0, c->st>>>(reads, n_bytes, sel, toff, prm->k, keys, pos);
+    k_sub_write<K><<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 8), SUB_NT, 0, c->st>>>(
+        win_args(c, prm, reads, n_bytes, d_offs, n_reads, bits), sel, toff, keys, pos, tiles);
     CK(cudaPeekAtLastError());
     WS(os_hist, unsigned long long, "win_os_hist", 16 * 256);
     WS(os_lb, unsigned long long, "win_os_lookback", onesweep_lookback_words(n + 1));
