@@ -440,7 +440,7 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
 
   WS(desc, uint64_t, "skm_desc_tile", cap_skm);
   WS(mm, uint32_t, "skm_mm_tile", cap_skm);
-  WS(packed, uint8_t, "packed", cap_bytes);
+  WS(packed, uint8_t, "packed", cap_bytes + 16);  // k-mers are cut from whole words
 
   PartArgs a;
   memset(&a, 0, sizeof(a));

@@ -41,26 +41,24 @@ namespace gkc {
 // ------------------------------------------------------------ key digits
 
 // Top 32 bits of a 2k-bit key, left-aligned when the key is shorter.
-template <typename K>
-GKC_DEV uint32_t key_top32(K x, int key_bits) {
-  return key_bits >= 32 ? (uint32_t)(x >> (key_bits - 32)) : (uint32_t)((uint64_t)x << (32 - key_bits));
+GKC_DEV uint32_t key_top32(uint64_t x, int key_bits) {
+  // (the clamping shift gives the high word at key_bits = 64)
+  return key_bits >= 32 ? __funnelshift_rc((uint32_t)x, (uint32_t)(x >> 32), key_bits - 32)
+                        : (uint32_t)x << (32 - key_bits);
 }
+GKC_DEV uint32_t key_top32(u128 x, int key_bits) { return (uint32_t)(x >> (key_bits - 32)); }  // k > 32
 
 // Order-preserving map of a canonical key's top 32 bits t that spreads
 // canonical keys evenly: the canonical key of a uniform k-mer is the smaller
 // of two near-independent uniform values, whose distribution function is
 // 1 - (1 - u)^2; v = 2^32 (1 - (1 - t / 2^32)^2), non-decreasing in t.
-GKC_DEV uint32_t eq_map(uint32_t t) {
-  if (t == 0) return 0;
-  const uint64_t s = (1ull << 32) - t;  // 1 .. 2^32 - 1
-  return (uint32_t)((0ull - s * s) >> 32);
-}
+GKC_DEV uint32_t eq_map(uint32_t t) { return ~__umulhi(~t, ~t); }
 
-GKC_DEV uint32_t coarse_of(uint32_t v, int cb) { return cb ? v >> (32 - cb) : 0u; }
+GKC_DEV uint32_t coarse_of(uint32_t v, int cb) { return __funnelshift_rc(v, 0u, 32 - cb); }  // 0 at cb = 0
 
 template <typename K>
 GKC_DEV uint32_t coarse_digit(K x, int key_bits, int cb) {
-  return coarse_of(eq_map(key_top32<K>(x, key_bits)), cb);
+  return coarse_of(eq_map(key_top32(x, key_bits)), cb);
 }
 
 // Bits of a key type, its leading zeros, and the sb bits that follow the
@@ -199,93 +197,123 @@ GKC_DEV uint64_t skm_of_kmer(const uint64_t *koff, uint64_t lo, uint64_t hi, uin
   return lo;
 }
 
-// Packed bases are read as aligned 8-byte words, byte-swapped so that the
-// stream's first base is in the top bits (2 bits per base, MSB first within
-// a byte).  A word is loaded only when it holds a wanted base, so reads end
-// within 7 bytes past the last superkmer.
-GKC_DEV uint64_t be_word(const uint8_t *packed, uint64_t w) {
-  const uint64_t x = __ldg(reinterpret_cast<const unsigned long long *>(packed) + w);
-  return ((uint64_t)__byte_perm((uint32_t)x, 0, 0x0123) << 32) | __byte_perm((uint32_t)(x >> 32), 0, 0x0123);
-}
-
-// nb <= 64 bits of the stream from bit position pos, left-aligned.
-GKC_DEV uint64_t stream_bits(const uint8_t *packed, uint64_t pos, int nb) {
-  const uint64_t w = pos >> 6;
-  const int r = (int)(pos & 63);
-  uint64_t v = be_word(packed, w) << r;
-  if (r + nb > 64) v |= be_word(packed, w + 1) >> (64 - r);
-  return v;
-}
-
-// The 2k bits of bases [o, o+k) of a packed superkmer at byte `off`.
+// A k-mer's 2k bits as 32-bit words of the packed bases (2 bits per base, MSB
+// first within a byte): its first base is in word 0, r bits below the top once
+// the word's bytes are swapped.  All words are loaded, so reads end within 16
+// bytes past the last superkmer (every packed buffer has them).
+template <typename K> struct PackedWords {
+  static constexpr int N = sizeof(K) / 4 + 1;
+  uint32_t w[N];
+  uint32_t r;
+};
 template <typename K>
-GKC_DEV K extract_kmer(const uint8_t *packed, uint64_t off, uint32_t o, int k);
-
-template <>
-GKC_DEV uint64_t extract_kmer<uint64_t>(const uint8_t *packed, uint64_t off, uint32_t o, int k) {
-  return stream_bits(packed, 8 * off + 2 * (uint64_t)o, 2 * k) >> (64 - 2 * k);
+GKC_DEV void load_packed(PackedWords<K> &p, const uint8_t *packed, uint64_t off, uint32_t o, bool valid) {
+  const uint64_t at = off + (o >> 2);
+  const uint32_t *src = reinterpret_cast<const uint32_t *>(packed + (at & ~3ull));
+  p.r = 8 * ((uint32_t)at & 3u) + 2 * (o & 3u);
+#pragma unroll
+  for (int t = 0; t < PackedWords<K>::N; t++) p.w[t] = valid ? __ldg(src + t) : 0u;
 }
 
-template <>
-GKC_DEV u128 extract_kmer<u128>(const uint8_t *packed, uint64_t off, uint32_t o, int k) {
-  const uint64_t pos = 8 * off + 2 * (uint64_t)o;
-  const int nb = 2 * k;  // 66 .. 128
-  const uint64_t hi = stream_bits(packed, pos, 64);
-  const uint64_t lo = stream_bits(packed, pos + 64, nb - 64);
-  const u128 v = ((u128)hi << 64) | lo;
-  return v >> (128 - nb);
+// Reverse complement of 16 bases.
+GKC_DEV uint32_t revcomp32(uint32_t x) {
+  const uint32_t y = __brev(x);
+  return 2 * (~y & 0x55555555u) + (~(y >> 1) & 0x55555555u);
+}
+// The canonical key: the smaller of the k-mer and its reverse complement.  The
+// reverse complement of the whole words holds that of the k-mer in its low 2k
+// bits.
+GKC_DEV uint64_t packed_canonical(const PackedWords<uint64_t> &p, int k) {
+  const uint32_t b0 = __byte_perm(p.w[0], 0, 0x0123), b1 = __byte_perm(p.w[1], 0, 0x0123),
+                 b2 = __byte_perm(p.w[2], 0, 0x0123);
+  const uint32_t hi = __funnelshift_l(b1, b0, p.r), lo = __funnelshift_l(b2, b1, p.r);
+  const uint64_t rc = ((uint64_t)revcomp32(lo) << 32) | revcomp32(hi);
+  uint64_t x;
+  const int s = 64 - 2 * k;
+  if (s <= 32) x = ((uint64_t)__funnelshift_rc(hi, 0u, s) << 32) | __funnelshift_rc(lo, hi, s);
+  else x = hi >> (s - 32);
+  const uint64_t r = rc & (~0ull >> s);
+  return x < r ? x : r;
+}
+GKC_DEV u128 packed_canonical(const PackedWords<u128> &p, int k) {
+  uint32_t b[5], w[4];
+#pragma unroll
+  for (int t = 0; t < 5; t++) b[t] = __byte_perm(p.w[t], 0, 0x0123);
+#pragma unroll
+  for (int t = 0; t < 4; t++) w[t] = __funnelshift_l(b[t + 1], b[t], p.r);
+  const uint64_t hi = ((uint64_t)w[0] << 32) | w[1], lo = ((uint64_t)w[2] << 32) | w[3];
+  const uint64_t rhi = ((uint64_t)revcomp32(w[3]) << 32) | revcomp32(w[2]),
+                 rlo = ((uint64_t)revcomp32(w[1]) << 32) | revcomp32(w[0]);
+  const int s = 128 - 2 * k;  // 0 .. 62
+  const u128 x = (((u128)hi << 64) | lo) >> s;
+  const u128 r = ((u128)(rhi & (~0ull >> s)) << 64) | rlo;
+  return x < r ? x : r;
 }
 
 // The k-mers [qa, qb) of one bin, taken by the calling warp 32 at a time,
-// lane i the i-th of each group: each lane finds its superkmer among the 32
-// from the group's first one (a search over their k-mer ends relative to the
-// group's first k-mer, held one per lane), extracts its k-mer and passes the
-// canonical key to emit(key, valid) (called by every lane; valid is false
-// past qb).  s0 is the superkmer holding k-mer qa, s_end the bin's end
-// (k-mer offsets up to koff[s_end] are read).  The next group's offsets are
-// loaded before this group's k-mers are extracted.
+// lane i the i-th of each group: the ends of the 32 superkmers from the
+// group's first one on, held one per lane, become a bitmap of the group's
+// positions, in which each lane finds its superkmer (bits up to its own) and
+// the k-mer's index in it (the distance to the last of them).  The canonical
+// keys go to emit(key, valid) (called by every lane; valid is false past qb).
+// s0 is the superkmer holding k-mer qa, s_end the bin's end (k-mer offsets up
+// to koff[s_end] are read).
+//
+// What bounds it is instruction issue and the latency of the packed bases,
+// which lie in tile order: positions are 32-bit, relative to qa, the next
+// group's ends and descriptors are loaded and this group's packed words
+// requested before the last group's k-mers are built.
 template <typename K, typename Emit>
 GKC_DEV void warp_kmers(const ExpandArgs &a, uint64_t qa, uint64_t qb, uint64_t s0, uint64_t s_end, Emit &&emit) {
   const uint32_t lane = threadIdx.x & 31u;
   const int k = a.k;
-  uint64_t base = s0;
-  uint64_t e = base + 1 + lane <= s_end ? __ldg(a.koff + base + 1 + lane) : ~0ull;  // end of superkmer base + lane
-  uint64_t kb = __ldg(a.koff + base);                                                // start of superkmer base
-  for (uint64_t q0 = qa; q0 < qb; q0 += 32) {
-    // superkmer `base` holds q0 or ends at it, so e >= q0
-    const uint32_t rel = (uint32_t)min(e - q0, (uint64_t)64);
-    uint32_t cnt = 0;  // superkmers from `base` on that end at or before q0 + lane
-#pragma unroll
-    for (uint32_t st = 16; st > 0; st >>= 1)
-      if (__shfl_sync(0xffffffffu, rel, cnt + st - 1) <= lane) cnt += st;
-    const uint32_t prev = __shfl_sync(0xffffffffu, rel, cnt ? cnt - 1 : 0);
-    const uint32_t r31 = __shfl_sync(0xffffffffu, rel, 31);
-    const bool valid = q0 + lane < qb;
-    uint64_t s = base + cnt;
-    uint64_t o = cnt ? (uint64_t)(lane - prev) : q0 - kb + lane;  // the k-mer's index in its superkmer
-    if (valid && lane >= r31) {  // 32 superkmers (some without k-mers) end before this k-mer
-      const uint64_t q = q0 + lane;
-      s = skm_of_kmer(a.koff, base + 32, s_end - 1, q);
-      o = q - __ldg(a.koff + s);
+  const uint32_t n = (uint32_t)(qb - qa);  // at most a chunk
+  // superkmers are counted from s0; their k-mer offsets differ from qa by less
+  // than 2^32 (a bin holds fewer k-mers), so the low words are enough
+  const uint32_t *koff = reinterpret_cast<const uint32_t *>(a.koff + s0);
+  const unsigned long long *desc = reinterpret_cast<const unsigned long long *>(a.desc + s0);
+  const uint32_t ns = (uint32_t)(s_end - s0), qa32 = (uint32_t)qa;
+  uint32_t base = 0;
+  // end of superkmer base + lane, and its descriptor
+  auto end_of = [&](uint32_t b) -> uint32_t { return b + lane < ns ? __ldg(koff + 2 * (b + lane) + 2) - qa32 : ~0u; };
+  auto desc_of = [&](uint32_t b) -> uint64_t { return b + lane < ns ? __ldg(desc + b + lane) : 0ull; };
+  uint32_t e = end_of(0);
+  uint64_t ds = desc_of(0);
+  uint32_t kb = __ldg(koff) - qa32;  // start of superkmer base (modulo 2^32: at most its length before qa)
+  const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);
+  PackedWords<K> pw;
+  bool pvalid = false;
+  for (uint32_t q = 0; q < n; q += 32) {
+    const uint32_t rel = e - q;  // superkmer `base` holds q or ends at it, so e >= q
+    const uint32_t inside = __ballot_sync(0xffffffffu, rel < 32u);
+    const uint32_t ends = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
+    const bool valid = q + lane < n;
+    uint64_t my;
+    uint32_t o;
+    if (__popc(ends) == __popc(inside) && inside != 0xFFFFFFFFu) {
+      const uint32_t le = ends & upto;
+      // the lane's superkmer: as many from `base` on as end at or before it
+      my = __shfl_sync(0xffffffffu, ds, __popc(le));
+      o = le ? lane + __clz((int)le) - 31 : q + lane - kb;
+      base += __popc(ends);  // holds the next group's first k-mer or precedes it
+      if (ends) kb = q + 31 - __clz((int)ends);
+    } else {
+      // superkmers without k-mers, or more than 31 ends: searched one by one
+      const uint64_t x = qa + min(q + lane, n - 1), s = skm_of_kmer(a.koff, s0 + base, s_end - 1, x);
+      o = (uint32_t)(x - __ldg(a.koff + s));
+      my = __ldg(a.desc + s);
+      base = (uint32_t)(__shfl_sync(0xffffffffu, s, 31) - s0);
+      kb = __ldg(koff + 2 * base) - qa32;
     }
-    const uint64_t nbase = __shfl_sync(0xffffffffu, s, 31);  // holds the next group's first k-mer or precedes it
-    uint64_t ne = e, nkb = kb;
-    if (q0 + 32 < qb) {
-      ne = nbase + 1 + lane <= s_end ? __ldg(a.koff + nbase + 1 + lane) : ~0ull;
-      nkb = __ldg(a.koff + nbase);
-    }
-    K key = 0;
-    if (valid) {
-      const uint64_t off = __ldg(a.desc + s) >> 24;
-      const K x = extract_kmer<K>(a.packed, off, (uint32_t)o, k);
-      const K r = revcomp_k<K>(x, k);
-      key = x < r ? x : r;
-    }
-    emit(key, valid);
-    base = nbase;
-    e = ne;
-    kb = nkb;
+    PackedWords<K> nw;
+    load_packed<K>(nw, a.packed, my >> 24, o, valid);
+    e = end_of(base);
+    ds = desc_of(base);
+    if (q) emit(pvalid ? packed_canonical(pw, k) : (K)0, pvalid);
+    pw = nw;
+    pvalid = valid;
   }
+  emit(pvalid ? packed_canonical(pw, k) : (K)0, pvalid);
 }
 
 // The k-mers of chunk c (bin b, j-th chunk of the bin) taken by warp w of W:

@@ -15,11 +15,11 @@ namespace gkc {
 constexpr int OS_NT = 256;
 constexpr int OS_WARPS = OS_NT / 32;
 constexpr int OS_RADIX = 256;
-// Keys per thread: a tile's keys fill 32 KB of shared memory, where they are
-// put in digit order before they are written.
-template <typename K> constexpr int os_items() { return sizeof(K) == 8 ? 16 : 8; }
-template <typename K> constexpr int os_tile() { return OS_NT * os_items<K>(); }
-constexpr int OS_TILE_MIN = OS_NT * 8;
+// Keys per thread: a tile's keys are put in digit order in shared memory
+// before they are written.  8 leave three CTAs on an SM (16 8-byte keys: two,
+// and the merged list of 60 M bases took 4.5 ms, not 4.3).
+constexpr int OS_ITEMS = 8;
+constexpr int OS_TILE = OS_NT * OS_ITEMS;
 constexpr int OS_WINDOW = 4;  // earlier tiles looked at together
 
 constexpr unsigned long long OS_AGG = 1ull << 62, OS_PRE = 2ull << 62;
@@ -97,12 +97,12 @@ __global__ void k_os_digit_offsets(unsigned long long *hist, int passes) {
 // from registers and one earlier tile a step: 424 us a pass of 13.9 M 16-byte
 // keys with values.)
 template <typename K, bool KV>
-__global__ void __launch_bounds__(OS_NT, sizeof(K) == 8 ? 2 : 3) k_os_pass(const K *in, K *out, const uint32_t *vin,
+__global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const uint32_t *vin,
                                                                            uint32_t *vout, const uint64_t *n_dev,
                                                                            int pass, const unsigned long long *digit_base,
                                                                            unsigned long long *lookback,
                                                                            unsigned long long *ticket, uint32_t *err) {
-  constexpr int ITEMS = os_items<K>(), TILE = os_tile<K>();
+  constexpr int ITEMS = OS_ITEMS, TILE = OS_TILE;
   __shared__ __align__(16) uint8_t sbuf[TILE * sizeof(K)];  // the tile in digit order; then its values
   __shared__ uint32_t warp_cnt[OS_WARPS][OS_RADIX];
   __shared__ uint32_t toff[OS_RADIX];               // first tile position of each digit
@@ -237,7 +237,7 @@ static OnesweepStatus onesweep_run(K *keys, K *alt, uint32_t *vals, uint32_t *va
                                    uint64_t n_max, int key_bits, OnesweepScratch s, cudaStream_t st,
                                    uint32_t *launches) {
   const int passes = (key_bits + 7) / 8;
-  const uint64_t tiles = (n_max + os_tile<K>() - 1) / os_tile<K>();
+  const uint64_t tiles = (n_max + OS_TILE - 1) / OS_TILE;
   cudaMemsetAsync(s.hist, 0, sizeof(unsigned long long) * 16 * OS_RADIX, st);
   unsigned grid_h = (unsigned)std::min<uint64_t>(std::max<uint64_t>(1, (n_max + OS_NT * 8 - 1) / (OS_NT * 8)), 148 * 16);
   k_os_histogram<K><<<grid_h, OS_NT, 0, st>>>(keys, n_dev, passes, s.hist);
@@ -276,7 +276,7 @@ OnesweepStatus onesweep_sort_kv(K *keys, K *alt, uint32_t *vals, uint32_t *valt,
 }
 
 size_t onesweep_lookback_words(uint64_t n_max) {
-  return ((n_max + OS_TILE_MIN - 1) / OS_TILE_MIN + 1) * OS_RADIX;
+  return ((n_max + OS_TILE - 1) / OS_TILE + 1) * OS_RADIX;
 }
 
 template OnesweepStatus onesweep_sort<uint64_t>(uint64_t *, uint64_t *, const uint64_t *, uint64_t,

@@ -445,7 +445,7 @@ constexpr uint64_t kMaxSkm = 1ull << 17;    // superkmers per call
 constexpr int kMaxDevices = 64;
 
 constexpr uint64_t round_up(uint64_t w) { return (w + 31) & ~31ull; }  // 256-byte steps
-constexpr uint64_t kOsTileMin = 2048;  // keys of the smallest onesweep tile (checked at set-up)
+constexpr uint64_t kOsTile = 2048;  // keys per onesweep tile (checked at set-up)
 constexpr uint64_t kRleBlocks = (kMaxKmers + RLE_TILE - 1) / RLE_TILE + 1;
 // word offsets of the parts of the array
 constexpr uint64_t W_SORT = 0;
@@ -458,7 +458,7 @@ constexpr uint64_t W_DESC = W_KOFF + round_up(kMaxSkm + 2);
 constexpr uint64_t W_STMP = W_DESC + round_up(kMaxSkm + 2);
 constexpr uint64_t W_HIST = W_STMP + round_up(kMaxSkm / 1024 + 16);
 constexpr uint64_t W_LB = W_HIST + round_up(16 * 256);
-constexpr uint64_t W_TICKET = W_LB + round_up(((kMaxKmers + kOsTileMin - 1) / kOsTileMin + 1) * 256);
+constexpr uint64_t W_TICKET = W_LB + round_up(((kMaxKmers + kOsTile - 1) / kOsTile + 1) * 256);
 constexpr uint64_t W_ERR = W_TICKET + 32;
 constexpr uint64_t W_RBLK = W_ERR + 32;
 constexpr uint64_t W_ROFF = W_RBLK + round_up(kRleBlocks + 1);
