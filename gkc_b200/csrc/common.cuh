@@ -6,6 +6,7 @@
 typedef unsigned __int128 u128;
 
 #define GKC_DEV __device__ __forceinline__
+#define GKC_HOST_DEV __host__ __device__ __forceinline__
 
 namespace gkc {
 

@@ -26,7 +26,7 @@ struct PartArgs {
 };
 
 constexpr int kPartThreads = 256;
-constexpr int kPartTile = 3584;
+constexpr int kPartTile = 3328;  // windows of the smallest tile
 size_t partition_smem_bytes(int nbins_smem);
 __global__ void k_partition(PartArgs a);
 constexpr int kBinChunk = 8192;          // superkmers per placement chunk (kBinRound where there are few)

@@ -24,20 +24,23 @@ namespace gkc {
 
 constexpr int PT_NT = TL_NT;
 constexpr int PT_PRE = 32;                       // local index of the first core window
-constexpr int PT_T = kPartTile;                  // core windows per tile; the rest find superkmer ends
+constexpr int PT_HALO = 224;                     // windows after the core, to find superkmer ends
+constexpr int PT_TMAX = TL_NW_MAX - PT_PRE - PT_HALO;  // core windows per tile (fewer where omega > 33)
 constexpr int PT_STG = 6144;                     // packed bytes of a tile staged in shared memory
-static_assert(PT_T % 32 == 0 && PT_PRE + PT_T < TL_NW && kPartThreads == TL_NT, "whole words, a halo after the core");
+static_assert(PT_TMAX % 32 == 0 && kPartThreads == TL_NT, "whole words");
+static_assert(kPartTile == TL_WARPS * 28 * TL_W - PT_PRE - PT_HALO, "the smallest tile");
 
 struct PartSmem {
   TileBases t;
-  uint32_t brkw[TL_WORDS];         // bit i: window i starts a superkmer or lies in none
-  uint32_t smm[PT_T];              // minimizer of each core superkmer
-  uint32_t boff[PT_T];             // its byte offset in the tile
-  uint16_t spos[PT_T];             // its first window
-  uint16_t send[PT_T];             // its end window (PT_EXT: ext_end)
+  uint32_t brkw[TL_NW_MAX / 32];   // bit i: window i starts a superkmer or lies in none
+  uint32_t smm[PT_TMAX];              // minimizer of each core superkmer
+  uint32_t boff[PT_TMAX];             // its byte offset in the tile
+  uint16_t spos[PT_TMAX];             // its first window
+  uint16_t send[PT_TMAX];             // its end window (PT_EXT: ext_end)
   alignas(16) uint8_t stg[PT_STG]; // the tile's packed superkmers before they are written out (read as uint4)
   uint32_t scan_tmp[64];
-  uint32_t lastmm[TL_WARPS], wcnt[TL_WARPS];
+  uint32_t lastmm[TL_WARPS], lastv[TL_WARPS], wcnt[TL_WARPS];
+  uint16_t redo[TL_WARPS][32];
   int ext_end;                     // local end window of an extended last superkmer
   unsigned long long base_skm, base_byte;
 };
@@ -53,7 +56,8 @@ __global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int k = a.k, p = a.p, omega = a.k - a.p + 1;
   if (a.nbytes_dev) a.nbytes = *a.nbytes_dev;
-  const uint64_t n_tiles = (a.nbytes + PT_T - 1) / PT_T;
+  const int strip = tile_strip(omega), NW = TL_WARPS * strip, T = NW - PT_PRE - PT_HALO;
+  const uint64_t n_tiles = (a.nbytes + T - 1) / T;
 
   // per-CTA bin histograms (small bin counts only): superkmers, k-mers
   uint32_t *h_skm = reinterpret_cast<uint32_t *>(smem_raw + sizeof(PartSmem));
@@ -62,62 +66,74 @@ __global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
 
   uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
   if (blockIdx.x < n_tiles && tid < TL_GROUPS)
-    bytes = tile_fetch(a.reads, a.nbytes, a.aligned16, (int64_t)blockIdx.x * PT_T - PT_PRE, tid);
+    bytes = tile_fetch(a.reads, a.nbytes, a.aligned16, (int64_t)blockIdx.x * T - PT_PRE, tid);
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int64_t G0 = (int64_t)(tile * PT_T) - PT_PRE;  // global position of local 0 (32-aligned)
+    const int64_t G0 = (int64_t)(tile * T) - PT_PRE;  // global position of local 0 (32-aligned)
     tile_store(S.t, bytes, a.rs_bits, a.rs_words, G0);
     if (tid == 0) S.ext_end = -1;
     __syncthreads();
     if (tile + gridDim.x < n_tiles && tid < TL_GROUPS)
-      bytes = tile_fetch(a.reads, a.nbytes, a.aligned16, (int64_t)((tile + gridDim.x) * PT_T) - PT_PRE, tid);
+      bytes = tile_fetch(a.reads, a.nbytes, a.aligned16, (int64_t)((tile + gridDim.x) * T) - PT_PRE, tid);
 
-    // ---- minimizers: lane l, register r hold window 32 (w0 + r) + l ----
-    const int w0 = warp * TL_TW;
-    uint32_t vw = 0, tw = 0;  // lane r + 1: word w0 + r; lane 0: the word before
-    if (lane <= TL_TW && w0 + lane >= 1)
-      tile_valid(S.t, w0 + lane - 1, G0, 0, (int64_t)a.nbytes, k, &vw, &tw);
-    uint32_t m[TL_TW + 2], none[1];
-    switch (a.filter) {
-      case FILTER_ALL: tile_minima<FILTER_ALL, false>(S.t, w0, p, omega, m, none); break;
-      case FILTER_NEW: tile_minima<FILTER_NEW, false>(S.t, w0, p, omega, m, none); break;
-      case FILTER_SIGNATURE: tile_minima<FILTER_SIGNATURE, false>(S.t, w0, p, omega, m, none); break;
-      default: tile_minima<FILTER_NEW2, false>(S.t, w0, p, omega, m, none); break;
+    // ---- minimizers: lane l holds windows P .. P + 15 ----
+    const int P0 = warp * strip, P = P0 + TL_W * lane;
+    const bool own = TL_W * lane < strip;  // the strip's last lanes only feed the others
+    uint32_t vw = 0, tw = 0;               // bit i: window P + i lies in a read; touches a byte that is no base
+    if (own) {
+      tile_valid(S.t, P >> 5, G0, 0, (int64_t)a.nbytes, k, &vw, &tw);
+      vw = (vw >> (P & 31)) & 0xFFFFu;
+      tw = (tw >> (P & 31)) & vw;
     }
-    if (__any_sync(0xffffffffu, (tw & vw) != 0u)) {
+    uint32_t m[TL_W], none[1];
+    tile_minima<false>(S.t, P0, k, p, a.filter, m, none);
+    if (__any_sync(0xffffffffu, tw != 0u))
+      tile_redo(tw, P0, S.redo[warp],
+                [&](int l, uint32_t &v, uint32_t &) {
+                  v = exact_window_minimizer([&](int i) { return tile_code(S.t, l + i); }, k, p, a.filter);
+                },
+                [&](int i, uint32_t v, uint32_t) {
 #pragma unroll
-      for (int r = 0; r < TL_TW; r++) {
-        const uint32_t t = __shfl_sync(0xffffffffu, tw & vw, r + 1);
-        if ((t >> lane) & 1u) {
-          const int l = 32 * (w0 + r) + lane;
-          m[r] = exact_window_minimizer([&](int i) { return tile_code(S.t, l + i); }, k, p, a.filter);
-        }
-      }
+                  for (int x = 0; x < TL_W; x++)
+                    if (x == i) m[x] = v;
+                });
+    if (P + TL_W == P0 + strip) {
+      S.lastmm[warp] = m[TL_W - 1];
+      S.lastv[warp] = vw >> 15;
     }
-    if (lane == 31) S.lastmm[warp] = m[TL_TW - 1];
     __syncthreads();
 
-    // ---- breaks and superkmer starts, 32 windows a word ----
-    uint32_t st[TL_TW], cnt = 0;
+    // ---- breaks and superkmer starts, 16 windows a lane ----
+    uint32_t st;
     {
-      uint32_t carry = warp ? S.lastmm[warp - 1] : 0u;  // minimizer of the window before
-      uint32_t pv = __shfl_sync(0xffffffffu, vw, 0);
-#pragma unroll
-      for (int r = 0; r < TL_TW; r++) {
-        const uint32_t before = __shfl_sync(0xffffffffu, m[r], (lane + 31) & 31);
-        const uint32_t diff = __ballot_sync(0xffffffffu, m[r] != (lane ? before : carry));
-        carry = before;  // lane 0: this word's last window
-        const uint32_t v = __shfl_sync(0xffffffffu, vw, r + 1);
-        const uint32_t start = v & (S.t.rsw[w0 + r] | diff | ~((v << 1) | (pv >> 31)));
-        pv = v;
-        if (lane == 0) S.brkw[w0 + r] = start | ~v;
-        const bool core = w0 + r >= PT_PRE / 32 && w0 + r < (PT_PRE + PT_T) / 32;
-        st[r] = core ? start : 0u;
-        cnt += __popc(st[r]);
+      uint32_t before = __shfl_up_sync(0xffffffffu, m[TL_W - 1], 1), pv = __shfl_up_sync(0xffffffffu, vw, 1) >> 15;
+      if (lane == 0) {
+        before = warp ? S.lastmm[warp - 1] : 0u;
+        pv = warp ? S.lastv[warp - 1] : 0u;
       }
+      uint32_t diff = 0;
+#pragma unroll
+      for (int i = 0; i < TL_W; i++) {
+        if (m[i] != before) diff |= 1u << i;
+        before = m[i];
+      }
+      const uint32_t rs = own ? S.t.rsw[P >> 5] >> (P & 31) : 0u;
+      st = vw & (rs | diff | ~((vw << 1) | pv));
+      const uint32_t brk = (st | ~vw) & 0xFFFFu;
+      const uint32_t other = __shfl_down_sync(0xffffffffu, brk, 1);
+      if (own && !(lane & 1)) S.brkw[P >> 5] = brk | (other << 16);
     }
-    if (lane == 0) S.wcnt[warp] = cnt;
+    if (P < PT_PRE || P >= PT_PRE + T) st = 0;  // core windows only (PT_PRE and T are multiples of 16)
+    uint32_t wtot = __popc(st), at = wtot;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, at, d);
+      if (lane >= d) at += y;
+    }
+    at -= wtot;
+    wtot = __shfl_sync(0xffffffffu, at + wtot, 31);
+    if (lane == 0) S.wcnt[warp] = wtot;
     __syncthreads();
-    uint32_t n_skm = 0, at = 0;
+    uint32_t n_skm = 0;
 #pragma unroll
     for (int x = 0; x < TL_WARPS; x++) {
       const uint32_t c = S.wcnt[x];
@@ -125,14 +141,12 @@ __global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
       n_skm += c;
     }
 #pragma unroll
-    for (int r = 0; r < TL_TW; r++) {
-      if ((st[r] >> lane) & 1u) {
-        const uint32_t i = at + __popc(st[r] & ((1u << lane) - 1u));
-        S.spos[i] = (uint16_t)(32 * (w0 + r) + lane);
-        S.smm[i] = m[r];
+    for (int i = 0; i < TL_W; i++)
+      if ((st >> i) & 1u) {
+        S.spos[at] = (uint16_t)(P + i);
+        S.smm[at] = m[i];
+        at++;
       }
-      at += __popc(st[r]);
-    }
     __syncthreads();
 
     // ---- ends, byte offsets: consecutive superkmers per thread ----
@@ -142,12 +156,12 @@ __global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
       const uint32_t l = S.spos[i];
       int w = (int)(l >> 5);
       uint32_t bits = S.brkw[w] & (0xFFFFFFFEu << (l & 31));
-      while (!bits && ++w < TL_WORDS) bits = S.brkw[w];
+      while (!bits && ++w < NW / 32) bits = S.brkw[w];
       uint32_t e = bits ? 32 * (uint32_t)w + __ffs((int)bits) - 1 : PT_EXT, end = e;
       if (!bits) {
         // the last superkmer runs past the tile: walk on with the exact rule until a break
         const uint32_t mv = S.smm[i];
-        uint64_t x = (uint64_t)(G0 + TL_NW);
+        uint64_t x = (uint64_t)(G0 + NW);
         while (x < a.nbytes) {
           if (global_rs(a.rs_bits, x) || !global_window_valid(a.rs_bits, a.nbytes, x, k)) break;
           const uint32_t v = exact_window_minimizer(

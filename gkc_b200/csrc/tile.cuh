@@ -1,16 +1,19 @@
 // Minimizers of a tile of windows, shared by the partition and the per-window
 // kernels.
 //
-// A CTA of TL_NT threads takes TL_NW consecutive windows of the concatenated
-// reads, every warp TL_TW words of 32.  The tile's bases are held as 16-base
+// A CTA takes a tile of consecutive windows of the concatenated reads, each
+// warp a strip of them and each lane 16.  The tile's bases are held as 16-base
 // words, each beside its reverse complement, so that any p-mer and its reverse
-// complement are one funnel shift each; lane l of a warp holds window (and
-// p-mer position) l of every word, and the minimum over the omega = k - p + 1
-// p-mers of a window is built in registers by doubling (shifts by 1, 2, 4, ..
-// positions between lanes), so no p-mer goes through shared memory.
-// What bounds it is instruction issue: about 50 instructions a window, against
-// 210 where p-mers rolled through bytes in shared memory and prefix and suffix
-// minima were kept per position.
+// complement are one funnel shift each, by a constant: lane l needs two words
+// for its 16 p-mers.  The minimum over the omega = k - p + 1 p-mers of a
+// window is built by doubling (shifts by 1, 2, 4, .. positions): most shifted
+// values are the lane's own registers, the rest come from the next lanes, so
+// no p-mer goes through shared memory.  The strip's last lanes only feed the
+// others: 30 lanes have windows of their own, 28 where omega > 33.
+// What bounds it is instruction issue (the ALU pipe): about 25 instructions a
+// window, against 50 with one window of every word per lane (each shift an
+// exchange and a select) and 210 where p-mers rolled through bytes in shared
+// memory and prefix and suffix minima were kept per position.
 #pragma once
 #include "common.cuh"
 #include "minimizer.cuh"
@@ -19,12 +22,21 @@ namespace gkc {
 
 constexpr int TL_NT = 256;
 constexpr int TL_WARPS = TL_NT / 32;
-constexpr int TL_TW = 15;                        // window words per warp
-constexpr int TL_WORDS = TL_WARPS * TL_TW;       // window words per tile
-constexpr int TL_NW = 32 * TL_WORDS;             // windows per tile
-constexpr int TL_BWORDS = TL_WORDS + 3;          // words with bases (k <= 64: a window reaches two words on)
+constexpr int TL_W = 16;                         // windows per lane
+constexpr int TL_BWORDS = 123;                   // 32-base words: the last strip's p-mers and windows reach 3936 bases
 constexpr int TL_GROUPS = 2 * TL_BWORDS;         // 16-base groups
+constexpr int TL_NW_MAX = TL_WARPS * 30 * TL_W;  // windows per tile
 static_assert(TL_GROUPS <= TL_NT, "one 16-base group per thread");
+GKC_HOST_DEV int tile_strip(int omega) { return omega > 33 ? 28 * TL_W : 30 * TL_W; }  // windows per warp
+GKC_HOST_DEV int tile_windows_n(int omega) { return TL_WARPS * tile_strip(omega); }    // windows per tile
+
+// Whether a 2p-bit p-mer value passes the filter (mm_filter for such values).
+template <int FILT>
+GKC_DEV bool tile_pass(uint32_t v, int p) {
+  // AAA, ACA or AGA on top: first base A, second below T, third A
+  if (FILT == FILTER_NEW2) return v >= (3u << (2 * p - 4)) || (v & (3u << (2 * p - 6))) != 0;
+  return mm_filter(v, p, FILT);
+}
 
 struct TileBases {
   uint2 pk[TL_GROUPS + 2];   // 16 bases, 2 bits each, first base in the top bits; their reverse complement
@@ -142,61 +154,139 @@ GKC_DEV uint32_t tile_code(const TileBases &S, int l) {
   return (S.pk[l >> 4].x >> (30 - 2 * (l & 15))) & 3u;
 }
 
-// Filtered minimum of the p-mer at base 32 w + lane and its reverse
-// complement; with POS also, in *code, the strand of the chosen one (0
-// forward, 1 reverse, 2 both).
+// m[i], i < 16: the filtered minimum of the p-mer at tile base P + i, P =
+// 16 (j0 + lane), and its reverse complement.  With POS q[i] holds 4 * (tile
+// base) + the strand of the chosen one (0 forward, 1 reverse, 2 both).
 template <int FILT, bool POS>
-GKC_DEV uint32_t tile_pmer(const TileBases &S, int w, int p, uint32_t M, uint32_t *code) {
-  const uint32_t lane = threadIdx.x & 31u, sh = 2 * (lane & 15u);
-  const uint2 a = S.pk[2 * w + (lane >> 4)], b = S.pk[2 * w + (lane >> 4) + 1];
-  const uint32_t f = __funnelshift_l(b.x, a.x, sh) >> (32 - 2 * p);
-  const uint32_t r = __funnelshift_r(a.y, b.y, sh) & M;
-  const uint32_t vf = mm_filter(f, p, FILT) ? f : M;
-  const uint32_t vr = mm_filter(r, p, FILT) ? r : M;
-  if (POS) *code = f == r ? 2u : (vr < vf ? 1u : 0u);
-  return vf < vr ? vf : vr;
+GKC_DEV void tile_pmers(const TileBases &S, int j0, int p, uint32_t (&m)[TL_W], uint32_t (&q)[POS ? TL_W : 1]) {
+  const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * p), lane = threadIdx.x & 31u;
+  const uint2 a = S.pk[j0 + lane], b = S.pk[j0 + lane + 1];
+#pragma unroll
+  for (int i = 0; i < TL_W; i++) {
+    const uint32_t f = __funnelshift_l(b.x, a.x, 2 * i) >> (32 - 2 * p);
+    const uint32_t r = __funnelshift_r(a.y, b.y, 2 * i) & M;
+    const uint32_t vf = tile_pass<FILT>(f, p) ? f : M;
+    const uint32_t vr = tile_pass<FILT>(r, p) ? r : M;
+    m[i] = min(vf, vr);
+    if (POS) q[POS ? i : 0] = 4 * (16 * (uint32_t)(j0 + lane) + i) + (f == r ? 2u : (vr < vf ? 1u : 0u));
+  }
 }
 
-// m[r], r < TL_TW: the minimum over the omega p-mers of window 32 (w0 + r) +
-// lane (the last two words of m only feed the others).  With POS q[r] holds
-// 4 * (tile base of the rightmost p-mer with that value) + its strand code.
-template <int FILT, bool POS>
-GKC_DEV void tile_minima(const TileBases &S, int w0, int p, int omega, uint32_t (&m)[TL_TW + 2],
-                         uint32_t (&q)[POS ? TL_TW + 2 : 1]) {
-  const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * p), lane = threadIdx.x & 31u;
-  const bool far = omega > 33;  // windows reach a second word
+// m[i] = min(m[i], the value 16 ls + T positions on); with POS the q of the
+// later one where they are equal.
+template <int T, bool POS>
+GKC_DEV void tile_shift(uint32_t (&m)[TL_W], uint32_t (&q)[POS ? TL_W : 1], int ls) {
+  uint32_t t[T > 0 ? T : 1], tq[POS && T > 0 ? T : 1];
 #pragma unroll
-  for (int r = 0; r < TL_TW + 2; r++) {
-    uint32_t code = 0;
-    m[r] = 0xFFFFFFFFu;
-    if (r < TL_TW + 1 || far) m[r] = tile_pmer<FILT, POS>(S, w0 + r, p, M, &code);
-    if (POS) q[POS ? r : 0] = 4 * (32 * (uint32_t)(w0 + r) + lane) + code;
+  for (int j = 0; j < T; j++) {
+    t[j] = __shfl_down_sync(0xffffffffu, m[j], ls + 1);
+    if (POS) tq[POS ? j : 0] = __shfl_down_sync(0xffffffffu, q[POS ? j : 0], ls + 1);
   }
-  int done = 1;
-  while (done < omega) {
-    // min over `done` positions -> over 2 * done, or (the last step) over omega
-    const int s = min(done, omega - done);  // 1 .. 32
-    const uint32_t from = (lane + (uint32_t)s) & 31u;
-    const bool same = lane + (uint32_t)s < 32u;
-    uint32_t t = __shfl_sync(0xffffffffu, m[0], from), tq = 0;
-    if (POS) tq = __shfl_sync(0xffffffffu, q[0], from);
 #pragma unroll
-    for (int r = 0; r < TL_TW + 2; r++) {
-      uint32_t tn = 0xFFFFFFFFu, tqn = 0;
-      if (r + 1 < TL_TW + 2) {
-        tn = __shfl_sync(0xffffffffu, m[r + 1], from);
-        if (POS) tqn = __shfl_sync(0xffffffffu, q[POS ? r + 1 : 0], from);
+  for (int i = 0; i < TL_W; i++) {
+    uint32_t y, yq = 0;
+    if (i + T < TL_W) {
+      const int x = i + T < TL_W ? i + T : 0;
+      y = m[x];
+      if (POS) yq = q[POS ? x : 0];
+      if (ls) {
+        y = __shfl_down_sync(0xffffffffu, y, ls);
+        if (POS) yq = __shfl_down_sync(0xffffffffu, yq, ls);
       }
-      const uint32_t y = same ? t : tn;
-      if (POS) {
-        const uint32_t yq = same ? tq : tqn;
-        if (y <= m[r]) q[POS ? r : 0] = yq;  // the rightmost of equal ones
-      }
-      m[r] = y < m[r] ? y : m[r];
-      t = tn;
-      tq = tqn;
+    } else {
+      const int x = i + T >= TL_W ? i + T - TL_W : 0;
+      y = t[T > 0 ? x : 0];
+      if (POS) yq = tq[POS && T > 0 ? x : 0];
     }
-    done += s;
+    if (POS) {
+      if (y <= m[i]) q[POS ? i : 0] = yq;
+    }
+    m[i] = min(m[i], y);
+  }
+}
+
+// The minimum over omega positions from p-mer minima (and, with POS, the
+// rightmost position that has it).
+template <bool POS>
+GKC_DEV void tile_slide(uint32_t (&m)[TL_W], uint32_t (&q)[POS ? TL_W : 1], int omega) {
+  if (omega >= 2) tile_shift<1, POS>(m, q, 0);
+  if (omega >= 4) tile_shift<2, POS>(m, q, 0);
+  if (omega >= 8) tile_shift<4, POS>(m, q, 0);
+  if (omega >= 16) tile_shift<8, POS>(m, q, 0);
+  if (omega >= 32) tile_shift<0, POS>(m, q, 1);
+  int done = 1;
+  while (2 * done <= omega) done *= 2;
+  const int s = omega - done;  // the last step overlaps; 0 .. 31
+  switch (s & 15) {
+    case 0: if (s) tile_shift<0, POS>(m, q, s >> 4); break;
+    case 1: tile_shift<1, POS>(m, q, s >> 4); break;
+    case 2: tile_shift<2, POS>(m, q, s >> 4); break;
+    case 3: tile_shift<3, POS>(m, q, s >> 4); break;
+    case 4: tile_shift<4, POS>(m, q, s >> 4); break;
+    case 5: tile_shift<5, POS>(m, q, s >> 4); break;
+    case 6: tile_shift<6, POS>(m, q, s >> 4); break;
+    case 7: tile_shift<7, POS>(m, q, s >> 4); break;
+    case 8: tile_shift<8, POS>(m, q, s >> 4); break;
+    case 9: tile_shift<9, POS>(m, q, s >> 4); break;
+    case 10: tile_shift<10, POS>(m, q, s >> 4); break;
+    case 11: tile_shift<11, POS>(m, q, s >> 4); break;
+    case 12: tile_shift<12, POS>(m, q, s >> 4); break;
+    case 13: tile_shift<13, POS>(m, q, s >> 4); break;
+    case 14: tile_shift<14, POS>(m, q, s >> 4); break;
+    default: tile_shift<15, POS>(m, q, s >> 4); break;
+  }
+}
+
+// Minimizers of the warp's strip from window P0 (a multiple of 32) on: lane
+// l's m[i] is that of window P0 + 16 l + i.
+template <bool POS>
+GKC_DEV void tile_minima(const TileBases &S, int P0, int k, int p, int filter, uint32_t (&m)[TL_W],
+                         uint32_t (&q)[POS ? TL_W : 1]) {
+  switch (filter) {
+    case FILTER_ALL: tile_pmers<FILTER_ALL, POS>(S, P0 >> 4, p, m, q); break;
+    case FILTER_NEW: tile_pmers<FILTER_NEW, POS>(S, P0 >> 4, p, m, q); break;
+    case FILTER_SIGNATURE: tile_pmers<FILTER_SIGNATURE, POS>(S, P0 >> 4, p, m, q); break;
+    default: tile_pmers<FILTER_NEW2, POS>(S, P0 >> 4, p, m, q); break;
+  }
+  tile_slide<POS>(m, q, k - p + 1);
+}
+
+// The windows of `mask` (bit i: the lane's window i) redone by the exact rule
+// of windows that touch a byte that is no base, spread over the warp's lanes
+// 32 at a time (a single such byte touches k windows in a row, which few
+// lanes hold).  exact(l) gives tile window l's value; `list` holds 32 entries
+// of the warp.
+template <typename Exact, typename Put>
+GKC_DEV void tile_redo(uint32_t mask, int P0, uint16_t *list, Exact &&exact, Put &&put) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t rank0 = __popc(mask);  // rank of the lane's first window among the warp's
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t y = __shfl_up_sync(0xffffffffu, rank0, d);
+    if (lane >= (uint32_t)d) rank0 += y;
+  }
+  const uint32_t total = __shfl_sync(0xffffffffu, rank0, 31);
+  rank0 -= __popc(mask);
+  for (uint32_t b = 0; b < total; b += 32) {
+    uint32_t left = mask, rk = rank0;
+    while (left) {
+      const int i = __ffs((int)left) - 1;
+      left &= left - 1;
+      if (rk - b < 32u) list[rk - b] = (uint16_t)(P0 + 16 * lane + i);
+      rk++;
+    }
+    __syncwarp();
+    uint32_t v = 0, v2 = 0;
+    if (b + lane < total) exact((int)list[lane], v, v2);
+    rk = rank0;
+#pragma unroll
+    for (int i = 0; i < TL_W; i++) {
+      const bool in = (mask >> i) & 1u;
+      const uint32_t x = __shfl_sync(0xffffffffu, v, (rk - b) & 31u), x2 = __shfl_sync(0xffffffffu, v2, (rk - b) & 31u);
+      if (in && rk - b < 32u) put(i, x, x2);
+      rk += in;
+    }
+    __syncwarp();
   }
 }
 

@@ -84,65 +84,96 @@ struct WinArgs {
   int k, p, filter;
 };
 
-// The warp's windows of a tile (tile.cuh): m[r] and, with POS, q[r] for word
-// w0 + r; valid and touched words in lane r of *vw and *tw.
-template <bool POS>
-GKC_DEV void tile_windows(const TileBases &S, const WinArgs &a, int64_t G0, int64_t lo, int64_t hi, int w0,
-                          uint32_t (&m)[TL_TW + 2], uint32_t (&q)[POS ? TL_TW + 2 : 1], uint32_t *vw, uint32_t *tw) {
-  const int lane = threadIdx.x & 31, omega = a.k - a.p + 1;
+// The lane's 16 windows of the warp's strip from tile window P0 on: bit i of
+// *vw and *tw: window i lies in a read; it touches a byte that is no base.
+GKC_DEV void lane_valid(const TileBases &S, const WinArgs &a, int64_t G0, int64_t lo, int64_t hi, int P0, int strip,
+                        uint32_t *vw, uint32_t *tw) {
+  const int x = TL_W * (threadIdx.x & 31), P = P0 + x;
   *vw = *tw = 0;
-  if (lane < TL_TW) tile_valid(S, w0 + lane, G0, lo, hi, a.k, vw, tw);
-  switch (a.filter) {
-    case FILTER_ALL: tile_minima<FILTER_ALL, POS>(S, w0, a.p, omega, m, q); break;
-    case FILTER_NEW: tile_minima<FILTER_NEW, POS>(S, w0, a.p, omega, m, q); break;
-    case FILTER_SIGNATURE: tile_minima<FILTER_SIGNATURE, POS>(S, w0, a.p, omega, m, q); break;
-    default: tile_minima<FILTER_NEW2, POS>(S, w0, a.p, omega, m, q); break;
+  if (x < strip) {
+    tile_valid(S, P >> 5, G0, lo, hi, a.k, vw, tw);
+    *vw = (*vw >> (P & 31)) & 0xFFFFu;
+    *tw = (*tw >> (P & 31)) & *vw;
   }
 }
 
-// Minimizer, position and strand of every window, one tile per CTA turn.
-// Windows with a byte that is no base follow the exact per-window rule, and so
-// do those whose minimizer is the largest p-mer value (it may stand for "none
-// passed", which has no position).
+// Minimizer, position and strand of every window, one tile per CTA turn; a
+// lane's 16 windows are written as whole 16-byte words.  Windows with a byte
+// that is no base follow the exact per-window rule, and so do those whose
+// minimizer is the largest p-mer value (it may stand for "none passed", which
+// has no position).
 __global__ void __launch_bounds__(TL_NT, 3) k_window_minimizers(WinArgs a, uint32_t *mm, uint8_t *pos,
-                                                                int8_t *strand) {
+                                                                int8_t *strand, int aligned) {
   __shared__ TileBases S;
+  __shared__ uint16_t redo[TL_WARPS][32];
   const uint64_t hi = a.offs[a.n_reads];
   const int64_t lo = (int64_t)a.offs[0], end = hi <= a.n_bytes ? (int64_t)hi : 0;
-  const uint64_t n_tiles = (a.n_bytes + TL_NW - 1) / TL_NW;
-  const int lane = threadIdx.x & 31, w0 = (threadIdx.x >> 5) * TL_TW;
+  const int strip = tile_strip(a.k - a.p + 1), NW = TL_WARPS * strip;
+  const uint64_t n_tiles = (a.n_bytes + NW - 1) / NW;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, P0 = warp * strip, P = P0 + TL_W * lane;
   const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * a.p);
   uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
   if (blockIdx.x < n_tiles && threadIdx.x < TL_GROUPS)
-    bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, (int64_t)blockIdx.x * TL_NW, threadIdx.x);
+    bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, (int64_t)blockIdx.x * NW, threadIdx.x);
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int64_t G0 = (int64_t)(tile * TL_NW);
+    const int64_t G0 = (int64_t)(tile * NW);
     tile_store(S, bytes, a.bits, a.bit_words, G0);
     __syncthreads();
     if (tile + gridDim.x < n_tiles && threadIdx.x < TL_GROUPS)
-      bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, (int64_t)((tile + gridDim.x) * TL_NW), threadIdx.x);
-    uint32_t m[TL_TW + 2], q[TL_TW + 2], vw, tw;
-    tile_windows<true>(S, a, G0, lo, end, w0, m, q, &vw, &tw);
+      bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, (int64_t)((tile + gridDim.x) * NW), threadIdx.x);
+    uint32_t vw, tw, m[TL_W], q[TL_W];
+    lane_valid(S, a, G0, lo, end, P0, strip, &vw, &tw);
+    tile_minima<true>(S, P0, a.k, a.p, a.filter, m, q);
 #pragma unroll
-    for (int r = 0; r < TL_TW; r++) {
-      const uint32_t v = __shfl_sync(0xffffffffu, vw, r), t = __shfl_sync(0xffffffffu, tw, r);
-      const uint32_t l = 32 * (uint32_t)(w0 + r) + lane;
-      const uint64_t i = (uint64_t)G0 + l;
-      if (i < a.n_bytes) {
-        WinMin w{0xFFFFFFFFu, 255, 0};
-        if ((v >> lane) & 1u) {
-          if (((t >> lane) & 1u) || m[r] == M) {
-            w = window_min_pos(a.reads, i, a.k, a.p, a.filter);
-          } else {
-            const uint32_t code = q[r] & 3u;
-            w.mm = m[r];
-            w.pos = (uint8_t)((q[r] >> 2) - l);
-            w.strand = (int8_t)(code == 2u ? -1 : (int)code);
-          }
+    for (int i = 0; i < TL_W; i++) {
+      if (m[i] == M) tw |= vw & (1u << i);
+      const uint32_t code = q[i] & 3u;
+      q[i] = ((q[i] >> 2) - (uint32_t)(P + i)) | (code == 2u ? 0xFF00u : code << 8);  // strand byte, position byte
+    }
+    if (__any_sync(0xffffffffu, tw != 0u))
+      tile_redo(tw, P0, redo[warp],
+                [&](int l, uint32_t &v, uint32_t &v2) {
+                  const WinMin w = window_min_pos(a.reads, (uint64_t)(G0 + l), a.k, a.p, a.filter);
+                  v = w.mm;
+                  v2 = (uint32_t)w.pos | ((uint32_t)(uint8_t)w.strand << 8);
+                },
+                [&](int i, uint32_t v, uint32_t v2) {
+#pragma unroll
+                  for (int x = 0; x < TL_W; x++)
+                    if (x == i) {
+                      m[x] = v;
+                      q[x] = v2;
+                    }
+                });
+#pragma unroll
+    for (int i = 0; i < TL_W; i++)
+      if (!((vw >> i) & 1u)) {
+        m[i] = 0xFFFFFFFFu;
+        q[i] = 255u;
+      }
+    const uint64_t at = (uint64_t)G0 + P;
+    if (TL_W * lane < strip) {
+      if (aligned && at + TL_W <= a.n_bytes) {
+        uint4 *om = reinterpret_cast<uint4 *>(mm + at);
+#pragma unroll
+        for (int x = 0; x < 4; x++) om[x] = make_uint4(m[4 * x], m[4 * x + 1], m[4 * x + 2], m[4 * x + 3]);
+        uint32_t pw[4], sw[4];
+#pragma unroll
+        for (int x = 0; x < 4; x++) {
+          const uint32_t lo2 = __byte_perm(q[4 * x], q[4 * x + 1], 0x5140), hi2 = __byte_perm(q[4 * x + 2], q[4 * x + 3], 0x5140);
+          pw[x] = __byte_perm(lo2, hi2, 0x5410);  // bytes: position 0, 1 (low halves of lo2), 2, 3
+          sw[x] = __byte_perm(lo2, hi2, 0x7632);
         }
-        mm[i] = w.mm;
-        if (pos) pos[i] = w.pos;
-        if (strand) strand[i] = w.strand;
+        if (pos) *reinterpret_cast<uint4 *>(pos + at) = make_uint4(pw[0], pw[1], pw[2], pw[3]);
+        if (strand) *reinterpret_cast<uint4 *>(strand + at) = make_uint4(sw[0], sw[1], sw[2], sw[3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < TL_W; i++)
+          if (at + i < a.n_bytes) {
+            mm[at + i] = m[i];
+            if (pos) pos[at + i] = (uint8_t)q[i];
+            if (strand) strand[at + i] = (int8_t)(q[i] >> 8);
+          }
       }
     }
     __syncthreads();  // before the next tile's bases
@@ -152,35 +183,45 @@ __global__ void __launch_bounds__(TL_NT, 3) k_window_minimizers(WinArgs a, uint3
 // ---- subsampling: windows whose minimizer % mod == 0, in window order ----
 
 constexpr int SUB_NT = TL_NT;
-constexpr int SUB_WORDS = TL_WORDS;  // selection words per tile
-constexpr int SUB_TILE = TL_NW;      // windows per tile
+constexpr int SUB_WORDS = TL_NW_MAX / 32;  // selection words kept per tile
 
-// Tile t covers windows [t*SUB_TILE, (t+1)*SUB_TILE): selection bitmap and count.
+// Selection bitmap (SUB_WORDS words a tile) and count of every tile.
 __global__ void __launch_bounds__(SUB_NT, 4) k_sub_flags(WinArgs a, uint32_t mod, uint32_t *sel,
                                                          unsigned long long *tile_cnt, uint64_t n_tiles) {
   __shared__ TileBases S;
+  __shared__ uint16_t redo[TL_WARPS][32];
   __shared__ uint32_t cnt[TL_WARPS];
   const uint64_t hi = a.offs[a.n_reads];
   const int64_t lo = (int64_t)a.offs[0], end = hi <= a.n_bytes ? (int64_t)hi : 0;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * TL_TW;
+  const int strip = tile_strip(a.k - a.p + 1), NW = TL_WARPS * strip;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, P0 = warp * strip, P = P0 + TL_W * lane;
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int64_t G0 = (int64_t)(tile * TL_NW);
+    const int64_t G0 = (int64_t)(tile * NW);
     uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < TL_GROUPS) bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, G0, threadIdx.x);
     tile_store(S, bytes, a.bits, a.bit_words, G0);
     __syncthreads();
-    uint32_t m[TL_TW + 2], none[1], vw, tw, c = 0;
-    tile_windows<false>(S, a, G0, lo, end, w0, m, none, &vw, &tw);
+    uint32_t vw, tw, m[TL_W], none[1];
+    lane_valid(S, a, G0, lo, end, P0, strip, &vw, &tw);
+    tile_minima<false>(S, P0, a.k, a.p, a.filter, m, none);
+    if (__any_sync(0xffffffffu, tw != 0u))
+      tile_redo(tw, P0, redo[warp],
+                [&](int l, uint32_t &v, uint32_t &) {
+                  v = exact_window_minimizer([&](int j) { return tile_code(S, l + j); }, a.k, a.p, a.filter);
+                },
+                [&](int i, uint32_t v, uint32_t) {
 #pragma unroll
-    for (int r = 0; r < TL_TW; r++) {
-      const uint32_t v = __shfl_sync(0xffffffffu, vw, r), t = __shfl_sync(0xffffffffu, tw & vw, r);
-      const int l = 32 * (w0 + r) + lane;
-      if ((t >> lane) & 1u)
-        m[r] = exact_window_minimizer([&](int j) { return tile_code(S, l + j); }, a.k, a.p, a.filter);
-      const uint32_t f = __ballot_sync(0xffffffffu, ((v >> lane) & 1u) && m[r] % mod == 0u);
-      if (lane == 0) sel[tile * SUB_WORDS + w0 + r] = f;
-      c += __popc(f);
-    }
+                  for (int x = 0; x < TL_W; x++)
+                    if (x == i) m[x] = v;
+                });
+    uint32_t f = 0;
+#pragma unroll
+    for (int i = 0; i < TL_W; i++)
+      if (m[i] % mod == 0u) f |= 1u << i;
+    f &= vw;
+    const uint32_t other = __shfl_down_sync(0xffffffffu, f, 1);
+    if (TL_W * lane < strip && !(lane & 1)) sel[tile * SUB_WORDS + (P >> 5)] = f | (other << 16);
+    const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(f));
     if (lane == 0) cnt[warp] = c;
     __syncthreads();  // also before the next tile's bases
     if (threadIdx.x == 0) {
@@ -214,19 +255,20 @@ __global__ void __launch_bounds__(SUB_NT) k_sub_write(WinArgs a, const uint32_t 
                                                       K *keys, uint32_t *posv, uint64_t n_tiles) {
   __shared__ TileBases S;
   __shared__ uint32_t cnt[TL_WARPS];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * TL_TW;
+  const int strip = tile_strip(a.k - a.p + 1), NW = TL_WARPS * strip, words = strip / 32;  // at most 15 words a warp
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * words;
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
-    const int64_t G0 = (int64_t)(tile * TL_NW);
+    const int64_t G0 = (int64_t)(tile * NW);
     uint4 bytes = make_uint4(0u, 0u, 0u, 0u);
     if (threadIdx.x < TL_GROUPS) bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, G0, threadIdx.x);
-    const uint32_t mine = lane < TL_TW ? sel[tile * SUB_WORDS + w0 + lane] : 0u;
+    const uint32_t mine = lane < words ? sel[tile * SUB_WORDS + w0 + lane] : 0u;
     tile_store(S, bytes, a.bits, a.bit_words, G0);
     const uint32_t c = __reduce_add_sync(0xffffffffu, __popc(mine));
     if (lane == 0) cnt[warp] = c;
     __syncthreads();
     uint64_t o = tile_off[tile];
     for (int x = 0; x < warp; x++) o += cnt[x];
-    for (int r = 0; r < TL_TW; r++) {
+    for (int r = 0; r < words; r++) {
       const uint32_t f = __shfl_sync(0xffffffffu, mine, r);
       if ((f >> lane) & 1u) {
         const int l = 32 * (w0 + r) + lane;
@@ -310,10 +352,12 @@ gkc_status gkc_minimizers_device(gkc_ctx *c, const gkc_params *prm, const char *
   uint32_t *bits, *err;
   s = mark_starts(c, d_offs, n_reads, n_bytes, &bits, &err);
   if (s != GKC_OK) return s;
-  const uint64_t tiles = (n_bytes + TL_NW - 1) / TL_NW;
+  const int nw = tile_windows_n(prm->k - prm->p + 1);
+  const uint64_t tiles = (n_bytes + nw - 1) / nw;
+  const int aligned = (((uintptr_t)d_minimizer | (uintptr_t)d_pos | (uintptr_t)d_strand) & 15) == 0;
   k_window_minimizers<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 3), TL_NT, 0, c->st>>>(
       win_args(c, prm, reinterpret_cast<const uint8_t *>(d_reads), n_bytes, d_offs, n_reads, bits), d_minimizer, d_pos,
-      d_strand);
+      d_strand, aligned);
   CK(cudaPeekAtLastError());
   return read_err(c, err);
 }
@@ -325,7 +369,8 @@ static gkc_status subsample_t(gkc_ctx *c, const gkc_params *prm, uint32_t mod, c
   uint32_t *bits, *err;
   gkc_status s = mark_starts(c, d_offs, n_reads, n_bytes, &bits, &err);
   if (s != GKC_OK) return s;
-  const uint64_t tiles = (n_bytes + SUB_TILE - 1) / SUB_TILE;
+  const int nw = tile_windows_n(prm->k - prm->p + 1);
+  const uint64_t tiles = (n_bytes + nw - 1) / nw;
   WS(sel, uint32_t, "win_sel", tiles * SUB_WORDS + 1);
   WS(tcnt, unsigned long long, "win_tile_cnt", tiles + 1);
   WS(toff, uint64_t, "win_tile_off", tiles + 2);
