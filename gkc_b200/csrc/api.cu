@@ -410,16 +410,11 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
   c->part_hpc_offs = nullptr;
   c->part_hpc_orig = nullptr;
   if (prm->hpc) {
-    WS(runlen, unsigned long long, "hpc_runlen", n_reads + 1);
     WS(hoffs, uint64_t, "hpc_offs", n_reads + 2);
     WS(hreads, uint8_t, "hpc_reads", n_bytes + 64);
     WS(horig, int32_t, "hpc_orig", n_bytes + 16);
-    WS(stmp, uint64_t, "scan_tmp", scan_u64_tmp_words(n_reads + 1) + 8);
-    k_hpc_count<<<c->n_sms * 8, 256, 0, c->st>>>(src, offs, n_reads, runlen);
-    LAUNCHED(c);
-    c->launches += scan_u64(runlen, hoffs, n_reads, stmp, c->st);
-    k_hpc_write<<<c->n_sms * 8, 256, 0, c->st>>>(src, offs, n_reads, hoffs, hreads, horig);
-    LAUNCHED(c);
+    const gkc_status hs = hpc_enqueue(c, src, n_bytes, offs, n_reads, hreads, hoffs, horig);
+    if (hs != GKC_OK) return hs;
     src = hreads;
     offs = hoffs;
     nbytes_dev = hoffs + n_reads;
@@ -428,7 +423,7 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
     c->part_hpc_orig = horig;
   }
   const uint64_t rs_words = (n_bytes + 1 + 31) / 32 + 2;
-  WS(rs, uint32_t, "rs_bits", rs_words);
+  WS(rs, uint32_t, "rs_bits", rs_words);  // with HPC: the original reads' bitmap until here
   WS(bin_nskm, unsigned long long, "bin_nskm", nbins + 1);
   WS(bin_nkm, unsigned long long, "bin_nkmers", nbins + 1);
   const ClearArgs ca{tot, err, bin_nskm, bin_nkm, nbins, rs, rs_words};

@@ -132,5 +132,8 @@ gkc_status count_plain_impl(gkc_ctx *c, const gkc_params *prm);
 gkc_status partition_device_impl(gkc_ctx *c, const gkc_params *prm, const char *d_reads,
                                  uint64_t n_bytes, const uint64_t *d_offs, uint64_t n_reads);
 gkc_status count_device_impl(gkc_ctx *c, const gkc_params *prm, gkc_mode mode);
+// Homopolymer compression of device reads, enqueued on the context's stream.
+gkc_status hpc_enqueue(gkc_ctx *c, const uint8_t *reads, uint64_t n_bytes, const uint64_t *offs, uint64_t n_reads,
+                       uint8_t *out, uint64_t *out_offs, int32_t *orig);
 gkc_status upload_reads(gkc_ctx *c, const char *reads, const uint64_t *offs, uint64_t n_reads,
                         char **d_reads, uint64_t **d_offs, uint64_t *n_bytes);

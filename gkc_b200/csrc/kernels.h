@@ -172,10 +172,6 @@ uint32_t scan_kmers_dev(const uint64_t *desc, int k, uint64_t *out, uint64_t n_c
 }  // namespace gkc
 
 namespace gkc {
-__global__ void k_hpc_count(const uint8_t *reads, const uint64_t *offs, uint64_t n_reads,
-                            unsigned long long *run_len);
-__global__ void k_hpc_write(const uint8_t *reads, const uint64_t *offs, uint64_t n_reads,
-                            const uint64_t *hpc_offs, uint8_t *out, int32_t *orig_pos);
 // Run-length pass over sorted keys (distinct keys + first indices).
 uint64_t rle_block_count(uint64_t n);
 template <typename K>

@@ -236,15 +236,11 @@ gkc_status partition_plain_impl(gkc_ctx *c, const gkc_params *prm, const char *d
   c->part_hpc_offs = nullptr;
   c->part_hpc_orig = nullptr;
   if (prm->hpc) {
-    WS(runlen, unsigned long long, "hpc_runlen", n_reads + 1);
     WS(hoffs, uint64_t, "hpc_offs", n_reads + 2);
     WS(hreads, uint8_t, "hpc_reads", n_bytes + 64);
     WS(horig, int32_t, "hpc_orig", n_bytes + 16);
-    WS(stmp, uint64_t, "scan_tmp", scan_u64_tmp_words(n_reads + 1) + 8);
-    k_hpc_count<<<grid, 256, 0, c->st>>>(src, offs, n_reads, runlen);
-    scan_u64(runlen, hoffs, n_reads, stmp, c->st);
-    k_hpc_write<<<grid, 256, 0, c->st>>>(src, offs, n_reads, hoffs, hreads, horig);
-    c->launches += 6;
+    const gkc_status hs = hpc_enqueue(c, src, n_bytes, offs, n_reads, hreads, hoffs, horig);
+    if (hs != GKC_OK) return hs;
     src = hreads;
     offs = hoffs;
     nbytes_dev = hoffs + n_reads;

@@ -93,3 +93,41 @@ def test_minimizer_tiles(ctx, k, p, filter_id, shift):
     assert np.array_equal(mm.cpu().numpy().view(np.uint32), want[0])
     assert np.array_equal(pos.cpu().numpy(), want[1])
     assert np.array_equal(strand.cpu().numpy(), want[2])
+
+
+@pytest.mark.parametrize("shift", [0, 5])
+@pytest.mark.parametrize("first", [0, 7])
+@pytest.mark.parametrize("total", [1, 15, 16, 33, 8191, 8192, 8193, 40_000])
+def test_hpc_tiles(ctx, total, first, shift):
+    """Homopolymer compression over its 8192-byte tiles: runs and reads that
+    end on tile, word and thread boundaries, empty reads, reads that do not
+    start at the first byte, unaligned addresses."""
+    import torch
+    r = np.random.default_rng(100 * total + first)
+    b = np.repeat(np.frombuffer(b"ACGTN", np.uint8)[r.integers(0, 5, total)], r.integers(1, 6, total))[:total].copy()
+    if total > 8200:
+        b[8100:8300] = ord("A")  # a run across a tile
+    first = min(first, total - 1)
+    cuts = np.unique(np.concatenate([r.integers(first, total + 1, 30), [first, total], np.arange(8192, total, 8192)]))
+    cuts = cuts[cuts >= first]
+    offs = np.concatenate([cuts[:1], cuts[:1], cuts, cuts[-1:]]).astype(np.uint64)  # empty reads at both ends
+    buf, d_reads, d_offs = on_device(b, offs, shift)
+    n = len(offs) - 1
+    out = torch.zeros(total + 16, dtype=torch.uint8, device="cuda")[shift:]
+    ooffs = torch.zeros(n + 1, dtype=torch.int64, device="cuda")
+    orig = torch.zeros(total + 1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ctx.hpc_device(d_reads, total, d_offs, n, out, ooffs, orig)
+    want, want_pos, want_offs = [], [], [0]
+    for i in range(n):
+        read = b[int(offs[i]):int(offs[i + 1])]
+        keep = np.ones(len(read), bool)
+        keep[1:] = read[1:] != read[:-1]
+        want.append(read[keep])
+        want_pos.append(np.flatnonzero(keep))
+        want_offs.append(want_offs[-1] + int(keep.sum()))
+    m = want_offs[-1]
+    assert ooffs.cpu().tolist() == want_offs
+    assert np.array_equal(out[:m].cpu().numpy(), np.concatenate(want))
+    assert np.array_equal(orig[:m].cpu().numpy(), np.concatenate(want_pos))
+    assert int(out[m:].sum()) == 0  # nothing written past the kept bytes
