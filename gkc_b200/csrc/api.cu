@@ -232,8 +232,10 @@ gkc_status gkc_ctx_create(int device_id, uint64_t hbm_budget_bytes, gkc_ctx **ou
       set_dyn_smem_limit((const void *)k_bin_place, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_sort<uint64_t>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_sort<u128>, c->max_smem_optin) != cudaSuccess ||
-      set_dyn_smem_limit((const void *)k_bucket_count<uint64_t>, c->max_smem_optin) != cudaSuccess ||
-      set_dyn_smem_limit((const void *)k_bucket_count<u128>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_open<uint64_t>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_open<u128>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_slices<uint64_t>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_slices<u128>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_scatter<uint64_t>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_scatter<u128>, c->max_smem_optin) != cudaSuccess) {
     cudaGetLastError();
@@ -639,8 +641,8 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   pl.bucket_base = bucket_base;
   pl.chunk_base = chunk_base;
   pl.hist_base = hist_base;
-  // [0] bucket ticket, [1] unused, [2] large buckets listed, [3] their ticket
-  WS(ticket, unsigned long long, "count_ticket", 4);
+  // [0] bucket ticket, [2] large buckets listed, [3] their ticket, [4] slices listed, [5] their ticket
+  WS(ticket, unsigned long long, "count_ticket", 6);
   pl.tickets = ticket;
   k_count_plan<<<1, kCountPlanThreads, 0, c->st>>>(pl);
   LAUNCHED(c);
@@ -686,12 +688,15 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   k_bucket_hist<K><<<c->n_sms * 8, kBucketHistThreads, 0, c->st>>>(ea);
   LAUNCHED(c);
   WS(big_list, uint32_t, "big_list", max_buckets + 1);
+  WS(bucket_head, uint32_t, "bucket_head", max_buckets + 1);
+  ea.bucket_head = bucket_head;
   ea.big_list = big_list;
   ea.big_count = ticket + 2;
   ea.big_min = bucket_count_cap<K>() + 1;
   k_bucket_scan<<<std::min<uint32_t>(nbins, 65535), kBucketScanThreads, 0, c->st>>>(ea, bstart, bsize);
   LAUNCHED(c);
-  k_bucket_offsets<<<(unsigned)std::min<uint64_t>((max_buckets + kBucketOffsetThreads - 1) / kBucketOffsetThreads, 65535),
+  k_bucket_offsets<<<(unsigned)std::min<uint64_t>((32 * max_buckets + kBucketOffsetThreads - 1) / kBucketOffsetThreads,
+                                                  (uint64_t)c->n_sms * 64),
                      kBucketOffsetThreads, 0, c->st>>>(ea, bstart);
   LAUNCHED(c);
   stage_mark(c, 4);
@@ -725,11 +730,19 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   sa.big_count = ticket + 2;
   sa.big_ticket = ticket + 3;
   sa.big_min = ea.big_min;
+  // an opened bucket of n > cap keys has at most 3 n / cap + 1 slices
+  const uint64_t task_cap = 4 * keys_cap / bucket_count_cap<K>() + 1024;
+  WS(tasks, uint4, "count_tasks", task_cap);
+  sa.tasks = tasks;
+  sa.task_cap = task_cap;
+  sa.task_count = ticket + 4;
+  sa.task_ticket = ticket + 5;
+  sa.bucket_head = bucket_head;
   sa.err = err;
   const size_t smem = bucket_count_smem_bytes<K>();
   if ((int)smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "count tables exceed shared memory");
   int occ = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bucket_count<K>, kBucketCountThreads, smem));
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bucket_slices<K>, kBucketCountThreads, smem));
   stage_mark(c, 5);
   const size_t sort_smem = bucket_sort_smem_bytes<K>();
   if ((int)sort_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "sort areas exceed shared memory");
@@ -739,7 +752,9 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   LAUNCHED(c);
   // the large and rejected buckets, persistent, taken by ticket
   const int ctas = std::max(1, std::min(occ, c->tune.count_ctas ? (int)c->tune.count_ctas : 2));
-  k_bucket_count<K><<<c->n_sms * ctas, kBucketCountThreads, smem, c->st>>>(sa);
+  k_bucket_open<K><<<c->n_sms * ctas, kBucketCountThreads, smem, c->st>>>(sa);
+  LAUNCHED(c);
+  k_bucket_slices<K><<<c->n_sms * ctas, kBucketCountThreads, smem, c->st>>>(sa);
   LAUNCHED(c);
   stage_mark(c, 6);
   // final offsets: the exclusive scan of the distinct counts (the bucket count is read on the device)
@@ -747,7 +762,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   WS(out_counts, uint32_t, slot_name(c, "counts").c_str(), keys_cap);
   WS(bin_out, uint64_t, slot_name(c, "bin_out").c_str(), nbins + 1);
   k_compact_runs<K><<<c->n_sms * 8, 256, 0, c->st>>>(keys, stage_counts, bstart, bucket_d, bucket_out, bucket_base,
-                                                      nbins, out_keys, out_counts, bin_out, err);
+                                                      nbins, out_keys, out_counts, bin_out, bucket_head, tasks, ticket + 4, err);
   LAUNCHED(c);
   c->count_keys_cap = keys_cap;
   return GKC_OK;

@@ -25,14 +25,15 @@
 //                         runs are staged at the bucket's own key range and
 //                         its distinct count recorded; k_compact_runs then
 //                         moves them to the scan of the counts;
-//      k_bucket_count   - the buckets too large for that, and those in which
+//      k_bucket_open    - the buckets too large for that, and those in which
 //                         copies of one key fill a group: the keys aggregated
 //                         in a shared-memory hash table and the distinct ones
 //                         sorted by a sample sort.  A bucket with too many
 //                         distinct keys is sorted by the digit that follows
 //                         the common prefix of its smallest and largest key
-//                         and counted in slices; a digit larger than a slice
-//                         is opened the same way, one prefix further on.
+//                         and cut into slices;
+//      k_bucket_slices  - counts the slices; a digit larger than a slice is
+//                         opened the same way, one prefix further on.
 #include "common.cuh"
 #include "kernels.h"
 
@@ -138,7 +139,7 @@ __global__ void __launch_bounds__(kCountPlanThreads) k_count_plan(CountPlan pl) 
     cb += nc;
     hb += nh;
   }
-  if (threadIdx.x < 4) pl.tickets[threadIdx.x] = 0;
+  if (threadIdx.x < 6) pl.tickets[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
     pl.bucket_base[pl.nbins] = bb;
     pl.chunk_base[pl.nbins] = cb;
@@ -434,21 +435,25 @@ __global__ void __launch_bounds__(BS_NT) k_bucket_scan(ExpandArgs a, uint64_t *b
       const uint64_t size = st == ~0u ? 0 : end - st;
       bucket_start[g0 + u] = a.bin_kstart[b] + (st == ~0u ? end : st);
       bucket_size[g0 + u] = size;
+      a.bucket_head[g0 + u] = 0;
       if (size >= a.big_min) a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)(g0 + u);
     }
     __syncthreads();
   }
 }
 
-// Every chunk's write offset per bucket, relative to the bin's first key: one
-// thread per bucket adds up its digits chunk after chunk and leaves each
-// offset at the count of the bucket's first digit.
+// Every chunk's write offset per bucket, relative to the bin's first key: a
+// warp per bucket adds up its digits in 32 chunks at a time, one a lane, and
+// leaves each offset at the count of the bucket's first digit.  (A thread per
+// bucket walked hundreds of chunks of a large bin one after the other: 524 us
+// where bins are uneven.)
 __global__ void __launch_bounds__(kBucketOffsetThreads) k_bucket_offsets(ExpandArgs a, const uint64_t *bucket_start) {
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   const uint64_t n_buckets = a.bucket_base[a.nbins];
-  for (uint64_t g = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; g < n_buckets;
-       g += (uint64_t)gridDim.x * blockDim.x) {
-    const uint32_t b = find_bin(a.bucket_base, a.nbins, g);
+  const uint32_t lane = threadIdx.x & 31u;
+  for (uint64_t g = (blockIdx.x * (uint64_t)blockDim.x + threadIdx.x) >> 5; g < n_buckets;
+       g += ((uint64_t)gridDim.x * blockDim.x) >> 5) {
+    const uint32_t b = (uint32_t)warp_last_le(a.bucket_base, 0, a.nbins - 1, g);
     const uint32_t u = (uint32_t)(g - a.bucket_base[b]), nd = 1u << a.bin_bits[b];
     // the bucket's digits [lo, hi): a run in the ascending table
     const uint16_t *lut = a.lut + ((uint64_t)b << a.max_bits);
@@ -466,12 +471,21 @@ __global__ void __launch_bounds__(kBucketOffsetThreads) k_bucket_offsets(ExpandA
     const uint64_t nch = a.chunk_base[b + 1] - a.chunk_base[b];
     uint32_t *M = a.hist + a.hist_base[b];
     uint32_t run = (uint32_t)(bucket_start[g] - a.bin_kstart[b]);
-#pragma unroll 4
-    for (uint64_t jj = 0; jj < nch; jj++) {
+    for (uint64_t j0 = 0; j0 < nch; j0 += 32) {
+      const uint64_t jj = j0 + lane;
       uint32_t v = 0;
-      for (uint32_t d = lo; d < hi; d++) v += M[jj * nd + d];
-      M[jj * nd + lo] = run;
-      run += v;
+      if (jj < nch) {
+#pragma unroll 4
+        for (uint32_t d = lo; d < hi; d++) v += M[jj * nd + d];
+      }
+      uint32_t inc = v;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= (uint32_t)d) inc += t;
+      }
+      if (jj < nch) M[jj * nd + lo] = run + inc - v;
+      run += __shfl_sync(0xffffffffu, inc, 31);
     }
   }
 }
@@ -1358,9 +1372,9 @@ __device__ __noinline__ uint32_t slice_count(SortArea<K, NT, CountShape<K>::CAP>
 }
 
 // Buckets of at most CAP keys, persistent, taken by ticket.  Those that
-// sort_count rejects join the list of large ones (k_bucket_count).  256
+// sort_count rejects join the list of large ones (k_bucket_open).  256
 // threads and 45 KB, so that five CTAs (four for 16-byte keys) on an SM hide
-// each other's barriers.  Count stage (this kernel and k_bucket_count) on a
+// each other's barriers.  Count stage (with the two kernels below) on a
 // B200, against counting each bucket in a 4096-slot hash table with a merge
 // sort, or by insertion and warp sorts of 4096 fixed digits: 720 M 31-mers at
 // 30x 9.7 ms (14.7), 134.7 M mostly distinct 21-mers 3.4 ms (10.6), 150.9 M
@@ -1480,9 +1494,107 @@ __device__ __noinline__ bool open_level(CountSmem<K> &S, const K *from, K *to, u
   return true;
 }
 
-// The listed buckets: larger than CAP, or rejected by k_bucket_sort.
+// Counts the keys [pos, end) of an oversized bucket (offsets from its key range
+// `start`; `from`: the buffer that holds them) and stages their runs from
+// start + pos on; returns their number.  The keys are sorted by digit into the
+// other buffer, then counted in slices of at most CAP keys in key order; a
+// digit of more keys is opened in turn, back into the first buffer.  Buffer 0
+// is the bucket's own key range, buffer 1 the same range of the scratch array
+// (the result's key array, written only after the count).  The staged runs
+// never pass the keys already counted.
 template <typename K>
-__global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_count(SortCountArgs a) {
+__device__ __noinline__ uint64_t count_range(CountSmem<K> &S, const SortCountArgs &a, uint64_t start, uint64_t pos,
+                                             uint64_t end, int from) {
+  constexpr int NT = CountShape<K>::NT, CAP = CountShape<K>::CAP;
+  const int tid = threadIdx.x;
+  K *const buf[2] = {reinterpret_cast<K *>(a.keys) + start, reinterpret_cast<K *>(a.scratch) + start};
+  start += pos;          // of the staged runs
+  uint64_t run = 0;      // [pos, end): what is opened next; the same in every thread
+  int level = 0;
+  while (true) {
+    int cp, sb;
+    K key;
+    if (open_level<K, NT>(S, buf[from], buf[from ^ 1], pos, end, &cp, &sb, &key)) {
+      if (level == CC_LEVELS) {  // not possible: every level fixes a bit of the key
+        if (tid == 0) atomicOr(a.err, ERR_BOUNDS);
+        break;
+      }
+      if (tid == 0) {
+        S.lend[level] = end;
+        S.lcp[level] = (uint8_t)cp;
+        S.lsb[level] = (uint8_t)sb;
+        S.lbuf[level] = (uint8_t)(from ^ 1);
+      }
+      level++;
+    } else {  // one key
+      if (tid == 0) {
+        if (start + run < a.stage_cap) {
+          reinterpret_cast<K *>(a.stage_keys)[start + run] = key;
+          a.stage_counts[start + run] = (uint32_t)(end - pos);
+        } else {
+          atomicOr(a.err, ERR_CAPACITY);
+        }
+      }
+      run++;
+      pos = end;
+    }
+    __syncthreads();
+    // slices of the innermost open level, until one has to be opened
+    bool open = false;
+    while (level > 0 && !open) {
+      const uint64_t lend = S.lend[level - 1];
+      if (pos == lend) {
+        level--;
+        continue;
+      }
+      const int lcp = S.lcp[level - 1], lsb = S.lsb[level - 1];
+      from = S.lbuf[level - 1];
+      const K *src = buf[from];
+      end = lend;
+      if (lend - pos > (uint64_t)CAP) {
+        // the digit of the first key that does not fit ends the slice
+        const uint32_t d = prefix_digit<K>(load_key(src + pos + CAP), lcp, lsb);
+        uint64_t l = pos, h = pos + CAP;  // first key of digit d
+        while (l < h) {
+          const uint64_t mid = (l + h) >> 1;
+          if (prefix_digit<K>(load_key(src + mid), lcp, lsb) < d) l = mid + 1; else h = mid;
+        }
+        end = l;
+        if (l == pos) {  // digit d alone is larger than a slice
+          l = pos + CAP + 1;
+          h = lend;
+          while (l < h) {
+            const uint64_t mid = (l + h) >> 1;
+            if (prefix_digit<K>(load_key(src + mid), lcp, lsb) <= d) l = mid + 1; else h = mid;
+          }
+          end = l;
+          open = true;
+          break;
+        }
+      }
+      const uint32_t ns = (uint32_t)(end - pos);
+      uint32_t D = slice_count<K, NT>(S.u.s, a, src + pos, ns, start + run);
+      if (D == SORT_REJECTED) {
+        hash_count<K, NT>(S, a, src + pos, ns, start + run);  // at most CAP keys: never too many
+        D = S.hfill;
+        __syncthreads();
+      }
+      run += D;
+      pos = end;
+    }
+    if (!open) break;
+    __syncthreads();  // the level's parameters are read before a new one is written
+  }
+  return run;
+}
+
+// The listed buckets: larger than CAP, or rejected by k_bucket_sort.  A bucket
+// that the table takes is counted here; another is sorted by digit into the
+// scratch array and its slices of at most CAP keys (and each digit of more)
+// become tasks of k_bucket_slices, so that a large bucket is counted by many
+// CTAs (by one, the largest of 150.9 M 25-mers kept the chip waiting: 1.9 ms).
+template <typename K>
+__global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_open(SortCountArgs a) {
   constexpr int NT = CountShape<K>::NT, CAP = CountShape<K>::CAP;
   extern __shared__ __align__(16) uint8_t smem_raw[];
   CountSmem<K> &S = *reinterpret_cast<CountSmem<K> *>(smem_raw);
@@ -1522,105 +1634,99 @@ __global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_count(SortCount
       __syncthreads();
       continue;
     }
-
-    // ---- oversized bucket: sorted by digit into the other buffer, then
-    // counted in slices of at most CAP keys in key order; a digit of more
-    // keys is opened in turn, back into the first buffer.  Buffer 0 is the
-    // bucket's own key range, buffer 1 the same range of the scratch array
-    // (the result's key array, written only after this kernel).  The runs are
-    // staged from the start of the key range on and never pass the keys
-    // already counted.
-    K *const buf[2] = {keys + start, reinterpret_cast<K *>(a.scratch) + start};
-    uint64_t pos = 0, end = n, run = 0;  // [pos, end): what is opened next; the same in every thread
-    int from = 0, level = 0;
-    while (true) {
-      int cp, sb;
-      K key;
-      if (open_level<K, NT>(S, buf[from], buf[from ^ 1], pos, end, &cp, &sb, &key)) {
-        if (level == CC_LEVELS) {  // not possible: every level fixes a bit of the key
-          if (tid == 0) atomicOr(a.err, ERR_BOUNDS);
-          break;
-        }
-        if (tid == 0) {
-          S.lend[level] = end;
-          S.lcp[level] = (uint8_t)cp;
-          S.lsb[level] = (uint8_t)sb;
-          S.lbuf[level] = (uint8_t)(from ^ 1);
-        }
-        level++;
-      } else {  // one key
-        if (tid == 0) {
-          if (start + run < a.stage_cap) {
-            reinterpret_cast<K *>(a.stage_keys)[start + run] = key;
-            a.stage_counts[start + run] = (uint32_t)(end - pos);
-          } else {
-            atomicOr(a.err, ERR_CAPACITY);
-          }
-        }
-        run++;
-        pos = end;
+    int cp, sb;
+    K key;
+    if (!open_level<K, NT>(S, keys + start, reinterpret_cast<K *>(a.scratch) + start, 0, n, &cp, &sb, &key)) {
+      if (tid == 0) {  // one key
+        reinterpret_cast<K *>(a.stage_keys)[start] = key;  // start + n <= stage_cap: the keys were there
+        a.stage_counts[start] = (uint32_t)n;
+        a.bucket_d[g] = 1;
       }
       __syncthreads();
-      // slices of the innermost open level, until one has to be opened
-      bool open = false;
-      while (level > 0 && !open) {
-        const uint64_t lend = S.lend[level - 1];
-        if (pos == lend) {
-          level--;
-          continue;
-        }
-        const int lcp = S.lcp[level - 1], lsb = S.lsb[level - 1];
-        from = S.lbuf[level - 1];
-        const K *src = buf[from];
-        end = lend;
-        if (lend - pos > (uint64_t)CAP) {
-          // the digit of the first key that does not fit ends the slice
-          const uint32_t d = prefix_digit<K>(load_key(src + pos + CAP), lcp, lsb);
-          uint64_t l = pos, h = pos + CAP;  // first key of digit d
-          while (l < h) {
-            const uint64_t mid = (l + h) >> 1;
-            if (prefix_digit<K>(load_key(src + mid), lcp, lsb) < d) l = mid + 1; else h = mid;
-          }
-          end = l;
-          if (l == pos) {  // digit d alone is larger than a slice
-            l = pos + CAP + 1;
-            h = lend;
-            while (l < h) {
-              const uint64_t mid = (l + h) >> 1;
-              if (prefix_digit<K>(load_key(src + mid), lcp, lsb) <= d) l = mid + 1; else h = mid;
-            }
-            end = l;
-            open = true;
-            break;
-          }
-        }
-        const uint32_t ns = (uint32_t)(end - pos);
-        uint32_t D = slice_count<K, NT>(S.u.s, a, src + pos, ns, start + run);
-        if (D == SORT_REJECTED) {
-          hash_count<K, NT>(S, a, src + pos, ns, start + run);  // at most CAP keys: never too many
-          D = S.hfill;
-          __syncthreads();
-        }
-        run += D;
-        pos = end;
-      }
-      if (!open) break;
-      __syncthreads();  // the level's parameters are read before a new one is written
+      continue;
     }
-    if (tid == 0) a.bucket_d[g] = run;
+    // S.u.sub[d] is now the end of digit d: as many digits a task as fit CAP
+    // keys, at least one; the first digits of the tasks are listed
+    uint16_t *first = reinterpret_cast<uint16_t *>(S.u.sub + CC_NSUB_MAX);
+    static_assert(sizeof(S.u) >= CC_NSUB_MAX * 6, "the list fits after the digits");
+    if (tid == 0) {
+      const uint32_t nsub = 1u << sb;
+      uint32_t m = 0, d = 0, s0 = 0;
+      while (d < nsub) {
+        uint32_t lo = d + 1, hi = nsub;
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi + 1) >> 1;
+          if (S.u.sub[mid - 1] - s0 <= (uint32_t)CAP) lo = mid; else hi = mid - 1;
+        }
+        if (S.u.sub[lo - 1] != s0) first[m++] = (uint16_t)d;
+        s0 = S.u.sub[lo - 1];
+        d = lo;
+      }
+      S.hfill = m;
+      S.n = atomicAdd(a.task_count, (unsigned long long)m);
+      a.bucket_d[g] = 0;
+      if (S.n + m > a.task_cap) atomicOr(a.err, ERR_BOUNDS);  // not possible: at most 3 n / CAP + 1 tasks
+      else a.bucket_head[g] = (uint32_t)S.n + 1;
+    }
     __syncthreads();
+    const uint32_t m = S.hfill;
+    const uint64_t t0 = S.n;
+    for (uint32_t i = tid; i < m && t0 + m <= a.task_cap; i += NT) {
+      const uint32_t b = first[i] ? S.u.sub[first[i] - 1] : 0u, e = i + 1 < m ? S.u.sub[first[i + 1] - 1] : (uint32_t)n;
+      a.tasks[t0 + i] = make_uint4((uint32_t)g, b, e - b, 0u);
+    }
+    __syncthreads();
+  }
+}
+
+// The tasks of k_bucket_open: slices of an opened bucket, each staged over its
+// own keys; k_compact_runs puts them together.
+template <typename K>
+__global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_slices(SortCountArgs a) {
+  constexpr int NT = CountShape<K>::NT, CAP = CountShape<K>::CAP;
+  extern __shared__ __align__(16) uint8_t smem_raw[];
+  CountSmem<K> &S = *reinterpret_cast<CountSmem<K> *>(smem_raw);
+  if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE | ERR_BOUNDS)) return;
+  const uint64_t n_tasks = *a.task_count;
+  while (true) {
+    if (threadIdx.x == 0) S.g = atomicAdd(a.task_ticket, 1ull);
+    __syncthreads();
+    const uint64_t t = S.g;
+    if (t >= n_tasks) break;
+    const uint4 task = a.tasks[t];
+    const uint64_t start = a.bucket_start[task.x];
+    uint64_t D;
+    if (task.z <= (uint32_t)CAP) {
+      const K *src = reinterpret_cast<const K *>(a.scratch) + start + task.y;
+      const uint32_t d = slice_count<K, NT>(S.u.s, a, src, task.z, start + task.y);
+      if (d != SORT_REJECTED) {
+        D = d;
+      } else {
+        hash_count<K, NT>(S, a, src, task.z, start + task.y);  // at most CAP keys: never too many
+        D = S.hfill;
+      }
+    } else {
+      D = count_range<K>(S, a, start, task.y, (uint64_t)task.y + task.z, 1);
+    }
+    __syncthreads();  // S.g and S.hfill are read
+    if (threadIdx.x == 0) {
+      a.tasks[t].w = (uint32_t)D;
+      atomicAdd(&a.bucket_d[task.x], (unsigned long long)D);
+    }
   }
 }
 
 // Moves each bucket's staged runs to its final offset (the exclusive scan of
 // the buckets' distinct counts); bin_out[b] is the offset of the bin's first
 // bucket.  A warp per bucket where there are buckets for every warp, else
-// several warps share one; four entries a lane in flight.
+// several warps share one; four entries a lane in flight.  An opened bucket's
+// runs lie task by task.
 template <typename K>
 __global__ void k_compact_runs(const K *stage_keys, const uint32_t *stage_counts, const uint64_t *bucket_start,
                                const unsigned long long *bucket_d, const uint64_t *bucket_out,
                                const uint64_t *bucket_base, uint32_t nbins, K *out_keys, uint32_t *out_counts,
-                               uint64_t *bin_out, const uint32_t *err) {
+                               uint64_t *bin_out, const uint32_t *bucket_head, const uint4 *tasks,
+                               const unsigned long long *task_count, const uint32_t *err) {
   if (*err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   constexpr int U = 4;
   const uint64_t nb = bucket_base[nbins];
@@ -1632,39 +1738,56 @@ __global__ void k_compact_runs(const K *stage_keys, const uint32_t *stage_counts
   const uint32_t parts = nb == 0 || nb >= warps ? 1 : (uint32_t)min(warps / nb, (uint64_t)32);
   for (uint64_t x = t >> 5; x < nb * parts; x += warps) {
     const uint64_t g = x / parts;
-    const uint64_t s = bucket_start[g], d = bucket_d[g], o = bucket_out[g];
-    for (uint64_t i0 = (x - g * parts) * 32 * U + lane; i0 < d; i0 += (uint64_t)parts * 32 * U) {
-      K kv[U];
-      uint32_t cv[U];
+    uint64_t s = bucket_start[g], d = bucket_d[g], o = bucket_out[g];
+    const uint64_t start = s;
+    uint64_t t = bucket_head[g];  // first task + 1, 0: none
+    const uint64_t nt2 = t ? *task_count : 0;
+    while (true) {
+      if (t) {
+        if (t > nt2 || tasks[t - 1].x != (uint32_t)g) break;
+        s = start + tasks[t - 1].y;
+        d = tasks[t - 1].w;
+        t++;
+      }
+      for (uint64_t i0 = (x - g * parts) * 32 * U + lane; i0 < d; i0 += (uint64_t)parts * 32 * U) {
+        K kv[U];
+        uint32_t cv[U];
 #pragma unroll
-      for (int u = 0; u < U; u++)
-        if (i0 + 32 * u < d) {
-          kv[u] = stage_keys[s + i0 + 32 * u];
-          cv[u] = stage_counts[s + i0 + 32 * u];
-        }
+        for (int u = 0; u < U; u++)
+          if (i0 + 32 * u < d) {
+            kv[u] = stage_keys[s + i0 + 32 * u];
+            cv[u] = stage_counts[s + i0 + 32 * u];
+          }
 #pragma unroll
-      for (int u = 0; u < U; u++)
-        if (i0 + 32 * u < d) {
-          out_keys[o + i0 + 32 * u] = kv[u];
-          out_counts[o + i0 + 32 * u] = cv[u];
-        }
+        for (int u = 0; u < U; u++)
+          if (i0 + 32 * u < d) {
+            out_keys[o + i0 + 32 * u] = kv[u];
+            out_counts[o + i0 + 32 * u] = cv[u];
+          }
+      }
+      if (!t) break;
+      o += d;
     }
   }
 }
 
 template __global__ void k_compact_runs<uint64_t>(const uint64_t *, const uint32_t *, const uint64_t *,
                                                   const unsigned long long *, const uint64_t *, const uint64_t *,
-                                                  uint32_t, uint64_t *, uint32_t *, uint64_t *, const uint32_t *);
+                                                  uint32_t, uint64_t *, uint32_t *, uint64_t *, const uint32_t *,
+                                                  const uint4 *, const unsigned long long *, const uint32_t *);
 template __global__ void k_compact_runs<u128>(const u128 *, const uint32_t *, const uint64_t *,
                                               const unsigned long long *, const uint64_t *, const uint64_t *,
-                                              uint32_t, u128 *, uint32_t *, uint64_t *, const uint32_t *);
+                                              uint32_t, u128 *, uint32_t *, uint64_t *, const uint32_t *,
+                                              const uint4 *, const unsigned long long *, const uint32_t *);
 template __global__ void k_bucket_hist<uint64_t>(ExpandArgs);
 template __global__ void k_bucket_hist<u128>(ExpandArgs);
 template __global__ void k_bucket_scatter<uint64_t>(ExpandArgs);
 template __global__ void k_bucket_scatter<u128>(ExpandArgs);
 template __global__ void k_bucket_sort<uint64_t>(SortCountArgs);
 template __global__ void k_bucket_sort<u128>(SortCountArgs);
-template __global__ void k_bucket_count<uint64_t>(SortCountArgs);
-template __global__ void k_bucket_count<u128>(SortCountArgs);
+template __global__ void k_bucket_open<uint64_t>(SortCountArgs);
+template __global__ void k_bucket_open<u128>(SortCountArgs);
+template __global__ void k_bucket_slices<uint64_t>(SortCountArgs);
+template __global__ void k_bucket_slices<u128>(SortCountArgs);
 
 }  // namespace gkc

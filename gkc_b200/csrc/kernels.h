@@ -75,7 +75,7 @@ struct CountPlan {
   uint64_t *bucket_base;       // first bucket of each bin (nbins+1)
   uint64_t *chunk_base;        // first chunk of each bin (nbins+1)
   uint64_t *hist_base;         // first (digit, chunk) entry of each bin (nbins+1)
-  unsigned long long *tickets; // 4, zeroed
+  unsigned long long *tickets; // 6, zeroed
 };
 __global__ void k_count_plan(CountPlan pl);
 constexpr int kCountPlanThreads = 1024;
@@ -105,6 +105,7 @@ struct ExpandArgs {
   uint32_t *big_list;          // buckets of at least big_min keys (listed by the scan, counted first)
   unsigned long long *big_count;  // zeroed
   uint64_t big_min;
+  uint32_t *bucket_head;      // zeroed by the scan
   uint32_t *err;
 };
 __global__ void k_chunk_first(ExpandArgs a);
@@ -133,20 +134,28 @@ struct SortCountArgs {
   uint32_t *big_list;             // buckets of at least big_min keys (from the scan), then rejected ones
   unsigned long long *big_count;
   unsigned long long *big_ticket;  // zeroed
+  // slices of opened buckets: bucket, offset in it, keys, distinct keys; a
+  // bucket's tasks follow one another
+  uint4 *tasks;
+  uint64_t task_cap;
+  unsigned long long *task_count, *task_ticket;  // zeroed
+  uint32_t *bucket_head;           // first task + 1 of each bucket, 0: none (zeroed by the scan)
   uint64_t big_min;
   uint32_t *err;
 };
 template <typename K> __global__ void k_bucket_sort(SortCountArgs a);
 template <typename K> size_t bucket_sort_smem_bytes();
 constexpr int kBucketSortThreads = 256;
-template <typename K> __global__ void k_bucket_count(SortCountArgs a);
+template <typename K> __global__ void k_bucket_open(SortCountArgs a);
+template <typename K> __global__ void k_bucket_slices(SortCountArgs a);
 template <typename K> size_t bucket_count_smem_bytes();
 template <typename K> uint64_t bucket_count_cap();  // largest bucket of k_bucket_sort
 template <typename K>
 __global__ void k_compact_runs(const K *stage_keys, const uint32_t *stage_counts, const uint64_t *bucket_start,
                                const unsigned long long *bucket_d, const uint64_t *bucket_out,
                                const uint64_t *bucket_base, uint32_t nbins, K *out_keys, uint32_t *out_counts,
-                               uint64_t *bin_out, const uint32_t *err);
+                               uint64_t *bin_out, const uint32_t *bucket_head, const uint4 *tasks,
+                               const unsigned long long *task_count, const uint32_t *err);
 constexpr int kBucketCountThreads = 512;
 constexpr uint32_t kCoarseTarget = 8192;
 // Keys of a bucket for a tuned target (an upper bound of the mean): at the

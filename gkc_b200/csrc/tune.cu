@@ -205,7 +205,7 @@ gkc_status gkc_autotune_device(gkc_ctx *c, const gkc_params *prm, const char *d_
     ps.nbins = std::max(1, (int)((double)prm->nbins * (double)nb / (double)n_bytes + 0.5));
   int occ = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-      &occ, prm->k <= 32 ? (const void *)gkc::k_bucket_count<uint64_t> : (const void *)gkc::k_bucket_count<u128>,
+      &occ, prm->k <= 32 ? (const void *)gkc::k_bucket_slices<uint64_t> : (const void *)gkc::k_bucket_slices<u128>,
       gkc::kBucketCountThreads,
       prm->k <= 32 ? gkc::bucket_count_smem_bytes<uint64_t>() : gkc::bucket_count_smem_bytes<u128>());
   gkc_tune_params cur = rep.defaults;
