@@ -607,9 +607,9 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   uint32_t max_bits = kCoarseMaxBits;
   while (max_bits > 0 && ((uint64_t)nbins << max_bits) > (1ull << 20)) max_bits--;
   const uint32_t bucket_keys = bucket_target<K>(c->tune.coarse_target ? c->tune.coarse_target : kCoarseTarget);
-  // a bin has a bucket per bucket_keys keys, or one per digit where the digits hold more than half of that
+  // any two neighbouring buckets of a bin hold more than bucket_keys keys
   const uint64_t max_buckets =
-      std::min<uint64_t>((uint64_t)nbins << max_bits, keys_cap / (bucket_keys / 2) + nbins + 1);
+      std::min<uint64_t>((uint64_t)nbins << max_bits, keys_cap / bucket_keys * 2 + 2 + nbins);
   const uint64_t cap_skm = std::max<uint64_t>(c->part_cap_skm, 1);
   WS(err, uint32_t, "err", 4);
   const unsigned long long *n_skm_dev = (const unsigned long long *)c->bufs["cursors"].p;
@@ -638,11 +638,11 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   pl.k = prm->k;
   pl.err = err;
   pl.bin_bits = bin_bits;
-  pl.bucket_base = bucket_base;
   pl.chunk_base = chunk_base;
   pl.hist_base = hist_base;
-  // [0] bucket ticket, [2] large buckets listed, [3] their ticket, [4] slices listed, [5] their ticket
-  WS(ticket, unsigned long long, "count_ticket", 6);
+  // [0] bucket ticket, [2] large buckets listed, [3] their ticket, [4] slices listed, [5] their ticket,
+  // [6] bins scanned
+  WS(ticket, unsigned long long, "count_ticket", 8);
   pl.tickets = ticket;
   k_count_plan<<<1, kCountPlanThreads, 0, c->st>>>(pl);
   LAUNCHED(c);
@@ -653,6 +653,8 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   WS(hist, uint32_t, "bucket_hist", max_chunks << max_bits);
   WS(lut, uint16_t, "bucket_lut", (uint64_t)nbins << max_bits);
   WS(digit_total, uint32_t, "digit_total", (uint64_t)nbins << max_bits);
+  WS(unit_start, uint32_t, "unit_start", (uint64_t)nbins << max_bits);
+  WS(bin_units, uint32_t, "bin_units", nbins);
   WS(keys, K, "keys", keys_cap);
   // the result's key array holds the k-mer-order keys until the count stage is done with them
   WS(out_keys, K, slot_name(c, "out_keys").c_str(), keys_cap);
@@ -676,6 +678,9 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   ea.hist = hist;
   ea.lut = lut;
   ea.digit_total = digit_total;
+  ea.unit_start = unit_start;
+  ea.bin_units = bin_units;
+  ea.scan_done = ticket + 6;
   ea.max_bits = max_bits;
   ea.bucket_keys = bucket_keys;
   ea.keys = keys;
@@ -685,7 +690,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   const uint64_t first_n = std::max(32 * max_chunks, ((uint64_t)nbins << max_bits) / 8);
   k_chunk_first<<<(unsigned)std::min<uint64_t>((first_n + 255) / 256, 65535), 256, 0, c->st>>>(ea);
   LAUNCHED(c);
-  k_bucket_hist<K><<<c->n_sms * 8, kBucketHistThreads, 0, c->st>>>(ea);
+  k_bucket_hist<K><<<(unsigned)std::min<uint64_t>(max_chunks, (uint64_t)c->n_sms * 8), kBucketHistThreads, 0, c->st>>>(ea);
   LAUNCHED(c);
   WS(big_list, uint32_t, "big_list", max_buckets + 1);
   WS(bucket_head, uint32_t, "bucket_head", max_buckets + 1);
@@ -693,16 +698,16 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   ea.big_list = big_list;
   ea.big_count = ticket + 2;
   ea.big_min = bucket_count_cap<K>() + 1;
-  k_bucket_scan<<<std::min<uint32_t>(nbins, 65535), kBucketScanThreads, 0, c->st>>>(ea, bstart, bsize);
+  k_bucket_scan<<<std::min<uint32_t>(nbins, 65535), kBucketScanThreads, 0, c->st>>>(ea);
   LAUNCHED(c);
   k_bucket_offsets<<<(unsigned)std::min<uint64_t>((32 * max_buckets + kBucketOffsetThreads - 1) / kBucketOffsetThreads,
                                                   (uint64_t)c->n_sms * 64),
-                     kBucketOffsetThreads, 0, c->st>>>(ea, bstart);
+                     kBucketOffsetThreads, 0, c->st>>>(ea, bstart, bsize);
   LAUNCHED(c);
   stage_mark(c, 4);
   const size_t sct_smem = bucket_scatter_smem_bytes<K>();
   if ((int)sct_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "scatter tile exceeds shared memory");
-  k_bucket_scatter<K><<<c->n_sms, kBucketScatterThreads, sct_smem, c->st>>>(ea);
+  k_bucket_scatter<K><<<(unsigned)std::min<uint64_t>(max_chunks, (uint64_t)c->n_sms), kBucketScatterThreads, sct_smem, c->st>>>(ea);
   LAUNCHED(c);
 
   // counting: buckets independently, each bucket's runs staged over its own
@@ -748,13 +753,14 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   if ((int)sort_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "sort areas exceed shared memory");
   int sort_occ = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sort_occ, k_bucket_sort<K>, kBucketSortThreads, sort_smem));
-  k_bucket_sort<K><<<c->n_sms * std::max(sort_occ, 1), kBucketSortThreads, sort_smem, c->st>>>(sa);
+  k_bucket_sort<K><<<(unsigned)std::min<uint64_t>(max_buckets, (uint64_t)c->n_sms * std::max(sort_occ, 1)), kBucketSortThreads, sort_smem, c->st>>>(sa);
   LAUNCHED(c);
   // the large and rejected buckets, persistent, taken by ticket
   const int ctas = std::max(1, std::min(occ, c->tune.count_ctas ? (int)c->tune.count_ctas : 2));
-  k_bucket_open<K><<<c->n_sms * ctas, kBucketCountThreads, smem, c->st>>>(sa);
+  const unsigned open_grid = (unsigned)std::min<uint64_t>(keys_cap / bucket_count_cap<K>() + 1, (uint64_t)c->n_sms * ctas);
+  k_bucket_open<K><<<open_grid, kBucketCountThreads, smem, c->st>>>(sa);
   LAUNCHED(c);
-  k_bucket_slices<K><<<c->n_sms * ctas, kBucketCountThreads, smem, c->st>>>(sa);
+  k_bucket_slices<K><<<open_grid, kBucketCountThreads, smem, c->st>>>(sa);
   LAUNCHED(c);
   stage_mark(c, 6);
   // final offsets: the exclusive scan of the distinct counts (the bucket count is read on the device)

@@ -102,46 +102,32 @@ GKC_DEV uint32_t plan_bits(uint64_t nk, uint32_t bucket_keys, uint32_t max_bits,
     while (bits < max_bits && bits < key_bits && (nk >> bits) > bucket_keys / 8) bits++;
   return bits;
 }
-// Whether each digit is a bucket of its own: digits too large to be packed.
-GKC_DEV bool plan_whole(uint64_t nk, uint32_t bucket_keys, uint32_t bits) {
-  return bits == 0 || (nk >> bits) > bucket_keys / 2;
-}
-// Buckets of the bin: a bucket takes the digits that start within its span of
-// bucket_keys keys.
-GKC_DEV uint64_t plan_buckets(uint64_t nk, uint32_t bucket_keys, uint32_t bits) {
-  return plan_whole(nk, bucket_keys, bits) ? 1ull << bits : (nk + bucket_keys - 1) / bucket_keys;
-}
-
-// One CTA: the digits, buckets and chunks of every bin and their prefixes
+// One CTA: the digits and chunks of every bin and the chunks' prefixes
 // (one bin per thread; one thread for all bins took 71-134 us at 256 bins).
 __global__ void __launch_bounds__(kCountPlanThreads) k_count_plan(CountPlan pl) {
   constexpr int NT = kCountPlanThreads;
   __shared__ uint64_t tmp[32];
   const bool dead = (*pl.err & (ERR_CAPACITY | ERR_BAD_READ)) != 0;
-  uint64_t bb = 0, cb = 0, hb = 0;
+  uint64_t cb = 0, hb = 0;
   for (uint32_t b0 = 0; b0 < pl.nbins; b0 += NT) {
     const uint32_t b = b0 + threadIdx.x;
     const bool in = b < pl.nbins;
     const uint64_t nk = dead || !in ? 0 : pl.bin_kstart[b + 1] - pl.bin_kstart[b];
     const uint32_t bits = plan_bits(nk, pl.bucket_keys, pl.max_bits, 2 * pl.k);
     const uint64_t nch = (nk + pl.chunk_kmers - 1) / pl.chunk_kmers;
-    uint64_t nb, nc, nh;
-    const uint64_t ob = block_exclusive_scan_u64<NT>(in ? plan_buckets(nk, pl.bucket_keys, bits) : 0ull, tmp, &nb);
+    uint64_t nc, nh;
     const uint64_t oc = block_exclusive_scan_u64<NT>(nch, tmp, &nc);
     const uint64_t oh = block_exclusive_scan_u64<NT>(nch << bits, tmp, &nh);
     if (in) {
       pl.bin_bits[b] = bits;
-      pl.bucket_base[b] = bb + ob;
       pl.chunk_base[b] = cb + oc;
       pl.hist_base[b] = hb + oh;
     }
-    bb += nb;
     cb += nc;
     hb += nh;
   }
-  if (threadIdx.x < 6) pl.tickets[threadIdx.x] = 0;
+  if (threadIdx.x < 8) pl.tickets[threadIdx.x] = 0;
   if (threadIdx.x == 0) {
-    pl.bucket_base[pl.nbins] = bb;
     pl.chunk_base[pl.nbins] = cb;
     pl.hist_base[pl.nbins] = hb;
   }
@@ -157,15 +143,6 @@ GKC_DEV uint64_t warp_last_le(const uint64_t *a, uint64_t lo, uint64_t hi, uint6
     const uint32_t le = __ballot_sync(0xffffffffu, at <= hi && __ldg(a + at) <= x);
     lo += (uint64_t)(__popc(le) - 1) * step;
     hi = min(hi, lo + step - 1);
-  }
-  return lo;
-}
-
-GKC_DEV uint32_t find_bin(const uint64_t *base, uint32_t nbins, uint64_t c) {
-  uint32_t lo = 0, hi = nbins - 1;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi + 1) >> 1;
-    if (base[mid] <= c) lo = mid; else hi = mid - 1;
   }
   return lo;
 }
@@ -383,29 +360,31 @@ __global__ void __launch_bounds__(HS_NT) k_bucket_hist(ExpandArgs a) {
 
 // ----------------------------------------------------------------- 2. scan
 
-// One CTA per bin: the exclusive scan of the bin's digit totals; the digits
-// packed into buckets (a bucket takes those that start within its span of
-// keys, so buckets are even where digits are not: the keys of a minimizer bin
-// crowd at the minimizers' own values); the buckets' starts and sizes.
+// One CTA per bin: the exclusive scan of the bin's digit totals, and the digits
+// packed into buckets: as many consecutive digits as hold at most bucket_keys
+// keys, at least one.  So buckets are full although digits are uneven (the
+// keys of a minimizer bin crowd at the minimizers' own values; with a bucket's
+// bounds at multiples of a span, 22% of the keys of compressed long reads lay
+// in buckets too large for k_bucket_sort).  Each digit's successor as the
+// first of a bucket is found by a search, the firsts from digit 0 on by
+// doubling.  The last CTA to finish adds up the bins' buckets.
 constexpr int BS_NT = 1024;
-__global__ void __launch_bounds__(BS_NT) k_bucket_scan(ExpandArgs a, uint64_t *bucket_start,
-                                                       uint64_t *bucket_size) {
-  __shared__ uint32_t tmp[64];
-  __shared__ uint32_t first[1 << kCoarseMaxBits];  // start of every bucket, relative to the bin
+__global__ void __launch_bounds__(BS_NT) k_bucket_scan(ExpandArgs a) {
   constexpr int DPT = (1 << kCoarseMaxBits) / BS_NT;
+  __shared__ uint32_t tmp[64];
+  __shared__ uint64_t tmp64[32];
+  __shared__ uint32_t start[(1 << kCoarseMaxBits) + 1];
+  __shared__ uint16_t jump[1 << kCoarseMaxBits];
+  __shared__ uint8_t mark[(1 << kCoarseMaxBits) + 1];
+  __shared__ bool done;
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
+  const int tid = threadIdx.x;
   for (uint32_t b = blockIdx.x; b < a.nbins; b += gridDim.x) {
     const uint32_t bits = a.bin_bits[b], nd = 1u << bits;
     const uint64_t nk = a.bin_kstart[b + 1] - a.bin_kstart[b];
-    const uint64_t g0 = a.bucket_base[b];
-    const uint32_t nu = (uint32_t)(a.bucket_base[b + 1] - g0);  // at most nd
-    if (nk >= (1ull << 32)) {  // offsets in a bin are 32-bit
-      if (threadIdx.x == 0) atomicOr(a.err, ERR_BIN_TOO_LARGE);
-      continue;
-    }
-    const bool whole = plan_whole(nk, a.bucket_keys, bits);
+    if (nk >= (1ull << 32) && tid == 0) atomicOr(a.err, ERR_BIN_TOO_LARGE);  // offsets in a bin are 32-bit
     // thread t holds the contiguous digits [t * DPT, t * DPT + DPT)
-    const uint32_t d0 = threadIdx.x * DPT;
+    const uint32_t d0 = tid * DPT;
     const uint32_t *total = a.digit_total + ((uint64_t)b << a.max_bits);
     uint32_t col[DPT], s = 0;
 #pragma unroll
@@ -413,41 +392,95 @@ __global__ void __launch_bounds__(BS_NT) k_bucket_scan(ExpandArgs a, uint64_t *b
       col[u] = d0 + u < nd ? total[d0 + u] : 0u;
       s += col[u];
     }
-    for (uint32_t u = threadIdx.x; u < nu; u += BS_NT) first[u] = ~0u;
     uint32_t tot;
-    uint32_t at = block_exclusive_scan<BS_NT>(s, tmp, &tot);  // ends with a barrier
+    uint32_t at = block_exclusive_scan<BS_NT>(s, tmp, &tot);
+#pragma unroll
+    for (int u = 0; u < DPT; u++) {
+      if (d0 + u < nd) {
+        start[d0 + u] = at;
+        mark[d0 + u] = d0 + u == 0;
+      }
+      at += col[u];
+    }
+    if (tid == 0) {
+      start[nd] = tot;
+      mark[nd] = 0;
+    }
+    __syncthreads();
+    uint32_t next[DPT];
+#pragma unroll
+    for (int u = 0; u < DPT; u++) {
+      const uint32_t d = d0 + u;
+      next[u] = nd;
+      if (d < nd) {
+        uint32_t lo = d + 1, hi = nd;  // the last first digit of a next bucket that leaves this one small enough
+        while (lo < hi) {
+          const uint32_t mid = (lo + hi + 1) >> 1;
+          if (start[mid] - start[d] <= a.bucket_keys) lo = mid; else hi = mid - 1;
+        }
+        next[u] = lo;
+        jump[d] = (uint16_t)lo;
+      }
+    }
+    __syncthreads();
+    for (uint32_t r = 0; r < bits; r++) {  // marks after 2^r, .. jumps; next[u] = jump[d], nd stays nd
+#pragma unroll
+      for (int u = 0; u < DPT; u++)
+        if (d0 + u < nd && mark[d0 + u]) mark[next[u]] = 1;
+#pragma unroll
+      for (int u = 0; u < DPT; u++)
+        if (next[u] < nd) next[u] = jump[next[u]];
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < DPT; u++)
+        if (d0 + u < nd) jump[d0 + u] = (uint16_t)next[u];
+      __syncthreads();
+    }
+    uint32_t begins = 0;
+#pragma unroll
+    for (int u = 0; u < DPT; u++)
+      if (d0 + u < nd && mark[d0 + u]) begins |= 1u << u;
+    uint32_t n_units;
+    uint32_t unit = block_exclusive_scan<BS_NT>(__popc(begins), tmp, &n_units);
 #pragma unroll
     for (int u = 0; u < DPT; u++) {
       const uint32_t d = d0 + u;
       if (d < nd) {
-        const uint32_t unit = whole ? d : min(at / a.bucket_keys, nu - 1);
-        a.lut[((uint64_t)b << a.max_bits) + d] = (uint16_t)unit;
-        atomicMin(&first[unit], at);
-        at += col[u];
+        unit += (begins >> u) & 1u;
+        a.lut[((uint64_t)b << a.max_bits) + d] = (uint16_t)(unit - 1);
+        if ((begins >> u) & 1u) a.unit_start[((uint64_t)b << a.max_bits) + unit - 1] = start[d];
       }
     }
-    __syncthreads();
-    for (uint32_t u = threadIdx.x; u < nu; u += BS_NT) {
-      const uint32_t st = first[u];
-      uint32_t next = u + 1;  // buckets in which no digit starts are empty
-      while (next < nu && first[next] == ~0u) next++;
-      const uint32_t end = next < nu ? first[next] : (uint32_t)nk;
-      const uint64_t size = st == ~0u ? 0 : end - st;
-      bucket_start[g0 + u] = a.bin_kstart[b] + (st == ~0u ? end : st);
-      bucket_size[g0 + u] = size;
-      a.bucket_head[g0 + u] = 0;
-      if (size >= a.big_min) a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)(g0 + u);
-    }
-    __syncthreads();
+    if (tid == 0) a.bin_units[b] = n_units;
+    __syncthreads();  // before the areas are written again
   }
+  // the last CTA: first bucket of every bin
+  if (tid == 0) {
+    __threadfence();
+    done = atomicAdd(a.scan_done, 1ull) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!done) return;
+  __threadfence();
+  uint64_t base = 0;
+  for (uint32_t b0 = 0; b0 < a.nbins; b0 += BS_NT) {
+    const uint32_t b = b0 + tid;
+    uint64_t n;
+    const uint64_t o = block_exclusive_scan_u64<BS_NT>(b < a.nbins ? *(volatile uint32_t *)(a.bin_units + b) : 0ull, tmp64, &n);
+    if (b < a.nbins) a.bucket_base[b] = base + o;
+    base += n;
+  }
+  if (tid == 0) a.bucket_base[a.nbins] = base;
 }
 
-// Every chunk's write offset per bucket, relative to the bin's first key: a
-// warp per bucket adds up its digits in 32 chunks at a time, one a lane, and
-// leaves each offset at the count of the bucket's first digit.  (A thread per
+// Each bucket's start and size, and every chunk's write offset per bucket,
+// relative to the bin's first key: a warp per bucket adds up its digits in 32
+// chunks at a time, one a lane, and leaves each offset at the count of the
+// bucket's first digit.  (A thread per
 // bucket walked hundreds of chunks of a large bin one after the other: 524 us
 // where bins are uneven.)
-__global__ void __launch_bounds__(kBucketOffsetThreads) k_bucket_offsets(ExpandArgs a, const uint64_t *bucket_start) {
+__global__ void __launch_bounds__(kBucketOffsetThreads) k_bucket_offsets(ExpandArgs a, uint64_t *bucket_start,
+                                                                         uint64_t *bucket_size) {
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   const uint64_t n_buckets = a.bucket_base[a.nbins];
   const uint32_t lane = threadIdx.x & 31u;
@@ -467,10 +500,19 @@ __global__ void __launch_bounds__(kBucketOffsetThreads) k_bucket_offsets(ExpandA
       const uint32_t mid = (hi + h) >> 1;
       if (lut[mid] <= u) hi = mid + 1; else h = mid;
     }
-    if (lo == hi) continue;  // no digit starts in it
+    const uint32_t *us = a.unit_start + ((uint64_t)b << a.max_bits) + u;
+    uint32_t run = us[0];
+    const uint64_t k0 = a.bin_kstart[b];
+    const uint32_t end = u + 1 < a.bin_units[b] ? us[1] : (uint32_t)(a.bin_kstart[b + 1] - k0), size = end - run;
+    if (lane == 0) {
+      bucket_start[g] = k0 + run;
+      bucket_size[g] = size;
+      a.bucket_head[g] = 0;
+      if (size >= a.big_min) a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)g;
+    }
+    if (size == 0) continue;
     const uint64_t nch = a.chunk_base[b + 1] - a.chunk_base[b];
     uint32_t *M = a.hist + a.hist_base[b];
-    uint32_t run = (uint32_t)(bucket_start[g] - a.bin_kstart[b]);
     for (uint64_t j0 = 0; j0 < nch; j0 += 32) {
       const uint64_t jj = j0 + lane;
       uint32_t v = 0;
@@ -1414,7 +1456,9 @@ __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket
         }
 #pragma unroll
         for (uint32_t j = 0; j < CC_TICKETS; j++)
-          if (sz[j] < a.big_min) {
+          if (sz[j] == 0) {
+            a.bucket_d[t0 + j] = 0;
+          } else if (sz[j] < a.big_min) {
             S.bg[bm] = t0 + j;
             S.bstart[bm] = st[j];
             S.bn[bm] = (uint32_t)sz[j];

@@ -65,17 +65,16 @@ struct CountPlan {
   uint32_t nbins;
   const uint64_t *bin_start;   // superkmers per bin (exclusive prefix, nbins+1)
   const uint64_t *bin_kstart;  // k-mers per bin (exclusive prefix, nbins+1)
-  uint32_t bucket_keys;        // keys of a bucket
+  uint32_t bucket_keys;        // most keys of a bucket of several digits
   uint32_t max_bits;           // digit bits cap (<= kCoarseMaxBits)
   uint64_t chunk_kmers;        // k-mers per expansion chunk
   int k;
   const uint32_t *err;         // nothing is planned after an upstream overflow
   // outputs
   uint32_t *bin_bits;          // digit bits per bin
-  uint64_t *bucket_base;       // first bucket of each bin (nbins+1)
   uint64_t *chunk_base;        // first chunk of each bin (nbins+1)
   uint64_t *hist_base;         // first (digit, chunk) entry of each bin (nbins+1)
-  unsigned long long *tickets; // 6, zeroed
+  unsigned long long *tickets; // 8, zeroed
 };
 __global__ void k_count_plan(CountPlan pl);
 constexpr int kCountPlanThreads = 1024;
@@ -89,7 +88,7 @@ struct ExpandArgs {
   const uint64_t *bin_kstart;
   const uint64_t *chunk_base;
   const uint64_t *hist_base;
-  const uint64_t *bucket_base;
+  uint64_t *bucket_base;       // first bucket of each bin (written by the scan)
   const uint32_t *bin_bits;
   uint64_t chunk_kmers;
   int k;
@@ -105,13 +104,16 @@ struct ExpandArgs {
   uint32_t *big_list;          // buckets of at least big_min keys (listed by the scan, counted first)
   unsigned long long *big_count;  // zeroed
   uint64_t big_min;
-  uint32_t *bucket_head;      // zeroed by the scan
+  uint32_t *bucket_head;       // zeroed with the offsets
+  uint32_t *unit_start;        // start of each bucket of a bin, 1 << max_bits entries per bin
+  uint32_t *bin_units;         // buckets of each bin
+  unsigned long long *scan_done;  // zeroed
   uint32_t *err;
 };
 __global__ void k_chunk_first(ExpandArgs a);
 template <typename K> __global__ void k_bucket_hist(ExpandArgs a);
-__global__ void k_bucket_scan(ExpandArgs a, uint64_t *bucket_start, uint64_t *bucket_size);
-__global__ void k_bucket_offsets(ExpandArgs a, const uint64_t *bucket_start);
+__global__ void k_bucket_scan(ExpandArgs a);
+__global__ void k_bucket_offsets(ExpandArgs a, uint64_t *bucket_start, uint64_t *bucket_size);
 constexpr int kBucketOffsetThreads = 128;
 template <typename K> __global__ void k_bucket_scatter(ExpandArgs a);
 constexpr int kBucketScanThreads = 1024;
@@ -139,7 +141,7 @@ struct SortCountArgs {
   uint4 *tasks;
   uint64_t task_cap;
   unsigned long long *task_count, *task_ticket;  // zeroed
-  uint32_t *bucket_head;           // first task + 1 of each bucket, 0: none (zeroed by the scan)
+  uint32_t *bucket_head;           // first task + 1 of each bucket, 0: none (zeroed before)
   uint64_t big_min;
   uint32_t *err;
 };
@@ -158,11 +160,14 @@ __global__ void k_compact_runs(const K *stage_keys, const uint32_t *stage_counts
                                const unsigned long long *task_count, const uint32_t *err);
 constexpr int kBucketCountThreads = 512;
 constexpr uint32_t kCoarseTarget = 8192;
-// Keys of a bucket for a tuned target (an upper bound of the mean): at the
-// default target 2816 8-byte or 1536 16-byte keys, so that with the digit
-// that passes the span a bucket still fits the 4096 (3072) of k_bucket_sort.
+// Most keys of a bucket of several digits for a tuned target (an upper bound of
+// the mean): at the default target 3584 8-byte or 3072 16-byte keys, of the
+// 4096 (3072) that k_bucket_sort takes.  (900 M bases at k 31: 28.8 ms with
+// 3072, 28.3 with 3584, 28.0 with 4096, but mostly distinct long reads 7.3 ms
+// with 3584 and 7.4 with either; k 63: 7.1 ms with 2048, 6.8 with 2560, 6.7
+// with 3072.)
 template <typename K> constexpr uint32_t bucket_target(uint32_t target) {
-  return sizeof(K) == 8 ? target / 16 * 11 / 2 : target / 16 * 3;
+  return sizeof(K) == 8 ? target / 16 * 7 : target / 8 * 3;
 }
 constexpr uint32_t kCoarseMaxBits = 12;
 constexpr uint64_t kChunkKmers = 65536;
