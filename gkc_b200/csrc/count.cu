@@ -544,19 +544,21 @@ template <typename K> constexpr int sc_tile() { return sizeof(K) == 8 ? 16384 : 
 // shared memory (a key's rank within its bucket from a shared-memory atomic),
 // then written out in that order, so the keys of one bucket leave as a
 // contiguous run at the chunk's write offset for the bucket (from the scan)
-// plus the bucket's keys of the chunk's earlier tiles.
+// plus the bucket's keys of the chunk's earlier tiles.  Bound by latency (one
+// CTA fills an SM's shared memory): the chunk's next tile is loaded into the
+// registers that this one's keys leave while it is written out.
 template <typename K>
 __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) {
   constexpr int SC_TILE = sc_tile<K>(), KPT = SC_TILE / SC_THREADS;
   constexpr int ND = 1 << kCoarseMaxBits;
   extern __shared__ __align__(16) uint8_t sc_smem[];
-  K *S = reinterpret_cast<K *>(sc_smem);                      // the tile, by digit
+  K *S = reinterpret_cast<K *>(sc_smem);                      // the tile, by bucket
   uint16_t *Sd = reinterpret_cast<uint16_t *>(S + SC_TILE);   // buckets of S
-  uint32_t *gbase = reinterpret_cast<uint32_t *>(Sd + SC_TILE);  // chunk's write offsets
-  uint32_t *done = gbase + ND;                                // bucket's keys of the chunk's earlier tiles
-  uint32_t *toff = done + ND;                                 // tile counts, then tile offsets (ND + 1)
-  uint16_t *lut = reinterpret_cast<uint16_t *>(toff + ND + 1 + 64);  // bucket of every digit
-  uint32_t *tmp = toff + ND + 1;                              // block scan
+  uint32_t *gbase = reinterpret_cast<uint32_t *>(Sd + SC_TILE);  // next write offset of every bucket
+  uint32_t *delta = gbase + ND;                               // write offset less tile position
+  uint32_t *toff = delta + ND;                                // tile counts, then tile offsets
+  uint32_t *tmp = toff + ND;                                  // block scan
+  uint16_t *lut = reinterpret_cast<uint16_t *>(tmp + 64);     // bucket of every digit
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   K *keys = reinterpret_cast<K *>(a.keys);
   const K *flat = reinterpret_cast<const K *>(a.flat);
@@ -571,52 +573,52 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
     const uint64_t kbase = a.bin_kstart[b];
     const uint64_t q0 = kbase + j * a.chunk_kmers;
     const uint64_t q1 = min(q0 + a.chunk_kmers, a.bin_kstart[b + 1]);
+    K xs[KPT];
+    auto load = [&](uint64_t t0) {
+#pragma unroll
+      for (int u = 0; u < KPT; u++) {
+        const uint64_t i = t0 + u * SC_THREADS + tid;
+        if (i < q1) xs[u] = flat[i];
+      }
+    };
+    load(q0);
     const uint32_t *row = a.hist + a.hist_base[b] + (j << cb);
-    for (uint32_t d = tid; d < nd; d += SC_THREADS) done[d] = 0;
     const uint16_t *glut = a.lut + ((uint64_t)b << a.max_bits);
     for (uint32_t d = tid; d < (1u << cb); d += SC_THREADS) {
       const uint16_t u = glut[d];
       lut[d] = u;
       if (d == 0 || glut[d - 1] != u) gbase[u] = row[d];  // the bucket's first digit holds its offset
     }
+    for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
+    __syncthreads();
     for (uint64_t t0 = q0; t0 < q1; t0 += SC_TILE) {
       const uint32_t tn = (uint32_t)min((uint64_t)SC_TILE, q1 - t0);
-      // the chunk's next tile into L2 while this one is sorted and written
-      constexpr int KPL = 128 / (int)sizeof(K);  // keys per line
-      for (uint64_t i = t0 + SC_TILE + (uint64_t)tid * KPL; i < q1 && i < t0 + 2 * (uint64_t)SC_TILE;
-           i += (uint64_t)SC_THREADS * KPL)
-        prefetch_l2(flat + i);
-      for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
-      __syncthreads();
-      K xs[KPT];
       uint32_t rk[KPT];  // bucket << 16 | rank within it (< SC_TILE)
 #pragma unroll
       for (int u = 0; u < KPT; u++) {
-        const uint32_t i = u * SC_THREADS + tid;
-        if (i < tn) {
-          xs[u] = flat[t0 + i];
+        if (u * SC_THREADS + tid < tn) {
           const uint32_t d = lut[coarse_digit<K>(xs[u], key_bits, cb)];
           rk[u] = (d << 16) | atomicAdd(&toff[d], 1u);
         }
       }
       __syncthreads();
-      // exclusive scan of the tile counts, thread-contiguous digits
+      // exclusive scan of the tile counts, thread-contiguous buckets
       const uint32_t per = (nd + SC_THREADS - 1) / SC_THREADS, d0 = tid * per;
       uint32_t sum = 0;
       for (uint32_t d = d0; d < d0 + per && d < nd; d++) sum += toff[d];
       uint32_t total;
       uint32_t run = block_exclusive_scan<SC_THREADS>(sum, tmp, &total);
       for (uint32_t d = d0; d < d0 + per && d < nd; d++) {
-        const uint32_t v = toff[d];
+        const uint32_t v = toff[d], g = gbase[d];
         toff[d] = run;
+        delta[d] = g - run;
+        gbase[d] = g + v;
         run += v;
       }
-      if (tid == 0) toff[nd] = total;
       __syncthreads();
 #pragma unroll
       for (int u = 0; u < KPT; u++) {
-        const uint32_t i = u * SC_THREADS + tid;
-        if (i < tn) {
+        if (u * SC_THREADS + tid < tn) {
           const uint32_t d = rk[u] >> 16;
           const uint32_t at = toff[d] + (rk[u] & 0xFFFFu);
           S[at] = xs[u];
@@ -624,15 +626,15 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
         }
       }
       __syncthreads();
+      if (t0 + SC_TILE < q1) load(t0 + SC_TILE);
+      for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
+#pragma unroll 4
       for (uint32_t i = tid; i < tn; i += SC_THREADS) {
-        const uint32_t d = Sd[i];
-        const uint64_t slot = kbase + gbase[d] + done[d] + (i - toff[d]);
+        const uint64_t slot = kbase + (uint32_t)(delta[Sd[i]] + i);
         if (slot < a.keys_cap) keys[slot] = S[i];
         else atomicOr(a.err, ERR_CAPACITY);
       }
-      __syncthreads();
-      for (uint32_t d = tid; d < nd; d += SC_THREADS) done[d] += toff[d + 1] - toff[d];
-      __syncthreads();  // before the next tile clears toff
+      __syncthreads();  // before the next tile's ranks and the next chunk's tables
     }
   }
 }
@@ -640,7 +642,7 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
 template <typename K> size_t bucket_scatter_smem_bytes() {
   constexpr int ND = 1 << kCoarseMaxBits;
   static_assert(sc_tile<K>() <= 65536 && sc_tile<K>() % SC_THREADS == 0, "16-bit ranks, whole rounds");
-  return (size_t)sc_tile<K>() * (sizeof(K) + 2) + 4 * (3 * ND + 1 + 64) + 2 * ND;
+  return (size_t)sc_tile<K>() * (sizeof(K) + 2) + 4 * (3 * ND + 64) + 2 * ND;
 }
 template size_t bucket_scatter_smem_bytes<uint64_t>();
 template size_t bucket_scatter_smem_bytes<u128>();
