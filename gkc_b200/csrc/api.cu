@@ -838,93 +838,110 @@ gkc_status gkc_count_device(gkc_ctx *c, const gkc_params *prm, gkc_mode mode, gk
 
 // -------------------------------------------------------------- pipeline
 
-// Batched: the whole partition -> count pipeline is enqueued once under
-// stream capture and replayed as a CUDA graph while inputs and parameters are
-// unchanged (one graph per buffer slot).  All sizes the kernels need are read
-// on the device.  With `async`, a replay is only enqueued: its totals land in
-// the slot's pinned totals and are checked by the caller after the stream.
+// The batched pipeline's launches, on the context stream.
+static gkc_status enqueue_pipeline(gkc_ctx *c, const gkc_params *prm, const GraphKey &key, const PipelineCaps &cap) {
+  c->launches = 0;
+  gkc_status s = enqueue_partition(c, prm, (const char *)key.reads, key.n_bytes, (const uint64_t *)key.offs, key.n_reads,
+                                   cap.skm, cap.bytes);
+  if (s == GKC_OK) s = enqueue_count(c, prm, cap.keys);
+  if (s == GKC_OK) s = read_totals(c, true, (uint32_t)prm->nbins);
+  return s;
+}
+
+// Grows the capacities to what the device reported.
+static void grow_caps(PipelineCaps *cap, const DevTotals *t) {
+  cap->skm = std::max<uint64_t>(cap->skm, t->n_skm + 16);
+  cap->bytes = std::max<uint64_t>(cap->bytes, t->n_packed + 64);
+  cap->keys = std::max<uint64_t>(cap->keys, t->n_kmers + 16);
+}
+
+// The launches as a graph: the workspaces were sized by a call with the same
+// key and capacities, and nothing was freed or grown since (G.seen).
+static gkc_status capture_pipeline(gkc_ctx *c, const gkc_params *prm, SlotGraph &G, bool async) {
+  // the replaced graph has ended: a streaming call waits for the slot's previous call before it comes here
+  if (!async) CK(cudaStreamSynchronize(c->st));
+  if (G.exec) {
+    cudaGraphExecDestroy(G.exec);
+    G.exec = nullptr;
+  }
+  cudaGraph_t g;
+  CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
+  c->capturing = true;
+  const gkc_status s = enqueue_pipeline(c, prm, G.key, G.cap);
+  const cudaError_t e = cudaStreamEndCapture(c->st, &g);
+  c->capturing = false;
+  if (s != GKC_OK) {
+    if (e == cudaSuccess) cudaGraphDestroy(g);
+    return s;
+  }
+  CK(e);
+  const cudaError_t ei = cudaGraphInstantiate(&G.exec, g, 0);
+  cudaGraphDestroy(g);
+  if (ei != cudaSuccess) G.exec = nullptr;
+  CK(ei);
+  G.launches = c->launches;
+  G.valid = true;
+  return GKC_OK;
+}
+
+// Batched: the first call with some inputs and parameters enqueues the
+// partition -> count pipeline launch by launch; the second one in a row (per
+// buffer slot) captures the same launches as a CUDA graph, which is replayed
+// from then on.  So inputs that are not run again pay for no capture, and a
+// streaming call of a new size waits for nothing: the sizing run, the wait for
+// it, the capture and the instantiation cost 1.7-2.7 ms of a 2.2 ms call when
+// every size was captured at its first call.  All sizes the kernels need are
+// read on the device.  With `async`, the pipeline is only enqueued: its totals
+// land in the slot's pinned totals and are checked by the caller after the
+// stream (`direct`, `cap_used`: how it was run, for a rerun).
 static gkc_status pipeline_batched(gkc_ctx *c, const gkc_params *prm, const char *d_reads,
                                    uint64_t n_bytes, const uint64_t *d_offs, uint64_t n_reads,
-                                   bool async = false) {
-  GraphKey key{d_reads, d_offs, n_bytes, n_reads, prm->k, prm->p, prm->hpc, prm->nbins, c->filter};
+                                   bool async = false, bool *direct = nullptr, PipelineCaps *cap_used = nullptr) {
+  const GraphKey key{d_reads, d_offs, n_bytes, n_reads, prm->k, prm->p, prm->hpc, prm->nbins, c->filter};
   SlotGraph &G = c->graphs[c->slot];
-  uint64_t cap_skm, cap_bytes;
-  partition_caps(prm, n_bytes, n_reads, &cap_skm, &cap_bytes);
-  const bool have = G.valid && G.key == key && G.exec;
-  if (have) {
-    cap_skm = c->part_cap_skm;
-    cap_bytes = c->part_cap_bytes;
+  PipelineCaps cap;
+  if (G.key == key && (G.seen || G.valid)) {
+    cap = G.cap;
+  } else {
+    partition_caps(prm, n_bytes, n_reads, &cap.skm, &cap.bytes);
+    cap.keys = std::max<uint64_t>(n_bytes, 16);
   }
-  uint64_t keys_cap = std::max<uint64_t>(n_bytes, 16);
-  if (have) keys_cap = c->count_keys_cap;
-  for (int attempt = 0; attempt < 3; attempt++) {
+  cudaStreamCaptureStatus cs;
+  CK(cudaStreamIsCapturing(c->st, &cs));
+  if (cs != cudaStreamCaptureStatusNone) return ctx_fail(c, GKC_ERR_INVALID_ARG, "stream already capturing");
+  for (int attempt = 0;; attempt++) {
+    gkc_status s = GKC_OK;
+    if (!(G.valid && G.key == key && G.exec) && G.seen && G.key == key && !c->one_shot) {
+      s = capture_pipeline(c, prm, G, async);
+      if (s != GKC_OK) {
+        G.seen = false;
+        return s;
+      }
+    }
     if (G.valid && G.key == key && G.exec) {
       CK(cudaGraphLaunch(G.exec, c->st));
       c->tm.graph_replayed = 1;
       c->launches = G.launches;
-      if (async) return GKC_OK;
     } else {
-      // allocate every workspace outside capture: one dry enqueue sizes them
-      c->launches = 0;
-      CK(cudaStreamSynchronize(c->st));
-      if (G.exec) {
-        cudaGraphExecDestroy(G.exec);
-        G.exec = nullptr;
-      }
-      cudaStreamCaptureStatus cs;
-      CK(cudaStreamIsCapturing(c->st, &cs));
-      if (cs != cudaStreamCaptureStatusNone) return ctx_fail(c, GKC_ERR_INVALID_ARG, "stream already capturing");
-      // size pass: plain enqueue (not captured) so that allocation happens now
-      gkc_status s = enqueue_partition(c, prm, d_reads, n_bytes, d_offs, n_reads, cap_skm, cap_bytes);
-      if (s == GKC_OK) s = enqueue_count(c, prm, keys_cap);
-      if (s == GKC_OK) s = read_totals(c, true, (uint32_t)prm->nbins);
+      G.valid = G.seen = false;
+      s = enqueue_pipeline(c, prm, key, cap);
       if (s != GKC_OK) return s;
-      CK(cudaStreamSynchronize(c->st));
-      if (c->one_shot && !(c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) {
-        c->tm.graph_replayed = 0;
-        break;
-      }
-      if (!(c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) {
-        // capture the same sequence into a graph for later replays
-        G.valid = true;
-        uint32_t launches = c->launches;
-        cudaGraph_t g;
-        CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-        c->capturing = true;
-        c->launches = 0;
-        s = enqueue_partition(c, prm, d_reads, n_bytes, d_offs, n_reads, cap_skm, cap_bytes);
-        if (s == GKC_OK) s = enqueue_count(c, prm, keys_cap);
-        if (s == GKC_OK) s = read_totals(c, true, (uint32_t)prm->nbins);
-        cudaError_t e = cudaStreamEndCapture(c->st, &g);
-        c->capturing = false;
-        if (s != GKC_OK) return s;
-        CK(e);
-        if (!G.valid) {  // a workspace moved during capture: do not keep it
-          cudaGraphDestroy(g);
-        } else {
-          CK(cudaGraphInstantiate(&G.exec, g, 0));
-          cudaGraphDestroy(g);
-          G.key = key;
-          G.launches = c->launches;
-        }
-        c->launches = launches;
-        c->tm.graph_replayed = 0;
-        break;
-      }
+      c->tm.graph_replayed = 0;
+      G.key = key;
+      G.cap = cap;
+      G.seen = true;
+    }
+    if (async) {
+      if (direct) *direct = !c->tm.graph_replayed;
+      if (cap_used) *cap_used = cap;
+      return GKC_OK;
     }
     CK(cudaStreamSynchronize(c->st));
     if (!(c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) break;
     // grow to the sizes the device reported and retry
     graphs_invalidate(c);
-    cap_skm = std::max<uint64_t>(cap_skm, c->h_tot->n_skm + 16);
-    cap_bytes = std::max<uint64_t>(cap_bytes, c->h_tot->n_packed + 64);
-    keys_cap = std::max<uint64_t>(keys_cap, c->h_tot->n_kmers + 16);
     if (attempt == 2) return ctx_fail(c, GKC_ERR_CAPACITY, "pipeline capacity");
-  }
-  CK(cudaStreamSynchronize(c->st));
-  if (c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH)) {
-    graphs_invalidate(c);
-    return ctx_fail(c, GKC_ERR_CAPACITY, "pipeline capacity");
+    grow_caps(&cap, c->h_tot);
   }
   gkc_status s = check_device_err(c);
   if (s != GKC_OK) return s;
@@ -1030,6 +1047,52 @@ __global__ void k_rebase_offs(uint64_t *offs, uint64_t n) {
   __syncthreads();
   if (threadIdx.x == 0) offs[0] = 0;
 }
+// The context on a streaming call's slot; every way out leaves it on slot 0.
+struct OnSlot {
+  gkc_ctx *c;
+  OnSlot(gkc_ctx *ctx, int slot) : c(ctx) {
+    c->slot = slot;
+    c->h_tot = c->h_tots[slot];
+  }
+  ~OnSlot() {
+    c->slot = 0;
+    c->h_tot = c->h_tots[0];
+  }
+};
+
+static void set_results(gkc_ctx *c, StreamCall &sc) {
+  sc.d_bin_off = c->bufs[slot_name(c, "bin_out")].p;
+  sc.d_keys = c->bufs[slot_name(c, "out_keys")].p;
+  sc.d_counts = c->bufs[slot_name(c, "counts")].p;
+}
+
+// A streaming call of a new size whose workspaces were too small for its
+// reads is run again with the sizes the device reported: its inputs stay in
+// the slot until its download is enqueued.  Waits for the device.
+static gkc_status rerun_larger(gkc_ctx *c, StreamCall &sc, int slot) {
+  OnSlot on(c, slot);
+  const int filter = c->filter;
+  c->filter = sc.key.filter;
+  gkc_status s = GKC_OK;
+  for (int attempt = 0; attempt < 2 && s == GKC_OK && (c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH)); attempt++) {
+    grow_caps(&sc.cap, c->h_tot);
+    graphs_invalidate(c);
+    s = enqueue_pipeline(c, &sc.prm, sc.key, sc.cap);
+    const cudaError_t e = cudaStreamSynchronize(c->st);
+    if (s == GKC_OK && e != cudaSuccess) s = ctx_cuda(c, e, "rerunning a streaming call");
+  }
+  c->filter = filter;
+  if (s != GKC_OK) return s;
+  set_results(c, sc);
+  SlotGraph &G = c->graphs[slot];
+  if (!(c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) {
+    G.key = sc.key;
+    G.cap = sc.cap;
+    G.seen = true;
+  }
+  return GKC_OK;
+}
+
 // The download of a streaming call: once its pipeline is done, its totals
 // (copied to page-locked memory inside the captured pipeline) give the exact
 // sizes, and three DMA copies on the download stream move the bin offsets,
@@ -1041,14 +1104,19 @@ static gkc_status issue_download(gkc_ctx *c, int rec) {
   if (sc.dl_issued) return GKC_OK;
   const int slot = (int)(sc.ticket & 1);
   CK(cudaEventSynchronize(c->ev_comp[slot]));
+  if (sc.direct && (c->h_tots[slot]->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) {
+    sc.status = rerun_larger(c, sc, slot);
+    if (sc.status != GKC_OK) sc.message = c->err;
+  }
   sc.tot = *c->h_tots[slot];  // the slot's next call overwrites them
   const DevTotals *h = &sc.tot;
-  const bool bad = (h->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH | ERR_BIN_TOO_LARGE | ERR_SPIN_TIMEOUT | ERR_BOUNDS |
+  const bool bad = sc.status != GKC_OK ||
+                   (h->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH | ERR_BIN_TOO_LARGE | ERR_SPIN_TIMEOUT | ERR_BOUNDS |
                               ERR_BAD_READ)) != 0;
   if (!bad) {
     const uint64_t nd = std::min<uint64_t>(h->n_distinct, sc.capacity);
     if (sc.h_bin_off)
-      CK(cudaMemcpyAsync(sc.h_bin_off, sc.d_bin_off, 8 * ((uint64_t)sc.nbins + 1), cudaMemcpyDeviceToHost, c->st_dl));
+      CK(cudaMemcpyAsync(sc.h_bin_off, sc.d_bin_off, 8 * ((uint64_t)sc.prm.nbins + 1), cudaMemcpyDeviceToHost, c->st_dl));
     if (sc.h_keys && nd)
       CK(cudaMemcpyAsync(sc.h_keys, sc.d_keys, nd * 8 * (uint64_t)sc.key_words, cudaMemcpyDeviceToHost, c->st_dl));
     if (sc.h_counts && nd)
@@ -1101,27 +1169,19 @@ gkc_status gkc_stream_submit(gkc_ctx *c, const gkc_params *prm, const char *read
   }
   // the slot's input buffers; growing them waits for everything in flight
   const uint64_t base = n_reads ? offs[0] : 0, nb = n_reads ? offs[n_reads] - base : 0;
-  c->slot = slot;
-  c->h_tot = c->h_tots[slot];
-  struct SlotReset {  // every return leaves the context on slot 0
-    gkc_ctx *c;
-    ~SlotReset() {
-      c->slot = 0;
-      c->h_tot = c->h_tots[0];
-    }
-  } reset{c};
-  const std::string rn = slot_name(c, "in_reads"), on = slot_name(c, "in_offs");
+  OnSlot on(c, slot);
+  const std::string rn = slot_name(c, "in_reads"), ofn = slot_name(c, "in_offs");
   auto fits = [&](const std::string &n, size_t bytes) {
     auto it = c->bufs.find(n);
     return it != c->bufs.end() && it->second.bytes >= bytes;
   };
-  if (!fits(rn, nb + 64) || !fits(on, 8 * (n_reads + 1))) {
+  if (!fits(rn, nb + 64) || !fits(ofn, 8 * (n_reads + 1))) {
     CK(cudaStreamSynchronize(c->st_up));
     CK(cudaStreamSynchronize(c->st_dl));
     CK(cudaStreamSynchronize(c->st));
   }
   WS(dr, char, rn.c_str(), nb + 64);
-  WS(doffs, uint64_t, on.c_str(), n_reads + 1);
+  WS(doffs, uint64_t, ofn.c_str(), n_reads + 1);
   // inputs of the slot's previous call must have been read before they are replaced
   if (t >= 2) CK(cudaStreamWaitEvent(c->st_up, c->ev_comp[slot], 0));
   if (nb) CK(cudaMemcpyAsync(dr, reads + base, nb, cudaMemcpyHostToDevice, c->st_up));
@@ -1135,20 +1195,19 @@ gkc_status gkc_stream_submit(gkc_ctx *c, const gkc_params *prm, const char *read
     LAUNCHED(c);
   }
   c->tm = gkc_timings{};
-  s = pipeline_batched(c, prm, dr, nb, doffs, n_reads, true);
+  StreamCall sc;
+  s = pipeline_batched(c, prm, dr, nb, doffs, n_reads, true, &sc.direct, &sc.cap);
   if (s != GKC_OK) return s;
   CK(cudaEventRecord(c->ev_comp[slot], c->st));
-  StreamCall sc;
+  sc.key = GraphKey{dr, doffs, nb, n_reads, prm->k, prm->p, prm->hpc, prm->nbins, c->filter};
+  sc.prm = *prm;
   sc.ticket = t;
   sc.capacity = capacity;
-  sc.nbins = (uint32_t)prm->nbins;
   sc.key_words = prm->k <= 32 ? 1 : 2;
   sc.h_bin_off = bin_off;
   sc.h_keys = keys;
   sc.h_counts = counts;
-  sc.d_bin_off = c->bufs[slot_name(c, "bin_out")].p;
-  sc.d_keys = c->bufs[slot_name(c, "out_keys")].p;
-  sc.d_counts = c->bufs[slot_name(c, "counts")].p;
+  set_results(c, sc);
   sc.dl_issued = false;
   sc.waited = false;
   c->calls[rec] = sc;
@@ -1176,6 +1235,7 @@ gkc_status gkc_stream_wait(gkc_ctx *c, uint64_t ticket, uint64_t *n_distinct, ui
   if (s != GKC_OK) return s;
   CK(cudaEventSynchronize(c->ev_dl[rec]));
   sc.waited = true;
+  if (sc.status != GKC_OK) return ctx_fail(c, sc.status, sc.message);
   const DevTotals *h = &sc.tot;
   if (n_distinct) *n_distinct = h->n_distinct;
   if (n_kmers) *n_kmers = h->n_kmers;

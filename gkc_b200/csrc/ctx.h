@@ -38,10 +38,17 @@ struct TuneChoice {
   uint32_t count_ctas = 0;     // count kernel CTAs per SM
 };
 
-// A captured batched pipeline for one buffer slot.
+// Capacities of the batched pipeline's workspaces.
+struct PipelineCaps {
+  uint64_t skm = 0, bytes = 0, keys = 0;
+};
+
+// The batched pipeline last run on a buffer slot.
 struct SlotGraph {
   bool valid = false;  // captured against the current workspaces and parameters
+  bool seen = false;   // run with `key` and `cap`; no workspace was freed or grown since
   GraphKey key{};
+  PipelineCaps cap;
   cudaGraphExec_t exec = nullptr;
   uint32_t launches = 0;
 };
@@ -50,8 +57,14 @@ struct SlotGraph {
 struct StreamCall {
   uint64_t ticket = ~0ull;
   uint64_t capacity = 0;
-  uint32_t nbins = 0;
+  gkc_params prm{};
   int key_words = 1;
+  // enqueued launch by launch, on these inputs and capacities: run again if they were too small
+  bool direct = false;
+  GraphKey key{};
+  PipelineCaps cap;
+  gkc_status status = GKC_OK;  // of that second run
+  std::string message;
   // the caller's page-locked outputs and the slot's device results
   uint64_t *h_bin_off = nullptr, *h_keys = nullptr;
   uint32_t *h_counts = nullptr;
@@ -117,7 +130,9 @@ struct gkc_ctx {
   std::vector<uint64_t> offs_tmp, desc_tmp;
 };
 
-inline void graphs_invalidate(gkc_ctx *c) { c->graphs[0].valid = c->graphs[1].valid = false; }
+inline void graphs_invalidate(gkc_ctx *c) {
+  for (SlotGraph &g : c->graphs) g.valid = g.seen = false;
+}
 // Workspace name of the current slot's copy of a per-slot buffer.
 inline std::string slot_name(const gkc_ctx *c, const char *n) { return c->slot ? std::string(n) + "#1" : std::string(n); }
 
