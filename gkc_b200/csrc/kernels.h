@@ -192,4 +192,8 @@ template <typename K>
 void rle_runs(const K *sorted, uint64_t n, unsigned long long *blk, uint64_t *blk_off, uint64_t *tmp,
               const unsigned long long *cursor, K *out_keys, uint64_t *starts, cudaStream_t st);
 
+// the same over the packed bytes of superkmers, given by length or by descriptor
+uint32_t scan_len_bytes(const uint32_t *len, uint64_t *out, uint64_t n, uint64_t *block_tmp, cudaStream_t st);
+uint32_t scan_desc_bytes(const uint64_t *desc, uint64_t *out, uint64_t n, uint64_t *block_tmp, cudaStream_t st);
+
 }  // namespace gkc

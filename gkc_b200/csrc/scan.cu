@@ -29,6 +29,16 @@ struct ScanKmers {
   }
 };
 
+// packed bytes of superkmers given by length, or by descriptor (its low 24 bits)
+struct ScanLenBytes {
+  const uint32_t *len;
+  GKC_DEV uint64_t operator()(uint64_t i) const { return ((uint64_t)len[i] + 3) / 4; }
+};
+struct ScanDescBytes {
+  const uint64_t *desc;
+  GKC_DEV uint64_t operator()(uint64_t i) const { return ((desc[i] & 0xFFFFFFu) + 3) / 4; }
+};
+
 GKC_DEV uint64_t scan_len(uint64_t n_cap, const uint64_t *n_dev) { return n_dev ? min(n_cap, *n_dev) : n_cap; }
 
 template <typename Src>
@@ -160,6 +170,14 @@ uint32_t scan_u64(const unsigned long long *in, uint64_t *out, uint64_t n, uint6
 uint32_t scan_kmers_dev(const uint64_t *desc, int k, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
                         uint64_t *block_tmp, cudaStream_t st) {
   return scan_any(ScanKmers{reinterpret_cast<const unsigned long long *>(desc), k}, out, n_cap, n_dev, block_tmp, st);
+}
+
+uint32_t scan_len_bytes(const uint32_t *len, uint64_t *out, uint64_t n, uint64_t *block_tmp, cudaStream_t st) {
+  return scan_any(ScanLenBytes{len}, out, n, nullptr, block_tmp, st);
+}
+
+uint32_t scan_desc_bytes(const uint64_t *desc, uint64_t *out, uint64_t n, uint64_t *block_tmp, cudaStream_t st) {
+  return scan_any(ScanDescBytes{desc}, out, n, nullptr, block_tmp, st);
 }
 
 }  // namespace gkc
