@@ -236,8 +236,10 @@ gkc_status gkc_ctx_create(int device_id, uint64_t hbm_budget_bytes, gkc_ctx **ou
       set_dyn_smem_limit((const void *)k_bucket_open<u128>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_slices<uint64_t>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_slices<u128>, c->max_smem_optin) != cudaSuccess ||
-      set_dyn_smem_limit((const void *)k_bucket_scatter<uint64_t>, c->max_smem_optin) != cudaSuccess ||
-      set_dyn_smem_limit((const void *)k_bucket_scatter<u128>, c->max_smem_optin) != cudaSuccess) {
+      set_dyn_smem_limit((const void *)k_bucket_scatter<uint64_t, 1>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_scatter<uint64_t, 2>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_scatter<u128, 1>, c->max_smem_optin) != cudaSuccess) {
+
     cudaGetLastError();
     delete c;
     return GKC_ERR_CUDA;
@@ -633,7 +635,11 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   pl.bin_kstart = bin_kstart;
   pl.bucket_keys = bucket_keys;
   pl.max_bits = max_bits;
-  const uint64_t chunk_kmers = c->tune.chunk_kmers ? c->tune.chunk_kmers : kChunkKmers;
+  uint64_t chunk_kmers = c->tune.chunk_kmers;
+  if (!chunk_kmers) {
+    chunk_kmers = kChunkKmers;
+    while (chunk_kmers > kChunkKmersMin && keys_cap / chunk_kmers < 8 * (uint64_t)c->n_sms) chunk_kmers /= 2;
+  }
   pl.chunk_kmers = chunk_kmers;
   pl.k = prm->k;
   pl.err = err;
@@ -705,9 +711,12 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
                      kBucketOffsetThreads, 0, c->st>>>(ea, bstart, bsize);
   LAUNCHED(c);
   stage_mark(c, 4);
-  const size_t sct_smem = bucket_scatter_smem_bytes<K>();
+  const int sc_ctas = sizeof(K) == 8 && keys_cap / nbins <= kScatterPairBin ? 2 : 1;
+  const size_t sct_smem = bucket_scatter_smem_bytes<K>(sc_ctas);
   if ((int)sct_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "scatter tile exceeds shared memory");
-  k_bucket_scatter<K><<<(unsigned)std::min<uint64_t>(max_chunks, (uint64_t)c->n_sms), kBucketScatterThreads, sct_smem, c->st>>>(ea);
+  const unsigned sc_grid = (unsigned)std::min<uint64_t>(max_chunks, (uint64_t)c->n_sms * sc_ctas);
+  if (sc_ctas == 2) k_bucket_scatter<uint64_t, 2><<<sc_grid, 512, sct_smem, c->st>>>(ea);
+  else k_bucket_scatter<K, 1><<<sc_grid, 1024, sct_smem, c->st>>>(ea);
   LAUNCHED(c);
 
   // counting: buckets independently, each bucket's runs staged over its own

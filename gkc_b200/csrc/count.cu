@@ -534,31 +534,36 @@ __global__ void __launch_bounds__(kBucketOffsetThreads) k_bucket_offsets(ExpandA
 
 // -------------------------------------------------------------- 3. scatter
 
-constexpr int SC_THREADS = 1024;
-// keys per scatter tile: the tile, its digits and three digit tables fill
-// most of the shared memory of one CTA per SM
-template <typename K> constexpr int sc_tile() { return sizeof(K) == 8 ? 16384 : 8192; }
+// threads of a scatter CTA and keys of its tile: one or two CTAs' tiles and
+// digit tables fill an SM's shared memory
+__host__ __device__ constexpr int sc_threads(int ctas) { return 1024 / ctas; }
+template <typename K> __host__ __device__ constexpr int sc_tile(int ctas) {
+  return sizeof(K) == 16 ? 8192 : ctas == 1 ? 16384 : 7168;
+}
 
 // Moves every key of `flat` to its bucket.  Each CTA takes whole chunks, a
 // tile of SC_TILE keys at a time: the tile is counting-sorted by bucket in
 // shared memory (a key's rank within its bucket from a shared-memory atomic),
 // then written out in that order, so the keys of one bucket leave as a
-// contiguous run at the chunk's write offset for the bucket (from the scan)
-// plus the bucket's keys of the chunk's earlier tiles.  Bound by latency (one
-// CTA fills an SM's shared memory): the chunk's next tile is loaded into the
-// registers that this one's keys leave while it is written out.
-template <typename K>
-__global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) {
-  constexpr int SC_TILE = sc_tile<K>(), KPT = SC_TILE / SC_THREADS;
+// contiguous run at the chunk's write offset for the bucket
+// (from the scan) plus the bucket's keys of the chunk's earlier tiles.  Bound
+// by the shared-memory accesses of phases that barriers separate, and by the
+// partial sectors at both ends of a run: one CTA an SM with as large a tile as
+// fits, or two that fill each other's gaps where runs stay long enough
+// (kScatterPairBin).  A tile is loaded into the registers that the previous
+// one's keys leave while that is written out.  720 M keys: 5.1 ms; 88 M of 16
+// bytes: 1.17 -> 0.98 ms with two digit tables instead of three.
+template <typename K, int CTAS>
+__global__ void __launch_bounds__(sc_threads(CTAS), CTAS) k_bucket_scatter(ExpandArgs a) {
+  constexpr int SC_THREADS = sc_threads(CTAS), SC_TILE = sc_tile<K>(CTAS), KPT = SC_TILE / SC_THREADS;
   constexpr int ND = 1 << kCoarseMaxBits;
   extern __shared__ __align__(16) uint8_t sc_smem[];
   K *S = reinterpret_cast<K *>(sc_smem);                      // the tile, by bucket
-  uint16_t *Sd = reinterpret_cast<uint16_t *>(S + SC_TILE);   // buckets of S
-  uint32_t *gbase = reinterpret_cast<uint32_t *>(Sd + SC_TILE);  // next write offset of every bucket
-  uint32_t *delta = gbase + ND;                               // write offset less tile position
-  uint32_t *toff = delta + ND;                                // tile counts, then tile offsets
+  uint32_t *gbase = reinterpret_cast<uint32_t *>(S + SC_TILE);  // end of every bucket's run of this tile
+  uint32_t *toff = gbase + ND;                                // tile counts, then tile ends
   uint32_t *tmp = toff + ND;                                  // block scan
-  uint16_t *lut = reinterpret_cast<uint16_t *>(tmp + 64);     // bucket of every digit
+  uint16_t *Sd = reinterpret_cast<uint16_t *>(tmp + 64);      // buckets of S
+  uint16_t *lut = Sd + SC_TILE;                               // bucket of every digit
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   K *keys = reinterpret_cast<K *>(a.keys);
   const K *flat = reinterpret_cast<const K *>(a.flat);
@@ -589,9 +594,9 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
       lut[d] = u;
       if (d == 0 || glut[d - 1] != u) gbase[u] = row[d];  // the bucket's first digit holds its offset
     }
-    for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
-    __syncthreads();
     for (uint64_t t0 = q0; t0 < q1; t0 += SC_TILE) {
+      for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
+      __syncthreads();  // also: the chunk's tables are there
       const uint32_t tn = (uint32_t)min((uint64_t)SC_TILE, q1 - t0);
       uint32_t rk[KPT];  // bucket << 16 | rank within it (< SC_TILE)
 #pragma unroll
@@ -602,50 +607,49 @@ __global__ void __launch_bounds__(SC_THREADS, 1) k_bucket_scatter(ExpandArgs a) 
         }
       }
       __syncthreads();
-      // exclusive scan of the tile counts, thread-contiguous buckets
+      // inclusive scan of the tile counts, thread-contiguous buckets
       const uint32_t per = (nd + SC_THREADS - 1) / SC_THREADS, d0 = tid * per;
       uint32_t sum = 0;
       for (uint32_t d = d0; d < d0 + per && d < nd; d++) sum += toff[d];
       uint32_t total;
       uint32_t run = block_exclusive_scan<SC_THREADS>(sum, tmp, &total);
       for (uint32_t d = d0; d < d0 + per && d < nd; d++) {
-        const uint32_t v = toff[d], g = gbase[d];
-        toff[d] = run;
-        delta[d] = g - run;
-        gbase[d] = g + v;
+        const uint32_t v = toff[d];
         run += v;
+        toff[d] = run;
+        gbase[d] += v;
       }
       __syncthreads();
 #pragma unroll
       for (int u = 0; u < KPT; u++) {
         if (u * SC_THREADS + tid < tn) {
           const uint32_t d = rk[u] >> 16;
-          const uint32_t at = toff[d] + (rk[u] & 0xFFFFu);
+          const uint32_t at = toff[d] - 1u - (rk[u] & 0xFFFFu);
           S[at] = xs[u];
           Sd[at] = (uint16_t)d;
         }
       }
       __syncthreads();
       if (t0 + SC_TILE < q1) load(t0 + SC_TILE);
-      for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
 #pragma unroll 4
       for (uint32_t i = tid; i < tn; i += SC_THREADS) {
-        const uint64_t slot = kbase + (uint32_t)(delta[Sd[i]] + i);
+        const uint32_t d = Sd[i];
+        const uint64_t slot = kbase + (uint32_t)(gbase[d] - toff[d] + i);
         if (slot < a.keys_cap) keys[slot] = S[i];
         else atomicOr(a.err, ERR_CAPACITY);
       }
-      __syncthreads();  // before the next tile's ranks and the next chunk's tables
+      __syncthreads();  // before the next tile's counts and the next chunk's tables
     }
   }
 }
 
-template <typename K> size_t bucket_scatter_smem_bytes() {
+template <typename K> size_t bucket_scatter_smem_bytes(int ctas) {
   constexpr int ND = 1 << kCoarseMaxBits;
-  static_assert(sc_tile<K>() <= 65536 && sc_tile<K>() % SC_THREADS == 0, "16-bit ranks, whole rounds");
-  return (size_t)sc_tile<K>() * (sizeof(K) + 2) + 4 * (3 * ND + 64) + 2 * ND;
+  static_assert(sc_tile<K>(1) % sc_threads(1) == 0 && sc_tile<K>(2) % sc_threads(2) == 0, "whole rounds");
+  return (size_t)sc_tile<K>(ctas) * (sizeof(K) + 2) + 4 * (2 * ND + 64) + 2 * ND;
 }
-template size_t bucket_scatter_smem_bytes<uint64_t>();
-template size_t bucket_scatter_smem_bytes<u128>();
+template size_t bucket_scatter_smem_bytes<uint64_t>(int);
+template size_t bucket_scatter_smem_bytes<u128>(int);
 
 // ---------------------------------------------------------------- 4. count
 
@@ -1827,8 +1831,9 @@ template __global__ void k_compact_runs<u128>(const u128 *, const uint32_t *, co
                                               const uint4 *, const unsigned long long *, const uint32_t *);
 template __global__ void k_bucket_hist<uint64_t>(ExpandArgs);
 template __global__ void k_bucket_hist<u128>(ExpandArgs);
-template __global__ void k_bucket_scatter<uint64_t>(ExpandArgs);
-template __global__ void k_bucket_scatter<u128>(ExpandArgs);
+template __global__ void k_bucket_scatter<uint64_t, 1>(ExpandArgs);
+template __global__ void k_bucket_scatter<uint64_t, 2>(ExpandArgs);
+template __global__ void k_bucket_scatter<u128, 1>(ExpandArgs);
 template __global__ void k_bucket_sort<uint64_t>(SortCountArgs);
 template __global__ void k_bucket_sort<u128>(SortCountArgs);
 template __global__ void k_bucket_open<uint64_t>(SortCountArgs);

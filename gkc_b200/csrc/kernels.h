@@ -115,11 +115,10 @@ template <typename K> __global__ void k_bucket_hist(ExpandArgs a);
 __global__ void k_bucket_scan(ExpandArgs a);
 __global__ void k_bucket_offsets(ExpandArgs a, uint64_t *bucket_start, uint64_t *bucket_size);
 constexpr int kBucketOffsetThreads = 128;
-template <typename K> __global__ void k_bucket_scatter(ExpandArgs a);
+template <typename K, int CTAS> __global__ void k_bucket_scatter(ExpandArgs a);
 constexpr int kBucketScanThreads = 1024;
 constexpr int kBucketHistThreads = 256;
-constexpr int kBucketScatterThreads = 1024;
-template <typename K> size_t bucket_scatter_smem_bytes();
+template <typename K> size_t bucket_scatter_smem_bytes(int ctas);
 
 struct SortCountArgs {
   uint32_t nbins;
@@ -171,6 +170,17 @@ template <typename K> constexpr uint32_t bucket_target(uint32_t target) {
 }
 constexpr uint32_t kCoarseMaxBits = 12;
 constexpr uint64_t kChunkKmers = 65536;
+// Halved down to this while there are fewer chunks than the histogram has CTAs
+// (histogram + scatter, 64 K / 32 K / 16 K: 20 M bases 389 / 319 / 269 us, 60 M
+// 718 / 684 / 678, 120 M 1331 / 1328 / 1387).
+constexpr uint64_t kChunkKmersMin = 16384;
+// Largest mean bin (k-mers) whose 8-byte keys are scattered by two CTAs an SM
+// with tiles of 7168 keys rather than one with 16384: their phases overlap,
+// but in larger bins a bucket's run of the smaller tile ends within few 32-byte
+// sectors (117 M k-mers, one CTA / two: 256 bins 0.91 / 0.86 ms, 64 bins 0.98 /
+// 0.95, 31 bins 1.06 / 1.27; 720 M in 1024 bins 4.72 / 4.26).  16-byte keys
+// gain nothing from it (88 M in 128 bins: 1.02 / 1.09).
+constexpr uint64_t kScatterPairBin = 2 << 20;
 
 // device-wide exclusive scan of uint64 counters (n <= 2^31); out[n] = total.
 // Returns the kernels launched.
