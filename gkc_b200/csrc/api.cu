@@ -230,8 +230,9 @@ gkc_status gkc_ctx_create(int device_id, uint64_t hbm_budget_bytes, gkc_ctx **ou
   // thread's setting and launch.
   if (set_dyn_smem_limit((const void *)k_partition, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bin_place, c->max_smem_optin) != cudaSuccess ||
-      set_dyn_smem_limit((const void *)k_bucket_sort<uint64_t>, c->max_smem_optin) != cudaSuccess ||
-      set_dyn_smem_limit((const void *)k_bucket_sort<u128>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_sort<uint64_t, false>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_sort<uint64_t, true>, c->max_smem_optin) != cudaSuccess ||
+      set_dyn_smem_limit((const void *)k_bucket_sort<u128, false>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_open<uint64_t>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_open<u128>, c->max_smem_optin) != cudaSuccess ||
       set_dyn_smem_limit((const void *)k_bucket_slices<uint64_t>, c->max_smem_optin) != cudaSuccess ||
@@ -602,6 +603,17 @@ gkc_status gkc_partition_device(gkc_ctx *c, const gkc_params *prm, const char *d
 
 // ------------------------------------------------------------------ count
 
+// Whether a group of some 96 keys of a bin of bin_keys k-mers mostly lies
+// within 2^29 consecutive values, so that no more than one in eight has keys
+// that differ in the upper word: counted from the k-mers' 2 k bits, as if they
+// were spread evenly (where they are not, more groups or fewer qualify; the
+// kernel looks at each).
+static bool narrow_groups(int k, uint64_t bin_keys) {
+  int bits = 2 * k;
+  for (uint64_t groups = bin_keys / 96; groups > 1; groups >>= 1) bits--;
+  return bits <= 29;
+}
+
 template <typename K>
 static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint64_t keys_cap,
                                         uint64_t) {
@@ -761,8 +773,11 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   const size_t sort_smem = bucket_sort_smem_bytes<K>();
   if ((int)sort_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "sort areas exceed shared memory");
   int sort_occ = 0;
-  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sort_occ, k_bucket_sort<K>, kBucketSortThreads, sort_smem));
-  k_bucket_sort<K><<<(unsigned)std::min<uint64_t>(max_buckets, (uint64_t)c->n_sms * std::max(sort_occ, 1)), kBucketSortThreads, sort_smem, c->st>>>(sa);
+  auto sort_kernel = k_bucket_sort<K, false>;
+  if constexpr (sizeof(K) == 8)
+    if (narrow_groups(prm->k, keys_cap / nbins)) sort_kernel = k_bucket_sort<uint64_t, true>;
+  CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&sort_occ, sort_kernel, kBucketSortThreads, sort_smem));
+  sort_kernel<<<(unsigned)std::min<uint64_t>(max_buckets, (uint64_t)c->n_sms * std::max(sort_occ, 1)), kBucketSortThreads, sort_smem, c->st>>>(sa);
   LAUNCHED(c);
   // the large and rejected buckets, persistent, taken by ticket
   const int ctas = std::max(1, std::min(occ, c->tune.count_ctas ? (int)c->tune.count_ctas : 2));

@@ -1142,6 +1142,23 @@ GKC_DEV uint32_t warp_exclusive_scan(uint32_t c, uint32_t *total) {
   return inc - c;
 }
 
+// Orders x and y (ascending if asc), and the smaller or the larger of two keys.
+template <typename K>
+GKC_DEV void compare_exchange(K &x, K &y, bool asc) {
+  const bool sw = (y < x) == asc;
+  const K a = sw ? y : x;
+  y = sw ? x : y;
+  x = a;
+}
+GKC_DEV void compare_exchange(uint32_t &x, uint32_t &y, bool asc) {
+  const uint32_t lo = min(x, y), hi = max(x, y);
+  x = asc ? lo : hi;
+  y = asc ? hi : lo;
+}
+template <typename K>
+GKC_DEV K pick(K x, K y, bool smaller) { return (y < x) == smaller ? y : x; }
+GKC_DEV uint32_t pick(uint32_t x, uint32_t y, bool smaller) { return smaller ? min(x, y) : max(x, y); }
+
 // Bitonic merge of each lane's R keys (ascending if asc).
 template <typename K, int R>
 GKC_DEV void lane_merge(K (&v)[R], bool asc) {
@@ -1149,12 +1166,7 @@ GKC_DEV void lane_merge(K (&v)[R], bool asc) {
   for (int stride = R / 2; stride > 0; stride >>= 1) {
 #pragma unroll
     for (int r = 0; r < R; r++)
-      if ((r & stride) == 0) {
-        const K x = v[r], y = v[r + stride];
-        const bool sw = (y < x) == asc;
-        v[r] = sw ? y : x;
-        v[r + stride] = sw ? x : y;
-      }
+      if ((r & stride) == 0) compare_exchange(v[r], v[r + stride], asc);
   }
 }
 
@@ -1174,13 +1186,7 @@ GKC_DEV void warp_bitonic(K (&v)[R]) {
     for (int stride = size >> 1; stride > 0; stride >>= 1) {
 #pragma unroll
       for (int r = 0; r < R; r++)
-        if ((r & stride) == 0) {
-          const bool asc = size < R ? (r & size) == 0 : (lane & 1u) == 0;
-          const K x = v[r], y = v[r + stride];
-          const bool sw = (y < x) == asc;
-          v[r] = sw ? y : x;
-          v[r + stride] = sw ? x : y;
-        }
+        if ((r & stride) == 0) compare_exchange(v[r], v[r + stride], size < R ? (r & size) == 0 : (lane & 1u) == 0);
     }
   }
 #pragma unroll 1
@@ -1191,30 +1197,25 @@ GKC_DEV void warp_bitonic(K (&v)[R]) {
       const bool keep_min = ((lane & lm) == 0) == asc;
 #pragma unroll
       for (int r = 0; r < R; r++) {
-        const K y = shfl_xor_k<K>(v[r], (int)lm);
-        v[r] = (y < v[r]) == keep_min ? y : v[r];
+        v[r] = pick(v[r], shfl_xor_k<K>(v[r], (int)lm), keep_min);
       }
     }
     lane_merge<K, R>(v, asc);
   }
 }
 
-// Sorts A[b0, b0 + n), n <= 32 R, with the calling warp and leaves its runs
-// there: the distinct keys in A, the first position of each in C.  Returns
-// their number.
-template <typename K, int R>
-GKC_DEV uint32_t warp_sort_runs(K *A, uint16_t *C, uint32_t b0, uint32_t n) {
+// The runs of the warp's sorted values (position e in lane e / R, register
+// e % R; the first n): the distinct keys, made of the values by `key`, to A,
+// the first position of each to C.  Returns their number.
+template <typename K, typename V, int R, typename F>
+GKC_DEV uint32_t warp_runs(const V (&v)[R], K *A, uint16_t *C, uint32_t b0, uint32_t n, F key) {
   const uint32_t lane = threadIdx.x & 31u;
-  K v[R];
-#pragma unroll
-  for (int r = 0; r < R; r++) v[r] = r * 32 + lane < n ? A[b0 + r * 32 + lane] : ~(K)0;
-  warp_bitonic<K, R>(v);
-  const K before = shfl_up_k<K>(v[R - 1], 1);
+  const V before = shfl_up_k<V>(v[R - 1], 1);
   uint32_t hb = 0;  // run heads among the first n positions
 #pragma unroll
   for (int r = 0; r < R; r++) {
     const uint32_t e = lane * R + r;
-    const K p = r == 0 ? before : v[r > 0 ? r - 1 : 0];
+    const V p = r == 0 ? before : v[r > 0 ? r - 1 : 0];
     if (e < n && (e == 0 || p != v[r])) hb |= 1u << r;
   }
   uint32_t D;
@@ -1222,12 +1223,43 @@ GKC_DEV uint32_t warp_sort_runs(K *A, uint16_t *C, uint32_t b0, uint32_t n) {
 #pragma unroll
   for (int r = 0; r < R; r++)
     if ((hb >> r) & 1u) {
-      A[rank] = v[r];
+      A[rank] = key(v[r]);
       C[rank] = (uint16_t)(lane * R + r);
       rank++;
     }
   __syncwarp();
   return D;
+}
+
+// Sorts A[b0, b0 + n), n <= 32 R, with the calling warp and leaves its runs
+// there: the distinct keys in A, the first position of each in C.  Returns
+// their number.  NARROW: 8-byte keys that share their upper word, as a group's
+// keys do where k is small, are sorted by the lower one, a third of the
+// network's instructions (count stage of 134.7 M distinct 21-mers 3.1 -> 2.6
+// ms; both networks in the kernel cost 25-mers, whose groups seldom qualify,
+// 3.9 -> 4.2, so the caller decides by k: narrow_groups).
+template <typename K, int R, bool NARROW>
+GKC_DEV uint32_t warp_sort_runs(K *A, uint16_t *C, uint32_t b0, uint32_t n) {
+  const uint32_t lane = threadIdx.x & 31u;
+  K v[R];
+#pragma unroll
+  for (int r = 0; r < R; r++) v[r] = r * 32 + lane < n ? A[b0 + r * 32 + lane] : ~(K)0;
+  if constexpr (NARROW) {
+    const uint32_t upper = (uint32_t)(A[b0] >> 32);
+    uint32_t diff = 0;
+#pragma unroll
+    for (int r = 0; r < R; r++)
+      if (r * 32 + lane < n) diff |= (uint32_t)(v[r] >> 32) ^ upper;
+    if (!__any_sync(0xffffffffu, diff)) {
+      uint32_t u[R];
+#pragma unroll
+      for (int r = 0; r < R; r++) u[r] = (uint32_t)v[r];
+      warp_bitonic<uint32_t, R>(u);
+      return warp_runs<K>(u, A, C, b0, n, [upper](uint32_t x) { return (K)upper << 32 | x; });
+    }
+  }
+  warp_bitonic<K, R>(v);
+  return warp_runs<K>(v, A, C, b0, n, [](K x) { return x; });
 }
 
 constexpr uint32_t SORT_REJECTED = ~0u;
@@ -1261,7 +1293,7 @@ struct TableKeys {
   }
 };
 
-template <typename K, int NT, typename Src, typename Area>
+template <typename K, int NT, bool NARROW, typename Src, typename Area>
 GKC_DEV uint32_t sort_count(Area &S, const SortCountArgs &a, const Src &src, uint32_t n, uint64_t out_at) {
   constexpr int CAP = Area::CAP, W = NT / 32, RMAX = SortShape<K>::RMAX;
   static_assert(CAP <= 65535 && (CS_GROUPS * SortShape<K>::GROUP) >= CAP, "16-bit positions");
@@ -1353,10 +1385,10 @@ GKC_DEV uint32_t sort_count(Area &S, const SortCountArgs &a, const Src &src, uin
     if (t >= G) break;
     const uint32_t b0 = goff[t], m = goff[t + 1] - b0;
     uint32_t d;
-    if (m <= 64) d = warp_sort_runs<K, 2>(S.A, S.C, b0, m);
-    else if (m <= 128) d = warp_sort_runs<K, 4>(S.A, S.C, b0, m);
-    else if (RMAX <= 8 || m <= 256) d = warp_sort_runs<K, 8>(S.A, S.C, b0, m);
-    else d = warp_sort_runs<K, RMAX>(S.A, S.C, b0, m);
+    if (m <= 64) d = warp_sort_runs<K, 2, NARROW>(S.A, S.C, b0, m);
+    else if (m <= 128) d = warp_sort_runs<K, 4, NARROW>(S.A, S.C, b0, m);
+    else if (RMAX <= 8 || m <= 256) d = warp_sort_runs<K, 8, NARROW>(S.A, S.C, b0, m);
+    else d = warp_sort_runs<K, RMAX, NARROW>(S.A, S.C, b0, m);
     if (lane == 0) S.gd[t] = (uint16_t)d;
   }
   __syncthreads();
@@ -1384,7 +1416,7 @@ GKC_DEV uint32_t sort_count(Area &S, const SortCountArgs &a, const Src &src, uin
 // A bucket of n <= 65535 8-byte keys, its distinct keys (their number is
 // returned; SORT_REJECTED when there are more than the table takes or sorted
 // groups are too large) aggregated in the table first and then sorted.
-template <int NT>
+template <int NT, bool NARROW>
 __device__ __noinline__ uint32_t dedup_count(SortSmem<uint64_t> &S, const SortCountArgs &a, const uint64_t *src,
                                              uint32_t n, uint64_t out_at) {
   DedupArea &H = S.u.d.t;
@@ -1406,9 +1438,9 @@ __device__ __noinline__ uint32_t dedup_count(SortSmem<uint64_t> &S, const SortCo
     H.L[pos++] = (uint16_t)(q * NT + threadIdx.x);
   }
   __syncthreads();
-  return sort_count<uint64_t, NT>(S.u.d.s, a, TableKeys{H}, D, out_at);
+  return sort_count<uint64_t, NT, NARROW>(S.u.d.s, a, TableKeys{H}, D, out_at);
 }
-template <int NT>
+template <int NT, bool NARROW>
 GKC_DEV uint32_t dedup_count(SortSmem<u128> &, const SortCountArgs &, const u128 *, uint32_t, uint64_t) {
   return SORT_REJECTED;
 }
@@ -1416,7 +1448,7 @@ GKC_DEV uint32_t dedup_count(SortSmem<u128> &, const SortCountArgs &, const u128
 template <typename K, int NT>
 __device__ __noinline__ uint32_t slice_count(SortArea<K, NT, CountShape<K>::CAP> &S, const SortCountArgs &a,
                                              const K *src, uint32_t n, uint64_t out_at) {
-  return sort_count<K, NT>(S, a, GlobalKeys<K>{src}, n, out_at);
+  return sort_count<K, NT, false>(S, a, GlobalKeys<K>{src}, n, out_at);
 }
 
 // Buckets of at most CAP keys, persistent, taken by ticket.  Those that
@@ -1427,7 +1459,7 @@ __device__ __noinline__ uint32_t slice_count(SortArea<K, NT, CountShape<K>::CAP>
 // sort, or by insertion and warp sorts of 4096 fixed digits: 720 M 31-mers at
 // 30x 9.7 ms (14.7), 134.7 M mostly distinct 21-mers 3.4 ms (10.6), 150.9 M
 // 25-mers of compressed long reads 4.5 ms (14.8), 112.8 M 63-mers 3.5 ms (9.9).
-template <typename K>
+template <typename K, bool NARROW>
 __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket_sort(SortCountArgs a) {
   constexpr int NT = SortShape<K>::NT;
   extern __shared__ __align__(16) uint8_t smem_raw[];
@@ -1493,9 +1525,9 @@ __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket
     // 16-byte keys have no table here: the next 15 such buckets go to the
     // list, then one is sorted again.
     uint32_t D = SORT_REJECTED;
-    if (sizeof(K) == 8 && repeats) D = dedup_count<NT>(S, a, keys + start, n, start);
+    if (sizeof(K) == 8 && repeats) D = dedup_count<NT, NARROW>(S, a, keys + start, n, start);
     if (D == SORT_REJECTED && (sizeof(K) == 8 || repeats == 0))
-      D = sort_count<K, NT>(S.u.s, a, GlobalKeys<K>{keys + start}, n, start);
+      D = sort_count<K, NT, NARROW>(S.u.s, a, GlobalKeys<K>{keys + start}, n, start);
     if (D != SORT_REJECTED) repeats = 3 * D <= n ? 15 : 0;
     else if (sizeof(K) == 8) repeats = 0;
     else if (repeats) repeats--;
@@ -1834,8 +1866,9 @@ template __global__ void k_bucket_hist<u128>(ExpandArgs);
 template __global__ void k_bucket_scatter<uint64_t, 1>(ExpandArgs);
 template __global__ void k_bucket_scatter<uint64_t, 2>(ExpandArgs);
 template __global__ void k_bucket_scatter<u128, 1>(ExpandArgs);
-template __global__ void k_bucket_sort<uint64_t>(SortCountArgs);
-template __global__ void k_bucket_sort<u128>(SortCountArgs);
+template __global__ void k_bucket_sort<uint64_t, false>(SortCountArgs);
+template __global__ void k_bucket_sort<uint64_t, true>(SortCountArgs);
+template __global__ void k_bucket_sort<u128, false>(SortCountArgs);
 template __global__ void k_bucket_open<uint64_t>(SortCountArgs);
 template __global__ void k_bucket_open<u128>(SortCountArgs);
 template __global__ void k_bucket_slices<uint64_t>(SortCountArgs);

@@ -144,7 +144,7 @@ struct SortCountArgs {
   uint64_t big_min;
   uint32_t *err;
 };
-template <typename K> __global__ void k_bucket_sort(SortCountArgs a);
+template <typename K, bool NARROW> __global__ void k_bucket_sort(SortCountArgs a);
 template <typename K> size_t bucket_sort_smem_bytes();
 constexpr int kBucketSortThreads = 256;
 template <typename K> __global__ void k_bucket_open(SortCountArgs a);
