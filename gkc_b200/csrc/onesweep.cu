@@ -7,6 +7,10 @@
 //
 // Keys: uint64 or unsigned __int128, sorted on their low `key_bits` bits,
 // 8-bit digits.  Every wait on another tile is bounded.
+#include <algorithm>
+#include <utility>
+#include <vector>
+
 #include "common.cuh"
 #include "onesweep.h"
 
@@ -37,8 +41,8 @@ GKC_DEV void os_st(unsigned long long *p, unsigned long long v) {
 }
 
 template <typename K>
-GKC_DEV uint32_t os_digit(K x, int pass) {
-  return (uint32_t)(x >> (8 * pass)) & 0xFFu;
+GKC_DEV uint32_t os_digit(K x, int shift) {
+  return (uint32_t)(x >> shift) & 0xFFu;
 }
 
 // The lanes whose digit equals this one's, among those with `in`: eight
@@ -54,17 +58,17 @@ GKC_DEV uint32_t os_peers(uint32_t d, bool in) {
   return peers;
 }
 
-// hist[pass][digit] over all keys, for every pass.
+// hist[pass][digit] over all keys, for every pass (digits from bit `bit0` on).
 template <typename K>
 __global__ void __launch_bounds__(OS_NT) k_os_histogram(const K *keys, const uint64_t *n_dev,
-                                                        int passes, unsigned long long *hist) {
+                                                        int passes, int bit0, unsigned long long *hist) {
   __shared__ uint32_t h[16][OS_RADIX];
   const uint64_t n = *n_dev;
   for (int i = threadIdx.x; i < passes * OS_RADIX; i += OS_NT) h[i / OS_RADIX][i % OS_RADIX] = 0;
   __syncthreads();
   for (uint64_t i = blockIdx.x * (uint64_t)OS_NT + threadIdx.x; i < n; i += (uint64_t)gridDim.x * OS_NT) {
     K x = keys[i];
-    for (int p = 0; p < passes; p++) atomicAdd(&h[p][os_digit<K>(x, p)], 1u);
+    for (int p = 0; p < passes; p++) atomicAdd(&h[p][os_digit<K>(x, bit0 + 8 * p)], 1u);
   }
   __syncthreads();
   for (int i = threadIdx.x; i < passes * OS_RADIX; i += OS_NT) {
@@ -99,7 +103,7 @@ __global__ void k_os_digit_offsets(unsigned long long *hist, int passes) {
 template <typename K, bool KV>
 __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const uint32_t *vin,
                                                                            uint32_t *vout, const uint64_t *n_dev,
-                                                                           int pass, const unsigned long long *digit_base,
+                                                                           int shift, const unsigned long long *digit_base,
                                                                            unsigned long long *lookback,
                                                                            unsigned long long *ticket, uint32_t *err) {
   constexpr int ITEMS = OS_ITEMS, TILE = OS_TILE;
@@ -136,7 +140,7 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
 #pragma unroll
     for (int r = 0; r < ITEMS; r++) {
       const bool v = seg + (uint64_t)r * 32 + lane < n;
-      const uint32_t d = os_digit<K>(key[r], pass);
+      const uint32_t d = os_digit<K>(key[r], shift);
       const uint32_t peers = os_peers(d, v);
       const uint32_t below = __popc(peers & ((1u << lane) - 1u));
       uint32_t base = 0;
@@ -165,7 +169,7 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
 #pragma unroll
     for (int r = 0; r < ITEMS; r++)
       if (seg + (uint64_t)r * 32 + lane < n) {
-        const uint32_t x = os_digit<K>(key[r], pass);
+        const uint32_t x = os_digit<K>(key[r], shift);
         rank[r] += toff[x] + warp_cnt[warp][x];
         S[rank[r]] = key[r];
       }
@@ -204,11 +208,11 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
       }
     }
     if (tile != 0) os_st(lb, OS_PRE | (excl + run));
-    gbase[d] = digit_base[pass * OS_RADIX + d] + excl;
+    gbase[d] = digit_base[d] + excl;
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < tn; i += OS_NT) {
       const K x = S[i];
-      const uint32_t y = os_digit<K>(x, pass);
+      const uint32_t y = os_digit<K>(x, shift);
       out[gbase[y] + (i - toff[y])] = x;
     }
     if (KV) {
@@ -220,7 +224,7 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
       for (int r = 0; r < ITEMS; r++)
         if (seg + (uint64_t)r * 32 + lane < n) {
           V[rank[r]] = val[KV ? r : 0];
-          D[rank[r]] = (uint8_t)os_digit<K>(key[r], pass);
+          D[rank[r]] = (uint8_t)os_digit<K>(key[r], shift);
         }
       __syncthreads();
       for (uint32_t i = threadIdx.x; i < tn; i += OS_NT) {
@@ -234,13 +238,13 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
 
 template <typename K, bool KV>
 static OnesweepStatus onesweep_run(K *keys, K *alt, uint32_t *vals, uint32_t *valt, const uint64_t *n_dev,
-                                   uint64_t n_max, int key_bits, OnesweepScratch s, cudaStream_t st,
+                                   uint64_t n_max, int bit0, int key_bits, OnesweepScratch s, cudaStream_t st,
                                    uint32_t *launches) {
-  const int passes = (key_bits + 7) / 8;
+  const int passes = (key_bits - bit0 + 7) / 8;
   const uint64_t tiles = (n_max + OS_TILE - 1) / OS_TILE;
   cudaMemsetAsync(s.hist, 0, sizeof(unsigned long long) * 16 * OS_RADIX, st);
   unsigned grid_h = (unsigned)std::min<uint64_t>(std::max<uint64_t>(1, (n_max + OS_NT * 8 - 1) / (OS_NT * 8)), 148 * 16);
-  k_os_histogram<K><<<grid_h, OS_NT, 0, st>>>(keys, n_dev, passes, s.hist);
+  k_os_histogram<K><<<grid_h, OS_NT, 0, st>>>(keys, n_dev, passes, bit0, s.hist);
   k_os_digit_offsets<<<1, 32 * 8, 0, st>>>(s.hist, passes);
   *launches += 2;
   K *src = keys, *dst = alt;
@@ -249,7 +253,7 @@ static OnesweepStatus onesweep_run(K *keys, K *alt, uint32_t *vals, uint32_t *va
     cudaMemsetAsync(s.lookback, 0, sizeof(unsigned long long) * (tiles + 1) * OS_RADIX, st);
     cudaMemsetAsync(s.ticket, 0, sizeof(unsigned long long), st);
     unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)s.max_ctas));
-    k_os_pass<K, KV><<<grid, OS_NT, 0, st>>>(src, dst, vsrc, vdst, n_dev, p, s.hist, s.lookback,
+    k_os_pass<K, KV><<<grid, OS_NT, 0, st>>>(src, dst, vsrc, vdst, n_dev, bit0 + 8 * p, s.hist + p * OS_RADIX, s.lookback,
                                               s.ticket, s.err);
     *launches += 1;
     K *t = src;
@@ -265,14 +269,199 @@ static OnesweepStatus onesweep_run(K *keys, K *alt, uint32_t *vals, uint32_t *va
 template <typename K>
 OnesweepStatus onesweep_sort(K *keys, K *alt, const uint64_t *n_dev, uint64_t n_max, int key_bits,
                              OnesweepScratch s, cudaStream_t st, uint32_t *launches) {
-  return onesweep_run<K, false>(keys, alt, nullptr, nullptr, n_dev, n_max, key_bits, s, st, launches);
+  return onesweep_run<K, false>(keys, alt, nullptr, nullptr, n_dev, n_max, 0, key_bits, s, st, launches);
+}
+
+// ---- pairs by their leading bits, then the rest run by run ----
+
+// Of n keys whose leading bits spread them well, few share some log2(n) + 5
+// leading bits with another one: passes over those bits leave runs of equal
+// leading bits, short ones, which one more kernel puts in order.  So a sort of
+// 126-bit keys takes four or five passes over memory, not 16.
+constexpr int OF_NT = 256;
+constexpr uint32_t OF_TILE = 1024;  // a tile's runs begin in it
+constexpr uint32_t OF_RUN = 512;    // and are ranked in shared memory up to this length
+constexpr uint32_t OF_LOAD = OF_TILE + OF_RUN;
+
+// Copies [s, e), a run too long to be ranked by its tile, as it is; lists it
+// unless all its keys are equal (they are in order then).
+template <typename K>
+GKC_DEV void os_long_run(const K *in, K *out, const uint32_t *vin, uint32_t *vout, uint64_t s, uint64_t e,
+                         unsigned long long *list) {
+  const K first = in[s];
+  bool mixed = false;
+  for (uint64_t i = s + threadIdx.x; i < e; i += OF_NT) {
+    const K x = in[i];
+    mixed = mixed || x != first;
+    out[i] = x;
+    vout[i] = vin[i];
+  }
+  if (__syncthreads_or(mixed) && threadIdx.x == 0) {
+    const unsigned long long at = atomicAdd(list, 1ull);
+    list[2 + 2 * at] = s;
+    list[3 + 2 * at] = e;
+  }
+}
+
+// Pairs in the order of their bits from `bit0` up, to `out` in the order of
+// all bits: each run of equal leading bits by ranking every key in it (equal
+// keys keep their order).  A tile takes the runs that begin in it.  list[0]
+// counts the runs left to the host, [begin, end) from list[2] on: longer than
+// OF_RUN, so at most n / OF_RUN.  Bound by the comparisons, a run's length for
+// each key: 13.9 M 16-byte keys in runs of about 17 take 0.48 ms, the twelve
+// passes it stands for 2.7; 8.7 M distinct 8-byte keys 0.08 for 0.47.
+template <typename K>
+__global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uint32_t *vin, uint32_t *vout,
+                                                  const uint64_t *n_dev, int bit0, unsigned long long *list) {
+  __shared__ __align__(16) K S[OF_LOAD];
+  __shared__ uint32_t heads[OF_LOAD / 32];  // bit i: a run begins at S[i] (or the keys end there)
+  __shared__ uint32_t n_long, long_s[4], long_e[4];
+  constexpr uint32_t OPEN = ~0u;
+  const uint64_t n = *n_dev;
+  const uint32_t tid = threadIdx.x;
+  for (uint64_t base = (uint64_t)blockIdx.x * OF_TILE; base < n; base += (uint64_t)gridDim.x * OF_TILE) {
+    const uint32_t m = (uint32_t)min(n - base, (uint64_t)OF_LOAD);
+    const bool closed = base + m == n;
+    for (uint32_t i = tid; i < m; i += OF_NT) S[i] = in[base + i];
+    if (tid == 0) n_long = 0;
+    __syncthreads();
+    for (uint32_t i = tid; i < OF_LOAD; i += OF_NT) {  // OF_LOAD is whole rounds
+      bool head = i == m;
+      if (i < m) {
+        const bool first = i == 0 && base == 0;
+        head = first || ((i ? S[i - 1] : in[base - 1]) >> bit0) != (S[i] >> bit0);
+      }
+      const uint32_t w = __ballot_sync(0xffffffffu, head);
+      if ((tid & 31u) == 0) heads[i >> 5] = w;
+    }
+    __syncthreads();
+    for (uint32_t i = tid; i < m; i += OF_NT) {
+      const uint32_t b = i & 31u;
+      uint32_t w = i >> 5, bits = heads[w] & (0xFFFFFFFFu >> (31 - b));
+      while (!bits && w > 0) bits = heads[--w];
+      if (!bits) continue;  // begins in an earlier tile
+      const uint32_t s = 32 * w + 31 - __clz(bits);
+      if (s >= OF_TILE) continue;  // in a later one
+      w = i >> 5;
+      bits = b == 31 ? 0u : heads[w] & (0xFFFFFFFFu << (b + 1));
+      while (!bits && w + 1 < OF_LOAD / 32) bits = heads[++w];
+      const uint32_t e = bits ? 32 * w + __ffs(bits) - 1 : closed ? m : OPEN;
+      if (e == OPEN || e - s > OF_RUN) {
+        if (i == s) {  // at most OF_TILE / OF_RUN + 1 of them
+          const uint32_t at = atomicAdd(&n_long, 1u);
+          long_s[at] = s;
+          long_e[at] = e;
+        }
+        continue;
+      }
+      const K x = S[i];
+      uint32_t at = s;
+      for (uint32_t j = s; j < e; j++) {
+        const K y = S[j];
+        at += y < x || (y == x && j < i) ? 1u : 0u;
+      }
+      out[base + at] = x;
+      vout[base + at] = vin[base + i];
+    }
+    __syncthreads();
+    for (uint32_t l = 0; l < n_long; l++) {
+      const uint64_t s = base + long_s[l];
+      uint64_t e = base + long_e[l];
+      if (long_e[l] == OPEN) {  // the first key after the loaded ones with other leading bits
+        const K lead = in[s] >> bit0;
+        uint64_t lo = base + m;
+        for (uint64_t hi = n; lo < hi;) {
+          const uint64_t mid = (lo + hi) >> 1;
+          if ((in[mid] >> bit0) == lead) lo = mid + 1;
+          else hi = mid;
+        }
+        e = lo;
+      }
+      os_long_run(in, out, vin, vout, s, e, list);
+    }
+    __syncthreads();  // before the next tile's keys
+  }
+}
+
+// The listed runs (begin, end, first place in the compact arrays) to the
+// compact arrays, or back.
+template <typename K>
+__global__ void __launch_bounds__(OF_NT) k_os_runs(K *keys, uint32_t *vals, K *ck, uint32_t *cv,
+                                                   const unsigned long long *runs, uint64_t n_runs, bool back) {
+  for (uint64_t r = blockIdx.x; r < n_runs; r += gridDim.x) {
+    const uint64_t s = runs[3 * r], n = runs[3 * r + 1] - s, at = runs[3 * r + 2];
+    for (uint64_t i = threadIdx.x; i < n; i += OF_NT) {
+      if (back) {
+        keys[s + i] = ck[at + i];
+        vals[s + i] = cv[at + i];
+      } else {
+        ck[at + i] = keys[s + i];
+        cv[at + i] = vals[s + i];
+      }
+    }
+  }
 }
 
 template <typename K>
-OnesweepStatus onesweep_sort_kv(K *keys, K *alt, uint32_t *vals, uint32_t *valt, const uint64_t *n_dev,
-                                uint64_t n_max, int key_bits, OnesweepScratch s, cudaStream_t st,
-                                uint32_t *launches) {
-  return onesweep_run<K, true>(keys, alt, vals, valt, n_dev, n_max, key_bits, s, st, launches);
+PairsStatus sort_pairs(K *keys, K *alt, uint32_t *vals, uint32_t *valt, const uint64_t *n_dev, uint64_t n, int key_bits,
+                       OnesweepScratch s, cudaStream_t st, uint32_t *launches) {
+  int lead = 5;
+  while (lead < 64 && (n >> (lead - 5))) lead++;
+  lead = (lead + 7) / 8 * 8;
+  if (lead + 8 >= key_bits)  // the last kernel would save a pass at most
+    return PairsStatus{onesweep_run<K, true>(keys, alt, vals, valt, n_dev, n, 0, key_bits, s, st, launches).result_in_alt,
+                       false};
+  const int bit0 = key_bits - lead;
+  const int in_alt = onesweep_run<K, true>(keys, alt, vals, valt, n_dev, n, bit0, key_bits, s, st, launches).result_in_alt;
+  // the look-back entries are free now: the list of long runs
+  cudaMemsetAsync(s.lookback, 0, 16, st);
+  const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + OF_TILE - 1) / OF_TILE, 1u << 20));
+  k_os_fix<K><<<grid, OF_NT, 0, st>>>(in_alt ? alt : keys, in_alt ? keys : alt, in_alt ? valt : vals,
+                                      in_alt ? vals : valt, n_dev, bit0, s.lookback);
+  *launches += 1;
+  return PairsStatus{!in_alt, true};
+}
+
+template <typename K>
+int sort_pairs_rest(PairsStatus done, uint64_t n_runs, K *keys, K *alt, uint32_t *vals, uint32_t *valt,
+                    const uint64_t *n_dev, uint64_t n, int key_bits, OnesweepScratch s, cudaStream_t st,
+                    uint32_t *launches) {
+  K *from = done.result_in_alt ? alt : keys, *free_k = done.result_in_alt ? keys : alt;
+  uint32_t *vfrom = done.result_in_alt ? valt : vals, *free_v = done.result_in_alt ? vals : valt;
+  std::vector<unsigned long long> list(2 * n_runs), runs(3 * n_runs);
+  cudaMemcpyAsync(list.data(), s.lookback + 2, 16 * n_runs, cudaMemcpyDeviceToHost, st);
+  cudaStreamSynchronize(st);
+  std::vector<std::pair<unsigned long long, unsigned long long>> r(n_runs);
+  for (uint64_t i = 0; i < n_runs; i++) r[i] = {list[2 * i], list[2 * i + 1]};
+  std::sort(r.begin(), r.end());
+  uint64_t u = 0;
+  for (uint64_t i = 0; i < n_runs; i++) {
+    runs[3 * i] = r[i].first;
+    runs[3 * i + 1] = r[i].second;
+    runs[3 * i + 2] = u;
+    u += r[i].second - r[i].first;
+  }
+  const uint64_t lb = onesweep_lookback_words(u);
+  if (2 * u > n || lb + 3 * n_runs + 1 > onesweep_lookback_words(n)) {
+    // no room for them beside their sort: all pairs (equal keys are in order, and stay so)
+    const int moved = onesweep_run<K, true>(from, free_k, vfrom, free_v, n_dev, n, 0, key_bits, s, st, launches).result_in_alt;
+    return moved ? !done.result_in_alt : done.result_in_alt;
+  }
+  // the runs compacted into the free buffer, sorted there (they keep their
+  // order among each other), and put back.  Their table lies behind the place
+  // of this sort's look-back entries.
+  unsigned long long *tab = s.lookback + lb;
+  runs.push_back(u);
+  cudaMemcpyAsync(tab, runs.data(), 8 * runs.size(), cudaMemcpyHostToDevice, st);
+  cudaStreamSynchronize(st);  // `runs` ends with this call
+  const unsigned grid = (unsigned)std::min<uint64_t>(n_runs, 148 * 8);
+  k_os_runs<K><<<grid, OF_NT, 0, st>>>(from, vfrom, free_k, free_v, tab, n_runs, false);
+  const int moved = onesweep_run<K, true>(free_k, free_k + u, free_v, free_v + u,
+                                          reinterpret_cast<const uint64_t *>(tab + 3 * n_runs), u, 0, key_bits, s, st,
+                                          launches).result_in_alt;
+  k_os_runs<K><<<grid, OF_NT, 0, st>>>(from, vfrom, free_k + (moved ? u : 0), free_v + (moved ? u : 0), tab, n_runs, true);
+  *launches += 2;
+  return done.result_in_alt;
 }
 
 size_t onesweep_lookback_words(uint64_t n_max) {
@@ -283,10 +472,13 @@ template OnesweepStatus onesweep_sort<uint64_t>(uint64_t *, uint64_t *, const ui
                                                 int, OnesweepScratch, cudaStream_t, uint32_t *);
 template OnesweepStatus onesweep_sort<u128>(u128 *, u128 *, const uint64_t *, uint64_t, int,
                                             OnesweepScratch, cudaStream_t, uint32_t *);
-template OnesweepStatus onesweep_sort_kv<uint64_t>(uint64_t *, uint64_t *, uint32_t *, uint32_t *,
-                                                   const uint64_t *, uint64_t, int, OnesweepScratch,
-                                                   cudaStream_t, uint32_t *);
-template OnesweepStatus onesweep_sort_kv<u128>(u128 *, u128 *, uint32_t *, uint32_t *, const uint64_t *,
-                                               uint64_t, int, OnesweepScratch, cudaStream_t, uint32_t *);
+template PairsStatus sort_pairs<uint64_t>(uint64_t *, uint64_t *, uint32_t *, uint32_t *, const uint64_t *, uint64_t, int,
+                                          OnesweepScratch, cudaStream_t, uint32_t *);
+template PairsStatus sort_pairs<u128>(u128 *, u128 *, uint32_t *, uint32_t *, const uint64_t *, uint64_t, int,
+                                      OnesweepScratch, cudaStream_t, uint32_t *);
+template int sort_pairs_rest<uint64_t>(PairsStatus, uint64_t, uint64_t *, uint64_t *, uint32_t *, uint32_t *,
+                                       const uint64_t *, uint64_t, int, OnesweepScratch, cudaStream_t, uint32_t *);
+template int sort_pairs_rest<u128>(PairsStatus, uint64_t, u128 *, u128 *, uint32_t *, uint32_t *, const uint64_t *,
+                                   uint64_t, int, OnesweepScratch, cudaStream_t, uint32_t *);
 
 }  // namespace gkc

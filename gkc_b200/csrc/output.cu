@@ -117,9 +117,8 @@ static gkc_status count_output_t(gkc_ctx *c, uint32_t lo, uint32_t hi, int merge
   CK(cudaMemsetAsync(err, 0, 16, c->st));
   OnesweepScratch os{os_hist, os_lb, os_ticket, err, c->n_sms * 4};
   uint32_t launches = 0;
-  OnesweepStatus r = onesweep_sort_kv<K>(mk, mk2, mv, mv2, nd, n, 2 * c->ck, os, c->st, &launches);
-  const K *sk = r.result_in_alt ? mk2 : mk;
-  const uint32_t *sv = r.result_in_alt ? mv2 : mv;
+  const PairsStatus r = sort_pairs<K>(mk, mk2, mv, mv2, nd, n, 2 * c->ck, os, c->st, &launches);
+  int in_alt = r.result_in_alt;
   const uint64_t nblk = rle_block_count(n);
   WS(rblk, unsigned long long, "merge_rle_blk", nblk + 1);
   WS(roff, uint64_t, "merge_rle_off", nblk + 2);
@@ -129,14 +128,21 @@ static gkc_status count_output_t(gkc_ctx *c, uint32_t lo, uint32_t hi, int merge
   WS(st, uint64_t, "merge_starts", n + 1);
   WS(us, uint32_t, "merge_sums", n + 1);
   WS(bo, uint64_t, "merge_bin_off", 2);
-  CK(cudaMemsetAsync(cur, 0, 16, c->st));
-  rle_runs<K>(sk, n, rblk, roff, rtmp, cur, uk, st, c->st);
   uint64_t d = 0;
   uint32_t e = 0;
-  if (nblk) CK(cudaMemcpyAsync(&d, roff + nblk, 8, cudaMemcpyDeviceToHost, c->st));
-  CK(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, c->st));
-  CK(cudaStreamSynchronize(c->st));
-  if (e & ERR_SPIN_TIMEOUT) return ctx_fail(c, GKC_ERR_DEVICE_TIMEOUT, "sort look-back timed out");
+  unsigned long long rest = 0;
+  for (int pass = 0; pass < 2; pass++) {  // once more where long runs were left
+    CK(cudaMemsetAsync(cur, 0, 16, c->st));
+    rle_runs<K>(in_alt ? mk2 : mk, n, rblk, roff, rtmp, cur, uk, st, c->st);
+    if (nblk) CK(cudaMemcpyAsync(&d, roff + nblk, 8, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaMemcpyAsync(&e, err, 4, cudaMemcpyDeviceToHost, c->st));
+    if (r.partial && pass == 0) CK(cudaMemcpyAsync(&rest, os_lb, 8, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    if (e & ERR_SPIN_TIMEOUT) return ctx_fail(c, GKC_ERR_DEVICE_TIMEOUT, "sort look-back timed out");
+    if (!rest || pass) break;
+    in_alt = sort_pairs_rest<K>(r, rest, mk, mk2, mv, mv2, nd, n, 2 * c->ck, os, c->st, &launches);
+  }
+  const uint32_t *sv = in_alt ? mv2 : mv;
   if (d) k_run_sums<<<grid, 256, 0, c->st>>>(sv, st, d, n, us);
   uint64_t hb[2] = {0, d};
   CK(cudaMemcpyAsync(bo, hb, 16, cudaMemcpyHostToDevice, c->st));

@@ -400,22 +400,28 @@ static gkc_status subsample_t(gkc_ctx *c, const gkc_params *prm, uint32_t mod, c
     // the selected count, on the device, for the sort
     const uint64_t *n_dev = toff + tiles;
     uint32_t launches = 0;
-    OnesweepStatus r = onesweep_sort_kv<K>(keys, alt, pos, palt, n_dev, n, 2 * prm->k, os, c->st, &launches);
-    const K *sk = r.result_in_alt ? alt : keys;
-    const uint32_t *sp = r.result_in_alt ? palt : pos;
+    const PairsStatus r = sort_pairs<K>(keys, alt, pos, palt, n_dev, n, 2 * prm->k, os, c->st, &launches);
+    int in_alt = r.result_in_alt;
     // distinct keys and their first indices (= the position-list offsets)
     const uint64_t nblk = rle_block_count(n);
     WS(rblk, unsigned long long, "win_rle_blk", nblk + 1);
     WS(roff, uint64_t, "win_rle_off", nblk + 2);
     WS(rtmp, uint64_t, "win_rle_tmp", scan_u64_tmp_words(nblk + 1) + 8);
     WS(cur, unsigned long long, "win_cursor", 2);
-    CK(cudaMemsetAsync(cur, 0, 16, c->st));
-    rle_runs<K>(sk, n, rblk, roff, rtmp, cur, out_keys, pos_off, c->st);
-    CK(cudaPeekAtLastError());
     uint64_t nd = 0;
-    CK(cudaMemcpyAsync(&nd, roff + nblk, 8, cudaMemcpyDeviceToHost, c->st));
-    s = read_err(c, err);
-    if (s != GKC_OK) return s;
+    unsigned long long rest = 0;
+    for (int pass = 0; pass < 2; pass++) {  // once more where long runs were left
+      CK(cudaMemsetAsync(cur, 0, 16, c->st));
+      rle_runs<K>(in_alt ? alt : keys, n, rblk, roff, rtmp, cur, out_keys, pos_off, c->st);
+      CK(cudaPeekAtLastError());
+      CK(cudaMemcpyAsync(&nd, roff + nblk, 8, cudaMemcpyDeviceToHost, c->st));
+      if (r.partial && pass == 0) CK(cudaMemcpyAsync(&rest, os_lb, 8, cudaMemcpyDeviceToHost, c->st));
+      s = read_err(c, err);
+      if (s != GKC_OK) return s;
+      if (!rest || pass) break;
+      in_alt = sort_pairs_rest<K>(r, rest, keys, alt, pos, palt, n_dev, n, 2 * prm->k, os, c->st, &launches);
+    }
+    const uint32_t *sp = in_alt ? palt : pos;
     uint64_t nn = n;
     CK(cudaMemcpyAsync(pos_off + nd, &nn, 8, cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
