@@ -283,6 +283,38 @@ constexpr uint32_t OF_TILE = 1024;  // a tile's runs begin in it
 constexpr uint32_t OF_RUN = 512;    // and are ranked in shared memory up to this length
 constexpr uint32_t OF_LOAD = OF_TILE + OF_RUN;
 
+// 1 where y at place j comes before x at place i (equal keys in their order):
+// the borrow of y - x less that of j - i, one subtraction a word.
+GKC_DEV uint32_t os_before(uint64_t y, uint32_t j, uint64_t x, uint32_t i) {
+  uint32_t t;
+  asm("{\n\t"
+      ".reg .u32 d;\n\t"
+      "sub.cc.u32 d, %1, %2;\n\t"
+      "subc.cc.u32 d, %3, %4;\n\t"
+      "subc.cc.u32 d, %5, %6;\n\t"
+      "subc.u32 %0, 0, 0;\n\t"
+      "}"
+      : "=r"(t)
+      : "r"(j), "r"(i), "r"((uint32_t)y), "r"((uint32_t)x), "r"((uint32_t)(y >> 32)), "r"((uint32_t)(x >> 32)));
+  return 0u - t;
+}
+GKC_DEV uint32_t os_before(u128 y, uint32_t j, u128 x, uint32_t i) {
+  uint32_t t;
+  asm("{\n\t"
+      ".reg .u32 d;\n\t"
+      "sub.cc.u32 d, %1, %2;\n\t"
+      "subc.cc.u32 d, %3, %4;\n\t"
+      "subc.cc.u32 d, %5, %6;\n\t"
+      "subc.cc.u32 d, %7, %8;\n\t"
+      "subc.cc.u32 d, %9, %10;\n\t"
+      "subc.u32 %0, 0, 0;\n\t"
+      "}"
+      : "=r"(t)
+      : "r"(j), "r"(i), "r"((uint32_t)y), "r"((uint32_t)x), "r"((uint32_t)(y >> 32)), "r"((uint32_t)(x >> 32)),
+        "r"((uint32_t)(y >> 64)), "r"((uint32_t)(x >> 64)), "r"((uint32_t)(y >> 96)), "r"((uint32_t)(x >> 96)));
+  return 0u - t;
+}
+
 // Copies [s, e), a run too long to be ranked by its tile, as it is; lists it
 // unless all its keys are equal (they are in order then).
 template <typename K>
@@ -308,8 +340,9 @@ GKC_DEV void os_long_run(const K *in, K *out, const uint32_t *vin, uint32_t *vou
 // keys keep their order).  A tile takes the runs that begin in it.  list[0]
 // counts the runs left to the host, [begin, end) from list[2] on: longer than
 // OF_RUN, so at most n / OF_RUN.  Bound by the comparisons, a run's length for
-// each key: 13.9 M 16-byte keys in runs of about 17 take 0.48 ms, the twelve
-// passes it stands for 2.7; 8.7 M distinct 8-byte keys 0.08 for 0.47.
+// each key (one subtraction a word: 0.48 -> 0.26 ms for 13.9 M 16-byte keys in
+// runs of about 17; the twelve
+// passes it stands for take 2.7.  8.7 M distinct 8-byte keys 0.08 for 0.47).
 template <typename K>
 __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uint32_t *vin, uint32_t *vout,
                                                   const uint64_t *n_dev, int bit0, unsigned long long *list) {
@@ -356,10 +389,8 @@ __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uin
       }
       const K x = S[i];
       uint32_t at = s;
-      for (uint32_t j = s; j < e; j++) {
-        const K y = S[j];
-        at += y < x || (y == x && j < i) ? 1u : 0u;
-      }
+#pragma unroll 4
+      for (uint32_t j = s; j < e; j++) at += os_before(S[j], j, x, i);
       out[base + at] = x;
       vout[base + at] = vin[base + i];
     }
