@@ -107,13 +107,16 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
                                                                            unsigned long long *lookback,
                                                                            unsigned long long *ticket, uint32_t *err) {
   constexpr int ITEMS = OS_ITEMS, TILE = OS_TILE;
-  __shared__ __align__(16) uint8_t sbuf[TILE * sizeof(K)];  // the tile in digit order; then its values
+  __shared__ __align__(16) uint8_t sbuf[TILE * sizeof(K)];
+  __shared__ uint8_t D[TILE];
   __shared__ uint32_t warp_cnt[OS_WARPS][OS_RADIX];
   __shared__ uint32_t toff[OS_RADIX];               // first tile position of each digit
-  __shared__ uint64_t gbase[OS_RADIX];              // where that position goes
+  __shared__ uint64_t gbase[OS_RADIX];              // where tile position 0 of each digit would go
   __shared__ uint32_t tmp[64];
   __shared__ uint64_t s_tile;
-  K *S = reinterpret_cast<K *>(sbuf);
+  K *S = reinterpret_cast<K *>(sbuf);               // the tile in digit order, D its digits
+  uint32_t *V = &warp_cnt[0][0];                    // and its values, once every rank is known
+  static_assert(TILE == OS_WARPS * OS_RADIX, "a value for every counter");
   const uint64_t n = *n_dev;
   const uint64_t n_tiles = (n + TILE - 1) / TILE;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -146,7 +149,7 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
       uint32_t base = 0;
       if (v) base = warp_cnt[warp][d];
       __syncwarp();
-      rank[r] = base + below;
+      rank[r] = d << 16 | (base + below);
       // the highest peer advances the warp's counter for this digit
       if (v && (peers >> lane) == 1u) warp_cnt[warp][d] = base + __popc(peers);
       __syncwarp();
@@ -164,15 +167,23 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
     }
     os_st(lb, (tile == 0 ? OS_PRE : OS_AGG) | run);
     uint32_t total;
-    toff[d] = block_exclusive_scan<OS_NT>(run, tmp, &total);
+    const uint32_t first = block_exclusive_scan<OS_NT>(run, tmp, &total);
+    toff[d] = first;
     __syncthreads();
 #pragma unroll
     for (int r = 0; r < ITEMS; r++)
       if (seg + (uint64_t)r * 32 + lane < n) {
-        const uint32_t x = os_digit<K>(key[r], shift);
-        rank[r] += toff[x] + warp_cnt[warp][x];
+        const uint32_t x = rank[r] >> 16;
+        rank[r] = (rank[r] & 0xFFFFu) + toff[x] + warp_cnt[warp][x];
         S[rank[r]] = key[r];
+        D[rank[r]] = (uint8_t)x;
       }
+    if (KV) {
+      __syncthreads();
+#pragma unroll
+      for (int r = 0; r < ITEMS; r++)
+        if (seg + (uint64_t)r * 32 + lane < n) V[rank[r]] = val[KV ? r : 0];
+    }
     // the earlier tiles' keys of this digit
     uint64_t excl = 0, j = tile;  // tiles [j, tile) are added up
     uint32_t it = 0;
@@ -208,29 +219,13 @@ __global__ void __launch_bounds__(OS_NT, 3) k_os_pass(const K *in, K *out, const
       }
     }
     if (tile != 0) os_st(lb, OS_PRE | (excl + run));
-    gbase[d] = digit_base[d] + excl;
+    gbase[d] = digit_base[d] + excl - first;
     __syncthreads();
+#pragma unroll 4
     for (uint32_t i = threadIdx.x; i < tn; i += OS_NT) {
-      const K x = S[i];
-      const uint32_t y = os_digit<K>(x, shift);
-      out[gbase[y] + (i - toff[y])] = x;
-    }
-    if (KV) {
-      // the values the same way; each one's digit beside it
-      __syncthreads();
-      uint32_t *V = reinterpret_cast<uint32_t *>(S);
-      uint8_t *D = reinterpret_cast<uint8_t *>(V + TILE);
-#pragma unroll
-      for (int r = 0; r < ITEMS; r++)
-        if (seg + (uint64_t)r * 32 + lane < n) {
-          V[rank[r]] = val[KV ? r : 0];
-          D[rank[r]] = (uint8_t)os_digit<K>(key[r], shift);
-        }
-      __syncthreads();
-      for (uint32_t i = threadIdx.x; i < tn; i += OS_NT) {
-        const uint32_t y = D[i];
-        vout[gbase[y] + (i - toff[y])] = V[i];
-      }
+      const uint64_t at = gbase[D[i]] + i;
+      out[at] = S[i];
+      if (KV) vout[at] = V[i];
     }
     __syncthreads();
   }
@@ -341,8 +336,7 @@ GKC_DEV void os_long_run(const K *in, K *out, const uint32_t *vin, uint32_t *vou
 // counts the runs left to the host, [begin, end) from list[2] on: longer than
 // OF_RUN, so at most n / OF_RUN.  Bound by the comparisons, a run's length for
 // each key (one subtraction a word: 0.48 -> 0.26 ms for 13.9 M 16-byte keys in
-// runs of about 17; the twelve
-// passes it stands for take 2.7.  8.7 M distinct 8-byte keys 0.08 for 0.47).
+// runs of about 17; the twelve passes it stands for take 2.7.  8.7 M distinct 8-byte keys 0.08 for 0.47).
 template <typename K>
 __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uint32_t *vin, uint32_t *vout,
                                                   const uint64_t *n_dev, int bit0, unsigned long long *list) {
