@@ -853,12 +853,13 @@ GKC_DEV uint32_t ht_slots(uint64_t n) {
 
 // Inserts the n keys into the table tab (S holds the fill counter and the
 // flag); false when they hold more than CAP distinct ones (only possible for
-// n > CAP).  At most CAP + NT slots are ever taken, so every probe chain ends
+// n > CAP).  At most CAP + B * NT slots are ever taken, so every probe chain ends
 // at a free slot.
 template <int NT, uint32_t CAP, uint32_t SLOTS, typename SM>
 GKC_DEV bool table_insert64(SM &S, uint64_t *tab, uint32_t *counts, const uint64_t *src, uint64_t n, uint32_t slots) {
-  constexpr int U = 8;  // keys in flight per thread
-  static_assert(CAP + NT < SLOTS, "a free slot is always left");
+  constexpr int U = 4;  // keys in flight per thread
+  constexpr int B = CAP + 4 * NT < SLOTS ? 4 : 2;  // first probes in flight, between looks at the flag
+  static_assert(CAP + B * NT < SLOTS, "a free slot is always left");
   const int tid = threadIdx.x;
   const bool limited = n > CAP;
   for (uint32_t i = tid; i < slots; i += NT) tab[i] = HT_EMPTY;
@@ -876,26 +877,35 @@ GKC_DEV bool table_insert64(SM &S, uint64_t *tab, uint32_t *counts, const uint64
       const uint64_t i = i0 + (uint64_t)u * NT;
       xs[u] = i < n ? __ldcg(reinterpret_cast<const unsigned long long *>(src) + i) : HT_EMPTY;
     }
-    if (limited && *(volatile int *)&S.flag) break;
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const uint64_t x = xs[u];
-      if (x == HT_EMPTY || (limited && *(volatile int *)&S.flag)) break;  // past the end, or given up
-      uint32_t h = ht_slot(x, slots);
-      while (true) {
-        uint64_t cur = T[h];
-        if (cur == HT_EMPTY) {
-          cur = atomicCAS(reinterpret_cast<unsigned long long *>(tab + h), (unsigned long long)HT_EMPTY,
-                          (unsigned long long)x);
-          if (cur == HT_EMPTY) {
-            if (limited && atomicAdd(&S.hfill, 1u) + 1 > CAP) S.flag = 1;
-            cur = x;
-          }
-        }
-        if (cur == x) break;
-        h = h + 1 == slots ? 0 : h + 1;
+    for (int u0 = 0; u0 < U; u0 += B) {
+      if (limited && *(volatile int *)&S.flag) break;
+      uint32_t h[B];
+      uint64_t cur[B];
+#pragma unroll
+      for (int u = 0; u < B; u++) {
+        h[u] = ht_slot(xs[u0 + u], slots);
+        cur[u] = T[h[u]];
       }
-      atomicAdd(&counts[h >> 1], 1u << (16 * (h & 1u)));
+#pragma unroll
+      for (int u = 0; u < B; u++) {
+        const uint64_t x = xs[u0 + u];
+        if (x == HT_EMPTY) break;  // past the end
+        while (cur[u] != x) {
+          if (cur[u] == HT_EMPTY) {
+            cur[u] = atomicCAS(reinterpret_cast<unsigned long long *>(tab + h[u]), (unsigned long long)HT_EMPTY,
+                               (unsigned long long)x);
+            if (cur[u] == HT_EMPTY) {
+              if (limited && atomicAdd(&S.hfill, 1u) + 1 > CAP) S.flag = 1;
+              break;
+            }
+            if (cur[u] == x) break;
+          }
+          h[u] = h[u] + 1 == slots ? 0 : h[u] + 1;
+          cur[u] = T[h[u]];
+        }
+        atomicAdd(&counts[h[u] >> 1], 1u << (16 * (h[u] & 1u)));
+      }
     }
   }
   __syncthreads();
@@ -1306,20 +1316,31 @@ GKC_DEV uint32_t sort_count(Area &S, const SortCountArgs &a, const Src &src, uin
     S.next = 0;
     if (lg == 0) S.same = 0;
   }
-  if (lg > 0 && w == 0) {
-    // splitter j (1 .. G - 1) is sample j * (samples / G); as a node of the
-    // tree it is number j >> (t + 1) of its level, t its trailing zero bits
-    K v[4];
-    uint32_t any = 0;
-    if (G <= 8) {  // n > 32 here: 32 samples, one a lane
-      K u[1] = {src.key(lane * n / 32)};
-      warp_bitonic<K, 1>(u);
-      const uint32_t j = lane * G / 32;
-      if (j > 0 && j * 32 == lane * G) {
-        const int t = __ffs((int)j) - 1;
-        S.spl[(1u << (lg - 1 - t)) + (j >> (t + 1))] = u[0];
+  if (lg > 0) {
+    // splitter j (1 .. G - 1) is sample j * (samples / G) in order; as a node
+    // of the tree it is number j >> (t + 1) of its level, t its trailing zero bits
+    auto put = [&](uint32_t j, K x) {
+      const int t = __ffs((int)j) - 1;
+      S.spl[(1u << (lg - 1 - t)) + (j >> (t + 1))] = x;
+    };
+    if (G <= 8) {  // n > 32 here: 32 samples, each ranked by a few threads (the block waits for them)
+      constexpr uint32_t T = NT / 32;
+      if (tid < 32) S.A[tid] = src.key(tid * n / 32);
+      if (tid == 0) S.same = 0;
+      __syncthreads();
+      const uint32_t i = tid / T;
+      const K x = S.A[i];
+      uint32_t r = 0;
+#pragma unroll
+      for (uint32_t j = tid % T; j < 32; j += T) {
+        const K y = S.A[j];
+        r += y < x || (y == x && j < i) ? 1u : 0u;
       }
-    } else {
+#pragma unroll
+      for (int d = 1; d < (int)T; d <<= 1) r += __shfl_xor_sync(0xffffffffu, r, d);
+      if (tid % T == 0 && r > 0 && r * G % 32 == 0) put(r * G / 32, x);
+    } else if (w == 0) {
+      K v[4];
 #pragma unroll
       for (int r = 0; r < 4; r++) v[r] = src.key((uint32_t)(r * 32 + lane) * n / 128);
       warp_bitonic<K, 4>(v);
@@ -1327,16 +1348,13 @@ GKC_DEV uint32_t sort_count(Area &S, const SortCountArgs &a, const Src &src, uin
 #pragma unroll
       for (int r = 0; r < 4; r += 2) {        // G = 64: every second one
         const uint32_t e = lane * 4 + r, jj = r ? e * G / 128 : j;
-        if (jj > 0 && jj * 128 == e * G) {
-          const int t = __ffs((int)jj) - 1;
-          S.spl[(1u << (lg - 1 - t)) + (jj >> (t + 1))] = v[r];
-        }
+        if (jj > 0 && jj * 128 == e * G) put(jj, v[r]);
       }
       // 32 equal samples: one key fills about a quarter of the bucket
       const K far = shfl_k<K>(v[0], min(lane + 8, 31u));
-      any = __any_sync(0xffffffffu, lane < 24 && v[0] == far && n > 4u * 32 * RMAX);
+      const uint32_t any = __any_sync(0xffffffffu, lane < 24 && v[0] == far && n > 4u * 32 * RMAX);
+      if (lane == 0) S.same = any;
     }
-    if (lane == 0) S.same = any;
   }
   __syncthreads();
   if (S.same) {
