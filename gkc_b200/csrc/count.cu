@@ -165,32 +165,24 @@ __global__ void k_chunk_first(ExpandArgs a) {
 
 // ------------------------------------------------------- k-mer runs
 
-// The superkmer of the bin holding k-mer q: the last one in [lo, hi] whose
-// k-mer prefix is at most q.
-GKC_DEV uint64_t skm_of_kmer(const uint64_t *koff, uint64_t lo, uint64_t hi, uint64_t q) {
-  while (lo < hi) {
-    const uint64_t mid = (lo + hi + 1) >> 1;
-    if (__ldg(koff + mid) <= q) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
+constexpr int KM_PIECE = 6;  // consecutive k-mers of a superkmer that a lane takes
 
-// A k-mer's 2k bits as 32-bit words of the packed bases (2 bits per base, MSB
-// first within a byte): its first base is in word 0, r bits below the top once
-// the word's bytes are swapped.  All words are loaded, so reads end within 16
-// bytes past the last superkmer (every packed buffer has them).
+// The bases of a piece as 32-bit words of the packed ones (2 bits per base,
+// MSB first within a byte): its first base is in word 0, r bits below the top
+// once the word's bytes are swapped.  All words are loaded, so reads end
+// within 16 bytes past the last superkmer (every packed buffer has them).
 template <typename K> struct PackedWords {
-  static constexpr int N = sizeof(K) / 4 + 1;
+  static constexpr int N = sizeof(K) / 4 + 2;  // 2 k + 2 (KM_PIECE - 1) + 30 bits
   uint32_t w[N];
-  uint32_t r;
+  uint32_t r, count;  // k-mers of the piece: 0 .. KM_PIECE
 };
 template <typename K>
-GKC_DEV void load_packed(PackedWords<K> &p, const uint8_t *packed, uint64_t off, uint32_t o, bool valid) {
+GKC_DEV void load_packed(PackedWords<K> &p, const uint8_t *packed, uint64_t off, uint32_t o) {
   const uint64_t at = off + (o >> 2);
   const uint32_t *src = reinterpret_cast<const uint32_t *>(packed + (at & ~3ull));
   p.r = 8 * ((uint32_t)at & 3u) + 2 * (o & 3u);
 #pragma unroll
-  for (int t = 0; t < PackedWords<K>::N; t++) p.w[t] = valid ? __ldg(src + t) : 0u;
+  for (int t = 0; t < PackedWords<K>::N; t++) p.w[t] = p.count ? __ldg(src + t) : 0u;
 }
 
 // Reverse complement of 16 bases.
@@ -198,51 +190,74 @@ GKC_DEV uint32_t revcomp32(uint32_t x) {
   const uint32_t y = __brev(x);
   return 2 * (~y & 0x55555555u) + (~(y >> 1) & 0x55555555u);
 }
-// The canonical key: the smaller of the k-mer and its reverse complement.  The
-// reverse complement of the whole words holds that of the k-mer in its low 2k
-// bits.
-GKC_DEV uint64_t packed_canonical(const PackedWords<uint64_t> &p, int k) {
-  const uint32_t b0 = __byte_perm(p.w[0], 0, 0x0123), b1 = __byte_perm(p.w[1], 0, 0x0123),
-                 b2 = __byte_perm(p.w[2], 0, 0x0123);
-  const uint32_t hi = __funnelshift_l(b1, b0, p.r), lo = __funnelshift_l(b2, b1, p.r);
-  const uint64_t rc = ((uint64_t)revcomp32(lo) << 32) | revcomp32(hi);
-  uint64_t x;
-  const int s = 64 - 2 * k;
-  if (s <= 32) x = ((uint64_t)__funnelshift_rc(hi, 0u, s) << 32) | __funnelshift_rc(lo, hi, s);
-  else x = hi >> (s - 32);
-  const uint64_t r = rc & (~0ull >> s);
-  return x < r ? x : r;
-}
-GKC_DEV u128 packed_canonical(const PackedWords<u128> &p, int k) {
-  uint32_t b[5], w[4];
+// The canonical keys (the smaller of a k-mer and its reverse complement) of a
+// piece, each to emit(key, valid).  The reverse complement of the piece's
+// words is taken once: that of a k-mer lies in it, as the k-mer in the words,
+// two bits further on for each k-mer.
+template <typename K, typename Emit>
+GKC_DEV void emit_piece(const PackedWords<K> &p, int k, Emit &&emit) {
+  constexpr int KW = sizeof(K) / 4;
+  uint32_t b[KW + 2], w[KW + 1], rc[KW + 1];
 #pragma unroll
-  for (int t = 0; t < 5; t++) b[t] = __byte_perm(p.w[t], 0, 0x0123);
+  for (int t = 0; t < KW + 2; t++) b[t] = __byte_perm(p.w[t], 0, 0x0123);
 #pragma unroll
-  for (int t = 0; t < 4; t++) w[t] = __funnelshift_l(b[t + 1], b[t], p.r);
-  const uint64_t hi = ((uint64_t)w[0] << 32) | w[1], lo = ((uint64_t)w[2] << 32) | w[3];
-  const uint64_t rhi = ((uint64_t)revcomp32(w[3]) << 32) | revcomp32(w[2]),
-                 rlo = ((uint64_t)revcomp32(w[1]) << 32) | revcomp32(w[0]);
-  const int s = 128 - 2 * k;  // 0 .. 62
-  const u128 x = (((u128)hi << 64) | lo) >> s;
-  const u128 r = ((u128)(rhi & (~0ull >> s)) << 64) | rlo;
-  return x < r ? x : r;
+  for (int t = 0; t <= KW; t++) {
+    w[t] = __funnelshift_l(b[t + 1], b[t], p.r);
+    rc[t] = revcomp32(w[t]);
+  }
+  const int s = 8 * (int)sizeof(K) - 2 * k;  // 0 .. 62
+  const uint32_t m0 = s < 32 ? 0xFFFFFFFFu >> s : 0u, m1 = s < 32 ? 0xFFFFFFFFu : 0xFFFFFFFFu >> (s - 32);
+#pragma unroll
+  for (int t = 0; t < KM_PIECE; t++) {
+    uint32_t m[KW], c[KW];  // the words from the k-mer's first base on; its reverse complement (both: word 0 on top)
+#pragma unroll
+    for (int i = 0; i < KW; i++) {
+      m[i] = __funnelshift_l(w[i + 1], w[i], 2 * t);
+      c[KW - 1 - i] = __funnelshift_r(rc[i], rc[i + 1], 2 * t);
+    }
+    c[0] &= m0;
+    c[1] &= m1;
+    K x = 0, r = 0;
+#pragma unroll
+    for (int i = 0; i < KW; i++) {
+      const uint32_t v = s < 32 ? __funnelshift_r(m[i], i > 0 ? m[i > 0 ? i - 1 : 0] : 0u, s)
+                                : i == 0 ? 0u : __funnelshift_r(m[i > 0 ? i - 1 : 0], i > 1 ? m[i > 1 ? i - 2 : 0] : 0u, s - 32);
+      x = (x << 32) | (K)v;
+      r = (r << 32) | (K)c[i];
+    }
+    emit(x < r ? x : r, (uint32_t)t < p.count);
+  }
 }
 
-// The k-mers [qa, qb) of one bin, taken by the calling warp 32 at a time,
-// lane i the i-th of each group: the ends of the 32 superkmers from the
-// group's first one on, held one per lane, become a bitmap of the group's
-// positions, in which each lane finds its superkmer (bits up to its own) and
-// the k-mer's index in it (the distance to the last of them).  The canonical
-// keys go to emit(key, valid) (called by every lane; valid is false past qb).
-// s0 is the superkmer holding k-mer qa, s_end the bin's end (k-mer offsets up
-// to koff[s_end] are read).
+GKC_DEV uint32_t warp_exclusive_scan(uint32_t c, uint32_t *total) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint32_t inc = c;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
+    if (lane >= (uint32_t)d) inc += t;
+  }
+  *total = __shfl_sync(0xffffffffu, inc, 31);
+  return inc - c;
+}
+
+// The k-mers [qa, qb) of one bin, taken by the calling warp: 32 superkmers,
+// one per lane, are cut into pieces of KM_PIECE consecutive k-mers, and each
+// round every lane takes a piece, found in a bitmap of the pieces that begin a
+// superkmer.  Whole rounds only: the pieces left over come first in the next
+// batch of superkmers, which begins with theirs.  The canonical keys go to
+// emit(key, valid) (called by every lane), in no order that matters.  s0 is
+// the superkmer holding k-mer qa, s_end the bin's end (k-mer offsets up to
+// koff[s_end] are read).
 //
 // What bounds it is instruction issue and the latency of the packed bases,
-// which lie in tile order: positions are 32-bit, relative to qa, the next
-// group's ends and descriptors are loaded and this group's packed words
-// requested before the last group's k-mers are built.
+// which lie in tile order: a lane's words, their bytes swapped, its place and
+// its reverse complement serve several k-mers; positions are 32-bit, relative to
+// qa; the next batch's ends and descriptors are loaded before this one's
+// rounds, and a piece's words requested before the piece before it is emitted.
 template <typename K, typename Emit>
 GKC_DEV void warp_kmers(const ExpandArgs &a, uint64_t qa, uint64_t qb, uint64_t s0, uint64_t s_end, Emit &&emit) {
+  constexpr uint32_t Q = KM_PIECE, FULL = 0xffffffffu;
   const uint32_t lane = threadIdx.x & 31u;
   const int k = a.k;
   const uint32_t n = (uint32_t)(qb - qa);  // at most a chunk
@@ -251,47 +266,59 @@ GKC_DEV void warp_kmers(const ExpandArgs &a, uint64_t qa, uint64_t qb, uint64_t 
   const uint32_t *koff = reinterpret_cast<const uint32_t *>(a.koff + s0);
   const unsigned long long *desc = reinterpret_cast<const unsigned long long *>(a.desc + s0);
   const uint32_t ns = (uint32_t)(s_end - s0), qa32 = (uint32_t)qa;
-  uint32_t base = 0;
   // end of superkmer base + lane, and its descriptor
   auto end_of = [&](uint32_t b) -> uint32_t { return b + lane < ns ? __ldg(koff + 2 * (b + lane) + 2) - qa32 : ~0u; };
   auto desc_of = [&](uint32_t b) -> uint64_t { return b + lane < ns ? __ldg(desc + b + lane) : 0ull; };
+  uint32_t base = 0, pos0 = 0;             // first superkmer of the batch, next k-mer to take
+  uint32_t kb = __ldg(koff) - qa32;        // start of superkmer base (modulo 2^32: at most its length before qa)
   uint32_t e = end_of(0);
   uint64_t ds = desc_of(0);
-  uint32_t kb = __ldg(koff) - qa32;  // start of superkmer base (modulo 2^32: at most its length before qa)
-  const uint32_t upto = 0xFFFFFFFFu >> (31 - lane);
+  const uint32_t upto = FULL >> (31 - lane);
   PackedWords<K> pw;
-  bool pvalid = false;
-  for (uint32_t q = 0; q < n; q += 32) {
-    const uint32_t rel = e - q;  // superkmer `base` holds q or ends at it, so e >= q
-    const uint32_t inside = __ballot_sync(0xffffffffu, rel < 32u);
-    const uint32_t ends = __reduce_or_sync(0xffffffffu, rel < 32u ? 1u << rel : 0u);
-    const bool valid = q + lane < n;
-    uint64_t my;
-    uint32_t o;
-    if (__popc(ends) == __popc(inside) && inside != 0xFFFFFFFFu) {
-      const uint32_t le = ends & upto;
-      // the lane's superkmer: as many from `base` on as end at or before it
-      my = __shfl_sync(0xffffffffu, ds, __popc(le));
-      o = le ? lane + __clz((int)le) - 31 : q + lane - kb;
-      base += __popc(ends);  // holds the next group's first k-mer or precedes it
-      if (ends) kb = q + 31 - __clz((int)ends);
+  bool have = false;
+  while (pos0 < n) {
+    const uint32_t ec = min(e, n), up = __shfl_up_sync(FULL, e, 1);
+    const uint32_t ks = lane ? up : kb, st = lane ? max(up, pos0) : pos0;  // start, and first k-mer to take
+    const uint32_t pieces = ec > st ? (ec - st + Q - 1) / Q : 0u;
+    uint32_t P;
+    const uint32_t S = warp_exclusive_scan(pieces, &P);
+    const uint32_t nz = __ballot_sync(FULL, pieces > 0);
+    const uint32_t all = __shfl_sync(FULL, ec, 31);  // the batch's k-mers end here
+    // the rounds of this batch, and where the next one begins
+    const uint32_t rounds = all == n || P < 32 ? (P + 31) / 32 : P / 32;
+    const uint64_t off = ds >> 24;
+    if (rounds * 32 >= P) {
+      pos0 = all;
+      base += 32;
+      kb = __shfl_sync(FULL, e, 31);
     } else {
-      // superkmers without k-mers, or more than 31 ends: searched one by one
-      const uint64_t x = qa + min(q + lane, n - 1), s = skm_of_kmer(a.koff, s0 + base, s_end - 1, x);
-      o = (uint32_t)(x - __ldg(a.koff + s));
-      my = __ldg(a.desc + s);
-      base = (uint32_t)(__shfl_sync(0xffffffffu, s, 31) - s0);
-      kb = __ldg(koff + 2 * base) - qa32;
+      const uint32_t j = 31 - __clz((int)__ballot_sync(FULL, pieces > 0 && S <= rounds * 32));
+      pos0 = __shfl_sync(FULL, st + Q * (rounds * 32 - S), j);
+      kb = __shfl_sync(FULL, ks, j);
+      base += j;
     }
-    PackedWords<K> nw;
-    load_packed<K>(nw, a.packed, my >> 24, o, valid);
     e = end_of(base);
     ds = desc_of(base);
-    if (q) emit(pvalid ? packed_canonical(pw, k) : (K)0, pvalid);
-    pw = nw;
-    pvalid = valid;
+    const uint32_t first = nz ? __ffs((int)nz) - 1 : 0, run = nz >> first;
+    const bool dense = (run & (run + 1)) == 0;  // superkmers without k-mers only before and after the others
+    for (uint32_t r = 0; r < rounds; r++) {
+      const uint32_t p = 32 * r + lane, rel = S - 32 * r;
+      const uint32_t before = __popc(__ballot_sync(FULL, pieces > 0 && S < 32 * r));
+      const uint32_t begins = __reduce_or_sync(FULL, pieces > 0 && rel < 32u ? 1u << rel : 0u);
+      const uint32_t at = before + __popc(begins & upto) - 1;  // the piece's superkmer, of those with pieces
+      const uint32_t j = dense ? first + at : __fns(nz, 0, (int)at + 1);
+      const uint32_t pos = __shfl_sync(FULL, st - Q * S, j) + Q * p, end = __shfl_sync(FULL, ec, j);
+      const uint32_t o = pos - __shfl_sync(FULL, ks, j);
+      const uint64_t src = __shfl_sync(FULL, off, j);
+      PackedWords<K> nw;
+      nw.count = p < P ? min(Q, end - pos) : 0u;
+      load_packed<K>(nw, a.packed, src, o);
+      if (have) emit_piece<K>(pw, k, emit);
+      pw = nw;
+      have = true;
+    }
   }
-  emit(pvalid ? packed_canonical(pw, k) : (K)0, pvalid);
+  if (have) emit_piece<K>(pw, k, emit);
 }
 
 // The k-mers of chunk c (bin b, j-th chunk of the bin) taken by warp w of W:
@@ -313,10 +340,13 @@ GKC_DEV uint64_t warp_run(const ExpandArgs &a, uint64_t c, uint32_t b, uint64_t 
 constexpr int HS_NT = 256;
 
 // Expands every k-mer once (k-mer extraction and canonical form:
-// kmer_counting.cu:99-112, 33-44) into `flat`, in k-mer order, and counts
-// the coarse digits of each chunk of a bin's k-mers; each warp takes a
-// contiguous share of the chunk, 32 consecutive k-mers at a time, so the
-// writes are coalesced.
+// kmer_counting.cu:99-112, 33-44) into `flat` and counts the coarse digits of
+// each chunk of a bin's k-mers.  Each warp takes a contiguous share of the
+// chunk and fills that share of `flat` front to back as its lanes emit keys,
+// so the writes are coalesced; their order within it is of no use to anyone.
+// 720 M 31-mers 5.9 -> 3.8 ms, 117 M 21-mers 1.02 -> 0.80, 88 M 63-mers 0.95 ->
+// 0.68 against one k-mer a lane and round (pieces of 3, 4, 5, 8 k-mers: 4.10,
+// 3.95, 3.85, 3.85 ms).
 template <typename K>
 __global__ void __launch_bounds__(HS_NT) k_bucket_hist(ExpandArgs a) {
   __shared__ uint32_t hist[1 << kCoarseMaxBits];
@@ -335,13 +365,15 @@ __global__ void __launch_bounds__(HS_NT) k_bucket_hist(ExpandArgs a) {
     uint64_t qa, qb;
     const uint64_t s0 = warp_run(a, c, b, j, w, HS_NT / 32, &qa, &qb);
     if (qa < qb && qb <= a.keys_cap) {
-      uint64_t q = qa + (threadIdx.x & 31u);
+      K *to = flat + qa;
+      const uint32_t below = (1u << (threadIdx.x & 31u)) - 1u;
       warp_kmers<K>(a, qa, qb, s0, a.bin_start[b + 1], [&](K key, bool valid) {
+        const uint32_t m = __ballot_sync(0xffffffffu, valid);
         if (valid) {
-          flat[q] = key;
+          to[__popc(m & below)] = key;
           atomicAdd(&hist[coarse_digit<K>(key, key_bits, cb)], 1u);
         }
-        q += 32;
+        to += __popc(m);
       });
     } else if (qa < qb && (threadIdx.x & 31u) == 0) {
       atomicOr(a.err, ERR_CAPACITY);
@@ -1138,18 +1170,6 @@ template <> GKC_DEV u128 shfl_up_k<u128>(u128 v, int d) {
   const uint64_t lo = __shfl_up_sync(0xffffffffu, (uint64_t)v, d);
   const uint64_t hi = __shfl_up_sync(0xffffffffu, (uint64_t)(v >> 64), d);
   return ((u128)hi << 64) | lo;
-}
-
-GKC_DEV uint32_t warp_exclusive_scan(uint32_t c, uint32_t *total) {
-  const uint32_t lane = threadIdx.x & 31u;
-  uint32_t inc = c;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
-    if (lane >= (uint32_t)d) inc += t;
-  }
-  *total = __shfl_sync(0xffffffffu, inc, 31);
-  return inc - c;
 }
 
 // Orders x and y (ascending if asc), and the smaller or the larger of two keys.
