@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(sc_threads(CTAS), CTAS) k_bucket_scatter(Expan
   constexpr int ND = 1 << kCoarseMaxBits;
   extern __shared__ __align__(16) uint8_t sc_smem[];
   K *S = reinterpret_cast<K *>(sc_smem);                      // the tile, by bucket
-  uint32_t *gbase = reinterpret_cast<uint32_t *>(S + SC_TILE);  // end of every bucket's run of this tile
+  uint32_t *gbase = reinterpret_cast<uint32_t *>(S + SC_TILE);  // next write offset of every bucket; in a tile less its start there
   uint32_t *toff = gbase + ND;                                // tile counts, then tile ends
   uint32_t *tmp = toff + ND;                                  // block scan
   uint16_t *Sd = reinterpret_cast<uint16_t *>(tmp + 64);      // buckets of S
@@ -624,11 +624,13 @@ __global__ void __launch_bounds__(sc_threads(CTAS), CTAS) k_bucket_scatter(Expan
     for (uint32_t d = tid; d < (1u << cb); d += SC_THREADS) {
       const uint16_t u = glut[d];
       lut[d] = u;
-      if (d == 0 || glut[d - 1] != u) gbase[u] = row[d];  // the bucket's first digit holds its offset
+      if (d == 0 || glut[d - 1] != u) {  // the bucket's first digit holds its offset
+        gbase[u] = row[d];
+        toff[u] = 0;
+      }
     }
+    __syncthreads();
     for (uint64_t t0 = q0; t0 < q1; t0 += SC_TILE) {
-      for (uint32_t d = tid; d < nd; d += SC_THREADS) toff[d] = 0;
-      __syncthreads();  // also: the chunk's tables are there
       const uint32_t tn = (uint32_t)min((uint64_t)SC_TILE, q1 - t0);
       uint32_t rk[KPT];  // bucket << 16 | rank within it (< SC_TILE)
 #pragma unroll
@@ -647,9 +649,9 @@ __global__ void __launch_bounds__(sc_threads(CTAS), CTAS) k_bucket_scatter(Expan
       uint32_t run = block_exclusive_scan<SC_THREADS>(sum, tmp, &total);
       for (uint32_t d = d0; d < d0 + per && d < nd; d++) {
         const uint32_t v = toff[d];
+        gbase[d] -= run;
         run += v;
         toff[d] = run;
-        gbase[d] += v;
       }
       __syncthreads();
 #pragma unroll
@@ -666,11 +668,16 @@ __global__ void __launch_bounds__(sc_threads(CTAS), CTAS) k_bucket_scatter(Expan
 #pragma unroll 4
       for (uint32_t i = tid; i < tn; i += SC_THREADS) {
         const uint32_t d = Sd[i];
-        const uint64_t slot = kbase + (uint32_t)(gbase[d] - toff[d] + i);
+        const uint64_t slot = kbase + (uint32_t)(gbase[d] + i);
         if (slot < a.keys_cap) keys[slot] = S[i];
         else atomicOr(a.err, ERR_CAPACITY);
       }
-      __syncthreads();  // before the next tile's counts and the next chunk's tables
+      __syncthreads();
+      for (uint32_t d = tid; d < nd; d += SC_THREADS) {  // for the next tile
+        gbase[d] += toff[d];
+        toff[d] = 0;
+      }
+      __syncthreads();  // also before the next chunk's tables
     }
   }
 }
