@@ -892,14 +892,20 @@ GKC_DEV uint32_t ht_slots(uint64_t n) {
 
 // Inserts the n keys into the table tab (S holds the fill counter and the
 // flag); false when they hold more than CAP distinct ones (only possible for
-// n > CAP).  At most CAP + B * NT slots are ever taken, so every probe chain ends
-// at a free slot.
+// n > CAP).  A key whose first slot holds it is counted at once; the others
+// (new ones, and those further down their chain) wait in the warp's queue
+// until 32 of them are there, so that the chains' loop runs with full warps
+// (720 M 31-mers at 30x: count stage 8.8 -> 8.1 ms).  A warp inserts at most 32
+// keys between looks at the flag, so at most CAP + NT slots are ever taken and
+// every probe chain ends at a free slot.
+constexpr int TQ_ROWS = 4;                       // keys in flight per thread
+constexpr uint32_t TQ_LEN = 32 * (TQ_ROWS + 1);  // a warp's queue: 31 keys left and a batch
 template <int NT, uint32_t CAP, uint32_t SLOTS, typename SM>
-GKC_DEV bool table_insert64(SM &S, uint64_t *tab, uint32_t *counts, const uint64_t *src, uint64_t n, uint32_t slots) {
-  constexpr int U = 4;  // keys in flight per thread
-  constexpr int B = CAP + 4 * NT < SLOTS ? 4 : 2;  // first probes in flight, between looks at the flag
-  static_assert(CAP + B * NT < SLOTS, "a free slot is always left");
+GKC_DEV bool table_insert64(SM &S, uint64_t *tab, uint32_t *counts, uint64_t *queue, const uint64_t *src, uint64_t n,
+                            uint32_t slots) {
+  static_assert(CAP + NT < SLOTS, "a free slot is always left");
   const int tid = threadIdx.x;
+  const uint32_t lane = tid & 31u, below = (1u << lane) - 1u;
   const bool limited = n > CAP;
   for (uint32_t i = tid; i < slots; i += NT) tab[i] = HT_EMPTY;
   for (uint32_t i = tid; i < slots / 2; i += NT) counts[i] = 0;
@@ -909,42 +915,54 @@ GKC_DEV bool table_insert64(SM &S, uint64_t *tab, uint32_t *counts, const uint64
   }
   __syncthreads();
   volatile uint64_t *T = tab;
-  for (uint64_t i0 = tid; i0 < n; i0 += (uint64_t)U * NT) {
-    uint64_t xs[U];
+  uint64_t *Q = queue + TQ_LEN * (tid >> 5);
+  uint32_t waiting = 0;  // the same in every lane
+  auto given_up = [&] { return limited && __any_sync(0xffffffffu, *(volatile int *)&S.flag); };
+  for (uint64_t i0 = 0; i0 < n && !given_up(); i0 += (uint64_t)TQ_ROWS * NT) {
+    uint64_t xs[TQ_ROWS], cur[TQ_ROWS];
+    uint32_t h[TQ_ROWS];
 #pragma unroll
-    for (int u = 0; u < U; u++) {
-      const uint64_t i = i0 + (uint64_t)u * NT;
+    for (int u = 0; u < TQ_ROWS; u++) {
+      const uint64_t i = i0 + (uint64_t)u * NT + tid;
       xs[u] = i < n ? __ldcg(reinterpret_cast<const unsigned long long *>(src) + i) : HT_EMPTY;
     }
 #pragma unroll
-    for (int u0 = 0; u0 < U; u0 += B) {
-      if (limited && *(volatile int *)&S.flag) break;
-      uint32_t h[B];
-      uint64_t cur[B];
+    for (int u = 0; u < TQ_ROWS; u++) {
+      h[u] = ht_slot(xs[u], slots);
+      cur[u] = T[h[u]];
+    }
 #pragma unroll
-      for (int u = 0; u < B; u++) {
-        h[u] = ht_slot(xs[u0 + u], slots);
-        cur[u] = T[h[u]];
-      }
-#pragma unroll
-      for (int u = 0; u < B; u++) {
-        const uint64_t x = xs[u0 + u];
-        if (x == HT_EMPTY) break;  // past the end
-        while (cur[u] != x) {
-          if (cur[u] == HT_EMPTY) {
-            cur[u] = atomicCAS(reinterpret_cast<unsigned long long *>(tab + h[u]), (unsigned long long)HT_EMPTY,
-                               (unsigned long long)x);
-            if (cur[u] == HT_EMPTY) {
+    for (int u = 0; u < TQ_ROWS; u++) {
+      const bool have = xs[u] != HT_EMPTY, hit = cur[u] == xs[u];
+      const uint32_t miss = __ballot_sync(0xffffffffu, have && !hit);
+      if (have && hit) atomicAdd(&counts[h[u] >> 1], 1u << (16 * (h[u] & 1u)));
+      if (have && !hit) Q[waiting + __popc(miss & below)] = xs[u];
+      waiting += __popc(miss);
+    }
+    const bool last = i0 + (uint64_t)TQ_ROWS * NT >= n;
+    while ((waiting >= 32 || (last && waiting > 0)) && !given_up()) {
+      const uint32_t m = min(waiting, 32u);
+      waiting -= m;
+      __syncwarp();
+      if (lane < m) {
+        const uint64_t x = Q[waiting + lane];
+        uint32_t s = ht_slot(x, slots);
+        while (true) {
+          uint64_t c = T[s];
+          if (c == HT_EMPTY) {
+            c = atomicCAS(reinterpret_cast<unsigned long long *>(tab + s), (unsigned long long)HT_EMPTY,
+                          (unsigned long long)x);
+            if (c == HT_EMPTY) {
               if (limited && atomicAdd(&S.hfill, 1u) + 1 > CAP) S.flag = 1;
-              break;
+              c = x;
             }
-            if (cur[u] == x) break;
           }
-          h[u] = h[u] + 1 == slots ? 0 : h[u] + 1;
-          cur[u] = T[h[u]];
+          if (c == x) break;
+          s = s + 1 == slots ? 0 : s + 1;
         }
-        atomicAdd(&counts[h[u] >> 1], 1u << (16 * (h[u] & 1u)));
+        atomicAdd(&counts[s >> 1], 1u << (16 * (s & 1u)));
       }
+      __syncwarp();
     }
   }
   __syncthreads();
@@ -952,7 +970,9 @@ GKC_DEV bool table_insert64(SM &S, uint64_t *tab, uint32_t *counts, const uint64
 }
 template <int NT>
 GKC_DEV bool table_insert(CountSmem<uint64_t> &S, const uint64_t *src, uint64_t n, uint32_t slots) {
-  return table_insert64<NT, CountShape<uint64_t>::CAP, CountShape<uint64_t>::SLOTS>(S, S.u.h.T, S.u.h.TC, src, n, slots);
+  static_assert(TQ_LEN * (NT / 32) <= CountShape<uint64_t>::CAP, "the groups' keys have room for the queues");
+  return table_insert64<NT, CountShape<uint64_t>::CAP, CountShape<uint64_t>::SLOTS>(S, S.u.h.T, S.u.h.TC, S.u.h.g.G, src,
+                                                                                  n, slots);
 }
 GKC_DEV bool slot_taken(const CountSmem<uint64_t> &S, uint32_t slot) { return S.u.h.T[slot] != HT_EMPTY; }
 GKC_DEV uint64_t slot_key(const CountSmem<uint64_t> &S, uint32_t slot) { return S.u.h.T[slot]; }
@@ -1467,7 +1487,8 @@ __device__ __noinline__ uint32_t dedup_count(SortSmem<uint64_t> &S, const SortCo
   DedupArea &H = S.u.d.t;
   constexpr int SPT = DedupArea::SLOTS / NT;
   static_assert(DedupArea::SLOTS % NT == 0 && SPT <= 32, "one mask per thread");
-  if (!table_insert64<NT, DedupArea::CAP, DedupArea::SLOTS>(S, H.T, H.TC, src, n, DedupArea::SLOTS)) {
+  static_assert(TQ_LEN * (NT / 32) <= DedupArea::CAP, "the sort's keys have room for the queues");
+  if (!table_insert64<NT, DedupArea::CAP, DedupArea::SLOTS>(S, H.T, H.TC, S.u.d.s.A, src, n, DedupArea::SLOTS)) {
     __syncthreads();
     return SORT_REJECTED;
   }
