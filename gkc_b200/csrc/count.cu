@@ -998,11 +998,18 @@ GKC_DEV bool table_insert(CountSmem<u128> &S, const u128 *src, uint64_t n, uint3
   HashArea<u128> &H = S.u.h;
   const int tid = threadIdx.x;
   if (n > (uint64_t)CountShape<u128>::CAP) return false;
-  for (uint32_t i = tid; i < (uint32_t)n; i += NT) {
-    const ulonglong2 v = __ldcg(reinterpret_cast<const ulonglong2 *>(src) + i);
-    H.A[i] = ((u128)v.y << 64) | v.x;
+  constexpr int CAP = CountShape<u128>::CAP, EPT = CAP / NT;
+  const uint32_t m = (uint32_t)n;
+  {
+    ulonglong2 v[EPT];
+#pragma unroll
+    for (int u = 0; u < EPT; u++)
+      if (u * NT + tid < m) v[u] = __ldcg(reinterpret_cast<const ulonglong2 *>(src) + u * NT + tid);
+    for (uint32_t i = tid; i < slots; i += NT) H.T[i] = 0;
+#pragma unroll
+    for (int u = 0; u < EPT; u++)
+      if (u * NT + tid < m) H.A[u * NT + tid] = ((u128)v[u].y << 64) | v[u].x;
   }
-  for (uint32_t i = tid; i < slots; i += NT) H.T[i] = 0;
   __syncthreads();
   volatile uint32_t *T = H.T;
   for (uint32_t i = tid; i < (uint32_t)n; i += NT) {
