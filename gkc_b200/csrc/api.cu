@@ -39,28 +39,20 @@ const char *gkc_status_string(gkc_status s) {
 
 int gkc_abi_version(void) { return GKC_ABI_VERSION; }
 
-// Stages of the batched pipeline, bounded by events sev[i] .. sev[i+1].
+// Stages of the batched pipeline.
 static const char *kStageNames[] = {"prepare", "partition", "bin_scatter", "coarse_hist",
                                     "coarse_scatter", "coarse_count", "finish"};
 constexpr int kNumStages = 7;
 const char *gkc_stage_name(int i) { return (i >= 0 && i < kNumStages) ? kStageNames[i] : ""; }
 
-// Records stage boundary i on the context stream (as a graph node while capturing).
-static void stage_mark(gkc_ctx *c, int i) {
-  if (c->capturing) cudaEventRecordWithFlags(c->sev[i], c->st, cudaEventRecordExternal);
-  else cudaEventRecord(c->sev[i], c->st);
-}
-
+// The first kernel of each stage writes the device's clock to its place (an
+// event between two kernels of a captured pipeline is a node of the graph that
+// both wait for:
+// without the eight a job of 100 k bases takes 163 us, with them 217).
 static void read_stage_times(gkc_ctx *c) {
   c->tm.n_stages = kNumStages;
-  for (int i = 0; i < kNumStages; i++) {
-    float ms = 0;
-    if (cudaEventElapsedTime(&ms, c->sev[i], c->sev[i + 1]) != cudaSuccess) {
-      cudaGetLastError();
-      ms = -1;
-    }
-    c->tm.stage_ms[i] = ms;
-  }
+  for (int i = 0; i < kNumStages; i++)
+    c->tm.stage_ms[i] = (float)((double)(int64_t)(c->h_tot->stamp[i + 1] - c->h_tot->stamp[i]) * 1e-6);
 }
 
 gkc_status ctx_fail(gkc_ctx *c, gkc_status s, const std::string &msg) {
@@ -254,7 +246,6 @@ gkc_status gkc_ctx_create(int device_id, uint64_t hbm_budget_bytes, gkc_ctx **ou
   c->h_tot = c->h_tots[0];
   c->own_stream = true;
   for (int i = 0; i < 4; i++) cudaEventCreate(&c->ev[i]);
-  for (int i = 0; i <= GKC_MAX_STAGES; i++) cudaEventCreate(&c->sev[i]);
   *out = c;
   return GKC_OK;
 }
@@ -267,8 +258,6 @@ void gkc_ctx_destroy(gkc_ctx *c) {
   trim_pool(c->dev);
   for (int i = 0; i < 4; i++)
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
-  for (int i = 0; i <= GKC_MAX_STAGES; i++)
-    if (c->sev[i]) cudaEventDestroy(c->sev[i]);
   if (c->h_tots[0]) cudaFreeHost(c->h_tots[0]);
   if (c->st_up) cudaStreamDestroy(c->st_up);
   if (c->st_dl) cudaStreamDestroy(c->st_dl);
@@ -346,13 +335,15 @@ static gkc_status check_params(gkc_ctx *c, const gkc_params *prm) {
 // The totals go straight to the slot's page-locked record (no copy follows).
 __global__ void k_finalize(DevTotals *t, const unsigned long long *cursors, const uint32_t *err,
                            const uint64_t *bin_kstart, uint32_t nbins, const uint64_t *n_bytes_dev,
-                           const uint64_t *bin_out) {
+                           const uint64_t *bin_out, const unsigned long long *stamp) {
+  for (int i = 0; i < kNumStages; i++) t->stamp[i] = stamp[i];
   t->n_skm = cursors[0];
   t->n_packed = cursors[1];
   t->err = *err;
   t->n_kmers = bin_kstart ? bin_kstart[nbins] : 0;
   t->n_bytes = n_bytes_dev ? *n_bytes_dev : 0;
   t->n_distinct = bin_out ? bin_out[nbins] : 0;
+  stamp_now(&t->stamp[kNumStages]);
   __threadfence_system();
 }
 
@@ -410,7 +401,7 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
   const uint64_t *nbytes_dev = nullptr;
   WS(tot, unsigned long long, "cursors", 4);
   WS(err, uint32_t, "err", 4);
-  stage_mark(c, 0);
+  WS(stamp, unsigned long long, "stamps", GKC_MAX_STAGES + 1);
   c->part_hpc_reads = nullptr;
   c->part_hpc_offs = nullptr;
   c->part_hpc_orig = nullptr;
@@ -418,7 +409,7 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
     WS(hoffs, uint64_t, "hpc_offs", n_reads + 2);
     WS(hreads, uint8_t, "hpc_reads", n_bytes + 64);
     WS(horig, int32_t, "hpc_orig", n_bytes + 16);
-    const gkc_status hs = hpc_enqueue(c, src, n_bytes, offs, n_reads, hreads, hoffs, horig);
+    const gkc_status hs = hpc_enqueue(c, src, n_bytes, offs, n_reads, hreads, hoffs, horig, stamp);
     if (hs != GKC_OK) return hs;
     src = hreads;
     offs = hoffs;
@@ -431,7 +422,7 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
   WS(rs, uint32_t, "rs_bits", rs_words);  // with HPC: the original reads' bitmap until here
   WS(bin_nskm, unsigned long long, "bin_nskm", nbins + 1);
   WS(bin_nkm, unsigned long long, "bin_nkmers", nbins + 1);
-  const ClearArgs ca{tot, err, bin_nskm, bin_nkm, nbins, rs, rs_words};
+  const ClearArgs ca{tot, err, bin_nskm, bin_nkm, nbins, rs, rs_words, prm->hpc ? nullptr : stamp};
   k_partition_clear<<<(unsigned)std::min<uint64_t>(rs_words / 1024 + 1, (uint64_t)c->n_sms * 8), 256, 0, c->st>>>(ca);
   LAUNCHED(c);
   k_read_start_bits<<<(unsigned)std::min<uint64_t>((n_reads + 256) / 256, 65535), 256, 0, c->st>>>(
@@ -471,14 +462,13 @@ static gkc_status enqueue_partition(gkc_ctx *c, const gkc_params *prm, const cha
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_partition, kPartThreads, smem));
   uint64_t tiles = (n_bytes + kPartTile - 1) / kPartTile;
   unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, (uint64_t)c->n_sms * std::max(occ, 1)));
-  stage_mark(c, 1);
+  a.stamp = stamp + 1;
   k_partition<<<grid, kPartThreads, smem, c->st>>>(a);
   LAUNCHED(c);
-  stage_mark(c, 2);
 
   WS(bin_start, uint64_t, "bin_start", nbins + 1);
   WS(bin_kstart, uint64_t, "bin_kstart", nbins + 1);
-  k_bin_prefix<<<1, kBinPrefixThreads, 0, c->st>>>(bin_nskm, bin_nkm, nbins, bin_start, bin_kstart);
+  k_bin_prefix<<<1, kBinPrefixThreads, 0, c->st>>>(bin_nskm, bin_nkm, nbins, bin_start, bin_kstart, stamp + 2);
   LAUNCHED(c);
   WS(bdesc, uint64_t, "skm_desc_bin", cap_skm);
   WS(bmm, uint32_t, "skm_mm_bin", cap_skm);
@@ -540,9 +530,9 @@ static gkc_status read_totals(gkc_ctx *c, bool with_count, uint32_t nbins) {
   const uint64_t *bk = (const uint64_t *)c->bufs["bin_kstart"].p;
   const uint64_t *bo = with_count ? (const uint64_t *)c->bufs[slot_name(c, "bin_out")].p : nullptr;
   k_finalize<<<1, 1, 0, c->st>>>(c->h_tot, (const unsigned long long *)c->bufs["cursors"].p,
-                                 (const uint32_t *)c->bufs["err"].p, bk, nbins, c->part_nbytes_dev, bo);
+                                 (const uint32_t *)c->bufs["err"].p, bk, nbins, c->part_nbytes_dev, bo,
+                                 (const unsigned long long *)c->bufs["stamps"].p);
   LAUNCHED(c);
-  stage_mark(c, 7);
   return GKC_OK;
 }
 
@@ -632,10 +622,10 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   const uint64_t *bin_kstart = (const uint64_t *)c->bufs["bin_kstart"].p;
 
   // k-mer offset of every bin-ordered superkmer
-  stage_mark(c, 3);
+  WS(stamp, unsigned long long, "stamps", GKC_MAX_STAGES + 1);
   WS(koff, uint64_t, "skm_koff", cap_skm + 2);
   WS(stmp, uint64_t, "scan_tmp2", scan_u64_tmp_words(cap_skm + 1) + 8);
-  c->launches += scan_kmers_dev(desc, prm->k, koff, cap_skm, (const uint64_t *)n_skm_dev, stmp, c->st);
+  c->launches += scan_kmers_dev(desc, prm->k, koff, cap_skm, (const uint64_t *)n_skm_dev, stmp, c->st, stamp + 3);
 
   WS(bin_bits, uint32_t, "bin_bits", nbins + 1);
   WS(bucket_base, uint64_t, "bucket_base", nbins + 1);
@@ -722,7 +712,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
                                                   (uint64_t)c->n_sms * 64),
                      kBucketOffsetThreads, 0, c->st>>>(ea, bstart, bsize);
   LAUNCHED(c);
-  stage_mark(c, 4);
+  ea.stamp = stamp + 4;
   const int sc_ctas = sizeof(K) == 8 && keys_cap / nbins <= kScatterPairBin ? 2 : 1;
   const size_t sct_smem = bucket_scatter_smem_bytes<K>(sc_ctas);
   if ((int)sct_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "scatter tile exceeds shared memory");
@@ -769,7 +759,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   if ((int)smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "count tables exceed shared memory");
   int occ = 0;
   CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_bucket_slices<K>, kBucketCountThreads, smem));
-  stage_mark(c, 5);
+  sa.stamp = stamp + 5;
   const size_t sort_smem = bucket_sort_smem_bytes<K>();
   if ((int)sort_smem > c->max_smem_optin) return ctx_fail(c, GKC_ERR_INTERNAL, "sort areas exceed shared memory");
   int sort_occ = 0;
@@ -786,9 +776,8 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   LAUNCHED(c);
   k_bucket_slices<K><<<open_grid, kBucketCountThreads, smem, c->st>>>(sa);
   LAUNCHED(c);
-  stage_mark(c, 6);
   // final offsets: the exclusive scan of the distinct counts (the bucket count is read on the device)
-  c->launches += scan_u64_dev(bucket_d, bucket_out, max_buckets, bucket_base + nbins, dtmp, c->st);
+  c->launches += scan_u64_dev(bucket_d, bucket_out, max_buckets, bucket_base + nbins, dtmp, c->st, stamp + 6);
   WS(out_counts, uint32_t, slot_name(c, "counts").c_str(), keys_cap);
   WS(bin_out, uint64_t, slot_name(c, "bin_out").c_str(), nbins + 1);
   k_compact_runs<K><<<c->n_sms * 8, 256, 0, c->st>>>(keys, stage_counts, bstart, bucket_d, bucket_out, bucket_base,

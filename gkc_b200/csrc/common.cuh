@@ -134,6 +134,16 @@ GKC_DEV uint32_t block_exclusive_scan(uint32_t v, uint32_t *tmp, uint32_t *total
   return res;
 }
 
+// The device's clock in ns to *stamp, by the first thread of a grid (a stage of
+// the pipeline begins with its first kernel; null: nothing to record).
+GKC_DEV void stamp_now(unsigned long long *stamp) {
+  if (stamp && blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+    *stamp = t;
+  }
+}
+
 // The same for one uint64 per thread; `tmp` holds >= 32 words.
 template <int NT>
 GKC_DEV uint64_t block_exclusive_scan_u64(uint64_t v, uint64_t *tmp, uint64_t *total) {

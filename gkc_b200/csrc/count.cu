@@ -596,6 +596,7 @@ __global__ void __launch_bounds__(sc_threads(CTAS), CTAS) k_bucket_scatter(Expan
   uint32_t *tmp = toff + ND;                                  // block scan
   uint16_t *Sd = reinterpret_cast<uint16_t *>(tmp + 64);      // buckets of S
   uint16_t *lut = Sd + SC_TILE;                               // bucket of every digit
+  stamp_now(a.stamp);
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   K *keys = reinterpret_cast<K *>(a.keys);
   const K *flat = reinterpret_cast<const K *>(a.flat);
@@ -1539,6 +1540,7 @@ __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket
   SortSmem<K> &S = *reinterpret_cast<SortSmem<K> *>(smem_raw);
   const K *keys = reinterpret_cast<const K *>(a.keys);
   const int tid = threadIdx.x;
+  stamp_now(a.stamp);
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   const uint64_t n_buckets = a.bucket_base[a.nbins];
   // several buckets per ticket only where every CTA gets many: with few, a

@@ -18,6 +18,7 @@ struct DevTotals {
   unsigned long long n_skm, n_packed;
   uint32_t err, pad;
   uint64_t n_kmers, n_bytes, n_distinct;
+  unsigned long long stamp[GKC_MAX_STAGES + 1];  // start of each stage, then the end (device clock, ns)
 };
 
 struct GraphKey {
@@ -89,7 +90,6 @@ struct gkc_ctx {
   DevTotals *h_tot = nullptr;                 // the current slot's
   int slot = 0;  // buffer set of the inputs and outputs in use (streaming form: 0 or 1)
   cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
-  cudaEvent_t sev[GKC_MAX_STAGES + 1] = {};  // stage boundaries of the batched pipeline
   bool capturing = false;
   uint32_t launches = 0;
   gkc_timings tm{};
@@ -149,6 +149,6 @@ gkc_status partition_device_impl(gkc_ctx *c, const gkc_params *prm, const char *
 gkc_status count_device_impl(gkc_ctx *c, const gkc_params *prm, gkc_mode mode);
 // Homopolymer compression of device reads, enqueued on the context's stream.
 gkc_status hpc_enqueue(gkc_ctx *c, const uint8_t *reads, uint64_t n_bytes, const uint64_t *offs, uint64_t n_reads,
-                       uint8_t *out, uint64_t *out_offs, int32_t *orig);
+                       uint8_t *out, uint64_t *out_offs, int32_t *orig, unsigned long long *stamp = nullptr);
 gkc_status upload_reads(gkc_ctx *c, const char *reads, const uint64_t *offs, uint64_t n_reads,
                         char **d_reads, uint64_t **d_offs, uint64_t *n_bytes);

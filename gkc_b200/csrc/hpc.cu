@@ -41,7 +41,8 @@ struct HpcArgs {
 };
 
 // One bit per read start inside [offs[0], offs[n]).
-__global__ void k_hpc_starts(HpcArgs a, uint32_t *starts) {
+__global__ void k_hpc_starts(HpcArgs a, uint32_t *starts, unsigned long long *stamp) {
+  stamp_now(stamp);
   const uint64_t lo = a.offs[0], hi = min(a.offs[a.n_reads], a.n_bytes);
   for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r < a.n_reads;
        r += (uint64_t)gridDim.x * blockDim.x) {
@@ -190,7 +191,7 @@ __global__ void k_hpc_offsets(HpcArgs a) {
   } while (0)
 
 gkc_status hpc_enqueue(gkc_ctx *c, const uint8_t *reads, uint64_t n_bytes, const uint64_t *offs, uint64_t n_reads,
-                       uint8_t *out, uint64_t *out_offs, int32_t *orig) {
+                       uint8_t *out, uint64_t *out_offs, int32_t *orig, unsigned long long *stamp) {
   using namespace gkc;
   const uint64_t tiles = std::max<uint64_t>(1, (n_bytes + HP_TILE - 1) / HP_TILE);
   // the bitmap of read starts; the partition's own, made afterwards, takes its place
@@ -205,7 +206,7 @@ gkc_status hpc_enqueue(gkc_ctx *c, const uint8_t *reads, uint64_t n_bytes, const
                   out, out_offs, orig};
   CK(cudaMemsetAsync(starts, 0, words * 4, c->st));
   const unsigned rgrid = (unsigned)std::min<uint64_t>((n_reads + 256) / 256, (uint64_t)c->n_sms * 16);
-  k_hpc_starts<<<rgrid, 256, 0, c->st>>>(a, starts);
+  k_hpc_starts<<<rgrid, 256, 0, c->st>>>(a, starts, stamp);
   k_hpc_flags<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 4), HP_NT, 0, c->st>>>(a);
   c->launches += 4 + scan_u64(cnt, off, tiles, stmp, c->st);
   k_hpc_write<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 4), HP_NT, 0, c->st>>>(a);

@@ -23,6 +23,7 @@ struct PartArgs {
   uint64_t cap_skm, cap_bytes;
   unsigned long long *bin_nskm, *bin_nkmers;
   uint32_t *err;
+  unsigned long long *stamp;    // start time, or null
 };
 
 constexpr int kPartThreads = 256;
@@ -47,6 +48,7 @@ struct ClearArgs {
   uint32_t nbins;
   uint32_t *rs_bits;
   uint64_t rs_words;
+  unsigned long long *stamp;  // start time, or null
 };
 __global__ void k_partition_clear(ClearArgs a);
 __global__ void k_read_start_bits(const uint64_t *offs, uint64_t n_reads, uint32_t *bits);
@@ -57,7 +59,7 @@ __global__ void k_bin_scatter(const unsigned long long *n_skm_ptr, const uint64_
 constexpr int kBinPrefixThreads = 1024;
 __global__ void k_bin_prefix(const unsigned long long *bin_nskm,
                              const unsigned long long *bin_nkmers, uint32_t nbins,
-                             uint64_t *bin_start, uint64_t *bin_kstart);
+                             uint64_t *bin_start, uint64_t *bin_kstart, unsigned long long *stamp);
 
 // ---- counting ----
 struct CountPlan {
@@ -109,6 +111,7 @@ struct ExpandArgs {
   uint32_t *bin_units;         // buckets of each bin
   unsigned long long *scan_done;  // zeroed
   uint32_t *err;
+  unsigned long long *stamp;   // start time of the scatter, or null
 };
 __global__ void k_chunk_first(ExpandArgs a);
 template <typename K> __global__ void k_bucket_hist(ExpandArgs a);
@@ -143,6 +146,7 @@ struct SortCountArgs {
   uint32_t *bucket_head;           // first task + 1 of each bucket, 0: none (zeroed before)
   uint64_t big_min;
   uint32_t *err;
+  unsigned long long *stamp;   // start time of k_bucket_sort, or null
 };
 template <typename K, bool NARROW> __global__ void k_bucket_sort(SortCountArgs a);
 template <typename K> size_t bucket_sort_smem_bytes();
@@ -188,10 +192,10 @@ uint32_t scan_u64(const unsigned long long *in, uint64_t *out, uint64_t n, uint6
 size_t scan_u64_tmp_words(uint64_t n);
 // the same over a device-side length min(*n_dev, n_cap)
 uint32_t scan_u64_dev(const unsigned long long *in, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
-                      uint64_t *block_tmp, cudaStream_t st);
+                      uint64_t *block_tmp, cudaStream_t st, unsigned long long *stamp = nullptr);
 // the same over the k-mers of each superkmer
 uint32_t scan_kmers_dev(const uint64_t *desc, int k, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
-                        uint64_t *block_tmp, cudaStream_t st);
+                        uint64_t *block_tmp, cudaStream_t st, unsigned long long *stamp = nullptr);
 
 }  // namespace gkc
 

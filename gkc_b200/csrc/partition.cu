@@ -53,6 +53,7 @@ constexpr uint32_t PT_EXT = 0xFFFFu;
 __global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PartSmem &S = *reinterpret_cast<PartSmem *>(smem_raw);
+  stamp_now(a.stamp);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int k = a.k, p = a.p, omega = a.k - a.p + 1;
   if (a.nbytes_dev) a.nbytes = *a.nbytes_dev;
@@ -286,6 +287,7 @@ size_t partition_smem_bytes(int nbins_smem) {
 }
 
 __global__ void k_partition_clear(ClearArgs a) {
+  stamp_now(a.stamp);
   const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
   if (t < 4) {
     a.cursors[t] = 0;
@@ -440,7 +442,8 @@ size_t bin_place_smem_bytes(uint32_t nbins) {
 // us at 256 bins).
 __global__ void __launch_bounds__(kBinPrefixThreads) k_bin_prefix(const unsigned long long *bin_nskm,
                                                                   const unsigned long long *bin_nkmers, uint32_t nbins,
-                                                                  uint64_t *bin_start, uint64_t *bin_kstart) {
+                                                                  uint64_t *bin_start, uint64_t *bin_kstart, unsigned long long *stamp) {
+  stamp_now(stamp);
   constexpr int NT = kBinPrefixThreads;
   __shared__ uint64_t tmp[32];
   uint64_t cs = 0, ck = 0;

@@ -326,7 +326,7 @@ gkc_status partition_plain_impl(gkc_ctx *c, const gkc_params *prm, const char *d
   CK(cudaMemcpyAsync(cur, hc, 16, cudaMemcpyHostToDevice, c->st));
   WS(bin_start, uint64_t, "bin_start", nbins + 1);
   WS(bin_kstart, uint64_t, "bin_kstart", nbins + 1);
-  k_bin_prefix<<<1, kBinPrefixThreads, 0, c->st>>>(bin_nskm, bin_nkm, nbins, bin_start, bin_kstart);
+  k_bin_prefix<<<1, kBinPrefixThreads, 0, c->st>>>(bin_nskm, bin_nkm, nbins, bin_start, bin_kstart, nullptr);
   WS(bfill, unsigned long long, "bin_fill", nbins + 1);
   CK(cudaMemsetAsync(bfill, 0, (nbins + 1) * 8, c->st));
   WS(bdesc, uint64_t, "skm_desc_bin", n_skm + 1);

@@ -42,7 +42,9 @@ struct ScanDescBytes {
 GKC_DEV uint64_t scan_len(uint64_t n_cap, const uint64_t *n_dev) { return n_dev ? min(n_cap, *n_dev) : n_cap; }
 
 template <typename Src>
-__global__ void __launch_bounds__(SCAN_ONE_NT) k_scan_one(Src in, uint64_t n_cap, const uint64_t *n_dev, uint64_t *out) {
+__global__ void __launch_bounds__(SCAN_ONE_NT) k_scan_one(Src in, uint64_t n_cap, const uint64_t *n_dev, uint64_t *out,
+                                                           unsigned long long *stamp) {
+  stamp_now(stamp);
   __shared__ uint64_t tmp[32];
   const uint64_t n = scan_len(n_cap, n_dev);
   uint64_t carry = 0;
@@ -68,7 +70,8 @@ __global__ void __launch_bounds__(SCAN_ONE_NT) k_scan_one(Src in, uint64_t n_cap
 
 template <typename Src>
 __global__ void __launch_bounds__(SCAN_NT) k_scan_reduce(Src in, uint64_t n_cap, const uint64_t *n_dev,
-                                                         uint64_t *tile_sum) {
+                                                         uint64_t *tile_sum, unsigned long long *stamp) {
+  stamp_now(stamp);
   __shared__ uint64_t tmp[32];
   const uint64_t n = scan_len(n_cap, n_dev), base = (uint64_t)blockIdx.x * SCAN_TILE;
   if (base >= n) return;  // not read by the next kernels
@@ -146,21 +149,21 @@ size_t scan_u64_tmp_words(uint64_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE +
 
 template <typename Src>
 static uint32_t scan_any(Src in, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev, uint64_t *block_tmp,
-                         cudaStream_t st) {
+                         cudaStream_t st, unsigned long long *stamp = nullptr) {
   if (n_cap <= SCAN_ONE_MAX) {
-    k_scan_one<Src><<<1, SCAN_ONE_NT, 0, st>>>(in, n_cap, n_dev, out);
+    k_scan_one<Src><<<1, SCAN_ONE_NT, 0, st>>>(in, n_cap, n_dev, out, stamp);
     return 1;
   }
   const unsigned tiles = (unsigned)((n_cap + SCAN_TILE - 1) / SCAN_TILE);
-  k_scan_reduce<Src><<<tiles, SCAN_NT, 0, st>>>(in, n_cap, n_dev, block_tmp);
+  k_scan_reduce<Src><<<tiles, SCAN_NT, 0, st>>>(in, n_cap, n_dev, block_tmp, stamp);
   k_scan_tiles<<<1, SCAN_ONE_NT, 0, st>>>(block_tmp, n_cap, n_dev, out);
   k_scan_apply<Src><<<tiles, SCAN_NT, 0, st>>>(in, n_cap, n_dev, block_tmp, out);
   return 3;
 }
 
 uint32_t scan_u64_dev(const unsigned long long *in, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
-                      uint64_t *block_tmp, cudaStream_t st) {
-  return scan_any(ScanArray{in}, out, n_cap, n_dev, block_tmp, st);
+                      uint64_t *block_tmp, cudaStream_t st, unsigned long long *stamp) {
+  return scan_any(ScanArray{in}, out, n_cap, n_dev, block_tmp, st, stamp);
 }
 
 uint32_t scan_u64(const unsigned long long *in, uint64_t *out, uint64_t n, uint64_t *block_tmp, cudaStream_t st) {
@@ -168,8 +171,8 @@ uint32_t scan_u64(const unsigned long long *in, uint64_t *out, uint64_t n, uint6
 }
 
 uint32_t scan_kmers_dev(const uint64_t *desc, int k, uint64_t *out, uint64_t n_cap, const uint64_t *n_dev,
-                        uint64_t *block_tmp, cudaStream_t st) {
-  return scan_any(ScanKmers{reinterpret_cast<const unsigned long long *>(desc), k}, out, n_cap, n_dev, block_tmp, st);
+                        uint64_t *block_tmp, cudaStream_t st, unsigned long long *stamp) {
+  return scan_any(ScanKmers{reinterpret_cast<const unsigned long long *>(desc), k}, out, n_cap, n_dev, block_tmp, st, stamp);
 }
 
 uint32_t scan_len_bytes(const uint32_t *len, uint64_t *out, uint64_t n, uint64_t *block_tmp, cudaStream_t st) {
