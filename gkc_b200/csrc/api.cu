@@ -47,8 +47,8 @@ const char *gkc_stage_name(int i) { return (i >= 0 && i < kNumStages) ? kStageNa
 
 // The first kernel of each stage writes the device's clock to its place (an
 // event between two kernels of a captured pipeline is a node of the graph that
-// both wait for:
-// without the eight a job of 100 k bases takes 163 us, with them 217).
+// the next one waits for: a job of 100 k bases takes 163 us, with eight of
+// them 217).
 static void read_stage_times(gkc_ctx *c) {
   c->tm.n_stages = kNumStages;
   for (int i = 0; i < kNumStages; i++)
@@ -387,7 +387,7 @@ uint64_t gkc_job_hbm_estimate(const gkc_params *prm, uint64_t n_bases, uint64_t 
   e += w * kc * 2 + 4 * kc * 2;                                          // keys, output keys, staged and output counts
   e += ((uint64_t)prm->nbins << max_bits) * (8 * 5 + 4 * 2);             // bucket starts, sizes, distinct counts,
                                                                          // offsets, scan; bins, large-bucket list
-  e += 8ull << 20;                                                       // count kernel's per-CTA slice starts
+  e += 8ull << 20;                                                       // tables of the buckets' digits, tasks
   return e + (64ull << 20);
 }
 

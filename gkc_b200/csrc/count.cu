@@ -4,27 +4,27 @@
 // every superkmer of a bin, canonicalised as min(x, revcomp(x)), sorted
 // ascending, run-length counted (count clamped to 2^32-1), per bin.
 //
-// The keys of a bin are split into buckets of about 3 K (1.5 K 16-byte) keys:
-// runs of digits, the digit being the top bits of an order-preserving map of
+// The keys of a bin are split into buckets of about 3 K keys: runs of digits, the digit being the top bits of an order-preserving map of
 // the key (eq_map), so a bin's sorted list is the concatenation of its
 // buckets' sorted lists.  Device stages:
-//   1. k_bucket_hist    - expands every k-mer once, in k-mer order, and per
-//                         chunk of a bin's k-mers counts the digits.  Warps take 32 consecutive k-mers at a time,
-//                         one per lane: each lane finds its superkmer by a
-//                         search over the next 32 superkmers' k-mer ends and
-//                         extracts its k-mer from aligned 8-byte words;
+//   1. k_bucket_hist    - expands every k-mer once and counts the digits of
+//                         each chunk of a bin's k-mers.  A lane takes a piece
+//                         of consecutive k-mers of a superkmer from one load
+//                         of aligned words;
 //   2. k_bucket_scan    - one CTA per bin packs the digits into buckets;
 //                         k_bucket_offsets turns the (chunk, digit) counts
 //                         into each chunk's write offset per bucket;
 //   3. k_bucket_scatter - moves every key to its chunk's offset for its
 //                         bucket plus its rank there;
 //   4. k_bucket_sort    - persistent, buckets taken by ticket, each counted
-//                         on its own: split into groups of about 100 keys by
-//                         splitters taken from its keys, the groups sorted
-//                         by warps in registers and run-length encoded.  The
-//                         runs are staged at the bucket's own key range and
-//                         its distinct count recorded; k_compact_runs then
-//                         moves them to the scan of the counts;
+//                         on its own (8-byte keys that mostly repeat: in a
+//                         small hash table first): split into groups of about
+//                         100 keys by splitters taken from its keys, the
+//                         groups sorted by warps in registers and run-length
+//                         encoded.  The runs are staged at the bucket's own
+//                         key range and its distinct count recorded;
+//                         k_compact_runs then moves them to the scan of the
+//                         counts;
 //      k_bucket_open    - the buckets too large for that, and those in which
 //                         copies of one key fill a group: the keys aggregated
 //                         in a shared-memory hash table and the distinct ones
@@ -344,7 +344,7 @@ constexpr int HS_NT = 256;
 // each chunk of a bin's k-mers.  Each warp takes a contiguous share of the
 // chunk and fills that share of `flat` front to back as its lanes emit keys,
 // so the writes are coalesced; their order within it is of no use to anyone.
-// 720 M 31-mers 5.9 -> 3.8 ms, 117 M 21-mers 1.02 -> 0.80, 88 M 63-mers 0.95 ->
+// 720 M 31-mers 5.9 -> 3.8 ms, 134.7 M 21-mers 1.02 -> 0.80, 112.8 M 63-mers 0.95 ->
 // 0.68 against one k-mer a lane and round (pieces of 3, 4, 5, 8 k-mers: 4.10,
 // 3.95, 3.85, 3.85 ms).
 template <typename K>
@@ -583,7 +583,7 @@ template <typename K> __host__ __device__ constexpr int sc_tile(int ctas) {
 // partial sectors at both ends of a run: one CTA an SM with as large a tile as
 // fits, or two that fill each other's gaps where runs stay long enough
 // (kScatterPairBin).  A tile is loaded into the registers that the previous
-// one's keys leave while that is written out.  720 M keys: 5.1 ms; 88 M of 16
+// one's keys leave while that is written out.  720 M keys: 5.1 ms; 112.8 M of 16
 // bytes: 1.17 -> 0.98 ms with two digit tables instead of three.
 template <typename K, int CTAS>
 __global__ void __launch_bounds__(sc_threads(CTAS), CTAS) k_bucket_scatter(ExpandArgs a) {
@@ -1531,8 +1531,8 @@ __device__ __noinline__ uint32_t slice_count(SortArea<K, NT, CountShape<K>::CAP>
 // each other's barriers.  Count stage (with the two kernels below) on a
 // B200, against counting each bucket in a 4096-slot hash table with a merge
 // sort, or by insertion and warp sorts of 4096 fixed digits: 720 M 31-mers at
-// 30x 9.7 ms (14.7), 134.7 M mostly distinct 21-mers 3.4 ms (10.6), 150.9 M
-// 25-mers of compressed long reads 4.5 ms (14.8), 112.8 M 63-mers 3.5 ms (9.9).
+// 30x 8.1 ms (14.7), 134.7 M mostly distinct 21-mers 2.7 ms (10.6), 150.9 M
+// 25-mers of compressed long reads 3.8 ms (14.8), 112.8 M 63-mers 2.8 ms (9.9).
 template <typename K, bool NARROW>
 __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket_sort(SortCountArgs a) {
   constexpr int NT = SortShape<K>::NT;

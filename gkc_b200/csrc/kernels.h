@@ -181,9 +181,9 @@ constexpr uint64_t kChunkKmersMin = 16384;
 // Largest mean bin (k-mers) whose 8-byte keys are scattered by two CTAs an SM
 // with tiles of 7168 keys rather than one with 16384: their phases overlap,
 // but in larger bins a bucket's run of the smaller tile ends within few 32-byte
-// sectors (117 M k-mers, one CTA / two: 256 bins 0.91 / 0.86 ms, 64 bins 0.98 /
+// sectors (134.7 M k-mers, one CTA / two: 256 bins 0.91 / 0.86 ms, 64 bins 0.98 /
 // 0.95, 31 bins 1.06 / 1.27; 720 M in 1024 bins 4.72 / 4.26).  16-byte keys
-// gain nothing from it (88 M in 128 bins: 1.02 / 1.09).
+// gain nothing from it (112.8 M in 128 bins: 1.02 / 1.09).
 constexpr uint64_t kScatterPairBin = 2 << 20;
 
 // device-wide exclusive scan of uint64 counters (n <= 2^31); out[n] = total.

@@ -336,7 +336,8 @@ GKC_DEV void os_long_run(const K *in, K *out, const uint32_t *vin, uint32_t *vou
 // counts the runs left to the host, [begin, end) from list[2] on: longer than
 // OF_RUN, so at most n / OF_RUN.  Bound by the comparisons, a run's length for
 // each key (one subtraction a word: 0.48 -> 0.26 ms for 13.9 M 16-byte keys in
-// runs of about 17; the twelve passes it stands for take 2.7.  8.7 M distinct 8-byte keys 0.08 for 0.47).
+// runs of about 17; the twelve passes it stands for take 2.7.  8.7 M distinct
+// 8-byte keys: 0.08, for passes of 0.47).
 template <typename K>
 __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uint32_t *vin, uint32_t *vout,
                                                   const uint64_t *n_dev, int bit0, unsigned long long *list) {

@@ -49,7 +49,8 @@ constexpr uint32_t PT_EXT = 0xFFFFu;
 // Bound by instruction issue and the barriers between its phases: 256 threads
 // and 64 registers, so that four CTAs on an SM overlap, the next tile's bytes
 // loaded while this one is worked on.  900 M bases of 150 b reads (k 31, p 11)
-// on a B200: see k_partition's figures at its launch.
+// on a B200: 4.4 ms (ALU pipe 66 % of its cycles, 110 instructions for 32
+// bases); every window searched from its bytes 8.7.
 __global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
   extern __shared__ __align__(16) uint8_t smem_raw[];
   PartSmem &S = *reinterpret_cast<PartSmem *>(smem_raw);

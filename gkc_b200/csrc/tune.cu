@@ -86,10 +86,12 @@ gkc_status gkc_tune_set(gkc_ctx *c, const gkc_tune_params *p) {
   if (!v.chunk_kmers) v.chunk_kmers = d.chunk_kmers;
   if (!v.count_ctas_per_sm) v.count_ctas_per_sm = d.count_ctas_per_sm;
   if (!valid(v)) return ctx_fail(c, GKC_ERR_INVALID_ARG, "tuning parameters out of range");
-  if (v.coarse_target != c->tune.coarse_target || v.chunk_kmers != c->tune.chunk_kmers ||
+  // the default chunk stays a default: small inputs take smaller ones
+  const uint32_t chunk = v.chunk_kmers == d.chunk_kmers ? 0 : v.chunk_kmers;
+  if (v.coarse_target != c->tune.coarse_target || chunk != c->tune.chunk_kmers ||
       v.count_ctas_per_sm != c->tune.count_ctas) {
     c->tune.coarse_target = v.coarse_target;
-    c->tune.chunk_kmers = v.chunk_kmers;
+    c->tune.chunk_kmers = chunk;
     c->tune.count_ctas = v.count_ctas_per_sm;
     graphs_invalidate(c);  // the captured pipeline holds the old shapes
   }
@@ -164,7 +166,7 @@ gkc_status gkc_tune_cache_load(const char *path) {
 static gkc_status time_count_stages(gkc_ctx *c, const gkc_params *prm, const char *d_reads, uint64_t nb,
                                     const uint64_t *d_offs, uint64_t nr, int reps, float *ms) {
   std::vector<float> t;
-  for (int r = 0; r < reps + 1; r++) {  // the first call captures the graph
+  for (int r = 0; r < reps + 1; r++) {  // the first call sizes the workspaces, the second is captured
     gkc_status s = gkc_pipeline_device(c, prm, GKC_MODE_BATCHED, d_reads, nb, d_offs, nr, nullptr, nullptr);
     if (s != GKC_OK) return s;
     if (r == 0) continue;

@@ -275,13 +275,13 @@ gkc_status gkc_db_read(const gkc_db *db, uint64_t first, uint64_t n, uint64_t *k
 /* ---- launch-shape tuning (the reference fixes its launch shape by hand:
  *      NUM_BLOCKS_PER_GRID, NUM_THREADS_PER_BLOCK and the stream count,
  *      experiment.cpp:234-238).  Shapes of the batched count stage that need
- *      no rebuild: the largest mean keys per count bucket (the coarse digit
- *      width of each bin follows from it), the k-mers per histogram chunk
- *      (a power of two) and the count kernel's CTAs per SM.  Zero fields
+ *      no rebuild: the keys per count bucket (digits are packed into buckets
+ *      of at most 7/16 of it, 3/8 for 16-byte keys), the k-mers per histogram
+ *      chunk (a power of two) and the CTAs per SM that count large buckets.  Zero fields
  *      mean the default. ---- */
 typedef struct gkc_tune_params {
   uint32_t coarse_target;      /* 256 .. 65536; default 8192 */
-  uint32_t chunk_kmers;        /* 4096 .. 2^22, a power of two; default 65536 */
+  uint32_t chunk_kmers;        /* 4096 .. 2^22, a power of two; default 65536, less for small inputs */
   uint32_t count_ctas_per_sm;  /* 1 .. 4; default 2 */
   uint32_t reserved;
 } gkc_tune_params;
