@@ -174,6 +174,9 @@ template <typename K> constexpr uint32_t bucket_target(uint32_t target) {
 }
 constexpr uint32_t kCoarseMaxBits = 12;
 constexpr uint64_t kChunkKmers = 65536;
+// Doubled where the histogram's CTAs get eight chunks each even so: fewer rows
+// of digits (720 M k-mers in bins of 2.8 M, 64 K / 128 K / 256 K: histogram +
+// scatter 8.85 / 8.56 / 8.71 ms; 151 M, which get 2.6: 2.00 / 2.04 / 2.19).
 // Halved down to this while there are fewer chunks than the histogram has CTAs
 // (histogram + scatter, 64 K / 32 K / 16 K: 20 M bases 389 / 319 / 269 us, 60 M
 // 718 / 684 / 678, 120 M 1331 / 1328 / 1387).
