@@ -1547,9 +1547,11 @@ __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket
   // batch would leave CTAs without any
   const uint32_t batch = n_buckets >= 16ull * CC_TICKETS * gridDim.x ? CC_TICKETS : 1;
   uint32_t bi = 0, bm = 0;          // thread 0: next and end of its batch of buckets
-  uint32_t repeats = 0;             // the same in every thread of the block
+  uint32_t repeats = 0;             // 8-byte keys: the same in every thread of the block
+  uint32_t skip = 0;                // thread 0, 16-byte keys: buckets to list before one is sorted again
+  uint32_t often = 0;               // thread 0, 16-byte keys: how many were listed last (0: the last one sorted held few repeats)
   while (true) {
-    if (tid == 0) {
+    if (tid == 0) while (true) {
       while (bi == bm) {  // a new batch, without the large ones
         const uint64_t t0 = atomicAdd(a.ticket, (unsigned long long)batch);
         bi = bm = 0;
@@ -1578,11 +1580,16 @@ __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket
             bm++;
           }
       }
+      if (sizeof(K) == 8 || skip == 0 || S.bg[bi] >= n_buckets) break;
+      a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)S.bg[bi++];
+      skip--;
+    }
+    if (tid == 0) {
       S.g = S.bg[bi];
       S.start = S.bstart[bi];
       S.n = S.bn[bi];
       bi++;
-      S.pf_n = bi < bm ? S.bn[bi] : 0;
+      S.pf_n = bi < bm && !often ? S.bn[bi] : 0;
       S.pf_start = bi < bm ? S.bstart[bi] : 0;
     }
     __syncthreads();
@@ -1597,20 +1604,22 @@ __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket
     // Which way is faster depends on how often keys repeat, which changes
     // little from bucket to bucket: the last bucket's share decides.  8-byte
     // keys: the table first where two keys in three or more are repeats.
-    // 16-byte keys have no table here: the next 15 such buckets go to the
-    // list, then one is sorted again.
+    // 16-byte keys have no table here: the next 15 buckets go to the list,
+    // unseen, then one is sorted again; 31 and 63 while that holds repeats
+    // too (count stage of 112.8 M 63-mers 2.84 ms with 15 each time, 2.71 so).
     uint32_t D = SORT_REJECTED;
     if (sizeof(K) == 8 && repeats) D = dedup_count<NT, NARROW>(S, a, keys + start, n, start);
-    if (D == SORT_REJECTED && (sizeof(K) == 8 || repeats == 0))
-      D = sort_count<K, NT, NARROW>(S.u.s, a, GlobalKeys<K>{keys + start}, n, start);
-    if (D != SORT_REJECTED) repeats = 3 * D <= n ? 15 : 0;
-    else if (sizeof(K) == 8) repeats = 0;
-    else if (repeats) repeats--;
-    if (tid == 0) {  // the counting's last barrier protects S.g too
+    if (D == SORT_REJECTED) D = sort_count<K, NT, NARROW>(S.u.s, a, GlobalKeys<K>{keys + start}, n, start);
+    const bool most = D != SORT_REJECTED && 3 * D <= n;
+    if (sizeof(K) == 8) repeats = most;
+    if (tid == 0) {  // sort_count's barriers lie between the reads of S.g and the next bucket's
       if (D != SORT_REJECTED) a.bucket_d[g] = D;
       else a.big_list[atomicAdd(a.big_count, 1ull)] = (uint32_t)g;
+      if (sizeof(K) == 16) {
+        often = most ? min(max(2 * often + 1, 15u), 63u) : 0;
+        skip = often;
+      }
     }
-    if (sizeof(K) == 16) __syncthreads();  // S.g is read before the next bucket, also where nothing was sorted
   }
 }
 
