@@ -695,7 +695,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   ea.flat = out_keys;
   ea.keys_cap = keys_cap;
   ea.err = err;
-  const uint64_t first_n = std::max(32 * max_chunks, ((uint64_t)nbins << max_bits) / 8);
+  const uint64_t first_n = 32 * std::max<uint64_t>(max_chunks, nbins);
   k_chunk_first<<<(unsigned)std::min<uint64_t>((first_n + 255) / 256, 65535), 256, 0, c->st>>>(ea);
   LAUNCHED(c);
   k_bucket_hist<K><<<(unsigned)std::min<uint64_t>(max_chunks, (uint64_t)c->n_sms * 8), kBucketHistThreads, 0, c->st>>>(ea);
@@ -780,7 +780,9 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   c->launches += scan_u64_dev(bucket_d, bucket_out, max_buckets, bucket_base + nbins, dtmp, c->st, stamp + 6);
   WS(out_counts, uint32_t, slot_name(c, "counts").c_str(), keys_cap);
   WS(bin_out, uint64_t, slot_name(c, "bin_out").c_str(), nbins + 1);
-  k_compact_runs<K><<<c->n_sms * 8, 256, 0, c->st>>>(keys, stage_counts, bstart, bucket_d, bucket_out, bucket_base,
+  // warps for every bucket and every 512 keys, at most what the chip holds
+  const uint64_t compact_n = std::max(max_buckets, keys_cap / 512) / 8 + 1;
+  k_compact_runs<K><<<(unsigned)std::min<uint64_t>(compact_n, (uint64_t)c->n_sms * 8), 256, 0, c->st>>>(keys, stage_counts, bstart, bucket_d, bucket_out, bucket_base,
                                                       nbins, out_keys, out_counts, bin_out, bucket_head, tasks, ticket + 4, err);
   LAUNCHED(c);
   c->count_keys_cap = keys_cap;

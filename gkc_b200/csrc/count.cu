@@ -152,8 +152,10 @@ GKC_DEV uint64_t warp_last_le(const uint64_t *a, uint64_t lo, uint64_t hi, uint6
 __global__ void k_chunk_first(ExpandArgs a) {
   if (*a.err & (ERR_CAPACITY | ERR_BAD_READ | ERR_BIN_TOO_LARGE)) return;
   const uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x, nt = (uint64_t)gridDim.x * blockDim.x;
-  const uint64_t n_tot = (uint64_t)a.nbins << a.max_bits;
-  for (uint64_t i = t; i < n_tot; i += nt) a.digit_total[i] = 0;
+  for (uint64_t b = t >> 5; b < a.nbins; b += nt >> 5) {  // a warp per bin, its digits only
+    uint32_t *tot = a.digit_total + (b << a.max_bits);
+    for (uint32_t d = threadIdx.x & 31u; d < 1u << a.bin_bits[b]; d += 32) tot[d] = 0;
+  }
   const uint64_t n_chunks = a.chunk_base[a.nbins];
   for (uint64_t c = t >> 5; c < n_chunks; c += nt >> 5) {  // a warp per chunk
     const uint32_t b = (uint32_t)warp_last_le(a.chunk_base, 0, a.nbins - 1, c);
