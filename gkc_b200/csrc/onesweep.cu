@@ -6,7 +6,9 @@
 // look-back, so keys are scattered in one read and one write per pass.
 //
 // Keys: uint64 or unsigned __int128, sorted on their low `key_bits` bits,
-// 8-bit digits.  Every wait on another tile is bounded.
+// 8-bit digits.  Every wait on another tile is bounded.  Long keys with values
+// (sort_pairs) take passes over their leading bits only; a kernel of its own
+// orders the runs that these leave.
 #include <algorithm>
 #include <utility>
 #include <vector>
