@@ -248,13 +248,16 @@ GKC_DEV K tile_kmer(const TileBases &S, int l, int k) {
 }
 
 // Writes (canonical key, window start) of the selected windows in window
-// order: a warp takes its words of the tile, each lane the k-mer of its own
-// window from the tile's packed bases.
+// order: a warp lists the selected windows of its words of the tile, then each
+// lane takes the k-mer of one of them from the tile's packed bases, so that
+// full warps cut and compare k-mers (13.9 M of 56 M windows at k 63: 171
+// us; each lane its own window, a quarter of them selected, 203).
 template <typename K>
 __global__ void __launch_bounds__(SUB_NT) k_sub_write(WinArgs a, const uint32_t *sel, const uint64_t *tile_off,
                                                       K *keys, uint32_t *posv, uint64_t n_tiles) {
   __shared__ TileBases S;
   __shared__ uint32_t cnt[TL_WARPS];
+  __shared__ uint16_t list[TL_NW_MAX];
   const int strip = tile_strip(a.k - a.p + 1), NW = TL_WARPS * strip, words = strip / 32;  // at most 15 words a warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * words;
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
@@ -268,16 +271,19 @@ __global__ void __launch_bounds__(SUB_NT) k_sub_write(WinArgs a, const uint32_t 
     __syncthreads();
     uint64_t o = tile_off[tile];
     for (int x = 0; x < warp; x++) o += cnt[x];
+    uint16_t *L = list + 32 * w0;
+    uint32_t n = 0;
     for (int r = 0; r < words; r++) {
       const uint32_t f = __shfl_sync(0xffffffffu, mine, r);
-      if ((f >> lane) & 1u) {
-        const int l = 32 * (w0 + r) + lane;
-        const K x = tile_kmer<K>(S, l, a.k), rc = revcomp_k<K>(x, a.k);
-        const uint64_t at = o + __popc(f & ((1u << lane) - 1u));
-        keys[at] = x < rc ? x : rc;
-        posv[at] = (uint32_t)(G0 + l);
-      }
-      o += __popc(f);
+      if ((f >> lane) & 1u) L[n + __popc(f & ((1u << lane) - 1u))] = (uint16_t)(32 * (w0 + r) + lane);
+      n += __popc(f);
+    }
+    __syncwarp();
+    for (uint32_t i = lane; i < n; i += 32) {
+      const int l = L[i];
+      const K x = tile_kmer<K>(S, l, a.k), rc = revcomp_k<K>(x, a.k);
+      keys[o + i] = x < rc ? x : rc;
+      posv[o + i] = (uint32_t)(G0 + l);
     }
     __syncthreads();  // before the next tile's bases
   }
