@@ -104,6 +104,8 @@ GKC_DEV uint32_t plan_bits(uint64_t nk, uint32_t bucket_keys, uint32_t max_bits,
 }
 // One CTA: the digits and chunks of every bin and the chunks' prefixes
 // (one bin per thread; one thread for all bins took 71-134 us at 256 bins).
+// A bin that is too large is flagged here, before the kernels that return at
+// the flag begin: threads of one block must not read it differently.
 __global__ void __launch_bounds__(kCountPlanThreads) k_count_plan(CountPlan pl) {
   constexpr int NT = kCountPlanThreads;
   __shared__ uint64_t tmp[32];
@@ -113,6 +115,7 @@ __global__ void __launch_bounds__(kCountPlanThreads) k_count_plan(CountPlan pl) 
     const uint32_t b = b0 + threadIdx.x;
     const bool in = b < pl.nbins;
     const uint64_t nk = dead || !in ? 0 : pl.bin_kstart[b + 1] - pl.bin_kstart[b];
+    if (nk >> 32) atomicOr(pl.err, ERR_BIN_TOO_LARGE);  // offsets in a bin are 32-bit
     const uint32_t bits = plan_bits(nk, pl.bucket_keys, pl.max_bits, 2 * pl.k);
     const uint64_t nch = (nk + pl.chunk_kmers - 1) / pl.chunk_kmers;
     uint64_t nc, nh;
@@ -415,8 +418,6 @@ __global__ void __launch_bounds__(BS_NT) k_bucket_scan(ExpandArgs a) {
   const int tid = threadIdx.x;
   for (uint32_t b = blockIdx.x; b < a.nbins; b += gridDim.x) {
     const uint32_t bits = a.bin_bits[b], nd = 1u << bits;
-    const uint64_t nk = a.bin_kstart[b + 1] - a.bin_kstart[b];
-    if (nk >= (1ull << 32) && tid == 0) atomicOr(a.err, ERR_BIN_TOO_LARGE);  // offsets in a bin are 32-bit
     // thread t holds the contiguous digits [t * DPT, t * DPT + DPT)
     const uint32_t d0 = tid * DPT;
     const uint32_t *total = a.digit_total + ((uint64_t)b << a.max_bits);

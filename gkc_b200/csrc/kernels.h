@@ -71,7 +71,7 @@ struct CountPlan {
   uint32_t max_bits;           // digit bits cap (<= kCoarseMaxBits)
   uint64_t chunk_kmers;        // k-mers per expansion chunk
   int k;
-  const uint32_t *err;         // nothing is planned after an upstream overflow
+  uint32_t *err;               // nothing is planned after an upstream overflow; flags a bin of 2^32 k-mers
   // outputs
   uint32_t *bin_bits;          // digit bits per bin
   uint64_t *chunk_base;        // first chunk of each bin (nbins+1)
