@@ -998,6 +998,20 @@ gkc_status gkc_pipeline_device(gkc_ctx *c, const gkc_params *prm, gkc_mode mode,
   return GKC_OK;
 }
 
+// A call with inputs in host memory that fails while they are being copied
+// ends only when they are no longer read: page-locked ones are copied after
+// the copy's own call has returned.
+struct SettleOnError {
+  gkc_ctx *c;
+  bool ok = false;
+  explicit SettleOnError(gkc_ctx *ctx) : c(ctx) {}
+  ~SettleOnError() {
+    if (ok) return;
+    if (c->st_up) cudaStreamSynchronize(c->st_up);
+    cudaStreamSynchronize(c->st);
+  }
+};
+
 // Host entry: H2D of reads and rebased offsets, then the device pipeline.
 gkc_status upload_reads(gkc_ctx *c, const char *reads, const uint64_t *offs, uint64_t n_reads,
                         char **d_reads, uint64_t **d_offs, uint64_t *n_bytes) {
@@ -1026,11 +1040,14 @@ gkc_status gkc_partition_host(gkc_ctx *c, const gkc_params *prm, const char *rea
   gkc_status s = check_params(c, prm);
   if (s != GKC_OK) return s;
   cudaSetDevice(c->dev);
+  SettleOnError settle(c);
   char *dr;
   uint64_t *doffs, nb;
   s = upload_reads(c, reads, offs, n_reads, &dr, &doffs, &nb);
   if (s != GKC_OK) return s;
-  return gkc_partition_device(c, prm, dr, nb, doffs, n_reads, out);
+  s = gkc_partition_device(c, prm, dr, nb, doffs, n_reads, out);
+  settle.ok = s == GKC_OK;
+  return s;
 }
 
 gkc_status gkc_pipeline_host(gkc_ctx *c, const gkc_params *prm, gkc_mode mode, const char *reads,
@@ -1040,12 +1057,14 @@ gkc_status gkc_pipeline_host(gkc_ctx *c, const gkc_params *prm, gkc_mode mode, c
   if (s != GKC_OK) return s;
   cudaSetDevice(c->dev);
   CK(cudaEventRecord(c->ev[3], c->st));
+  SettleOnError settle(c);
   char *dr;
   uint64_t *doffs, nb;
   s = upload_reads(c, reads, offs, n_reads, &dr, &doffs, &nb);
   if (s != GKC_OK) return s;
   s = gkc_pipeline_device(c, prm, mode, dr, nb, doffs, n_reads, nullptr, cnt);
   if (s != GKC_OK) return s;
+  settle.ok = true;
   float ms = 0;
   cudaEventElapsedTime(&ms, c->ev[3], c->ev[0]);
   c->tm.h2d_ms = ms;
@@ -1197,6 +1216,7 @@ gkc_status gkc_stream_submit(gkc_ctx *c, const gkc_params *prm, const char *read
   }
   WS(dr, char, rn.c_str(), nb + 64);
   WS(doffs, uint64_t, ofn.c_str(), n_reads + 1);
+  SettleOnError settle(c);
   // inputs of the slot's previous call must have been read before they are replaced
   if (t >= 2) CK(cudaStreamWaitEvent(c->st_up, c->ev_comp[slot], 0));
   if (nb) CK(cudaMemcpyAsync(dr, reads + base, nb, cudaMemcpyHostToDevice, c->st_up));
@@ -1228,6 +1248,7 @@ gkc_status gkc_stream_submit(gkc_ctx *c, const gkc_params *prm, const char *read
   c->calls[rec] = sc;
   c->next_ticket = t + 1;
   *ticket = t;
+  settle.ok = true;  // the call is in flight: its inputs are read until its wait
   // the previous call (the other slot), if its pipeline is already done:
   // start its download now
   if (t >= 1) {
@@ -1403,6 +1424,7 @@ gkc_status gkc_count_superkmers_host(gkc_ctx *c, int k, const uint32_t *skm_len,
   uint32_t *dl = dmm;
   WS(boff, uint64_t, "skm_koff", n_skm + 3);
   WS(btmp, uint64_t, "scan_tmp2", scan_u64_tmp_words(n_skm + 1) + 8);
+  SettleOnError settle(c);
   // both copies before the kernels: a copy from pageable memory waits for the stream
   if (n_skm) CK(cudaMemcpyAsync(dl, skm_len, n_skm * 4, cudaMemcpyHostToDevice, c->st));
   if (off) CK(cudaMemcpyAsync(dp, packed, off, cudaMemcpyHostToDevice, c->st));
@@ -1432,6 +1454,7 @@ gkc_status gkc_count_superkmers_host(gkc_ctx *c, int k, const uint32_t *skm_len,
   graphs_invalidate(c);
   gkc_status s = gkc_count_device(c, &prm, mode, nullptr);
   if (s != GKC_OK) return s;
+  settle.ok = true;
   if (n_distinct) *n_distinct = c->cv.n_distinct;
   return GKC_OK;
 }
