@@ -536,8 +536,7 @@ static gkc_status read_totals(gkc_ctx *c, bool with_count, uint32_t nbins) {
   return GKC_OK;
 }
 
-static gkc_status check_device_err(gkc_ctx *c) {
-  uint32_t e = c->h_tot->err;
+static gkc_status device_err(gkc_ctx *c, uint32_t e) {
   if (e & ERR_BIN_TOO_LARGE)
     return ctx_fail(c, GKC_ERR_CAPACITY, "a bin holds 2^32 or more k-mers: use more bins");
   if (e & ERR_BOUNDS) return ctx_fail(c, GKC_ERR_INTERNAL, "device bounds check failed");
@@ -545,6 +544,7 @@ static gkc_status check_device_err(gkc_ctx *c) {
   if (e & ERR_BAD_READ) return ctx_fail(c, GKC_ERR_INVALID_ARG, "read longer than supported");
   return GKC_OK;
 }
+static gkc_status check_device_err(gkc_ctx *c) { return device_err(c, c->h_tot->err); }
 
 gkc_status partition_device_impl(gkc_ctx *c, const gkc_params *prm, const char *d_reads,
                                  uint64_t n_bytes, const uint64_t *d_offs, uint64_t n_reads) {
@@ -1277,9 +1277,8 @@ gkc_status gkc_stream_wait(gkc_ctx *c, uint64_t ticket, uint64_t *n_distinct, ui
   if (n_kmers) *n_kmers = h->n_kmers;
   if (h->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))
     return ctx_fail(c, GKC_ERR_CAPACITY, "the call's input outgrew the captured pipeline: run it with gkc_pipeline_host");
-  if (h->err & ERR_BIN_TOO_LARGE) return ctx_fail(c, GKC_ERR_CAPACITY, "a bin holds 2^32 or more k-mers");
-  if (h->err & ERR_SPIN_TIMEOUT) return ctx_fail(c, GKC_ERR_DEVICE_TIMEOUT, "device look-back wait timed out");
-  if (h->err & (ERR_BOUNDS | ERR_BAD_READ)) return ctx_fail(c, GKC_ERR_INTERNAL, "device check failed");
+  s = device_err(c, h->err);
+  if (s != GKC_OK) return s;
   if (h->n_distinct > sc.capacity)
     return ctx_fail(c, GKC_ERR_CAPACITY, "result larger than the output capacity (bin offsets and the first entries copied)");
   return GKC_OK;
