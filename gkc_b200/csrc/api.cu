@@ -908,10 +908,10 @@ static gkc_status capture_pipeline(gkc_ctx *c, const gkc_params *prm, SlotGraph 
 // every size was captured at its first call.  All sizes the kernels need are
 // read on the device.  With `async`, the pipeline is only enqueued: its totals
 // land in the slot's pinned totals and are checked by the caller after the
-// stream (`direct`, `cap_used`: how it was run, for a rerun).
+// stream (`cap_used`: what it was run with, for a rerun).
 static gkc_status pipeline_batched(gkc_ctx *c, const gkc_params *prm, const char *d_reads,
                                    uint64_t n_bytes, const uint64_t *d_offs, uint64_t n_reads,
-                                   bool async = false, bool *direct = nullptr, PipelineCaps *cap_used = nullptr) {
+                                   bool async = false, PipelineCaps *cap_used = nullptr) {
   const GraphKey key{d_reads, d_offs, n_bytes, n_reads, prm->k, prm->p, prm->hpc, prm->nbins, c->filter};
   SlotGraph &G = c->graphs[c->slot];
   PipelineCaps cap;
@@ -947,7 +947,6 @@ static gkc_status pipeline_batched(gkc_ctx *c, const gkc_params *prm, const char
       G.seen = true;
     }
     if (async) {
-      if (direct) *direct = !c->tm.graph_replayed;
       if (cap_used) *cap_used = cap;
       return GKC_OK;
     }
@@ -1100,9 +1099,10 @@ static void set_results(gkc_ctx *c, StreamCall &sc) {
   sc.d_counts = c->bufs[slot_name(c, "counts")].p;
 }
 
-// A streaming call of a new size whose workspaces were too small for its
-// reads is run again with the sizes the device reported: its inputs stay in
-// the slot until its download is enqueued.  Waits for the device.
+// A streaming call whose workspaces were too small for its reads (sized from
+// their number of bases, or by an earlier call of that size) is run again with
+// the sizes the device reported: its inputs stay in the slot until its
+// download is enqueued.  Waits for the device.
 static gkc_status rerun_larger(gkc_ctx *c, StreamCall &sc, int slot) {
   OnSlot on(c, slot);
   const int filter = c->filter;
@@ -1138,7 +1138,7 @@ static gkc_status issue_download(gkc_ctx *c, int rec) {
   if (sc.dl_issued) return GKC_OK;
   const int slot = (int)(sc.ticket & 1);
   CK(cudaEventSynchronize(c->ev_comp[slot]));
-  if (sc.direct && (c->h_tots[slot]->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) {
+  if (c->h_tots[slot]->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH)) {
     sc.status = rerun_larger(c, sc, slot);
     if (sc.status != GKC_OK) sc.message = c->err;
   }
@@ -1231,7 +1231,7 @@ gkc_status gkc_stream_submit(gkc_ctx *c, const gkc_params *prm, const char *read
   }
   c->tm = gkc_timings{};
   StreamCall sc;
-  s = pipeline_batched(c, prm, dr, nb, doffs, n_reads, true, &sc.direct, &sc.cap);
+  s = pipeline_batched(c, prm, dr, nb, doffs, n_reads, true, &sc.cap);
   if (s != GKC_OK) return s;
   CK(cudaEventRecord(c->ev_comp[slot], c->st));
   sc.key = GraphKey{dr, doffs, nb, n_reads, prm->k, prm->p, prm->hpc, prm->nbins, c->filter};
@@ -1276,7 +1276,7 @@ gkc_status gkc_stream_wait(gkc_ctx *c, uint64_t ticket, uint64_t *n_distinct, ui
   if (n_distinct) *n_distinct = h->n_distinct;
   if (n_kmers) *n_kmers = h->n_kmers;
   if (h->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))
-    return ctx_fail(c, GKC_ERR_CAPACITY, "the call's input outgrew the captured pipeline: run it with gkc_pipeline_host");
+    return ctx_fail(c, GKC_ERR_CAPACITY, "pipeline capacity");
   s = device_err(c, h->err);
   if (s != GKC_OK) return s;
   if (h->n_distinct > sc.capacity)

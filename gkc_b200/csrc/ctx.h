@@ -60,8 +60,7 @@ struct StreamCall {
   uint64_t capacity = 0;
   gkc_params prm{};
   int key_words = 1;
-  // enqueued launch by launch, on these inputs and capacities: run again if they were too small
-  bool direct = false;
+  // its inputs and capacities: run again if they were too small
   GraphKey key{};
   PipelineCaps cap;
   gkc_status status = GKC_OK;  // of that second run

@@ -336,9 +336,10 @@ gkc_status gkc_pipeline_host(gkc_ctx *ctx, const gkc_params *prm, gkc_mode mode,
  *      for `capacity` pairs).  The reads of a call may be cut from a larger
  *      CSR (offs[0] need not be 0).  A call whose reads have the size of the
  *      call two before (the same buffer slot) runs as a captured pipeline;
- *      another size is enqueued launch by launch, and run a second time (in
- *      its gkc_stream_wait or a later submit) if its reads need more room
- *      than their number of bases suggests.
+ *      another size is enqueued launch by launch.  Either is run a second
+ *      time (in its gkc_stream_wait or a later submit) if its reads need more
+ *      room than their number of bases, or the earlier call of that size,
+ *      suggests.
  *      gkc_stream_wait blocks until the call's results are in host memory
  *      and returns its status; at most two calls may be in flight, and the
  *      context's device views do not describe them.  (No reference
