@@ -1296,7 +1296,7 @@ gkc_status gkc_partition_copy_out(gkc_ctx *c, uint64_t *bin_skm_off, uint32_t *s
   if (minimizer && v.n_superkmers) {
     if (v.skm_minimizer)
       CK(cudaMemcpyAsync(minimizer, v.skm_minimizer, v.n_superkmers * 4, cudaMemcpyDeviceToHost, c->st));
-    else  // an imported partition carries no minimizers
+    else  // an imported partition and superkmers from the host have no minimizers
       memset(minimizer, 0xFF, v.n_superkmers * 4);
   }
   if (packed && v.n_packed_bytes)
@@ -1414,14 +1414,12 @@ gkc_status gkc_count_superkmers_host(gkc_ctx *c, int k, const uint32_t *skm_len,
   if (longest > 0xFFFFFFu) return ctx_fail(c, GKC_ERR_INVALID_ARG, "superkmer too long");
   WS(dd, uint64_t, "skm_desc_bin", n_skm + 1);
   WS(dp, uint8_t, "packed_bin", off + 16);
-  WS(dmm, uint32_t, "skm_mm_bin", n_skm + 1);
+  WS(dl, uint32_t, "skm_mm_bin", n_skm + 1);  // the lengths, where a partition keeps its minimizers
   WS(bs, uint64_t, "bin_start", 2);
   WS(bk, uint64_t, "bin_kstart", 2);
   WS(cur, unsigned long long, "cursors", 4);
   WS(err, uint32_t, "err", 4);
-  // no buffer of their own: these superkmers have no minimizers, and the count stage fills its offsets afterwards
-  uint32_t *dl = dmm;
-  WS(boff, uint64_t, "skm_koff", n_skm + 3);
+  WS(boff, uint64_t, "skm_koff", n_skm + 3);  // filled again by the count stage
   WS(btmp, uint64_t, "scan_tmp2", scan_u64_tmp_words(n_skm + 1) + 8);
   SettleOnError settle(c);
   // both copies before the kernels: a copy from pageable memory waits for the stream
@@ -1440,7 +1438,7 @@ gkc_status gkc_count_superkmers_host(gkc_ctx *c, int k, const uint32_t *skm_len,
   c->pv.bin_skm_off = bs;
   c->pv.bin_kmer_off = bk;
   c->pv.skm_desc = dd;
-  c->pv.skm_minimizer = dmm;
+  c->pv.skm_minimizer = nullptr;  // these superkmers come without
   c->pv.packed = dp;
   c->part_nbytes_dev = nullptr;
   // the count path sizes its per-superkmer arrays from the partition's

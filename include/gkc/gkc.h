@@ -129,7 +129,8 @@ gkc_status gkc_partition_host(gkc_ctx *ctx, const gkc_params *prm, const char *r
 /* Copies the context's partition to host arrays sized from the view:
  * bin_skm_off[nbins+1], skm_len[n_superkmers], skm_byte_off[n_superkmers]
  * (into `packed`), packed[n_packed_bytes], minimizer[n_superkmers] (may be NULL;
- * all 0xFFFFFFFF for an imported partition, which carries none). */
+ * all 0xFFFFFFFF for an imported partition and after
+ * gkc_count_superkmers_host, which have none). */
 gkc_status gkc_partition_copy_out(gkc_ctx *ctx, uint64_t *bin_skm_off, uint32_t *skm_len,
                                   uint64_t *skm_byte_off, uint8_t *packed, uint32_t *minimizer);
 
