@@ -637,11 +637,7 @@ static gkc_status enqueue_count_batched(gkc_ctx *c, const gkc_params *prm, uint6
   pl.bin_kstart = bin_kstart;
   pl.bucket_keys = bucket_keys;
   pl.max_bits = max_bits;
-  uint64_t chunk_kmers = c->tune.chunk_kmers;
-  if (!chunk_kmers) {
-    chunk_kmers = keys_cap / kChunkKmers >= 64 * (uint64_t)c->n_sms ? 2 * kChunkKmers : kChunkKmers;
-    while (chunk_kmers > kChunkKmersMin && keys_cap / chunk_kmers < 8 * (uint64_t)c->n_sms) chunk_kmers /= 2;
-  }
+  const uint64_t chunk_kmers = c->tune.chunk_kmers ? c->tune.chunk_kmers : default_chunk(keys_cap, c->n_sms);
   pl.chunk_kmers = chunk_kmers;
   pl.k = prm->k;
   pl.err = err;

@@ -35,7 +35,7 @@ struct GraphKey {
 // zero means the built-in default).
 struct TuneChoice {
   uint32_t coarse_target = 0;  // keys per count bucket (bucket_target)
-  uint32_t chunk_kmers = 0;    // k-mers per histogram chunk (a power of two)
+  uint32_t chunk_kmers = 0;    // k-mers per histogram chunk (a power of two; 0: by the input's size)
   uint32_t count_ctas = 0;     // count kernel CTAs per SM
 };
 

@@ -181,6 +181,11 @@ constexpr uint64_t kChunkKmers = 65536;
 // (histogram + scatter, 64 K / 32 K / 16 K: 20 M bases 389 / 319 / 269 us, 60 M
 // 718 / 684 / 678, 120 M 1331 / 1328 / 1387).
 constexpr uint64_t kChunkKmersMin = 16384;
+inline uint64_t default_chunk(uint64_t keys, int n_sms) {
+  uint64_t chunk = keys / kChunkKmers >= 64 * (uint64_t)n_sms ? 2 * kChunkKmers : kChunkKmers;
+  while (chunk > kChunkKmersMin && keys / chunk < 8 * (uint64_t)n_sms) chunk /= 2;
+  return chunk;
+}
 // Largest mean bin (k-mers) whose 8-byte keys are scattered by two CTAs an SM
 // with tiles of 7168 keys rather than one with 16384: their phases overlap,
 // but in larger bins a bucket's run of the smaller tile ends within few 32-byte

@@ -54,16 +54,17 @@ TuneKey key_for(int sms, const gkc_params *prm, uint64_t n_bases, uint64_t n_rea
 gkc_tune_params defaults() {
   gkc_tune_params d;
   d.coarse_target = gkc::kCoarseTarget;
-  d.chunk_kmers = (uint32_t)gkc::kChunkKmers;
+  d.chunk_kmers = 0;  // by the input's size
   d.count_ctas_per_sm = 2;
   d.reserved = 0;
   return d;
 }
 
 bool valid(const gkc_tune_params &p) {
-  const bool pow2 = p.chunk_kmers && (p.chunk_kmers & (p.chunk_kmers - 1)) == 0;
-  return p.coarse_target >= 256 && p.coarse_target <= 65536 && pow2 && p.chunk_kmers >= 4096 &&
-         p.chunk_kmers <= (1u << 22) && p.count_ctas_per_sm >= 1 && p.count_ctas_per_sm <= 4;
+  const bool pow2 = (p.chunk_kmers & (p.chunk_kmers - 1)) == 0;
+  const bool chunk = p.chunk_kmers == 0 || (pow2 && p.chunk_kmers >= 4096 && p.chunk_kmers <= (1u << 22));
+  return p.coarse_target >= 256 && p.coarse_target <= 65536 && chunk && p.count_ctas_per_sm >= 1 &&
+         p.count_ctas_per_sm <= 4;
 }
 
 }  // namespace
@@ -72,7 +73,7 @@ gkc_status gkc_tune_get(const gkc_ctx *c, gkc_tune_params *out) {
   if (!c || !out) return GKC_ERR_INVALID_ARG;
   gkc_tune_params d = defaults();
   out->coarse_target = c->tune.coarse_target ? c->tune.coarse_target : d.coarse_target;
-  out->chunk_kmers = c->tune.chunk_kmers ? c->tune.chunk_kmers : d.chunk_kmers;
+  out->chunk_kmers = c->tune.chunk_kmers;
   out->count_ctas_per_sm = c->tune.count_ctas ? c->tune.count_ctas : d.count_ctas_per_sm;
   out->reserved = 0;
   return GKC_OK;
@@ -83,15 +84,12 @@ gkc_status gkc_tune_set(gkc_ctx *c, const gkc_tune_params *p) {
   gkc_tune_params v = p ? *p : defaults();
   const gkc_tune_params d = defaults();
   if (!v.coarse_target) v.coarse_target = d.coarse_target;
-  if (!v.chunk_kmers) v.chunk_kmers = d.chunk_kmers;
   if (!v.count_ctas_per_sm) v.count_ctas_per_sm = d.count_ctas_per_sm;
   if (!valid(v)) return ctx_fail(c, GKC_ERR_INVALID_ARG, "tuning parameters out of range");
-  // the default chunk stays a default: small inputs take smaller ones
-  const uint32_t chunk = v.chunk_kmers == d.chunk_kmers ? 0 : v.chunk_kmers;
-  if (v.coarse_target != c->tune.coarse_target || chunk != c->tune.chunk_kmers ||
+  if (v.coarse_target != c->tune.coarse_target || v.chunk_kmers != c->tune.chunk_kmers ||
       v.count_ctas_per_sm != c->tune.count_ctas) {
     c->tune.coarse_target = v.coarse_target;
-    c->tune.chunk_kmers = chunk;
+    c->tune.chunk_kmers = v.chunk_kmers;
     c->tune.count_ctas = v.count_ctas_per_sm;
     graphs_invalidate(c);  // the captured pipeline holds the old shapes
   }
@@ -234,6 +232,7 @@ gkc_status gkc_autotune_device(gkc_ctx *c, const gkc_params *prm, const char *d_
       uint32_t *field = dim == 0 ? &cand.count_ctas_per_sm : dim == 1 ? &cand.coarse_target : &cand.chunk_kmers;
       if (*field == vals[i]) continue;
       if (dim == 0 && vals[i] > (uint32_t)std::max(occ, 1)) continue;
+      if (dim == 2 && vals[i] == gkc::default_chunk(std::max<uint64_t>(nb, 16), c->n_sms)) continue;  // timed as the default
       *field = vals[i];
       float ms = 0;
       s = gkc_tune_set(c, &cand);

@@ -282,7 +282,7 @@ gkc_status gkc_db_read(const gkc_db *db, uint64_t first, uint64_t n, uint64_t *k
  *      mean the default. ---- */
 typedef struct gkc_tune_params {
   uint32_t coarse_target;      /* 256 .. 65536; default 8192 */
-  uint32_t chunk_kmers;        /* 4096 .. 2^22, a power of two; default 65536, less for small inputs, twice that for large ones */
+  uint32_t chunk_kmers;        /* 4096 .. 2^22, a power of two; default 0: by the input's size, 16384 .. 131072 */
   uint32_t count_ctas_per_sm;  /* 1 .. 4; default 2 */
   uint32_t reserved;
 } gkc_tune_params;
