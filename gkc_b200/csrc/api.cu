@@ -362,11 +362,14 @@ static void partition_caps(const gkc_params *prm, uint64_t n_bytes, uint64_t n_r
   *cap_bytes = (w + s * (uint64_t)(prm->k - 1)) / 4 + s + tiles * 16 + 64;
 }
 
-// Device bytes one pipeline run over n_bases bases in n_reads reads needs:
-// the workspaces the batched pipeline sizes for it (reads uploaded from the
-// host, optional HPC copies, the read-start bitmap, superkmers in tile and bin
-// order, k-mer offsets, coarse-bucket matrices, keys, runs, counts, sort
-// scratch) plus a fixed allowance for the small per-bin arrays.
+// Device bytes one pipeline run over n_bases bases in n_reads reads needs: a
+// bound over the workspaces that the batched pipeline sizes for it, with room
+// (64 MB and more) for reads that hold more superkmers than that.  The room
+// comes from terms charged above their size: two words a superkmer for one
+// k-mer offset, chunks of 32 K k-mers (small inputs have smaller ones, but few),
+// buckets for every digit.  It also takes what is not named here: the flags and
+// prefixes of HPC, the placement matrices of small chunks, the slices of
+// opened buckets.
 uint64_t gkc_job_hbm_estimate(const gkc_params *prm, uint64_t n_bases, uint64_t n_reads) {
   if (!prm || prm->k < 1 || prm->k > 64 || prm->nbins < 1) return 0;
   const uint64_t B = n_bases, R = n_reads, w = prm->k <= 32 ? 8 : 16;
@@ -382,12 +385,13 @@ uint64_t gkc_job_hbm_estimate(const gkc_params *prm, uint64_t n_bases, uint64_t 
   const uint64_t kc = std::max<uint64_t>(B, 16);
   uint32_t max_bits = kCoarseMaxBits;
   while (max_bits > 0 && ((uint64_t)prm->nbins << max_bits) > (1ull << 20)) max_bits--;
-  const uint64_t chunks = kc / 32768 + prm->nbins + 1;  // the smallest chunk the tuner picks
+  const uint64_t chunks = kc / 32768 + prm->nbins + 1;
   e += 4 * (chunks << max_bits) + 8 * chunks;                            // chunk matrix, first superkmers
   e += w * kc * 2 + 4 * kc * 2;                                          // keys, output keys, staged and output counts
   e += ((uint64_t)prm->nbins << max_bits) * (8 * 5 + 4 * 2);             // bucket starts, sizes, distinct counts,
                                                                          // offsets, scan; bins, large-bucket list
   e += 8ull << 20;                                                       // tables of the buckets' digits, tasks
+  e += 80 * (uint64_t)prm->nbins;                                        // counters, prefixes and offsets per bin
   return e + (64ull << 20);
 }
 
