@@ -707,7 +707,7 @@ constexpr int CC_NSUB_MAX = 1 << CC_SB_MAX;
 // GROUP keys on average, sorted by one warp with at most RMAX keys a lane.
 template <typename K> struct SortShape;
 template <> struct SortShape<uint64_t> { static constexpr int NT = 256, GROUP = 128, RMAX = 16, CTAS = 5; };
-template <> struct SortShape<u128> { static constexpr int NT = 256, GROUP = 64, RMAX = 8, CTAS = 4; };
+template <> struct SortShape<u128> { static constexpr int NT = 256, GROUP = 64, RMAX = 8, CTAS = 3; };
 constexpr int CS_GROUPS = 64;       // most groups of a bucket
 constexpr uint32_t CC_SPLIT_MAX = 512;  // groups of the sample sort (one per thread)
 constexpr uint32_t CC_TICKETS = 4;     // buckets taken per ticket
@@ -817,7 +817,10 @@ template <typename K> struct SortSmem {
   uint64_t pf_start;                  // the next bucket's keys, prefetched into L2
   uint32_t pf_n;
 };
-static_assert(sizeof(SortSmem<uint64_t>) <= 45568, "five CTAs per SM");
+// an SM's 228 KB less 1 KB a CTA
+template <typename K> constexpr size_t sort_smem_room() { return 228 * 1024 / SortShape<K>::CTAS - 1024; }
+static_assert(sizeof(SortSmem<uint64_t>) <= sort_smem_room<uint64_t>() && sizeof(SortSmem<u128>) <= sort_smem_room<u128>(),
+              "as many CTAs on an SM as the registers are shared out for");
 template <typename K> size_t bucket_sort_smem_bytes() { return sizeof(SortSmem<K>); }
 template size_t bucket_sort_smem_bytes<uint64_t>();
 template size_t bucket_sort_smem_bytes<u128>();
@@ -1530,7 +1533,7 @@ __device__ __noinline__ uint32_t slice_count(SortArea<K, NT, CountShape<K>::CAP>
 
 // Buckets of at most CAP keys, persistent, taken by ticket.  Those that
 // sort_count rejects join the list of large ones (k_bucket_open).  256
-// threads and 45 KB, so that five CTAs (four for 16-byte keys) on an SM hide
+// threads and 45 KB (58 KB), so that five CTAs (three for 16-byte keys) on an SM hide
 // each other's barriers.  Count stage (with the two kernels below) on a
 // B200, against counting each bucket in a 4096-slot hash table with a merge
 // sort, or by insertion and warp sorts of 4096 fixed digits: 720 M 31-mers at
