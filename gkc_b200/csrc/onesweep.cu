@@ -312,48 +312,67 @@ GKC_DEV uint32_t os_before(u128 y, uint32_t j, u128 x, uint32_t i) {
   return 0u - t;
 }
 
-// Copies [s, e), a run too long to be ranked by its tile, as it is; lists it
-// unless all its keys are equal (they are in order then).
+// What k_os_fix leaves behind it, in the look-back words: the number of runs
+// listed for the host, their [begin, end) from word 2 on (longer than OF_RUN,
+// so at most n / OF_RUN), then for every tile the long run that begins in it and
+// goes on past it (its end 0: none) and whether keys of that run differ.
+struct FixLists {
+  unsigned long long *list, *cand, *mixed;
+};
+static uint64_t fix_tiles(uint64_t n) { return (n + OF_TILE - 1) / OF_TILE; }
+static FixLists fix_lists(unsigned long long *words, uint64_t n) {
+  unsigned long long *cand = words + 2 + 2 * (n / OF_RUN + 1);
+  return FixLists{words, cand, cand + 2 * fix_tiles(n)};
+}
+GKC_DEV void os_list_run(unsigned long long *list, uint64_t s, uint64_t e) {
+  const unsigned long long at = atomicAdd(list, 1ull);
+  list[2 + 2 * at] = s;
+  list[3 + 2 * at] = e;
+}
+
+// The first place in [0, base) whose key has the leading bits `lead` (keys in
+// their order, the last one of them has), by the calling warp.
 template <typename K>
-GKC_DEV void os_long_run(const K *in, K *out, const uint32_t *vin, uint32_t *vout, uint64_t s, uint64_t e,
-                         unsigned long long *list) {
-  const K first = in[s];
-  bool mixed = false;
-  for (uint64_t i = s + threadIdx.x; i < e; i += OF_NT) {
-    const K x = in[i];
-    mixed = mixed || x != first;
-    out[i] = x;
-    vout[i] = vin[i];
+GKC_DEV uint64_t os_run_start(const K *in, uint64_t base, K lead, int bit0) {
+  const uint32_t lane = threadIdx.x & 31u;
+  uint64_t lo = 0, hi = base;
+  while (lo < hi) {
+    const uint64_t step = (hi - lo + 31) / 32, at = lo + lane * step;
+    const uint32_t c = __popc(__ballot_sync(0xffffffffu, at < hi && (in[at] >> bit0) < lead));
+    hi = min(hi, lo + c * step);
+    if (c) lo += (c - 1) * step + 1;
   }
-  if (__syncthreads_or(mixed) && threadIdx.x == 0) {
-    const unsigned long long at = atomicAdd(list, 1ull);
-    list[2 + 2 * at] = s;
-    list[3 + 2 * at] = e;
-  }
+  return lo;
 }
 
 // Pairs in the order of their bits from `bit0` up, to `out` in the order of
 // all bits: each run of equal leading bits by ranking every key in it (equal
-// keys keep their order).  A tile takes the runs that begin in it.  list[0]
-// counts the runs left to the host, [begin, end) from list[2] on: longer than
-// OF_RUN, so at most n / OF_RUN.  Bound by the comparisons, a run's length for
-// each key (one subtraction a word: 0.48 -> 0.26 ms for 13.9 M 16-byte keys in
-// runs of about 17; the twelve passes it stands for take 2.7.  8.7 M distinct
-// 8-byte keys: 0.08, for passes of 0.47).
+// keys keep their order).  A tile takes the runs that begin in it.  Longer ones
+// than OF_RUN are copied as they are, each tile its own part, and listed for
+// the host where their keys differ.  Bound by the comparisons, a run's length
+// for each key (one subtraction a word: 0.48 -> 0.26 ms for 13.9 M 16-byte keys
+// in runs of about 17; the twelve passes it stands for take 2.7.  8.7 M
+// distinct 8-byte keys: 0.08, for passes of 0.47).  Reads of few letters, 12 M
+// keys, most in one run: position lists 34.6 ms where one block copied a run, 2.6 so.
 template <typename K>
 __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uint32_t *vin, uint32_t *vout,
-                                                  const uint64_t *n_dev, int bit0, unsigned long long *list) {
+                                                  const uint64_t *n_dev, int bit0, FixLists lists) {
   __shared__ __align__(16) K S[OF_LOAD];
   __shared__ uint32_t heads[OF_LOAD / 32];  // bit i: a run begins at S[i] (or the keys end there)
-  __shared__ uint32_t n_long, long_s[4], long_e[4];
+  __shared__ uint32_t n_long, long_s[4], long_e[4], before;
   constexpr uint32_t OPEN = ~0u;
   const uint64_t n = *n_dev;
   const uint32_t tid = threadIdx.x;
   for (uint64_t base = (uint64_t)blockIdx.x * OF_TILE; base < n; base += (uint64_t)gridDim.x * OF_TILE) {
+    const uint64_t tile = base / OF_TILE;
     const uint32_t m = (uint32_t)min(n - base, (uint64_t)OF_LOAD);
     const bool closed = base + m == n;
     for (uint32_t i = tid; i < m; i += OF_NT) S[i] = in[base + i];
-    if (tid == 0) n_long = 0;
+    if (tid == 0) {
+      n_long = 0;
+      before = 0;
+      lists.cand[2 * tile + 1] = 0;
+    }
     __syncthreads();
     for (uint32_t i = tid; i < OF_LOAD; i += OF_NT) {  // OF_LOAD is whole rounds
       bool head = i == m;
@@ -365,6 +384,13 @@ __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uin
       if ((tid & 31u) == 0) heads[i >> 5] = w;
     }
     __syncthreads();
+    if (tid == 0 && !(heads[0] & 1u)) {  // a run of an earlier tile goes on: `before`, its keys here if it is a long one
+      uint32_t w = 0;
+      while (w + 1 < OF_LOAD / 32 && !heads[w]) w++;
+      const uint32_t e = heads[w] ? 32 * w + __ffs(heads[w]) - 1 : closed ? m : OPEN;
+      if (e == OPEN || (base + e > OF_RUN && (in[base + e - OF_RUN - 1] >> bit0) == (S[0] >> bit0)))
+        before = min(e, min(m, OF_TILE));
+    }
     for (uint32_t i = tid; i < m; i += OF_NT) {
       const uint32_t b = i & 31u;
       uint32_t w = i >> 5, bits = heads[w] & (0xFFFFFFFFu >> (31 - b));
@@ -392,23 +418,50 @@ __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uin
       vout[base + at] = vin[base + i];
     }
     __syncthreads();
-    for (uint32_t l = 0; l < n_long; l++) {
-      const uint64_t s = base + long_s[l];
-      uint64_t e = base + long_e[l];
-      if (long_e[l] == OPEN) {  // the first key after the loaded ones with other leading bits
-        const K lead = in[s] >> bit0;
-        uint64_t lo = base + m;
-        for (uint64_t hi = n; lo < hi;) {
-          const uint64_t mid = (lo + hi) >> 1;
-          if ((in[mid] >> bit0) == lead) lo = mid + 1;
-          else hi = mid;
-        }
-        e = lo;
+    // the tile's part of long runs: of the one from before, then of those that begin here
+    for (uint32_t l = 0; l < n_long + 1; l++) {
+      const uint32_t s = l ? long_s[l - 1] : 0u, e = l ? long_e[l - 1] : before, stop = min(e, min(m, OF_TILE));
+      if (s >= stop) continue;  // the same in every thread
+      bool differ = false;
+      for (uint32_t i = s + tid; i < stop; i += OF_NT) {
+        const K x = S[i];
+        if (i > s || l == 0) differ = differ || x != (i ? S[i - 1] : in[base - 1]);
+        out[base + i] = x;
+        vout[base + i] = vin[base + i];
       }
-      os_long_run(in, out, vin, vout, s, e, list);
+      const bool any = __syncthreads_or(differ);
+      if (l == 0) {
+        if (any && tid < 32) {
+          const uint64_t first = os_run_start<K>(in, base, S[0] >> bit0, bit0);
+          if (tid == 0) lists.mixed[first / OF_TILE] = 1;
+        }
+      } else if (tid == 0 && e <= OF_TILE) {
+        if (any) os_list_run(lists.list, base + s, base + e);
+      } else if (tid == 0) {
+        uint64_t end = base + e;
+        if (e == OPEN) {  // the first key after the loaded ones with other leading bits
+          const K lead = S[s] >> bit0;
+          end = base + m;
+          for (uint64_t hi = n; end < hi;) {
+            const uint64_t mid = (end + hi) >> 1;
+            if ((in[mid] >> bit0) == lead) end = mid + 1;
+            else hi = mid;
+          }
+        }
+        lists.cand[2 * tile] = base + s;
+        lists.cand[2 * tile + 1] = end;
+        if (any) lists.mixed[tile] = 1;
+      }
     }
     __syncthreads();  // before the next tile's keys
   }
+}
+
+// Lists the runs that go on past their tile and whose keys differ.
+__global__ void k_os_fix_list(const uint64_t *n_dev, FixLists lists) {
+  const uint64_t tiles = (*n_dev + OF_TILE - 1) / OF_TILE;
+  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < tiles; t += (uint64_t)gridDim.x * blockDim.x)
+    if (lists.mixed[t] && lists.cand[2 * t + 1]) os_list_run(lists.list, lists.cand[2 * t], lists.cand[2 * t + 1]);
 }
 
 // The listed runs (begin, end, first place in the compact arrays) to the
@@ -441,12 +494,15 @@ PairsStatus sort_pairs(K *keys, K *alt, uint32_t *vals, uint32_t *valt, const ui
                        false};
   const int bit0 = key_bits - lead;
   const int in_alt = onesweep_run<K, true>(keys, alt, vals, valt, n_dev, n, bit0, key_bits, s, st, launches).result_in_alt;
-  // the look-back entries are free now: the list of long runs
-  cudaMemsetAsync(s.lookback, 0, 16, st);
+  // the look-back entries are free now: the lists of long runs
+  const FixLists lists = fix_lists(s.lookback, n);
+  cudaMemsetAsync(lists.list, 0, 16, st);
+  cudaMemsetAsync(lists.mixed, 0, 8 * fix_tiles(n), st);
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + OF_TILE - 1) / OF_TILE, 1u << 20));
   k_os_fix<K><<<grid, OF_NT, 0, st>>>(in_alt ? alt : keys, in_alt ? keys : alt, in_alt ? valt : vals,
-                                      in_alt ? vals : valt, n_dev, bit0, s.lookback);
-  *launches += 1;
+                                      in_alt ? vals : valt, n_dev, bit0, lists);
+  k_os_fix_list<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(fix_tiles(n) / 256 + 1, 148 * 8)), 256, 0, st>>>(n_dev, lists);
+  *launches += 2;
   return PairsStatus{!in_alt, true};
 }
 
