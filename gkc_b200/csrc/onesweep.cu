@@ -313,21 +313,15 @@ GKC_DEV uint32_t os_before(u128 y, uint32_t j, u128 x, uint32_t i) {
 }
 
 // What k_os_fix leaves behind it, in the look-back words: the number of runs
-// listed for the host, their [begin, end) from word 2 on (longer than OF_RUN,
-// so at most n / OF_RUN), then for every tile the long run that begins in it and
-// goes on past it (its end 0: none) and whether keys of that run differ.
+// listed for the host, a word for every tile (whether the run that begins in it
+// and goes on past it is listed), and the runs' [begin, end), each longer than
+// OF_RUN, so at most n / OF_RUN.
 struct FixLists {
-  unsigned long long *list, *cand, *mixed;
+  unsigned long long *count, *claimed, *runs;
 };
 static uint64_t fix_tiles(uint64_t n) { return (n + OF_TILE - 1) / OF_TILE; }
 static FixLists fix_lists(unsigned long long *words, uint64_t n) {
-  unsigned long long *cand = words + 2 + 2 * (n / OF_RUN + 1);
-  return FixLists{words, cand, cand + 2 * fix_tiles(n)};
-}
-GKC_DEV void os_list_run(unsigned long long *list, uint64_t s, uint64_t e) {
-  const unsigned long long at = atomicAdd(list, 1ull);
-  list[2 + 2 * at] = s;
-  list[3 + 2 * at] = e;
+  return FixLists{words, words + 2, words + 2 + fix_tiles(n)};
 }
 
 // The first place in [0, base) whose key has the leading bits `lead` (keys in
@@ -348,8 +342,8 @@ GKC_DEV uint64_t os_run_start(const K *in, uint64_t base, K lead, int bit0) {
 // Pairs in the order of their bits from `bit0` up, to `out` in the order of
 // all bits: each run of equal leading bits by ranking every key in it (equal
 // keys keep their order).  A tile takes the runs that begin in it.  Longer ones
-// than OF_RUN are copied as they are, each tile its own part, and listed for
-// the host where their keys differ.  Bound by the comparisons, a run's length
+// than OF_RUN are copied as they are, each tile its own part; the first tile
+// that sees keys of a run differ lists it for the host.  Bound by the comparisons, a run's length
 // for each key (one subtraction a word: 0.48 -> 0.26 ms for 13.9 M 16-byte keys
 // in runs of about 17; the twelve passes it stands for take 2.7.  8.7 M
 // distinct 8-byte keys: 0.08, for passes of 0.47).  Reads of few letters, 12 M
@@ -359,19 +353,17 @@ __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uin
                                                   const uint64_t *n_dev, int bit0, FixLists lists) {
   __shared__ __align__(16) K S[OF_LOAD];
   __shared__ uint32_t heads[OF_LOAD / 32];  // bit i: a run begins at S[i] (or the keys end there)
-  __shared__ uint32_t n_long, long_s[4], long_e[4], before;
+  __shared__ uint32_t n_long, long_s[4], long_e[4], before;  // before: end of a long run that goes on here
   constexpr uint32_t OPEN = ~0u;
   const uint64_t n = *n_dev;
   const uint32_t tid = threadIdx.x;
   for (uint64_t base = (uint64_t)blockIdx.x * OF_TILE; base < n; base += (uint64_t)gridDim.x * OF_TILE) {
-    const uint64_t tile = base / OF_TILE;
     const uint32_t m = (uint32_t)min(n - base, (uint64_t)OF_LOAD);
     const bool closed = base + m == n;
     for (uint32_t i = tid; i < m; i += OF_NT) S[i] = in[base + i];
     if (tid == 0) {
       n_long = 0;
       before = 0;
-      lists.cand[2 * tile + 1] = 0;
     }
     __syncthreads();
     for (uint32_t i = tid; i < OF_LOAD; i += OF_NT) {  // OF_LOAD is whole rounds
@@ -384,12 +376,12 @@ __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uin
       if ((tid & 31u) == 0) heads[i >> 5] = w;
     }
     __syncthreads();
-    if (tid == 0 && !(heads[0] & 1u)) {  // a run of an earlier tile goes on: `before`, its keys here if it is a long one
+    if (tid == 0 && !(heads[0] & 1u)) {  // a run of an earlier tile goes on
       uint32_t w = 0;
       while (w + 1 < OF_LOAD / 32 && !heads[w]) w++;
       const uint32_t e = heads[w] ? 32 * w + __ffs(heads[w]) - 1 : closed ? m : OPEN;
       if (e == OPEN || (base + e > OF_RUN && (in[base + e - OF_RUN - 1] >> bit0) == (S[0] >> bit0)))
-        before = min(e, min(m, OF_TILE));
+        before = e;
     }
     for (uint32_t i = tid; i < m; i += OF_NT) {
       const uint32_t b = i & 31u;
@@ -429,39 +421,28 @@ __global__ void __launch_bounds__(OF_NT) k_os_fix(const K *in, K *out, const uin
         out[base + i] = x;
         vout[base + i] = vin[base + i];
       }
-      const bool any = __syncthreads_or(differ);
-      if (l == 0) {
-        if (any && tid < 32) {
-          const uint64_t first = os_run_start<K>(in, base, S[0] >> bit0, bit0);
-          if (tid == 0) lists.mixed[first / OF_TILE] = 1;
-        }
-      } else if (tid == 0 && e <= OF_TILE) {
-        if (any) os_list_run(lists.list, base + s, base + e);
-      } else if (tid == 0) {
-        uint64_t end = base + e;
-        if (e == OPEN) {  // the first key after the loaded ones with other leading bits
-          const K lead = S[s] >> bit0;
-          end = base + m;
-          for (uint64_t hi = n; end < hi;) {
-            const uint64_t mid = (end + hi) >> 1;
-            if ((in[mid] >> bit0) == lead) end = mid + 1;
-            else hi = mid;
+      if (__syncthreads_or(differ) && tid < 32) {
+        const uint64_t first = l ? base + s : os_run_start<K>(in, base, S[0] >> bit0, bit0);
+        const bool whole = l && e <= OF_TILE;  // no other tile sees it
+        if (tid == 0 && (whole || atomicExch(lists.claimed + first / OF_TILE, 1ull) == 0)) {
+          uint64_t end = base + e;
+          if (e == OPEN) {  // the first key after the loaded ones with other leading bits
+            const K lead = S[s] >> bit0;
+            end = base + m;
+            for (uint64_t hi = n; end < hi;) {
+              const uint64_t mid = (end + hi) >> 1;
+              if ((in[mid] >> bit0) == lead) end = mid + 1;
+              else hi = mid;
+            }
           }
+          const unsigned long long at = atomicAdd(lists.count, 1ull);
+          lists.runs[2 * at] = first;
+          lists.runs[2 * at + 1] = end;
         }
-        lists.cand[2 * tile] = base + s;
-        lists.cand[2 * tile + 1] = end;
-        if (any) lists.mixed[tile] = 1;
       }
     }
     __syncthreads();  // before the next tile's keys
   }
-}
-
-// Lists the runs that go on past their tile and whose keys differ.
-__global__ void k_os_fix_list(const uint64_t *n_dev, FixLists lists) {
-  const uint64_t tiles = (*n_dev + OF_TILE - 1) / OF_TILE;
-  for (uint64_t t = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; t < tiles; t += (uint64_t)gridDim.x * blockDim.x)
-    if (lists.mixed[t] && lists.cand[2 * t + 1]) os_list_run(lists.list, lists.cand[2 * t], lists.cand[2 * t + 1]);
 }
 
 // The listed runs (begin, end, first place in the compact arrays) to the
@@ -496,13 +477,11 @@ PairsStatus sort_pairs(K *keys, K *alt, uint32_t *vals, uint32_t *valt, const ui
   const int in_alt = onesweep_run<K, true>(keys, alt, vals, valt, n_dev, n, bit0, key_bits, s, st, launches).result_in_alt;
   // the look-back entries are free now: the lists of long runs
   const FixLists lists = fix_lists(s.lookback, n);
-  cudaMemsetAsync(lists.list, 0, 16, st);
-  cudaMemsetAsync(lists.mixed, 0, 8 * fix_tiles(n), st);
+  cudaMemsetAsync(lists.count, 0, 8 * (2 + fix_tiles(n)), st);
   const unsigned grid = (unsigned)std::max<uint64_t>(1, std::min<uint64_t>((n + OF_TILE - 1) / OF_TILE, 1u << 20));
   k_os_fix<K><<<grid, OF_NT, 0, st>>>(in_alt ? alt : keys, in_alt ? keys : alt, in_alt ? valt : vals,
                                       in_alt ? vals : valt, n_dev, bit0, lists);
-  k_os_fix_list<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(fix_tiles(n) / 256 + 1, 148 * 8)), 256, 0, st>>>(n_dev, lists);
-  *launches += 2;
+  *launches += 1;
   return PairsStatus{!in_alt, true};
 }
 
@@ -513,7 +492,7 @@ int sort_pairs_rest(PairsStatus done, uint64_t n_runs, K *keys, K *alt, uint32_t
   K *from = done.result_in_alt ? alt : keys, *free_k = done.result_in_alt ? keys : alt;
   uint32_t *vfrom = done.result_in_alt ? valt : vals, *free_v = done.result_in_alt ? vals : valt;
   std::vector<unsigned long long> list(2 * n_runs), runs(3 * n_runs);
-  cudaMemcpyAsync(list.data(), s.lookback + 2, 16 * n_runs, cudaMemcpyDeviceToHost, st);
+  cudaMemcpyAsync(list.data(), fix_lists(s.lookback, n).runs, 16 * n_runs, cudaMemcpyDeviceToHost, st);
   cudaStreamSynchronize(st);
   std::vector<std::pair<unsigned long long, unsigned long long>> r(n_runs);
   for (uint64_t i = 0; i < n_runs; i++) r[i] = {list[2 * i], list[2 * i + 1]};
