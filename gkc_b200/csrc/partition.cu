@@ -33,14 +33,18 @@ static_assert(kPartTile == TL_WARPS * 28 * TL_W - PT_PRE - PT_HALO, "the smalles
 struct PartSmem {
   TileBases t;
   uint32_t brkw[TL_NW_MAX / 32];   // bit i: window i starts a superkmer or lies in none
-  uint32_t smm[PT_TMAX];              // minimizer of each core superkmer
-  uint32_t boff[PT_TMAX];             // its byte offset in the tile
-  uint16_t spos[PT_TMAX];             // its first window
-  uint16_t send[PT_TMAX];             // its end window (PT_EXT: ext_end)
+  union {
+    struct {
+      uint32_t smm[PT_TMAX];       // minimizer of each core superkmer
+      uint32_t boff[PT_TMAX];      // its byte offset in the tile
+      uint16_t spos[PT_TMAX];      // its first window
+      uint16_t send[PT_TMAX];      // its end window (PT_EXT: ext_end)
+    };
+    RedoArea redo[TL_WARPS];       // before them
+  };
   alignas(16) uint8_t stg[PT_STG]; // the tile's packed superkmers before they are written out (read as uint4)
   uint32_t scan_tmp[64];
   uint32_t lastmm[TL_WARPS], lastv[TL_WARPS], wcnt[TL_WARPS];
-  uint16_t redo[TL_WARPS][32];
   int ext_end;                     // local end window of an extended last superkmer
   int halo;                        // a break lies in the halo
   unsigned long long base_skm, base_byte;
@@ -93,15 +97,7 @@ __global__ void __launch_bounds__(PT_NT, 4) k_partition(PartArgs a) {
     uint32_t m[TL_W], none[1];
     tile_minima<false>(S.t, P0, k, p, a.filter, m, none);
     if (__any_sync(0xffffffffu, tw != 0u))
-      tile_redo(tw, P0, S.redo[warp],
-                [&](int l, uint32_t &v, uint32_t &) {
-                  v = exact_window_minimizer([&](int i) { return tile_code(S.t, l + i); }, k, p, a.filter);
-                },
-                [&](int i, uint32_t v, uint32_t) {
-#pragma unroll
-                  for (int x = 0; x < TL_W; x++)
-                    if (x == i) m[x] = v;
-                });
+      tile_redo(S.t, tw, P0, S.redo[warp], k, p, a.filter, m);
     if (P + TL_W == P0 + strip) {
       S.lastmm[warp] = m[TL_W - 1];
       S.lastv[warp] = vw >> 15;

@@ -28,7 +28,6 @@ constexpr int TL_GROUPS = 2 * TL_BWORDS;         // 16-base groups
 constexpr int TL_NW_MAX = TL_WARPS * 30 * TL_W;  // windows per tile
 static_assert(TL_GROUPS <= TL_NT, "one 16-base group per thread");
 GKC_HOST_DEV int tile_strip(int omega) { return omega > 33 ? 28 * TL_W : 30 * TL_W; }  // windows per warp
-GKC_HOST_DEV int tile_windows_n(int omega) { return TL_WARPS * tile_strip(omega); }    // windows per tile
 
 // Whether a 2p-bit p-mer value passes the filter (mm_filter for such values).
 template <int FILT>
@@ -154,6 +153,80 @@ GKC_DEV uint32_t tile_code(const TileBases &S, int l) {
   return (S.pk[l >> 4].x >> (30 - 2 * (l & 15))) & 3u;
 }
 
+// The (up to) 64 bases from tile base l on, in registers.
+struct WindowBases {
+  uint64_t hi, lo, bad;  // bases 0 .. 31 and 32 .. 63, the first on top (no base: 3); bit i: base i is no base
+};
+GKC_DEV WindowBases window_bases(const TileBases &S, int l) {
+  const int j = l >> 4, q = l >> 5;
+  const uint32_t sh = 2 * (uint32_t)(l & 15), bs = (uint32_t)(l & 31);
+  uint32_t w[5];
+#pragma unroll
+  for (int t = 0; t < 5; t++) w[t] = S.pk[j + t].x;
+  WindowBases b;
+  b.hi = (uint64_t)__funnelshift_l(w[1], w[0], sh) << 32 | __funnelshift_l(w[2], w[1], sh);
+  b.lo = (uint64_t)__funnelshift_l(w[3], w[2], sh) << 32 | __funnelshift_l(w[4], w[3], sh);
+  const uint32_t b1 = S.badw[q + 1];
+  b.bad = (uint64_t)__funnelshift_r(b1, S.badw[q + 2], bs) << 32 | __funnelshift_r(S.badw[q], b1, bs);
+  return b;
+}
+// The bases [j, k) in order, 16 taken from the registers at a time:
+// step(code, whether it is no base) for each.
+template <typename Step>
+GKC_DEV void each_base(WindowBases b, int j, int k, Step &&step) {
+  if (j > 0) {  // 0 < j <= 16
+    b.hi = b.hi << (2 * j) | b.lo >> (64 - 2 * j);
+    b.lo <<= 2 * j;
+    b.bad >>= j;
+  }
+  for (; j < k; j += 16) {
+    uint32_t w = (uint32_t)(b.hi >> 32), x = (uint32_t)b.bad;
+    const int n = min(16, k - j);
+#pragma unroll 4
+    for (int t = 0; t < n; t++) {
+      step(w >> 30, (x & 1u) != 0u);
+      w <<= 2;
+      x >>= 1;
+    }
+    b.hi = b.hi << 32 | b.lo >> 32;
+    b.lo <<= 32;
+    b.bad >>= 16;
+  }
+}
+
+// exact_window_minimizer from the window's bases in registers (codes of bytes
+// that are no base: 255, as there).  A window costs k + p codes, each some 25
+// instructions; 15 M bases with 30% N, k 31: partition 0.67 ms, with every code
+// read from shared memory and the filter chosen at each 1.36.
+template <int FILT>
+GKC_DEV uint32_t exact_minimizer(const WindowBases &b, int k, int p) {
+  const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * p);
+  uint32_t f = 0, r = 0;
+  each_base(b, 0, p, [&](uint32_t c, bool bad) { f = (f << 2) | (bad ? 255u : c); });
+  uint32_t w = (uint32_t)(b.hi >> 32) >> (32 - 2 * p), x = (uint32_t)b.bad << (32 - p);
+  for (int j = 0; j < p; j++) {  // from base p - 1 down
+    r = (r << 2) | ((int32_t)x < 0 ? 255u : 3u - (w & 3u));
+    w >>= 2;
+    x <<= 1;
+  }
+  uint32_t best = min(mm_filter(f, p, FILT) ? f : M, mm_filter(r, p, FILT) ? r : M);
+  each_base(b, p, k, [&](uint32_t c, bool bad) {
+    f = ((f << 2) | (bad ? 255u : c)) & M;
+    r = (r >> 2) | ((bad ? 255u : 3u - c) << (2 * p - 2));
+    if (mm_filter(f, p, FILT)) best = min(best, f);
+    if (mm_filter(r, p, FILT)) best = min(best, r);
+  });
+  return best;
+}
+GKC_DEV uint32_t exact_minimizer(const WindowBases &b, int k, int p, int filter) {
+  switch (filter) {
+    case FILTER_ALL: return exact_minimizer<FILTER_ALL>(b, k, p);
+    case FILTER_NEW: return exact_minimizer<FILTER_NEW>(b, k, p);
+    case FILTER_SIGNATURE: return exact_minimizer<FILTER_SIGNATURE>(b, k, p);
+    default: return exact_minimizer<FILTER_NEW2>(b, k, p);
+  }
+}
+
 // m[i], i < 16: the filtered minimum of the p-mer at tile base P + i, P =
 // 16 (j0 + lane), and its reverse complement.  With POS q[i] holds 4 * (tile
 // base) + the strand of the chosen one (0 forward, 1 reverse, 2 both).
@@ -251,43 +324,45 @@ GKC_DEV void tile_minima(const TileBases &S, int P0, int k, int p, int filter, u
   tile_slide<POS>(m, q, k - p + 1);
 }
 
-// The windows of `mask` (bit i: the lane's window i) redone by the exact rule
-// of windows that touch a byte that is no base, spread over the warp's lanes
-// 32 at a time (a single such byte touches k windows in a row, which few
-// lanes hold).  exact(l) gives tile window l's value; `list` holds 32 entries
-// of the warp.
-template <typename Exact, typename Put>
-GKC_DEV void tile_redo(uint32_t mask, int P0, uint16_t *list, Exact &&exact, Put &&put) {
+// The windows of `mask` (bit i: the lane's window i) listed for the whole warp,
+// so that those that touch a byte that is no base are redone by the exact rule
+// 32 at a time (a single such byte touches k windows in a row, which few lanes
+// hold).  Returns their number; *rank: that of the lane's first one.
+constexpr int TL_REDO = 30 * TL_W;  // windows a warp may have to redo
+GKC_DEV uint32_t tile_list(uint32_t mask, int P0, uint16_t *list, uint32_t *rank) {
   const uint32_t lane = threadIdx.x & 31u;
-  uint32_t rank0 = __popc(mask);  // rank of the lane's first window among the warp's
+  uint32_t rk = __popc(mask);
 #pragma unroll
   for (int d = 1; d < 32; d <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, rank0, d);
-    if (lane >= (uint32_t)d) rank0 += y;
+    const uint32_t y = __shfl_up_sync(0xffffffffu, rk, d);
+    if (lane >= (uint32_t)d) rk += y;
   }
-  const uint32_t total = __shfl_sync(0xffffffffu, rank0, 31);
-  rank0 -= __popc(mask);
-  for (uint32_t b = 0; b < total; b += 32) {
-    uint32_t left = mask, rk = rank0;
-    while (left) {
-      const int i = __ffs((int)left) - 1;
-      left &= left - 1;
-      if (rk - b < 32u) list[rk - b] = (uint16_t)(P0 + 16 * lane + i);
-      rk++;
-    }
-    __syncwarp();
-    uint32_t v = 0, v2 = 0;
-    if (b + lane < total) exact((int)list[lane], v, v2);
-    rk = rank0;
+  const uint32_t total = __shfl_sync(0xffffffffu, rk, 31);
+  rk -= __popc(mask);
+  *rank = rk;
+  for (uint32_t left = mask; left; left &= left - 1) list[rk++] = (uint16_t)(P0 + TL_W * lane + __ffs((int)left) - 1);
+  __syncwarp();
+  return total;
+}
+// Their minimizers: m[i] for the lane's window i of the mask.
+struct RedoArea {
+  uint32_t v[TL_REDO / 16 * 17];  // in the list's order, so that lanes 16 apart meet in no bank
+  uint16_t list[TL_REDO];
+};
+GKC_DEV void tile_redo(const TileBases &S, uint32_t mask, int P0, RedoArea &R, int k, int p, int filter,
+                       uint32_t (&m)[TL_W]) {
+  uint32_t rank;
+  const uint32_t total = tile_list(mask, P0, R.list, &rank);
+  for (uint32_t r = threadIdx.x & 31u; r < total; r += 32)
+    R.v[r + (r >> 4)] = exact_minimizer(window_bases(S, R.list[r]), k, p, filter);
+  __syncwarp();
 #pragma unroll
-    for (int i = 0; i < TL_W; i++) {
-      const bool in = (mask >> i) & 1u;
-      const uint32_t x = __shfl_sync(0xffffffffu, v, (rk - b) & 31u), x2 = __shfl_sync(0xffffffffu, v2, (rk - b) & 31u);
-      if (in && rk - b < 32u) put(i, x, x2);
-      rk += in;
+  for (int i = 0; i < TL_W; i++)
+    if ((mask >> i) & 1u) {
+      m[i] = R.v[rank + (rank >> 4)];
+      rank++;
     }
-    __syncwarp();
-  }
+  __syncwarp();
 }
 
 }  // namespace gkc

@@ -40,37 +40,27 @@ __global__ void k_window_starts(const uint64_t *offs, uint64_t n_reads, uint64_t
   }
 }
 
-struct WinMin {
-  uint32_t mm;
-  uint8_t pos;
-  int8_t strand;
-};
-
-// Minimizer, position and strand of the window at i (inside a read).
-GKC_DEV WinMin window_min_pos(const uint8_t *reads, uint64_t i, int k, int p, int filter) {
-  WinMin w;
-  w.mm = exact_window_minimizer([&](int j) { return code_of_byte(reads[i + j]); }, k, p, filter);
+// Minimizer (x), position (y, lowest byte) and strand (the byte above) of
+// tile window l, inside a read.
+GKC_DEV uint2 window_min_pos(const TileBases &S, int l, int k, int p, int filter) {
+  const WindowBases b = window_bases(S, l);
+  const uint32_t mm = exact_minimizer(b, k, p, filter);
   const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * p);
   uint32_t f = 0, r = 0;
-  int bpos = 255, bstr = 0;
-  for (int j = 0; j < k; j++) {
-    const uint32_t c0 = code_of_byte(reads[i + j]);
-    const uint32_t c = c0 & 3u;                          // N counts as T here
-    const uint32_t cc = (c0 == 255u ? 255u : 3u - c0) & 3u;  // and its complement as T
+  int bpos = 255, bstr = 0, at = 1 - p;
+  each_base(b, 0, k, [&](uint32_t c, bool bad) {  // a byte that is no base counts as T here, and so does its complement
     f = ((f << 2) | c) & M;
-    r = (r >> 2) | (cc << (2 * p - 2));
-    if (j + 1 >= p) {
-      const bool mf = mm_filter(f, p, filter) && f == w.mm;
-      const bool mr = mm_filter(r, p, filter) && r == w.mm;
+    r = (r >> 2) | ((bad ? 3u : 3u - c) << (2 * p - 2));
+    if (at >= 0 && (f == mm || r == mm)) {
+      const bool mf = f == mm && mm_filter(f, p, filter), mr = r == mm && mm_filter(r, p, filter);
       if (mf || mr) {
-        bpos = j + 1 - p;
+        bpos = at;
         bstr = (f == r) ? -1 : (mr ? 1 : 0);
       }
     }
-  }
-  w.pos = (uint8_t)bpos;
-  w.strand = (int8_t)bstr;
-  return w;
+    at++;
+  });
+  return make_uint2(mm, (uint32_t)bpos | (uint32_t)(uint8_t)bstr << 8);
 }
 
 struct WinArgs {
@@ -82,6 +72,7 @@ struct WinArgs {
   const uint32_t *bits;  // read starts
   uint64_t bit_words;
   int k, p, filter;
+  int strip;             // windows per warp (window_strip)
 };
 
 // The lane's 16 windows of the warp's strip from tile window P0 on: bit i of
@@ -105,10 +96,10 @@ GKC_DEV void lane_valid(const TileBases &S, const WinArgs &a, int64_t G0, int64_
 __global__ void __launch_bounds__(TL_NT, 3) k_window_minimizers(WinArgs a, uint32_t *mm, uint8_t *pos,
                                                                 int8_t *strand, int aligned) {
   __shared__ TileBases S;
-  __shared__ uint16_t redo[TL_WARPS][32];
+  __shared__ uint16_t redo[TL_WARPS][TL_REDO];
   const uint64_t hi = a.offs[a.n_reads];
   const int64_t lo = (int64_t)a.offs[0], end = hi <= a.n_bytes ? (int64_t)hi : 0;
-  const int strip = tile_strip(a.k - a.p + 1), NW = TL_WARPS * strip;
+  const int strip = a.strip, NW = TL_WARPS * strip;
   const uint64_t n_tiles = (a.n_bytes + NW - 1) / NW;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, P0 = warp * strip, P = P0 + TL_W * lane;
   const uint32_t M = 0xFFFFFFFFu >> (32 - 2 * a.p);
@@ -121,30 +112,15 @@ __global__ void __launch_bounds__(TL_NT, 3) k_window_minimizers(WinArgs a, uint3
     __syncthreads();
     if (tile + gridDim.x < n_tiles && threadIdx.x < TL_GROUPS)
       bytes = tile_fetch(a.reads, a.n_bytes, a.aligned16, (int64_t)((tile + gridDim.x) * NW), threadIdx.x);
-    uint32_t vw, tw, m[TL_W], q[TL_W];
+    uint32_t vw, tw, m[TL_W] = {}, q[TL_W] = {};
     lane_valid(S, a, G0, lo, end, P0, strip, &vw, &tw);
-    tile_minima<true>(S, P0, a.k, a.p, a.filter, m, q);
+    if (__any_sync(0xffffffffu, vw != 0u)) tile_minima<true>(S, P0, a.k, a.p, a.filter, m, q);
 #pragma unroll
     for (int i = 0; i < TL_W; i++) {
       if (m[i] == M) tw |= vw & (1u << i);
       const uint32_t code = q[i] & 3u;
       q[i] = ((q[i] >> 2) - (uint32_t)(P + i)) | (code == 2u ? 0xFF00u : code << 8);  // strand byte, position byte
     }
-    if (__any_sync(0xffffffffu, tw != 0u))
-      tile_redo(tw, P0, redo[warp],
-                [&](int l, uint32_t &v, uint32_t &v2) {
-                  const WinMin w = window_min_pos(a.reads, (uint64_t)(G0 + l), a.k, a.p, a.filter);
-                  v = w.mm;
-                  v2 = (uint32_t)w.pos | ((uint32_t)(uint8_t)w.strand << 8);
-                },
-                [&](int i, uint32_t v, uint32_t v2) {
-#pragma unroll
-                  for (int x = 0; x < TL_W; x++)
-                    if (x == i) {
-                      m[x] = v;
-                      q[x] = v2;
-                    }
-                });
 #pragma unroll
     for (int i = 0; i < TL_W; i++)
       if (!((vw >> i) & 1u)) {
@@ -176,6 +152,17 @@ __global__ void __launch_bounds__(TL_NT, 3) k_window_minimizers(WinArgs a, uint3
           }
       }
     }
+    if (__any_sync(0xffffffffu, tw != 0u)) {  // over what was written above: the lanes' registers are free again
+      uint32_t rank;
+      const uint32_t total = tile_list(tw, P0, redo[warp], &rank);  // its barrier orders the writes
+      for (uint32_t r = lane; r < total; r += 32) {
+        const int l = redo[warp][r];
+        const uint2 w = window_min_pos(S, l, a.k, a.p, a.filter);
+        mm[G0 + l] = w.x;
+        if (pos) pos[G0 + l] = (uint8_t)w.y;
+        if (strand) strand[G0 + l] = (int8_t)(w.y >> 8);
+      }
+    }
     __syncthreads();  // before the next tile's bases
   }
 }
@@ -189,11 +176,11 @@ constexpr int SUB_WORDS = TL_NW_MAX / 32;  // selection words kept per tile
 __global__ void __launch_bounds__(SUB_NT, 4) k_sub_flags(WinArgs a, uint32_t mod, uint32_t *sel,
                                                          unsigned long long *tile_cnt, uint64_t n_tiles) {
   __shared__ TileBases S;
-  __shared__ uint16_t redo[TL_WARPS][32];
+  __shared__ RedoArea redo[TL_WARPS];
   __shared__ uint32_t cnt[TL_WARPS];
   const uint64_t hi = a.offs[a.n_reads];
   const int64_t lo = (int64_t)a.offs[0], end = hi <= a.n_bytes ? (int64_t)hi : 0;
-  const int strip = tile_strip(a.k - a.p + 1), NW = TL_WARPS * strip;
+  const int strip = a.strip, NW = TL_WARPS * strip;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, P0 = warp * strip, P = P0 + TL_W * lane;
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const int64_t G0 = (int64_t)(tile * NW);
@@ -205,15 +192,7 @@ __global__ void __launch_bounds__(SUB_NT, 4) k_sub_flags(WinArgs a, uint32_t mod
     lane_valid(S, a, G0, lo, end, P0, strip, &vw, &tw);
     tile_minima<false>(S, P0, a.k, a.p, a.filter, m, none);
     if (__any_sync(0xffffffffu, tw != 0u))
-      tile_redo(tw, P0, redo[warp],
-                [&](int l, uint32_t &v, uint32_t &) {
-                  v = exact_window_minimizer([&](int j) { return tile_code(S, l + j); }, a.k, a.p, a.filter);
-                },
-                [&](int i, uint32_t v, uint32_t) {
-#pragma unroll
-                  for (int x = 0; x < TL_W; x++)
-                    if (x == i) m[x] = v;
-                });
+      tile_redo(S, tw, P0, redo[warp], a.k, a.p, a.filter, m);
     uint32_t f = 0;
 #pragma unroll
     for (int i = 0; i < TL_W; i++)
@@ -258,7 +237,7 @@ __global__ void __launch_bounds__(SUB_NT) k_sub_write(WinArgs a, const uint32_t 
   __shared__ TileBases S;
   __shared__ uint32_t cnt[TL_WARPS];
   __shared__ uint16_t list[TL_NW_MAX];
-  const int strip = tile_strip(a.k - a.p + 1), NW = TL_WARPS * strip, words = strip / 32;  // at most 15 words a warp
+  const int strip = a.strip, NW = TL_WARPS * strip, words = strip / 32;  // at most 15 words a warp
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, w0 = warp * words;
   for (uint64_t tile = blockIdx.x; tile < n_tiles; tile += gridDim.x) {
     const int64_t G0 = (int64_t)(tile * NW);
@@ -332,10 +311,18 @@ static gkc_status mark_starts(gkc_ctx *c, const uint64_t *d_offs, uint64_t n_rea
   return GKC_OK;
 }
 
+// Windows per warp: what a warp can take, less where that leaves SMs without a
+// tile (15 kB of reads with 3% N, k 31: 112 us with full strips, 48 so).
+static int window_strip(const gkc_ctx *c, const gkc_params *prm, uint64_t n_bytes) {
+  int strip = tile_strip(prm->k - prm->p + 1);
+  while (strip > 64 && n_bytes < (uint64_t)TL_WARPS * strip * c->n_sms) strip = strip / 2 & ~31;
+  return strip;
+}
+
 static WinArgs win_args(const gkc_ctx *c, const gkc_params *prm, const uint8_t *reads, uint64_t n_bytes,
                         const uint64_t *offs, uint64_t n_reads, const uint32_t *bits) {
   return WinArgs{reads,  n_bytes, ((uintptr_t)reads % 16) == 0, offs,   n_reads, bits, (n_bytes + 1) / 32 + 3,
-                 prm->k, prm->p,  c->filter};
+                 prm->k, prm->p,  c->filter, window_strip(c, prm, n_bytes)};
 }
 
 static gkc_status read_err(gkc_ctx *c, const uint32_t *err) {
@@ -358,7 +345,7 @@ gkc_status gkc_minimizers_device(gkc_ctx *c, const gkc_params *prm, const char *
   uint32_t *bits, *err;
   s = mark_starts(c, d_offs, n_reads, n_bytes, &bits, &err);
   if (s != GKC_OK) return s;
-  const int nw = tile_windows_n(prm->k - prm->p + 1);
+  const int nw = TL_WARPS * window_strip(c, prm, n_bytes);
   const uint64_t tiles = (n_bytes + nw - 1) / nw;
   const int aligned = (((uintptr_t)d_minimizer | (uintptr_t)d_pos | (uintptr_t)d_strand) & 15) == 0;
   k_window_minimizers<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 3), TL_NT, 0, c->st>>>(
@@ -375,7 +362,7 @@ static gkc_status subsample_t(gkc_ctx *c, const gkc_params *prm, uint32_t mod, c
   uint32_t *bits, *err;
   gkc_status s = mark_starts(c, d_offs, n_reads, n_bytes, &bits, &err);
   if (s != GKC_OK) return s;
-  const int nw = tile_windows_n(prm->k - prm->p + 1);
+  const int nw = TL_WARPS * window_strip(c, prm, n_bytes);
   const uint64_t tiles = (n_bytes + nw - 1) / nw;
   WS(sel, uint32_t, "win_sel", tiles * SUB_WORDS + 1);
   WS(tcnt, unsigned long long, "win_tile_cnt", tiles + 1);
