@@ -1629,41 +1629,112 @@ __global__ void __launch_bounds__(SortShape<K>::NT, SortShape<K>::CTAS) k_bucket
   }
 }
 
+// What open_level found: the digit's place; the only key (where there is just
+// one); the keys left, and the copies left out of them and of which key.
+template <typename K> struct Opened {
+  int cp, sb;
+  K key, crowd;
+  uint64_t kept;
+  uint32_t extra;
+};
+
+// A key that fills a quarter of [b, e) or more, by 32 samples: in S.red[0],
+// S.flag tells whether there may be one.  Barriers around it are the caller's.
+template <typename K>
+GKC_DEV void crowd_sample(CountSmem<K> &S, const K *from, uint64_t b, uint64_t e) {
+  if (threadIdx.x >= 32) return;
+  const uint32_t lane = threadIdx.x;
+  const K x = load_key(from + b + (e - b) * lane / 32);
+  uint32_t same = 0;
+#pragma unroll 4
+  for (int l = 0; l < 32; l++) same += shfl_k<K>(x, l) == x ? 1u : 0u;
+  const uint32_t most = __reduce_max_sync(0xffffffffu, same << 5 | lane);
+  if (lane == (most & 31u)) {
+    S.red[0] = x;
+    S.flag = (most >> 5) >= 8;
+    S.tmp[0] = 0;
+  }
+}
+
 // Opens the keys [b, e) of an oversized bucket (`from`: its keys, `to`: the
 // same range of the other buffer): sorted into `to` by the up to 12 bits after
 // their common prefix, so that at least the first differing bit is among
-// them.  Returns false when all keys are equal (*key), nothing moved then.
+// them.  Returns false when all keys are equal (o->key), nothing moved then.
+// Buckets grow large because keys crowd, often at one key, whose copies would
+// be moved from level to level by one CTA: of a key that is a quarter of them or
+// more one copy is left in, and the caller adds the others to its run (15 M
+// bases, 98.5% A: k 21 in 31 bins 34.6 -> 15.6 ms, k 31 in 256 51.8 -> 18.4).
 template <typename K, int NT>
-__device__ __noinline__ bool open_level(CountSmem<K> &S, const K *from, K *to, uint64_t b, uint64_t e, int *cp, int *sb,
-                                        K *key) {
+__device__ __noinline__ bool open_level(CountSmem<K> &S, const K *from, K *to, uint64_t b, uint64_t e, Opened<K> *o) {
   constexpr int U = sizeof(K) == 8 ? 8 : 4;  // keys in flight per thread
   const int tid = threadIdx.x;
   uint32_t *sub = S.u.sub;
+  bool crowded = false;  // the same in every thread
+  K crowd = 0;
+  if (e - b > 4 * (uint64_t)CountShape<K>::CAP) {
+    crowd_sample<K>(S, from, b, e);
+    __syncthreads();
+    crowded = S.flag;
+    crowd = S.red[0];
+    __syncthreads();
+  }
   K lo = ~(K)0, hi = 0;
+  uint32_t copies = 0;
 #pragma unroll U
   for (uint64_t i = b + tid; i < e; i += NT) {
     const K x = load_key(from + i);
     lo = x < lo ? x : lo;
     hi = x > hi ? x : hi;
+    copies += x == crowd ? 1u : 0u;
+  }
+  if (crowded) {
+    copies = __reduce_add_sync(0xffffffffu, copies);
+    if ((tid & 31) == 0) atomicAdd(&S.tmp[0], copies);
   }
   block_minmax<K, NT>(S, lo, hi);
-  *key = lo;
+  o->key = lo;
   if (lo == hi) return false;
-  prefix_split<K>(lo, hi, e - b, CC_SB_MAX, cp, sb);
-  const uint32_t nsub = 1u << *sb;
+  copies = crowded ? S.tmp[0] : 0u;
+  crowded = copies >= (e - b) / 4 && copies > 16;
+  int cp, sb;
+  prefix_split<K>(lo, hi, e - b, CC_SB_MAX, &cp, &sb);
+  const uint32_t nsub = 1u << sb;
   for (uint32_t jj = tid; jj < nsub; jj += NT) sub[jj] = 0;
   __syncthreads();
-#pragma unroll U
-  for (uint64_t i = b + tid; i < e; i += NT) atomicAdd(&sub[prefix_digit<K>(load_key(from + i), *cp, *sb)], 1u);
-  __syncthreads();
-  scan_sub<NT>(sub, S.tmp, nsub);
+  if (crowded && tid == 0) atomicAdd(&sub[prefix_digit<K>(crowd, cp, sb)], 1u);
 #pragma unroll U
   for (uint64_t i = b + tid; i < e; i += NT) {
     const K x = load_key(from + i);
-    to[b + atomicAdd(&sub[prefix_digit<K>(x, *cp, *sb)], 1u)] = x;
+    if (!crowded || x != crowd) atomicAdd(&sub[prefix_digit<K>(x, cp, sb)], 1u);
   }
   __syncthreads();
+  scan_sub<NT>(sub, S.tmp, nsub);
+  if (crowded && tid == 0) to[b + atomicAdd(&sub[prefix_digit<K>(crowd, cp, sb)], 1u)] = crowd;
+#pragma unroll U
+  for (uint64_t i = b + tid; i < e; i += NT) {
+    const K x = load_key(from + i);
+    if (!crowded || x != crowd) to[b + atomicAdd(&sub[prefix_digit<K>(x, cp, sb)], 1u)] = x;
+  }
+  __syncthreads();
+  o->cp = cp;
+  o->sb = sb;
+  o->crowd = crowd;
+  o->extra = crowded ? copies - 1 : 0u;
+  o->kept = e - b - o->extra;
   return true;
+}
+
+// Adds the copies left out of key x to its run, one of the staged runs [lo, hi).
+// By one thread.
+template <typename K>
+GKC_DEV void add_copies(const SortCountArgs &a, uint64_t lo, uint64_t hi, K x, uint32_t extra) {
+  const K *keys = reinterpret_cast<const K *>(a.stage_keys);
+  while (lo < hi) {
+    const uint64_t mid = (lo + hi) >> 1;
+    if (load_key(keys + mid) < x) lo = mid + 1; else hi = mid;
+  }
+  if (lo < a.stage_cap && load_key(keys + lo) == x) a.stage_counts[lo] = __ldcg(a.stage_counts + lo) + extra;
+  else atomicOr(a.err, ERR_BOUNDS);  // not possible: one copy was left in
 }
 
 // Counts the keys [pos, end) of an oversized bucket (offsets from its key range
@@ -1684,24 +1755,30 @@ __device__ __noinline__ uint64_t count_range(CountSmem<K> &S, const SortCountArg
   uint64_t run = 0;      // [pos, end): what is opened next; the same in every thread
   int level = 0;
   while (true) {
-    int cp, sb;
-    K key;
-    if (open_level<K, NT>(S, buf[from], buf[from ^ 1], pos, end, &cp, &sb, &key)) {
+    Opened<K> o;
+    if (open_level<K, NT>(S, buf[from], buf[from ^ 1], pos, end, &o)) {
       if (level == CC_LEVELS) {  // not possible: every level fixes a bit of the key
         if (tid == 0) atomicOr(a.err, ERR_BOUNDS);
         break;
       }
       if (tid == 0) {
-        S.lend[level] = end;
-        S.lcp[level] = (uint8_t)cp;
-        S.lsb[level] = (uint8_t)sb;
-        S.lbuf[level] = (uint8_t)(from ^ 1);
+        S.lend[level] = pos + o.kept;
+        S.lcp[level] = (uint8_t)o.cp;
+        S.lsb[level] = (uint8_t)o.sb;
+        S.lbuf[level] = (uint8_t)((from ^ 1) | (o.extra ? 2 : 0));
+        if (o.extra) {  // more than 16, so there is room where the copies were
+          K *x = buf[from ^ 1] + pos + o.kept;
+          x[0] = o.crowd;
+          x[1] = (K)o.extra;
+          x[2] = (K)run;
+          x[3] = (K)end;
+        }
       }
       level++;
     } else {  // one key
       if (tid == 0) {
         if (start + run < a.stage_cap) {
-          reinterpret_cast<K *>(a.stage_keys)[start + run] = key;
+          reinterpret_cast<K *>(a.stage_keys)[start + run] = o.key;
           a.stage_counts[start + run] = (uint32_t)(end - pos);
         } else {
           atomicOr(a.err, ERR_CAPACITY);
@@ -1717,10 +1794,16 @@ __device__ __noinline__ uint64_t count_range(CountSmem<K> &S, const SortCountArg
       const uint64_t lend = S.lend[level - 1];
       if (pos == lend) {
         level--;
+        const uint32_t lb = S.lbuf[level];
+        if (lb & 2u) {
+          const K *x = buf[lb & 1u] + lend;
+          if (tid == 0) add_copies<K>(a, start + (uint64_t)load_key(x + 2), start + run, load_key(x), (uint32_t)load_key(x + 1));
+          pos = (uint64_t)load_key(x + 3);
+        }
         continue;
       }
       const int lcp = S.lcp[level - 1], lsb = S.lsb[level - 1];
-      from = S.lbuf[level - 1];
+      from = S.lbuf[level - 1] & 1;
       const K *src = buf[from];
       end = lend;
       if (lend - pos > (uint64_t)CAP) {
@@ -1806,11 +1889,10 @@ __global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_open(SortCountA
       __syncthreads();
       continue;
     }
-    int cp, sb;
-    K key;
-    if (!open_level<K, NT>(S, keys + start, reinterpret_cast<K *>(a.scratch) + start, 0, n, &cp, &sb, &key)) {
+    Opened<K> o;
+    if (!open_level<K, NT>(S, keys + start, reinterpret_cast<K *>(a.scratch) + start, 0, n, &o)) {
       if (tid == 0) {  // one key
-        reinterpret_cast<K *>(a.stage_keys)[start] = key;  // start + n <= stage_cap: the keys were there
+        reinterpret_cast<K *>(a.stage_keys)[start] = o.key;  // start + n <= stage_cap: the keys were there
         a.stage_counts[start] = (uint32_t)n;
         a.bucket_d[g] = 1;
       }
@@ -1822,7 +1904,7 @@ __global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_open(SortCountA
     uint16_t *first = reinterpret_cast<uint16_t *>(S.u.sub + CC_NSUB_MAX);
     static_assert(sizeof(S.u) >= CC_NSUB_MAX * 6, "the list fits after the digits");
     if (tid == 0) {
-      const uint32_t nsub = 1u << sb;
+      const uint32_t nsub = 1u << o.sb;
       uint32_t m = 0, d = 0, s0 = 0;
       while (d < nsub) {
         uint32_t lo = d + 1, hi = nsub;
@@ -1844,8 +1926,17 @@ __global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_open(SortCountA
     const uint32_t m = S.hfill;
     const uint64_t t0 = S.n;
     for (uint32_t i = tid; i < m && t0 + m <= a.task_cap; i += NT) {
-      const uint32_t b = first[i] ? S.u.sub[first[i] - 1] : 0u, e = i + 1 < m ? S.u.sub[first[i + 1] - 1] : (uint32_t)n;
-      a.tasks[t0 + i] = make_uint4((uint32_t)g, b, e - b, 0u);
+      const uint32_t b = first[i] ? S.u.sub[first[i] - 1] : 0u;
+      const uint32_t e = i + 1 < m ? S.u.sub[first[i + 1] - 1] : (uint32_t)o.kept;
+      // the slice with the key whose copies were left out: it and they, behind the bucket's keys
+      const uint32_t d = o.extra ? prefix_digit<K>(o.crowd, o.cp, o.sb) : 0u;
+      const bool crowd = o.extra && first[i] <= d && (i + 1 == m || d < first[i + 1]);
+      if (crowd) {
+        K *x = reinterpret_cast<K *>(a.scratch) + start + n;
+        x[-1] = o.crowd;
+        x[-2] = (K)o.extra;
+      }
+      a.tasks[t0 + i] = make_uint4((uint32_t)g, b, e - b, crowd ? 1u : 0u);
     }
     __syncthreads();
   }
@@ -1882,6 +1973,10 @@ __global__ void __launch_bounds__(CountShape<K>::NT, 2) k_bucket_slices(SortCoun
     }
     __syncthreads();  // S.g and S.hfill are read
     if (threadIdx.x == 0) {
+      if (task.w) {
+        const K *x = reinterpret_cast<const K *>(a.scratch) + start + a.bucket_size[task.x];
+        add_copies<K>(a, start + task.y, start + task.y + D, load_key(x - 1), (uint32_t)load_key(x - 2));
+      }
       a.tasks[t].w = (uint32_t)D;
       atomicAdd(&a.bucket_d[task.x], (unsigned long long)D);
     }

@@ -138,8 +138,8 @@ struct SortCountArgs {
   uint32_t *big_list;             // buckets of at least big_min keys (from the scan), then rejected ones
   unsigned long long *big_count;
   unsigned long long *big_ticket;  // zeroed
-  // slices of opened buckets: bucket, offset in it, keys, distinct keys; a
-  // bucket's tasks follow one another
+  // slices of opened buckets: bucket, offset in it, keys, distinct keys (until
+  // then: 1 where copies of a key are to be added); a bucket's tasks follow one another
   uint4 *tasks;
   uint64_t task_cap;
   unsigned long long *task_count, *task_ticket;  // zeroed
