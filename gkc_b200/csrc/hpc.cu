@@ -92,6 +92,26 @@ __global__ void __launch_bounds__(HP_NT) k_hpc_flags(HpcArgs a) {
   }
 }
 
+// Compressed offset of every read: the kept bytes before its first one.
+GKC_DEV void hpc_offsets(const HpcArgs &a) {
+  const uint64_t lo = a.offs[0], hi = min(a.offs[a.n_reads], a.n_bytes);
+  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r <= a.n_reads;
+       r += (uint64_t)gridDim.x * blockDim.x) {
+    const uint64_t pos = a.offs[r];
+    uint64_t o;
+    if (pos <= lo) o = 0;
+    else if (pos >= hi) o = a.tile_off[a.n_tiles];
+    else o = a.tile_off[pos / HP_TILE] + a.pre[pos >> 5] + __popc(a.flags[pos >> 5] & ((1u << (pos & 31)) - 1u));
+    a.out_offs[r] = o;
+  }
+}
+
+__global__ void __launch_bounds__(256) k_hpc_offsets(HpcArgs a) { hpc_offsets(a); }
+
+// OFFSETS: the reads' offsets as well, where a launch costs more than what they
+// take from this kernel's registers (one tile a CTA: 15 kB 67 -> 63 us; 150 M
+// bytes, many tiles: 494 -> 604).
+template <bool OFFSETS>
 __global__ void __launch_bounds__(HP_NT) k_hpc_write(HpcArgs a) {
   __shared__ uint8_t sb[HP_TILE];
   __shared__ int32_t so[HP_TILE];
@@ -159,20 +179,7 @@ __global__ void __launch_bounds__(HP_NT) k_hpc_write(HpcArgs a) {
     for (uint64_t x = lead + 4 * nw + threadIdx.x; x < n; x += HP_NT) a.out[o + x] = sb[x];
     __syncthreads();
   }
-}
-
-// Compressed offset of every read: the kept bytes before its first one.
-__global__ void k_hpc_offsets(HpcArgs a) {
-  const uint64_t lo = a.offs[0], hi = min(a.offs[a.n_reads], a.n_bytes);
-  for (uint64_t r = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; r <= a.n_reads;
-       r += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t pos = a.offs[r];
-    uint64_t o;
-    if (pos <= lo) o = 0;
-    else if (pos >= hi) o = a.tile_off[a.n_tiles];
-    else o = a.tile_off[pos / HP_TILE] + a.pre[pos >> 5] + __popc(a.flags[pos >> 5] & ((1u << (pos & 31)) - 1u));
-    a.out_offs[r] = o;
-  }
+  if (OFFSETS) hpc_offsets(a);
 }
 
 }  // namespace gkc
@@ -208,9 +215,15 @@ gkc_status hpc_enqueue(gkc_ctx *c, const uint8_t *reads, uint64_t n_bytes, const
   const unsigned rgrid = (unsigned)std::min<uint64_t>((n_reads + 256) / 256, (uint64_t)c->n_sms * 16);
   k_hpc_starts<<<rgrid, 256, 0, c->st>>>(a, starts, stamp);
   k_hpc_flags<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 4), HP_NT, 0, c->st>>>(a);
-  c->launches += 4 + scan_u64(cnt, off, tiles, stmp, c->st);
-  k_hpc_write<<<(unsigned)std::min<uint64_t>(tiles, (uint64_t)c->n_sms * 4), HP_NT, 0, c->st>>>(a);
-  k_hpc_offsets<<<rgrid, 256, 0, c->st>>>(a);
+  c->launches += 3 + scan_u64(cnt, off, tiles, stmp, c->st);
+  const uint64_t most = (uint64_t)c->n_sms * 4;
+  if (tiles <= most) {
+    k_hpc_write<true><<<(unsigned)tiles, HP_NT, 0, c->st>>>(a);
+  } else {
+    k_hpc_write<false><<<(unsigned)most, HP_NT, 0, c->st>>>(a);
+    k_hpc_offsets<<<rgrid, 256, 0, c->st>>>(a);
+    c->launches++;
+  }
   CK(cudaPeekAtLastError());
   return GKC_OK;
 }
