@@ -951,7 +951,7 @@ static gkc_status pipeline_batched(gkc_ctx *c, const gkc_params *prm, const char
       return GKC_OK;
     }
     CK(cudaStreamSynchronize(c->st));
-    if (!(c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) break;
+    if (!(c->h_tot->err & ERR_CAPACITY)) break;
     // grow to the sizes the device reported and retry
     graphs_invalidate(c);
     if (attempt == 2) return ctx_fail(c, GKC_ERR_CAPACITY, "pipeline capacity");
@@ -1108,7 +1108,7 @@ static gkc_status rerun_larger(gkc_ctx *c, StreamCall &sc, int slot) {
   const int filter = c->filter;
   c->filter = sc.key.filter;
   gkc_status s = GKC_OK;
-  for (int attempt = 0; attempt < 2 && s == GKC_OK && (c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH)); attempt++) {
+  for (int attempt = 0; attempt < 2 && s == GKC_OK && (c->h_tot->err & ERR_CAPACITY); attempt++) {
     grow_caps(&sc.cap, c->h_tot);
     graphs_invalidate(c);
     s = enqueue_pipeline(c, &sc.prm, sc.key, sc.cap);
@@ -1119,7 +1119,7 @@ static gkc_status rerun_larger(gkc_ctx *c, StreamCall &sc, int slot) {
   if (s != GKC_OK) return s;
   set_results(c, sc);
   SlotGraph &G = c->graphs[slot];
-  if (!(c->h_tot->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))) {
+  if (!(c->h_tot->err & ERR_CAPACITY)) {
     G.key = sc.key;
     G.cap = sc.cap;
     G.seen = true;
@@ -1138,14 +1138,14 @@ static gkc_status issue_download(gkc_ctx *c, int rec) {
   if (sc.dl_issued) return GKC_OK;
   const int slot = (int)(sc.ticket & 1);
   CK(cudaEventSynchronize(c->ev_comp[slot]));
-  if (c->h_tots[slot]->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH)) {
+  if (c->h_tots[slot]->err & ERR_CAPACITY) {
     sc.status = rerun_larger(c, sc, slot);
     if (sc.status != GKC_OK) sc.message = c->err;
   }
   sc.tot = *c->h_tots[slot];  // the slot's next call overwrites them
   const DevTotals *h = &sc.tot;
   const bool bad = sc.status != GKC_OK ||
-                   (h->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH | ERR_BIN_TOO_LARGE | ERR_SPIN_TIMEOUT | ERR_BOUNDS |
+                   (h->err & (ERR_CAPACITY | ERR_BIN_TOO_LARGE | ERR_SPIN_TIMEOUT | ERR_BOUNDS |
                               ERR_BAD_READ)) != 0;
   if (!bad) {
     const uint64_t nd = std::min<uint64_t>(h->n_distinct, sc.capacity);
@@ -1275,7 +1275,7 @@ gkc_status gkc_stream_wait(gkc_ctx *c, uint64_t ticket, uint64_t *n_distinct, ui
   const DevTotals *h = &sc.tot;
   if (n_distinct) *n_distinct = h->n_distinct;
   if (n_kmers) *n_kmers = h->n_kmers;
-  if (h->err & (ERR_CAPACITY | ERR_OVERSIZE_SCRATCH))
+  if (h->err & ERR_CAPACITY)
     return ctx_fail(c, GKC_ERR_CAPACITY, "pipeline capacity");
   s = device_err(c, h->err);
   if (s != GKC_OK) return s;

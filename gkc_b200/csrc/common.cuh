@@ -14,14 +14,10 @@ namespace gkc {
 enum : uint32_t {
   ERR_SPIN_TIMEOUT = 1u << 0,   // a bounded wait ran out (look-back / tile chain)
   ERR_CAPACITY = 1u << 1,       // an output buffer sized in advance was too small
-  ERR_OVERSIZE_SCRATCH = 1u << 2,
   ERR_BAD_READ = 1u << 3,       // a read longer than the supported superkmer length
   ERR_BOUNDS = 1u << 4,         // a device bounds check failed (access skipped)
   ERR_BIN_TOO_LARGE = 1u << 5,  // a bin holds 2^32 or more k-mers
 };
-
-// Bounded spin limit for any wait on another CTA (~0.5-2 s with backoff).
-constexpr uint32_t kSpinLimit = 1u << 22;
 
 // ASCII -> 2-bit code with the reference's mapping (A/a/U/u 0, C/c 1, G/g 2,
 // T/t 3, anything else 255), built once into shared memory per CTA.
@@ -92,14 +88,6 @@ GKC_DEV u128 revcomp_k<u128>(u128 x, int k) { return revcomp128(x, k); }
 template <typename K>
 GKC_DEV K kmer_mask(int k) {
   return (2 * k >= (int)(8 * sizeof(K))) ? ~(K)0 : (((K)1 << (2 * k)) - 1);
-}
-
-// Top `nbits` bits of a 2k-bit key, below the `skip` most significant bits.
-template <typename K>
-GKC_DEV uint32_t key_digit(K x, int key_bits, int skip, int nbits) {
-  if (nbits <= 0) return 0u;
-  int sh = key_bits - skip - nbits;
-  return (uint32_t)(x >> sh) & ((1u << nbits) - 1u);
 }
 
 GKC_DEV uint32_t lane_id() { return threadIdx.x & 31u; }

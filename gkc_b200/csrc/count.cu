@@ -718,11 +718,10 @@ constexpr int CC_LEVELS = 130;      // open levels of an oversized bucket: each 
 // and 16-bit counts beside them; an element's handle is its slot.
 template <typename K> struct HashArea {
   static constexpr int CAP = CountShape<K>::CAP, SLOTS = CountShape<K>::SLOTS;
-  typedef uint64_t Member;     // groups hold the keys themselves
   K T[SLOTS];                  // keys; at the end the sorted keys
   uint32_t TC[SLOTS / 2];      // counts, two 16-bit halves a word; at the end the sorted counts
   union {
-    Member G[CAP];             // the distinct keys, group after group
+    uint64_t G[CAP];            // the distinct keys, group after group
     K spl[2 * CC_SPLIT_MAX];   // samples (runs of 32), then the sorted splitters
   } g;
   uint16_t L[CAP];             // handles of the distinct keys, then the group of every G entry
@@ -733,7 +732,6 @@ template <typename K> struct HashArea {
 // claimant + 1) and the count in one word; an element's handle is that index.
 template <> struct HashArea<u128> {
   static constexpr int CAP = CountShape<u128>::CAP, SLOTS = CountShape<u128>::SLOTS;
-  typedef uint16_t Member;     // groups hold handles
   u128 A[CAP];                 // the bucket's keys
   uint32_t T[SLOTS];           // 0: free, else (index + 1) | count << 13
   union {

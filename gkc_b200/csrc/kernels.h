@@ -174,9 +174,12 @@ template <typename K> constexpr uint32_t bucket_target(uint32_t target) {
 }
 constexpr uint32_t kCoarseMaxBits = 12;
 constexpr uint64_t kChunkKmers = 65536;
-// Doubled where the histogram's CTAs get eight chunks each even so: fewer rows
-// of digits (720 M k-mers in bins of 2.8 M, 64 K / 128 K / 256 K: histogram +
-// scatter 8.85 / 8.56 / 8.71 ms; 151 M, which get 2.6: 2.00 / 2.04 / 2.19).
+// Doubled where there are eight for each of the histogram's CTAs (eight an SM),
+// which leaves four: fewer rows of digits (720 M k-mers in bins of 2.8 M, 9.3
+// for each, 64 K / 128 K / 256 K: histogram + scatter 8.85 / 8.56 / 8.71 ms; 151 M,
+// 1.9 for each: 2.00 / 2.04 / 2.19).  What lies between was not measured.  `keys`
+// is the room for keys: the bases where a whole pipeline runs, the k-mers where a
+// partition is counted.
 // Halved down to this while there are fewer chunks than the histogram has CTAs
 // (histogram + scatter, 64 K / 32 K / 16 K: 20 M bases 389 / 319 / 269 us, 60 M
 // 718 / 684 / 678, 120 M 1331 / 1328 / 1387).
@@ -186,7 +189,7 @@ inline uint64_t default_chunk(uint64_t keys, int n_sms) {
   while (chunk > kChunkKmersMin && keys / chunk < 8 * (uint64_t)n_sms) chunk /= 2;
   return chunk;
 }
-// Largest mean bin (k-mers) whose 8-byte keys are scattered by two CTAs an SM
+// Largest mean bin (room for keys, as above) whose 8-byte keys are scattered by two CTAs an SM
 // with tiles of 7168 keys rather than one with 16384: their phases overlap,
 // but in larger bins a bucket's run of the smaller tile ends within few 32-byte
 // sectors (134.7 M k-mers, one CTA / two: 256 bins 0.91 / 0.86 ms, 64 bins 0.98 /
